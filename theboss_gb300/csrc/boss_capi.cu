@@ -88,6 +88,11 @@ int ensure_pinned(Context* cx, size_t bytes) {
 
 static inline size_t align_up(size_t x, size_t a) { return (x + a - 1) & ~(a - 1); }
 
+// D's rows as the FP64 permanent and all-minors sweeps take them (pack_row).
+static void pack_rows(const std::vector<longlong2>& D, longlong2* out) {
+  for (size_t i = 0; i < D.size(); ++i) out[i] = longlong2{pack_row(D[i].x), pack_row(D[i].y)};
+}
+
 // A list of sweeps that share one factor count, uploaded and ready to launch.
 struct SweepBatch {
   int n = 0, nf = 0;
@@ -137,9 +142,10 @@ static int sweeps_prepare(Context* cx, const std::vector<HostSweep>& sweeps, boo
     P.nf = h.nf;
     P.kind = h.kind;
     P.parity0 = h.parity0;
-    P.fx = h.fx;
+    P.fx = -h.fx_sum;
     P.has_base = h.has_base;
     P.out_idx = p;
+    P.align = range_align((int64_t)h.total_codes, nthr[p], h.nb);
     P.n_codes = (int64_t)h.total_codes;
     P.thread_begin = threads;
     P.n_threads = nthr[p];
@@ -175,9 +181,11 @@ static int sweeps_prepare(Context* cx, const std::vector<HostSweep>& sweeps, boo
   longlong2* hp = (longlong2*)(h + o_pool);
   for (int p = 0; p < n; ++p) {
     const HostSweep& hs = sweeps[p];
-    std::copy(hs.D.begin(), hs.D.end(), hp + probs[p].mat_off);
     std::copy(hs.base.begin(), hs.base.end(), hp + probs[p].base_off);
-    if (B.ff) {
+    if (!B.ff) {
+      pack_rows(hs.D, hp + probs[p].mat_off);
+    } else {
+      std::copy(hs.D.begin(), hs.D.end(), hp + probs[p].mat_off);
       float4* df = reinterpret_cast<float4*>(hp + probs[p].ff_off);
       for (int d = 0; d < hs.nb; ++d)
         for (int f = 0; f < hs.nf; ++f) {
@@ -270,16 +278,26 @@ static int choose_fx(double bound) {
   int ex = 0;
   std::frexp(bound, &ex);  // bound < 2^ex
   int fx = 61 - ex;
-  return std::max(-900, std::min(fx, 200));
+  return std::max(-1000, std::min(fx, 1000));
 }
 
-static inline long long to_fixed(double v, int fx) { return std::llrint(std::ldexp(v, fx)); }
+// v * 2^fx rounded to the nearest integer (ties to even); |v * 2^fx| < 2^62.
+static inline long long to_fixed(double v, double scale) {
+  double x = v * scale;  // exact: scale is a power of two
+  const double t = std::copysign(4503599627370496.0, x);  // 2^52: adding it rounds to an integer
+  if (std::fabs(x) < 4503599627370496.0) x = (x + t) - t;
+  return (long long)x;
+}
 
 // Fills a sweep that iterates `dig` and multiplies over the particles of `col`
 // (a mode occupied p times gives p factors).  entry(a, l) is the matrix element
-// between digit mode a and product mode l.
+// between digit mode a and product mode l.  Every factor f has its own fixed-point
+// scale 2^fx_f, chosen so that its largest possible sum fills 61 bits (a shared
+// scale would leave the factors of small rows with fewer significant bits);
+// shared_fx: one scale for all of them.
 template <class F>
-static int fill_sweep(HostSweep& hs, const Side& dig, const Side& col, int kind, bool halve, F entry) {
+static int fill_sweep(HostSweep& hs, const Side& dig, const Side& col, int kind, bool halve, bool shared_fx,
+                      F entry) {
   int drop = -1;
   if (halve && dig.nb > 0) drop = dig.nb - 1;  // a binary digit fixed at r = 0
   hs.kind = kind;
@@ -309,64 +327,50 @@ static int fill_sweep(HostSweep& hs, const Side& dig, const Side& col, int kind,
     hs.total_codes *= b;
     ++a_out;
   }
-  // |row sum| <= sum_a mult_a * max component of the entries
-  double bound = 0.0;
+  // |row sum| <= sum_a mult_a * max component of the entries (of one factor, or of all)
+  double bound[kMaxFactors] = {}, shared = 0.0;
   for (size_t a = 0; a < dig.modes.size(); ++a) {
     double mx = 0.0;
     for (int f = 0; f < hs.nf; ++f) {
       const double2 z = entry(dig.modes[a], fmode[f]);
-      mx = std::max(mx, std::max(std::fabs(z.x), std::fabs(z.y)));
+      const double c = std::max(std::fabs(z.x), std::fabs(z.y));
+      bound[f] += dig.mult[a] * c;
+      mx = std::max(mx, c);
     }
-    bound += dig.mult[a] * mx;
+    shared += dig.mult[a] * mx;
   }
-  hs.fx = choose_fx(bound);
+  hs.fx = choose_fx(shared);
   hs.D.resize((size_t)hs.nd * hs.nf);
-  const long long fsign = (kind == kGlynn) ? -2 : 1;  // Glynn: s = base - 2 sum r U
-  a_out = 0;
-  for (size_t a = 0; a < dig.modes.size(); ++a) {
-    if ((int)a == drop) continue;
-    for (int f = 0; f < hs.nf; ++f) {
-      const double2 z = entry(dig.modes[a], fmode[f]);
-      longlong2 v;
-      v.x = fsign * to_fixed(z.x, hs.fx);
-      v.y = fsign * to_fixed(z.y, hs.fx);
-      hs.D[(size_t)a_out * hs.nf + f] = v;
-    }
-    ++a_out;
-  }
   hs.has_base = (kind == kGlynn);
-  if (hs.has_base) {
-    hs.base.assign(hs.nf, longlong2{0, 0});
-    for (int f = 0; f < hs.nf; ++f) {
-      long long re = 0, im = 0;
-      for (size_t a = 0; a < dig.modes.size(); ++a) {
-        const double2 z = entry(dig.modes[a], fmode[f]);
-        re += (long long)dig.mult[a] * to_fixed(z.x, hs.fx);
-        im += (long long)dig.mult[a] * to_fixed(z.y, hs.fx);
-      }
-      hs.base[f].x = re;
-      hs.base[f].y = im;
-    }
-    hs.scale = std::ldexp(1.0, -dig.n) * (drop >= 0 ? 2.0 : 1.0);
-    hs.parity0 = 0;
-  } else {
-    hs.scale = 1.0;
-    hs.parity0 = dig.n & 1;
-  }
+  if (hs.has_base) hs.base.assign(hs.nf, longlong2{0, 0});
   hs.fbias.assign(hs.nf, 189);
   hs.ff_exp = 0;
+  hs.fx_sum = 0;
+  const long long fsign = (kind == kGlynn) ? -2 : 1;  // Glynn: s = base - 2 sum r U
   for (int f = 0; f < hs.nf; ++f) {
+    const int fx = shared_fx ? hs.fx : choose_fx(bound[f]);
+    const double scale = std::ldexp(1.0, fx);
+    long long re = 0, im = 0;
     unsigned long long bx = 0, by = 0;
+    a_out = 0;
     for (size_t a = 0; a < dig.modes.size(); ++a) {
       const double2 z = entry(dig.modes[a], fmode[f]);
-      bx += (unsigned long long)dig.mult[a] * (unsigned long long)std::llabs(to_fixed(z.x, hs.fx));
-      by += (unsigned long long)dig.mult[a] * (unsigned long long)std::llabs(to_fixed(z.y, hs.fx));
+      const long long x = to_fixed(z.x, scale), y = to_fixed(z.y, scale);
+      re += (long long)dig.mult[a] * x;
+      im += (long long)dig.mult[a] * y;
+      bx += (unsigned long long)dig.mult[a] * (unsigned long long)std::llabs(x);
+      by += (unsigned long long)dig.mult[a] * (unsigned long long)std::llabs(y);
+      if ((int)a != drop) hs.D[(size_t)(a_out++) * hs.nf + f] = longlong2{fsign * x, fsign * y};
     }
+    if (hs.has_base) hs.base[f] = longlong2{re, im};
     const unsigned long long b = std::max(bx, by);
     const int p = b ? 63 - __builtin_clzll(b) : 0;
     hs.fbias[f] = 189 - p;
-    hs.ff_exp += p + 1 - hs.fx;
+    hs.ff_exp += p + 1 - fx;
+    hs.fx_sum += fx;
   }
+  hs.scale = hs.has_base ? std::ldexp(1.0, -dig.n) * (drop >= 0 ? 2.0 : 1.0) : 1.0;
+  hs.parity0 = hs.has_base ? 0 : (dig.n & 1);
   return kOk;
 }
 
@@ -407,7 +411,7 @@ void host_fx_to_ff(long long x, int fbias, float& hi, float& lo) {
 // One permanent request.  Returns kOk and either fills `hs` (needs_sweep = true)
 // or sets `value` directly for the edge cases theboss special-cases.
 int plan_permanent(const double* U, int m, const int32_t* S, const int32_t* T, int len, int variant,
-                          HostSweep& hs, bool& needs_sweep, double2& value) {
+                          HostSweep& hs, bool& needs_sweep, double2& value, bool shared_fx) {
   needs_sweep = false;
   if (len > m || len < 0) {  // bs_permanent_calculator_base.py:61-72
     set_error("state length exceeds matrix dimension");
@@ -433,7 +437,7 @@ int plan_permanent(const double* U, int m, const int32_t* S, const int32_t* T, i
         return kOk;
       }
       const bool ch = (variant == BOSS_CHIN_HUH);
-      const int st = fill_sweep(hs, in, out, ch ? kGlynn : kRyser, ch && in.n == out.n, entry_in_out);
+      const int st = fill_sweep(hs, in, out, ch ? kGlynn : kRyser, ch && in.n == out.n, shared_fx, entry_in_out);
       if (st) return st;
       needs_sweep = true;
       return kOk;
@@ -457,10 +461,10 @@ int plan_permanent(const double* U, int m, const int32_t* S, const int32_t* T, i
       const uint64_t co = out.nb ? out.codes / 2 : out.codes;
       int st;
       bool outs = co < ci;
-      st = outs ? fill_sweep(hs, out, in, kGlynn, true, entry_out_in) : fill_sweep(hs, in, out, kGlynn, true, entry_in_out);
+      st = outs ? fill_sweep(hs, out, in, kGlynn, true, shared_fx, entry_out_in) : fill_sweep(hs, in, out, kGlynn, true, shared_fx, entry_in_out);
       if (st == kErrLimit) {  // try the other orientation
         outs = !outs;
-        st = outs ? fill_sweep(hs, out, in, kGlynn, true, entry_out_in) : fill_sweep(hs, in, out, kGlynn, true, entry_in_out);
+        st = outs ? fill_sweep(hs, out, in, kGlynn, true, shared_fx, entry_out_in) : fill_sweep(hs, in, out, kGlynn, true, shared_fx, entry_in_out);
       }
       if (st) return st;
       hs.digits_are_outputs = outs;
@@ -540,7 +544,7 @@ static int plan_minors(const double* U, int m, const int32_t* S, const int32_t* 
   // from one sweep, one single-occupied digit held at r = 0); the kernel
   // accumulates half of each, hence the factor 2.
   auto entry = [&](int i_mode, int j_mode) { return U_at(U, m, j_mode, i_mode); };
-  const int st = fill_sweep(hs, in, out, kGlynn, true, entry);
+  const int st = fill_sweep(hs, in, out, kGlynn, true, false, entry);
   if (st) return st;
   hs.scale *= 2.0;
   needs_sweep = true;
@@ -713,7 +717,7 @@ int boss_perm_grad_batch(const double* matrix, int32_t m, const int32_t* input_s
     double2 v = make_double2(0.0, 0.0);
     const int32_t* S = input_states + (size_t)k * len;
     const int32_t* T = output_states + (size_t)k * len;
-    int st = plan_permanent(matrix, m, S, T, len, BOSS_GLYNN, hs, need, v);
+    int st = plan_permanent(matrix, m, S, T, len, BOSS_GLYNN, hs, need, v, true);
     if (st) return st;
     if (!need) {  // no particles: perm = 1, gradient 0
       P2[k] = v;
@@ -1110,14 +1114,15 @@ extern "C" int boss_perm_batch_noalloc(const double* matrix, int32_t m, const in
       P.nf = h.nf;
       P.kind = h.kind;
       P.parity0 = h.parity0;
-      P.fx = h.fx;
+      P.fx = -h.fx_sum;
+      P.align = range_align((int64_t)h.total_codes, G.nthr[p], h.nb);
       P.has_base = h.has_base;
       P.out_idx = which[nf][p];  // the reduction writes straight into the caller's buffer
       P.n_codes = (int64_t)h.total_codes;
       P.thread_begin = thread_at;
       P.n_threads = G.nthr[p];
       P.mat_off = pool_at;
-      std::copy(h.D.begin(), h.D.end(), hpool + pool_at);
+      pack_rows(h.D, hpool + pool_at);
       pool_at += (int64_t)h.D.size();
       P.base_off = pool_at;
       std::copy(h.base.begin(), h.base.end(), hpool + pool_at);

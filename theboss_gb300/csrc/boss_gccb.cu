@@ -151,6 +151,7 @@ static inline uint32_t mask_for(uint32_t n) {
 struct Draws {
   int n = 0;                       // row stride: the most input particles of a sample
   bool binned = false;             // some input mode holds more than one particle
+  bool one_input = false;          // every sample has the same input state
   std::vector<uint8_t> particles;  // [sample][n] particle -> mode of the sample's input (ascending)
   std::vector<uint8_t> nparticles; // [sample] particles of the sample's input
   std::vector<int32_t> L;          // [sample] particles kept
@@ -167,6 +168,7 @@ static void same_input(Draws& D, const std::vector<uint8_t>& particles, int n_sa
   for (int s = 0; s < n_samples; ++s)
     if (n) memcpy(&D.particles[(size_t)s * n], particles.data(), n);
   D.nparticles.assign(n_samples, (uint8_t)n);
+  D.one_input = true;
 }
 
 // The popped modes from the randint results: remove the idx-th remaining particle.
@@ -637,6 +639,7 @@ struct LevelSample {  // host-computed layout of one sample's sweep at one level
   int64_t n_threads;
   int64_t part_off;
   int64_t pool_off;
+  int64_t align;  // range_align of its split
 };
 
 struct FinalizeArgs {
@@ -645,8 +648,8 @@ struct FinalizeArgs {
   int A_next;  // active samples at level k + 1
   int m;
   int n;       // row stride of idx / uni
-  int fx;      // fixed-point fraction bits of the sweep rows
-  const longlong2* Ufx;   // m x m, U * 2^fx rounded
+  const longlong2* Ufx;   // m x m, row o of U * 2^rowfx[o] rounded
+  const int32_t* rowfx;   // [output mode] fixed-point fraction bits of that row (per matrix)
   const float4* Uff;      // float-pair pmf: m x m transposed, Uff[i * m + o] = U[o][i] as float pairs
                           // (re hi, re lo, im hi, im lo)
   const int4* Ulimb;      // FP64 pmf: m x m transposed, U[o][i] * 2^lfx rounded, as 27-bit limbs
@@ -869,7 +872,8 @@ __global__ void __launch_bounds__(kFinWarps * 32, 8) gccb_finalize_kernel(Finali
   const int j = blockIdx.x * kFinWarps + w;
   if (j >= a.A) return;
   const int m = a.m;
-  const longlong2* Ufxs = a.Ufx + (size_t)j * a.mstride;  // and its fixed-point copy
+  const longlong2* Ufxs = a.Ufx + (size_t)j * a.mstride;  // the sample's fixed-point matrix
+  const int32_t* rowfx = a.rowfx + (a.mstride ? (size_t)j * m : 0);
   uint8_t* S = a.S + (size_t)j * m;
   uint8_t* T = a.T + (size_t)j * m;
   // Everything the particle bookkeeping needs, loaded up front (independent
@@ -1490,6 +1494,7 @@ __global__ void __launch_bounds__(kFinWarps * 32, 8) gccb_finalize_kernel(Finali
     ls.thread_begin = (int64_t)j * a.next_uni.n_threads;
     ls.part_off = (int64_t)j * a.next_uni.part_off;
     ls.pool_off = (int64_t)j * a.next_uni.pool_off;
+    ls.align = a.next_uni.align;
   }
   // rows: -2 U[out][in] for the sweep's digits; base sums: sum_i S_i U[out][i]
   // over every input mode (all signs +1 at r = 0), exact in fixed point
@@ -1498,7 +1503,7 @@ __global__ void __launch_bounds__(kFinWarps * 32, 8) gccb_finalize_kernel(Finali
   for (int e = lane; e < nds * nf; e += 32) {
     const int d = e / nf, f = e - d * nf;
     const longlong2 u = Ufxs[(size_t)fm_s[w][f] * m + dm_s[w][d]];
-    D[e] = make_longlong2(-2 * u.x, -2 * u.y);
+    D[e] = a.next_ff ? make_longlong2(-2 * u.x, -2 * u.y) : make_longlong2(pack_row(-2 * u.x), pack_row(-2 * u.y));
   }
   longlong2* B = D + (size_t)nds * nf;
   // Float-pair sweeps: factor f is scaled by 2^-(p_f + 1), 2^p_f <= its bound
@@ -1506,7 +1511,8 @@ __global__ void __launch_bounds__(kFinWarps * 32, 8) gccb_finalize_kernel(Finali
   // so |s_f| < 1 in that scale; fx_to_ff takes the bias 189 - p_f.
   float4* DF = reinterpret_cast<float4*>(B + nf);
   int* fbias = reinterpret_cast<int*>(DF + (size_t)(nb - held) * nf);
-  int esum = 0;  // sum_f (p_f + 1)
+  int esum = 0;   // sum_f (p_f + 1)
+  int fxsum = 0;  // sum_f fx_f
   for (int f = lane; f < nf; f += 32) {
     long long bx = 0, by = 0;
     unsigned long long ax = 0, ay = 0;
@@ -1519,6 +1525,7 @@ __global__ void __launch_bounds__(kFinWarps * 32, 8) gccb_finalize_kernel(Finali
       ay += (unsigned long long)mult_s[w][d] * (unsigned long long)(u.y < 0 ? -u.y : u.y);
     }
     B[f] = make_longlong2(bx, by);
+    fxsum += rowfx[fm_s[w][f]];
     if (a.next_ff) {
       const unsigned long long bnd = ax > ay ? ax : ay;
       const int p = bnd ? 63 - __clzll((long long)bnd) : 0;
@@ -1526,6 +1533,8 @@ __global__ void __launch_bounds__(kFinWarps * 32, 8) gccb_finalize_kernel(Finali
       esum += p + 1;
     }
   }
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) fxsum += __shfl_xor_sync(0xffffffffu, fxsum, off);
   if (a.next_ff) {
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) esum += __shfl_xor_sync(0xffffffffu, esum, off);
@@ -1552,7 +1561,8 @@ __global__ void __launch_bounds__(kFinWarps * 32, 8) gccb_finalize_kernel(Finali
     P.nf = nf;
     P.kind = kGlynn;
     P.parity0 = 0;
-    P.fx = a.fx;
+    P.fx = -fxsum;
+    P.align = (int32_t)ls.align;
     P.has_base = 1;
     P.out_idx = j;
     P.n_codes = ls.n_codes;
@@ -1561,9 +1571,9 @@ __global__ void __launch_bounds__(kFinWarps * 32, 8) gccb_finalize_kernel(Finali
     P.mat_off = ls.pool_off;
     P.base_off = ls.pool_off + (int64_t)nds * nf;
     P.part_off = ls.part_off;
-    // float pairs: the factors' scales 2^(p_f + 1 - fx) multiply the product
+    // float pairs: the factors' scales 2^(p_f + 1 - fx_f) multiply the product
     P.ff_off = a.next_ff ? ls.pool_off + (int64_t)(nds + 1) * nf : 0;
-    const int e2 = (held ? -(nf - 1) : -nf) + (a.next_ff ? esum - nf * a.fx : 0);
+    const int e2 = (held ? -(nf - 1) : -nf) + (a.next_ff ? esum - fxsum : 0);
     P.scale = (e2 >= -1022 && e2 <= 1023) ? __longlong_as_double((long long)(e2 + 1023) << 52) : ldexp(1.0, e2);
     P.fixed_digit = held;
     P.group = a.next_tab ? 1 : a.next_group;
@@ -1642,9 +1652,49 @@ __global__ void transpose_matrices_kernel(const double2* __restrict__ U, void* _
   uabs[t] = __double2float_ru(fabs(v.x) + fabs(v.y));  // rounded up: an upper bound
 }
 
-__global__ void to_fixed_kernel(const double* __restrict__ x, long long* __restrict__ y, int64_t count, int fx) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < count) y[i] = __double2ll_rn(ldexp(x[i], fx));  // exact scaling, round to nearest even
+// One warp per row o of a matrix (n_mats x m rows): the row's fixed-point scale,
+// the largest 2^rowfx for which its possible sums, sum_i w_i max(|Re U[o][i]|,
+// |Im U[o][i]|) over the input's particles, stay below 2^61, and the row in it.
+// weight: each mode's particle count at most (one matrix for all samples); else
+// the sample's own particles (pmode row of its draws, `order` as everywhere).
+__global__ void __launch_bounds__(128) fixed_rows_kernel(const double2* __restrict__ U, longlong2* __restrict__ out,
+                                                         int32_t* __restrict__ rowfx, int m, int64_t rows,
+                                                         const uint8_t* __restrict__ weight,
+                                                         const int32_t* __restrict__ order,
+                                                         const uint8_t* __restrict__ pmode,
+                                                         const uint8_t* __restrict__ npart, int n) {
+  const int64_t r = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  if (r >= rows) return;
+  const double2* row = U + r * m;
+  int np = 0, pm = -1;
+  if (!weight) {
+    const int64_t s = order[r / m];
+    np = npart[s];
+    if (lane < np) pm = pmode[s * n + lane];  // at most 32 particles
+  }
+  double bound = 0.0;
+  for (int base = 0; base < m; base += 32) {
+    const int i = base + lane;
+    int w = 0;
+    if (weight) {
+      if (i < m) w = weight[i];
+    } else {
+      for (int p = 0; p < np; ++p) w += (__shfl_sync(0xffffffffu, pm, p) == i) ? 1 : 0;
+    }
+    if (i < m && w) {
+      const double2 v = row[i];
+      bound += (double)w * fmax(fabs(v.x), fabs(v.y));
+    }
+  }
+  bound = warp_sum(bound) * (1.0 + 0x1p-40);  // the sums' own rounding
+  int fx = 56;
+  if (bound > 0.0 && bound < 1.7e308) fx = max(-1000, min(60 - ilogb(bound), 1000));  // bound < 2^(ilogb + 1)
+  if (lane == 0) rowfx[r] = fx;
+  for (int i = lane; i < m; i += 32) {
+    const double2 v = row[i];
+    out[r * m + i] = make_longlong2(__double2ll_rn(ldexp(v.x, fx)), __double2ll_rn(ldexp(v.y, fx)));
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -1784,12 +1834,8 @@ static int gccb_prepare(Context* cx, const double* matrix, int n_mats, int m, Dr
   }
   const std::vector<int>& order = R.order;
   R.Lmax = Lmax;
-  // fixed point: |row sum| <= n * max |component of U|
   double umax = 0.0;
   for (size_t i = 0; i < (size_t)2 * m * m * n_mats; ++i) umax = std::max(umax, std::fabs(matrix[i]));
-  int ex = 0;
-  std::frexp(std::max(umax, 1e-300) * std::max(n, 1), &ex);
-  const int fx = std::max(-900, std::min(61 - ex, 200));
   // the Laplace step's fixed point: |U| * 2^lfx < 2^53 (umax < 2^eu)
   int eu = 0;
   std::frexp(std::max(umax, 1e-300), &eu);
@@ -1897,6 +1943,7 @@ static int gccb_prepare(Context* cx, const double* matrix, int n_mats, int m, Dr
       uni_lvl[k].n_threads = tps;
       uni_lvl[k].part_off = tps * nd0;
       uni_lvl[k].pool_off = pool_units(nd0);
+      uni_lvl[k].align = range_align((int64_t)code0, tps, k);
       if (!ffl[k] && tps / G >= kReduceMinParts && Ak <= kReduceMaxSamples && nd0 <= 32) {
         red[k] = 1;
         max_red = std::max<int64_t>(max_red, Ak);
@@ -1922,6 +1969,7 @@ static int gccb_prepare(Context* cx, const double* matrix, int n_mats, int m, Dr
       ls.n_threads = nthr[jj];
       ls.part_off = parts;
       ls.pool_off = pool;
+      ls.align = range_align(ls.n_codes, ls.n_threads, k);
       threads += nthr[jj];
       parts += nthr[jj] * ndv[jj];
       pool += pool_units(ndv[jj]);
@@ -1946,6 +1994,7 @@ static int gccb_prepare(Context* cx, const double* matrix, int n_mats, int m, Dr
   const size_t o_idx = off; off = al(off + (size_t)N * n);
   const size_t o_pm = off; off = al(off + (size_t)N * n);
   const size_t o_np = off; off = al(off + (size_t)N);
+  const size_t o_cap = off; off = al(off + (size_t)m);
   const size_t o_uni = off; off = al(off + sizeof(double) * (size_t)N * n);
   const size_t o_U = off; off = al(off + sizeof(double2) * (size_t)m * m * n_mats);
   const size_t arena = off;
@@ -1959,8 +2008,8 @@ static int gccb_prepare(Context* cx, const double* matrix, int n_mats, int m, Dr
   if ((st = ensure(B[4], sizeof(longlong2) * (size_t)max_pool * 2 + 512))) return st;  // rows x2
   if ((st = ensure(B[5], sizeof(double2) * (size_t)(max_parts + 32 * max_red)))) return st;  // partials | sums
   if ((st = ensure(B[6], sizeof(uint32_t) * 8 * (size_t)N))) return st;                // particles left
-  // U fixed point | U^T (doubles or float pairs) | U^T 1-norms
-  if ((st = ensure(B[7], 36 * (size_t)m * m * n_mats + 256))) return st;
+  // U fixed point | U^T (limbs or float pairs) | U^T 1-norms | rows' fraction bits
+  if ((st = ensure(B[7], (36 * (size_t)m * m + 4 * (size_t)m) * n_mats + 256))) return st;
   if ((st = ensure_slot_pinned(slot, std::max(arena, al((size_t)N * m) + 256)))) return st;
   char* h = (char*)g_gccb_pinned[slot];
   memset(h, 0, o_ord);
@@ -1971,6 +2020,16 @@ static int gccb_prepare(Context* cx, const double* matrix, int n_mats, int m, Dr
   memcpy(h + o_idx, D.idx.data(), (size_t)N * n);
   memcpy(h + o_pm, D.particles.data(), (size_t)N * n);
   memcpy(h + o_np, D.nparticles.data(), (size_t)N);
+  {  // each mode's particles at most, over the samples' inputs
+    uint8_t* cap = (uint8_t*)(h + o_cap);
+    memset(cap, 0, (size_t)m);
+    uint8_t occ[256] = {};
+    for (int s = 0; s < (n_mats > 1 ? 0 : (D.one_input ? std::min(N, 1) : N)); ++s) {
+      const uint8_t* ps = D.particles.data() + (size_t)s * n;
+      for (int k = 0; k < D.nparticles[s]; ++k) cap[ps[k]] = std::max(cap[ps[k]], ++occ[ps[k]]);
+      for (int k = 0; k < D.nparticles[s]; ++k) occ[ps[k]] = 0;
+    }
+  }
   memcpy(h + o_uni, D.u.data(), sizeof(double) * (size_t)N * n);
   const size_t mm = (size_t)m * m;
   if (n_mats > 1) {  // instances: matrices in level order
@@ -1994,9 +2053,12 @@ static int gccb_prepare(Context* cx, const double* matrix, int n_mats, int m, Dr
   longlong2* dUfx = (longlong2*)B[7].ptr;
   void* dUt = (void*)(dUfx + mm * n_mats);  // 16 bytes per entry either way
   float* dUabs = (float*)((char*)dUt + 16 * mm * n_mats);
+  int32_t* drowfx = (int32_t*)(dUabs + mm * n_mats);
   {
-    const int64_t cnt = (int64_t)2 * mm * n_mats;
-    to_fixed_kernel<<<(unsigned)((cnt + 255) / 256), 256, 0, s>>>((const double*)(d + o_U), (long long*)dUfx, cnt, fx);
+    const int64_t rows = (int64_t)m * n_mats;
+    fixed_rows_kernel<<<(unsigned)((rows + 3) / 4), 128, 0, s>>>(
+        (const double2*)(d + o_U), dUfx, drowfx, m, rows, n_mats > 1 ? nullptr : (const uint8_t*)(d + o_cap),
+        (const int32_t*)(d + o_ord), (const uint8_t*)(d + o_pm), (const uint8_t*)(d + o_np), n);
     if ((e = cudaGetLastError()) != cudaSuccess) return fail_cuda(e, "fixed-point matrices");
     const int64_t cnt2 = (int64_t)mm * n_mats;
     transpose_matrices_kernel<<<(unsigned)((cnt2 + 255) / 256), 256, 0, s>>>((const double2*)(d + o_U), dUt, dUabs,
@@ -2050,8 +2112,8 @@ static int gccb_prepare(Context* cx, const double* matrix, int n_mats, int m, Dr
     fa.A_next = (k < Lmax) ? A[k + 1] : 0;
     fa.m = m;
     fa.n = n;
-    fa.fx = fx;
     fa.Ufx = dUfx;
+    fa.rowfx = drowfx;
     fa.Uff = f64 ? nullptr : (const float4*)dUt;
     fa.Ulimb = f64 ? (const int4*)dUt : nullptr;
     fa.lfx = lfx;

@@ -49,6 +49,11 @@ cudaError_t launch_minors_reduce(const SweepProblem* probs, int n_probs, const d
 // least one thread per sweep and at least kMinCodesPerThread codes per thread.
 constexpr int64_t kMinCodesPerThread = 8;
 void partition_threads(const std::vector<uint64_t>& n_codes, int64_t resident, std::vector<int64_t>& n_threads);
+// log2 of the codes every range of a sweep starts at a multiple of: the largest
+// (at most 6, at most the nb binary digits) that makes the longest range at most
+// 1/32 longer than an even split.  Lanes of a warp then flip the same low digit
+// at each step and read the same row (one broadcast instead of several lines).
+int range_align(int64_t n_codes, int64_t n_threads, int nb);
 
 // ---------------------------------------------------------------------------
 // Host-side sweep description.
@@ -58,7 +63,8 @@ struct HostSweep {
   int parity0 = 0;
   int nd = 0, nb = 0, nf = 0;
   int has_base = 0;
-  int fx = 56;
+  int fx = 56;                 // fraction bits shared by all factors (gradients)
+  int fx_sum = 0;              // sum of the factors' own fraction bits (permanents, all-minors)
   uint8_t mult[kMaxDigits] = {};
   std::vector<longlong2> D;     // nd x nf
   std::vector<longlong2> base;  // nf (has_base)
@@ -71,7 +77,7 @@ struct HostSweep {
   // Float-pair all-minors: factor f's bound 2^p <= max(sum mult |Re|, sum mult |Im|) < 2^(p+1)
   // over every digit (held one included), in fixed-point units; fx_to_ff takes 189 - p.
   std::vector<int> fbias;
-  int ff_exp = 0;  // sum_f (p_f + 1) - nf * fx: the float-pair products' scale
+  int ff_exp = 0;  // sum_f (p_f + 1 - fx_f): the float-pair products' scale
 };
 
 // Arithmetic of the all-minors sweeps (boss_minors_arithmetic): 0 float pairs
@@ -132,7 +138,8 @@ int small_perm_batch(Context* cx, const double* matrix, int m, int len, const in
 // One permanent request (theboss's variant semantics).  Returns kOk and either
 // fills `hs` (needs_sweep = true) or sets `value` for the edge cases theboss
 // special-cases.
+// shared_fx: one scale for all factors (the gradient sweeps) instead of one each.
 int plan_permanent(const double* U, int m, const int32_t* S, const int32_t* T, int len, int variant, HostSweep& hs,
-                   bool& needs_sweep, double2& value);
+                   bool& needs_sweep, double2& value, bool shared_fx = false);
 
 }  // namespace boss

@@ -94,6 +94,17 @@ void partition_threads(const std::vector<uint64_t>& n_codes, int64_t resident, s
   }
 }
 
+int range_align(int64_t n_codes, int64_t n_threads, int nb) {
+  int c = 0;
+  while (c < 6 && c < nb) {
+    const int64_t units = (n_codes + (2ll << c) - 1) >> (c + 1);
+    const int64_t longest = ((units + n_threads - 1) / n_threads) << (c + 1);
+    if (32.0 * (double)longest * (double)n_threads > 33.0 * (double)n_codes) break;
+    ++c;
+  }
+  return c;
+}
+
 // One block per sweep: fixed-order sum of its threads' partials.
 // ff: the partials are float pairs (float4), as the float-pair sweep writes them.
 __global__ void perm_reduce_kernel(const SweepProblem* __restrict__ probs, const double2* __restrict__ partials,

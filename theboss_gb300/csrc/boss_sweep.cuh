@@ -17,16 +17,14 @@
 // The binomial weight follows bs_permanent_calculator_base.py:151-164.
 //
 // GB300 mapping.  The FP64 pipe issues 2 lanes/clk/SM, 1/64 of FP32, so only
-// products and sums of products use it, and the integer pipes take what they can:
-//   * the row sums are exact 64-bit fixed-point integers (value = int * 2^-fx),
-//     updated with integer adds and converted to FP64 with integer instructions
-//     (fx_to_double), so the 2 adds per factor and code leave the FP64 pipe and
-//     the sums never drift;
-//   * the first factors of every product are multiplied in block floating point
-//     on the integer pipe (62-bit mantissas, accumulate_product_bf), the rest on
-//     the FP64 pipe, 4 instructions per factor (accumulate_product);
-//   * the last multiply of every product is fused into the accumulation (4 DFMA);
+// sums over codes use it, and the integer pipes take everything else:
+//   * the row sums are exact 64-bit fixed-point integers (value = int * 2^-fx_f,
+//     every factor in its own scale), so they never drift;
+//   * the products are formed in block floating point on the integer pipe (62-bit
+//     mantissas, accumulate_product_bf), rounded to FP64 once per code;
 //   * sign flips are integer XORs on the sign bit.
+// (The gradient sweep multiplies on the FP64 pipe, its factors converted with
+// integer instructions, fx_to_double.)
 //
 // Work split: the codes of a sweep are cut into one contiguous range per thread
 // (lengths differ by at most one), each thread decodes its start code in closed
@@ -54,7 +52,8 @@ struct SweepProblem {
   int32_t nf;        // product factors
   int32_t kind;      // SweepKind
   int32_t parity0;   // sign parity of the r = 0 code
-  int32_t fx;        // fixed-point fraction bits of the row sums
+  int32_t fx;        // permanents, all-minors: minus the sum of the factors' fraction bits (every factor has
+                     // its own scale 2^fx_f); gradients: the fraction bits shared by all factors
   int32_t has_base;  // base sums present
   int32_t out_idx;   // result index
   int64_t n_codes;       // codes in the sweep
@@ -71,8 +70,18 @@ struct SweepProblem {
                      // launch's threads fill whole blocks) sums its minors, so the partials are
                      // (n_threads / group) x nd; n_threads and thread_begin are multiples of it, and
                      // every sweep of the launch has the same
+  int32_t align;     // permanents, all-minors: ranges start at multiples of 2^align codes (range_align)
   uint8_t mult[kMaxDigits];
 };
+
+// A row entry of D for the integer-pipe sweeps (permanents, all-minors): the
+// 64-bit value hi 2^32 + lo with lo taken as a SIGNED word (hi carries its sign
+// bit), so that adding sg times it (sg = +-1) is one 32 x 32 + 64-bit multiply-add
+// and one 32-bit one per component, on the FMA pipe, instead of two exclusive-ors
+// and two carry-linked adds on the ALU pipe, which bounds these sweeps.
+__host__ __device__ __forceinline__ long long pack_row(long long v) {
+  return (long long)((unsigned long long)v + (((unsigned long long)v & 0x80000000ull) << 1));
+}
 
 // ---------------------------------------------------------------------------
 // Integer-pipe helpers
@@ -126,9 +135,41 @@ __device__ __forceinline__ uint32_t digit_value(const SweepProblem& P, uint64_t 
   return r;
 }
 
+// a b and a b + c, 32 x 32 -> 64 bits signed: one instruction each.  (Written as
+// 64-bit C products of sign-extended words the compiler expanded part of them to
+// full 64 x 64-bit products: 64 instead of 45 instructions per factor.)
+__host__ __device__ __forceinline__ long long mul_wide(int a, int b) {
+#ifdef __CUDA_ARCH__
+  long long r;
+  asm("mul.wide.s32 %0, %1, %2;" : "=l"(r) : "r"(a), "r"(b));
+  return r;
+#else
+  return (long long)a * (long long)b;
+#endif
+}
+__host__ __device__ __forceinline__ long long mad_wide(int a, int b, long long c) {
+#ifdef __CUDA_ARCH__
+  long long r;
+  asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(r) : "r"(a), "r"(b), "l"(c));
+  return r;
+#else
+  return (long long)((unsigned long long)((long long)a * (long long)b) + (unsigned long long)c);
+#endif
+}
+
+// acc + sg * d for a packed row component d (pack_row): one 32 x 32 + 64-bit and
+// one 32-bit multiply-add.  sg is a small integer (+-1, or a digit's value).
+__device__ __forceinline__ long long add_packed(long long acc, long long d, int sg) {
+  const int lo = (int)(unsigned)(unsigned long long)d, hi = (int)((unsigned long long)d >> 32);
+  const unsigned long long t = (unsigned long long)mad_wide(lo, sg, acc);
+  const unsigned th = (unsigned)(t >> 32) + (unsigned)hi * (unsigned)sg;
+  return (long long)(((unsigned long long)th << 32) | (unsigned)t);
+}
+
 // Full state at code t: fixed-point sums, sign parity, binomial weight of the
-// multi-valued digits, and the bits of the binary digits.
-template <int NF>
+// multi-valued digits, and the bits of the binary digits.  kPacked: the rows are
+// packed (pack_row), as the integer-pipe sweeps take them.
+template <int NF, bool kPacked = false>
 __device__ __forceinline__ void decode_code(const SweepProblem& P, const longlong2* __restrict__ D,
                                             const longlong2* __restrict__ base, uint64_t t, long long (&sr)[NF],
                                             long long (&si)[NF], uint64_t& gbits, uint32_t& parity, double& weight) {
@@ -157,8 +198,8 @@ __device__ __forceinline__ void decode_code(const SweepProblem& P, const longlon
     for (int f = 0; f < NF; ++f) {
       if (f > 0 && (f & 7) == 0) load_fence();
       const longlong2 d = row[f];
-      sr[f] += d.x;
-      si[f] += d.y;
+      sr[f] = kPacked ? add_packed(sr[f], d.x, 1) : sr[f] + d.x;
+      si[f] = kPacked ? add_packed(si[f], d.y, 1) : si[f] + d.y;
     }
   }
   uint64_t th = t >> P.nb;
@@ -176,8 +217,8 @@ __device__ __forceinline__ void decode_code(const SweepProblem& P, const longlon
 #pragma unroll
       for (int f = 0; f < NF; ++f) {
         const longlong2 d = row[f];
-        sr[f] += (long long)r * d.x;
-        si[f] += (long long)r * d.y;
+        sr[f] = kPacked ? add_packed(sr[f], d.x, (int)r) : sr[f] + (long long)r * d.x;
+        si[f] = kPacked ? add_packed(si[f], d.y, (int)r) : si[f] + (long long)r * d.y;
       }
     }
   }
@@ -196,6 +237,21 @@ __device__ __forceinline__ void flip_binary(const longlong2* __restrict__ D, int
     const longlong2 d = row[f];
     sr[f] = sr[f] + (d.x ^ sgn) + one;
     si[f] = si[f] + (d.y ^ sgn) + one;
+  }
+}
+
+// The same with packed rows.
+template <int NF>
+__device__ __forceinline__ void flip_packed(const longlong2* __restrict__ D, int i, uint32_t bit, long long (&sr)[NF],
+                                            long long (&si)[NF]) {
+  const longlong2* row = D + (size_t)i * NF;
+  const int sg = 1 - 2 * (int)bit;
+#pragma unroll
+  for (int f = 0; f < NF; ++f) {
+    if (f > 0 && (f & 7) == 0) load_fence();
+    const longlong2 d = row[f];
+    sr[f] = add_packed(sr[f], d.x, sg);
+    si[f] = add_packed(si[f], d.y, sg);
   }
 }
 
@@ -242,19 +298,28 @@ __host__ __device__ __forceinline__ I128 sub128(I128 x, I128 y) {
 // ---------------------------------------------------------------------------
 // Block floating point on the integer pipe.  A complex value is (re + i im) 2^e,
 // two 64-bit integers sharing one exponent, normalised so that the larger
-// component lies in [2^61, 2^62] in magnitude.  GB300 issues the 64-bit integer
-// multiplies on its FMA pipe and the shifts and adds on its ALU pipe, both far
-// faster than its FP64 pipe (2 lanes/clk/SM), so a chain of factors can be
-// multiplied with no FP64 instruction at all:
-//   * bf_pair: the exact 128-bit product of two fixed-point factors, truncated
-//     once to 62 bits (relative error below 2^-60);
-//   * bf_mul: the product of two normalised values from the high halves of the
-//     four 64 x 64 -> 128-bit products (|product| >= 2^122 before the shift, two
-//     truncations of one unit per component: relative error below 2^-56.5 of
-//     the product's magnitude);
+// component lies in [2^61, 2^62].  GB300 issues the 32 x 32 + 64-bit multiply-add
+// on its FMA pipe and shifts and adds on its ALU pipe, both far faster than its
+// FP64 pipe (2 lanes/clk/SM), so whole products are formed without it:
+//   * bf_mul: the high half of the product from two signed 32-bit limbs per
+//     component, 12 multiply-adds (4 high x high, 8 cross; low x low, below half
+//     a unit, is dropped), then one normalising shift.  Of two normal values
+//     |product| >= 2^122 before the >> 64, off by less than 2 units a component:
+//     relative error below 2^-56.5 of the product's magnitude;
+//   * bf_mul with a fixed-point factor as it is (|re|, |im| < 2^61, its own scale
+//     2^fx_f such that its largest possible sum has 61 bits): the same absolute
+//     error, under 2^-58 of (the first value's magnitude times that largest
+//     sum), so a factor that happens to be small costs nothing extra to scale;
 //   * bf_to_double: one rounding to FP64 (2^-53) at the end.
 // An FP64 complex product errs by up to about 2^-52 of its magnitude, so a chain
-// of these products is at least as accurate as the FP64 chain it replaces.
+// of these products is more accurate than the FP64 chain it replaces (64
+// permanents at n = 28: 9.9e-14 from 64-bit values against 1.5e-13 with the last
+// 8 factors multiplied in FP64).
+// Measured, 64 permanents (input-side digits, 2^(n-1) codes each): n = 20 1.71 ms,
+// n = 24 33.5 ms, against 2.08 and 39.3 ms with the limb products left to the
+// compiler and 3.5 and 62 ms with exact 128-bit leaves and 8 FP64 products.
+// Bound by the FMA pipe (a 32 x 32 + 64-bit multiply-add holds it for 4 cycles a
+// warp, 66 % busy) and dependent latency at 3 warps per scheduler.
 // ---------------------------------------------------------------------------
 struct BFloat {
   long long re, im;
@@ -313,18 +378,52 @@ __host__ __device__ __forceinline__ unsigned mag_hi32(long long x) {
   const unsigned h = hi32(x);
   return h ^ (unsigned)((int)h >> 31);
 }
+// Two signed 32-bit limbs of a 64-bit value: x = h 2^32 + l.
+struct Limbs {
+  int h, l;
+};
+__host__ __device__ __forceinline__ Limbs limbs_of(long long x) {
+  Limbs v;
+  v.l = (int)lo32(x);
+  v.h = (int)(hi32(x) + (lo32(x) >> 31));
+  return v;
+}
+// Position of the leading bit that differs from the sign, -1 if none.
+__host__ __device__ __forceinline__ int lead_bit(int x) {
+#ifdef __CUDA_ARCH__
+  int p;
+  asm("bfind.s32 %0, %1;" : "=r"(p) : "r"(x));
+  return p;
+#else
+  return 31 - clz_u32((unsigned)(x ^ (x >> 31)));
+#endif
+}
+// (x y) 2^-64 within 2 units a component, for |x|'s components <= 2^62 and |y|'s
+// <= 2^62 (normal values or fixed-point factors).  Every sum of cross products
+// stays below 2^63: a limb pair (h, l) with |h| = 2^30 has l of the sign that
+// keeps |value| <= 2^62.
+__host__ __device__ __forceinline__ void bf_mul_high(long long xr, long long xi, long long yr, long long yi,
+                                                     long long& re, long long& im) {
+  const Limbs a = limbs_of(xr), b = limbs_of(xi), c = limbs_of(yr), d = limbs_of(yi);
+  const long long p = mad_wide(a.l, c.h, mul_wide(a.h, c.l)), q = mad_wide(b.l, d.h, mul_wide(b.h, d.l));
+  const long long r = mad_wide(b.l, c.h, mad_wide(b.h, c.l, mad_wide(a.l, d.h, mul_wide(a.h, d.l))));
+  re = mad_wide(-b.h, d.h, mul_wide(a.h, c.h)) + (long long)((int)hi32(p) - (int)hi32(q));
+  im = mad_wide(b.h, c.h, mul_wide(a.h, d.h)) + (long long)(int)hi32(r);
+}
+// The normalising shift of a product's high half: the leading bit (in the high
+// word, or below it when the product is tiny) moves up to bit 61; zero stays zero.
+__host__ __device__ __forceinline__ int bf_renorm(long long& re, long long& im) {
+  const int pr = lead_bit((int)hi32(re)), pi = lead_bit((int)hi32(im));
+  const int p = pr > pi ? pr : pi;
+  const int s = 29 - p;  // 0 .. 30
+  re = join32(fshl32(lo32(re), hi32(re), s), lo32(re) << (s & 31));
+  im = join32(fshl32(lo32(im), hi32(im), s), lo32(im) << (s & 31));
+  return p;  // the exponent grows by 64 - s = p + 35
+}
 __host__ __device__ __forceinline__ BFloat bf_mul(const BFloat& x, const BFloat& y) {
-  // |x.re| ... |y.im| <= 2^62: every high half lies in [-2^60, 2^60], the sums in [-2^61, 2^61]
-  const long long re = mulhi_s64(x.re, y.re) - mulhi_s64(x.im, y.im);
-  const long long im = mulhi_s64(x.re, y.im) + mulhi_s64(x.im, y.re);
-  // |x|, |y| >= 2^61, so |x y| 2^-64 >= 2^58 and the larger component is at least
-  // 2^57: its leading bit is in the high word and the normalising shift is 0..5
-  // (30 for a zero product, which stays zero).
-  const int s = clz_u32(mag_hi32(re) | mag_hi32(im)) - 2;
   BFloat z;
-  z.re = join32(fshl32(lo32(re), hi32(re), s), lo32(re) << (s & 31));
-  z.im = join32(fshl32(lo32(im), hi32(im), s), lo32(im) << (s & 31));
-  z.e = x.e + y.e + 64 - s;
+  bf_mul_high(x.re, x.im, y.re, y.im, z.re, z.im);
+  z.e = x.e + y.e + 35 + bf_renorm(z.re, z.im);
   return z;
 }
 // The 128-bit value (hi, lo) shifted right by r (arithmetic; 1 <= r <= 63), low 64 bits.
@@ -384,83 +483,40 @@ __host__ __device__ __forceinline__ double bf_to_double(long long x, int e) {
   if (be >= 1 && be <= 2046 && ax != 0) return bits_to_double((sgn << 63) | ((unsigned long long)be << 52) | mant);
   return ax ? ldexp((double)x, e) : 0.0;
 }
-// Product of the fixed-point factors [LO, HI) (unit 2^efx each) as a balanced
-// tree: exact pairs at the leaves, bf_mul above them.
-template <int LO, int HI, int NF>
-__host__ __device__ __forceinline__ BFloat bf_product(const long long (&sr)[NF], const long long (&si)[NF], int efx) {
-  if constexpr (HI - LO == 1) {
-    return bf_norm(sr[LO], si[LO], efx);
-  } else if constexpr (HI - LO == 2) {
-    return bf_pair(sr[LO], si[LO], sr[LO + 1], si[LO + 1], 2 * efx);
-  } else {
-    constexpr int MID = LO + 2 * ((HI - LO + 2) / 4);
-    return bf_mul(bf_product<LO, MID, NF>(sr, si, efx), bf_product<MID, HI, NF>(sr, si, efx));
-  }
-}
-
-// acc += sign * prod_f s_f with the first K factors multiplied in block floating
-// point on the integer pipe and the others on the FP64 pipe (the last one fused
-// into the accumulation).  K = NF leaves 2 FP64 adds per code.
-template <int NF, int K>
-__device__ __forceinline__ void accumulate_product_bf(const long long (&sr)[NF], const long long (&si)[NF],
-                                                      int bias_exp, uint32_t neg_mask, double& ar, double& ai) {
-  static_assert(K >= 2 && K <= NF, "block-float factors");
-  const int efx = bias_exp - 1086;  // a factor's unit: 2^-fx
-  const BFloat p = bf_product<0, K, NF>(sr, si, efx);
-  double pr = bf_to_double(p.re, p.e), pi = bf_to_double(p.im, p.e);
-  if constexpr (K == NF) {
-    ar += xor_sign(pr, neg_mask);
-    ai += xor_sign(pi, neg_mask);
-  } else {
-#pragma unroll
-    for (int f = K; f < NF - 1; ++f) {
-      const double br = fx_to_double(sr[f], bias_exp);
-      const double bi = fx_to_double(si[f], bias_exp);
-      const double t_re = fma(pr, br, -(pi * bi));
-      const double t_im = fma(pr, bi, pi * br);
-      pr = t_re;
-      pi = t_im;
-    }
-    pr = xor_sign(pr, neg_mask);
-    pi = xor_sign(pi, neg_mask);
-    const double br = fx_to_double(sr[NF - 1], bias_exp);
-    const double bi = fx_to_double(si[NF - 1], bias_exp);
-    ar = fma(pr, br, ar);
-    ar = fma(-pi, bi, ar);
-    ai = fma(pr, bi, ai);
-    ai = fma(pi, br, ai);
-  }
-}
-
-// acc += sign * prod_f s_f on the FP64 pipe: complex products (4 instructions
-// each), the last fused with the accumulation (4 DFMA): 4 (nf - 1) FP64
-// instructions per code.
+// acc += sign * prod_f s_f, every product on the integer pipe, two FP64 adds.  The
+// factors are split over two chains (two independent chains of dependent
+// instructions hide each other's latency); a chain starts from a normalised
+// factor and takes the others as they are.  e0: minus the factors' fraction bits.
 template <int NF>
-__device__ __forceinline__ void accumulate_product(const long long (&sr)[NF], const long long (&si)[NF], int bias_exp,
-                                                   uint32_t neg_mask, double& ar, double& ai) {
-  if (NF == 1) {
-    ar += xor_sign(fx_to_double(sr[0], bias_exp), neg_mask);
-    ai += xor_sign(fx_to_double(si[0], bias_exp), neg_mask);
-    return;
-  }
-  double pr = fx_to_double(sr[0], bias_exp), pi = fx_to_double(si[0], bias_exp);
+__device__ __forceinline__ void accumulate_product_bf(const long long (&sr)[NF], const long long (&si)[NF], int e0,
+                                                      uint32_t neg_mask, double& ar, double& ai) {
+  if constexpr (NF == 1) {
+    ar += xor_sign(bf_to_double(sr[0], e0), neg_mask);
+    ai += xor_sign(bf_to_double(si[0], e0), neg_mask);
+  } else {
+    constexpr int H = NF < 4 ? NF : (NF + 1) / 2;  // first chain: factors 0 .. H - 1
+    long long xr = sr[0], xi = si[0], yr, yi;
+    int e = e0;
+    e += bf_renorm(xr, xi) - 29;
+    if constexpr (H < NF) {
+      yr = sr[H];
+      yi = si[H];
+      e += bf_renorm(yr, yi) - 29;
+    }
 #pragma unroll
-  for (int f = 1; f < NF - 1; ++f) {
-    const double br = fx_to_double(sr[f], bias_exp);
-    const double bi = fx_to_double(si[f], bias_exp);
-    const double t_re = fma(pr, br, -(pi * bi));
-    const double t_im = fma(pr, bi, pi * br);
-    pr = t_re;
-    pi = t_im;
+    for (int k = 1; k < H; ++k) {
+      bf_mul_high(xr, xi, sr[k], si[k], xr, xi);
+      if (k < H - 1 || H < NF) e += 35 + bf_renorm(xr, xi);
+      if (H + k < NF) {
+        bf_mul_high(yr, yi, sr[H + k], si[H + k], yr, yi);
+        e += 35 + bf_renorm(yr, yi);
+      }
+    }
+    if constexpr (H < NF) bf_mul_high(xr, xi, yr, yi, xr, xi);
+    e += 64;  // the last product stays unnormalised: each component is rounded on its own
+    ar += xor_sign(bf_to_double(xr, e), neg_mask);
+    ai += xor_sign(bf_to_double(xi, e), neg_mask);
   }
-  pr = xor_sign(pr, neg_mask);
-  pi = xor_sign(pi, neg_mask);
-  const double br = fx_to_double(sr[NF - 1], bias_exp);
-  const double bi = fx_to_double(si[NF - 1], bias_exp);
-  ar = fma(pr, br, ar);
-  ar = fma(-pi, bi, ar);
-  ai = fma(pr, bi, ai);
-  ai = fma(pi, br, ai);
 }
 
 // ---------------------------------------------------------------------------

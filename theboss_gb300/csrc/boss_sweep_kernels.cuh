@@ -6,20 +6,6 @@
 
 namespace boss {
 
-// Factors of a single permanent's product chain multiplied in block floating
-// point on the integer pipe (0: all on the FP64 pipe, accumulate_product<NF>).
-template <int NF>
-constexpr int kPermBF = NF >= 10 ? NF - 8 : (NF >= 2 ? NF : 0);
-
-template <int NF>
-__device__ __forceinline__ void perm_product(const long long (&sr)[NF], const long long (&si)[NF], int bias_exp,
-                                             uint32_t neg_mask, double& ar, double& ai) {
-  if constexpr (kPermBF<NF> >= 2)
-    accumulate_product_bf<NF, kPermBF<NF>>(sr, si, bias_exp, neg_mask, ar, ai);
-  else
-    accumulate_product<NF>(sr, si, bias_exp, neg_mask, ar, ai);
-}
-
 // One permanent per sweep problem; every thread writes one complex partial.
 template <int NF>
 __global__ void __launch_bounds__(128, 3) perm_sweep_kernel(const SweepProblem* __restrict__ probs, int n_probs,
@@ -30,36 +16,36 @@ __global__ void __launch_bounds__(128, 3) perm_sweep_kernel(const SweepProblem* 
   const SweepProblem& P = probs[find_problem(probs, n_probs, gt)];
   const int64_t q = gt - P.thread_begin;
   int64_t a, len;
-  thread_range(P, q, a, len);
+  thread_range_aligned(P, q, P.align, a, len);
   double tr = 0.0, ti = 0.0;
   if (len > 0) {
     const longlong2* D = pool + P.mat_off;
     const longlong2* base = pool + P.base_off;
-    const int bias = 1023 + 63 - P.fx;
+    const int e0 = P.fx;
     const int nb = P.nb;
     long long sr[NF], si[NF];
     uint64_t g;
     uint32_t parity;
     double w;
-    decode_code<NF>(P, D, base, (uint64_t)a, sr, si, g, parity, w);
+    decode_code<NF, true>(P, D, base, (uint64_t)a, sr, si, g, parity, w);
     double ar = 0.0, ai = 0.0;
-    perm_product<NF>(sr, si, bias, parity << 31, ar, ai);
+    accumulate_product_bf<NF>(sr, si, e0, parity << 31, ar, ai);
     const uint64_t end = (uint64_t)(a + len);
     for (uint64_t t = (uint64_t)a + 1; t < end; ++t) {
       const int i = __ffsll((long long)t) - 1;
       if (i < nb) {
         const uint32_t bit = (uint32_t)(g >> i) & 1u;
         g ^= 1ull << i;
-        flip_binary<NF>(D, i, bit, sr, si);
+        flip_packed<NF>(D, i, bit, sr, si);
         parity ^= 1u;
       } else {  // a multi-valued digit moves: settle the weight and re-decode
         tr = fma(w, ar, tr);
         ti = fma(w, ai, ti);
         ar = 0.0;
         ai = 0.0;
-        decode_code<NF>(P, D, base, t, sr, si, g, parity, w);
+        decode_code<NF, true>(P, D, base, t, sr, si, g, parity, w);
       }
-      perm_product<NF>(sr, si, bias, parity << 31, ar, ai);
+      accumulate_product_bf<NF>(sr, si, e0, parity << 31, ar, ai);
     }
     tr = fma(w, ar, tr);
     ti = fma(w, ai, ti);
@@ -97,26 +83,11 @@ __device__ __forceinline__ void settle_minors(const SweepProblem& P, double2* M,
   }
 }
 
-// Factors of the all-minors product chain multiplied in block floating point on
-// the integer pipe (0: all on the FP64 pipe, accumulate_product<NF>): 8 up to 16
-// factors (4 blocks per SM), nf - 8 above (3 blocks, more registers per thread).
-template <int NF>
-constexpr int kMinorsBF = NF >= 2 ? (NF < 8 ? NF : (NF <= 16 ? 8 : NF - 8)) : 0;
-
 // Blocks of 128 threads per SM the all-minors kernel is compiled for: 4 (128
-// registers, a few spilled words at NF 11..16) up to NF = 16, where the fourth
+// registers, some spilled words from NF 12 on) up to NF = 16, where the fourth
 // block's warps hide more latency than the spills cost; 3 above.
 template <int NF>
 constexpr int kMinorsMinBlocks = NF <= 16 ? 4 : 3;
-
-template <int NF>
-__device__ __forceinline__ void minors_product(const long long (&sr)[NF], const long long (&si)[NF], int bias_exp,
-                                               uint32_t neg_mask, double& ar, double& ai) {
-  if constexpr (kMinorsBF<NF> >= 2)
-    accumulate_product_bf<NF, kMinorsBF<NF>>(sr, si, bias_exp, neg_mask, ar, ai);
-  else
-    accumulate_product<NF>(sr, si, bias_exp, neg_mask, ar, ai);
-}
 
 // All-minors sweep (C&C-B), in Glynn form.  theboss sums each minor over the
 // Ryser codes with r_i = 0 (bs_cc_ryser_submatrices_permanent_calculator.py:96-119).
@@ -140,9 +111,9 @@ __device__ __forceinline__ void minors_walk(const SweepProblem& P, const longlon
   const int nd = P.nd + P.fixed_digit;
   for (int j = 0; j < nd; ++j) M[j * STRIDE] = make_double2(0.0, 0.0);
   int64_t a, len;
-  thread_range(P, q, a, len);
+  thread_range_aligned(P, q, P.align, a, len);
   if (len > 0) {
-    const int bias = 1023 + 63 - P.fx;
+    const int e0 = P.fx;
     const int nb = P.nb;
     const int low = nb < kSegLog ? nb : kSegLog;
     const bool weighted = P.nd > P.nb;
@@ -150,9 +121,9 @@ __device__ __forceinline__ void minors_walk(const SweepProblem& P, const longlon
     uint64_t g, t_seg = (uint64_t)a;
     uint32_t parity;
     double w;
-    decode_code<NF>(P, D, base, (uint64_t)a, sr, si, g, parity, w);
+    decode_code<NF, true>(P, D, base, (uint64_t)a, sr, si, g, parity, w);
     double Rr = 0.0, Ri = 0.0;
-    minors_product<NF>(sr, si, bias, parity << 31, Rr, Ri);
+    accumulate_product_bf<NF>(sr, si, e0, parity << 31, Rr, Ri);
     const uint64_t end = (uint64_t)(a + len);
     for (uint64_t t = (uint64_t)a + 1; t < end; ++t) {
       const int i = __ffsll((long long)t) - 1;
@@ -168,7 +139,7 @@ __device__ __forceinline__ void minors_walk(const SweepProblem& P, const longlon
         v.y += xor_sign(vi, bit << 31);
         M[i * STRIDE] = v;
         g ^= 1ull << i;
-        flip_binary<NF>(D, i, bit, sr, si);
+        flip_packed<NF>(D, i, bit, sr, si);
         parity ^= 1u;
       } else {
         settle_minors<STRIDE>(P, M, Rr, Ri, w, g, t_seg);
@@ -178,13 +149,13 @@ __device__ __forceinline__ void minors_walk(const SweepProblem& P, const longlon
         if (i < nb) {
           const uint32_t bit = (uint32_t)(g >> i) & 1u;
           g ^= 1ull << i;
-          flip_binary<NF>(D, i, bit, sr, si);
+          flip_packed<NF>(D, i, bit, sr, si);
           parity ^= 1u;
         } else {
-          decode_code<NF>(P, D, base, t, sr, si, g, parity, w);
+          decode_code<NF, true>(P, D, base, t, sr, si, g, parity, w);
         }
       }
-      minors_product<NF>(sr, si, bias, parity << 31, Rr, Ri);
+      accumulate_product_bf<NF>(sr, si, e0, parity << 31, Rr, Ri);
     }
     settle_minors<STRIDE>(P, M, Rr, Ri, w, g, t_seg);
   }
