@@ -13,6 +13,7 @@
 
 #include "../../include/boss.h"
 #include "boss_internal.h"
+#include "boss_quad.cuh"
 
 namespace boss {
 
@@ -88,9 +89,32 @@ int ensure_pinned(Context* cx, size_t bytes) {
 
 static inline size_t align_up(size_t x, size_t a) { return (x + a - 1) & ~(a - 1); }
 
-// D's rows as the FP64 permanent and all-minors sweeps take them (pack_row).
-static void pack_rows(const std::vector<longlong2>& D, longlong2* out) {
-  for (size_t i = 0; i < D.size(); ++i) out[i] = longlong2{pack_row(D[i].x), pack_row(D[i].y)};
+// The device description of a planned sweep, but for its place in the launch.
+static void describe_sweep(const HostSweep& h, int64_t n_threads, SweepProblem& P) {
+  memset(&P, 0, sizeof(P));
+  P.low = h.layout == kRowsQuad ? 2 : 0;
+  P.nd = h.nd - P.low;
+  P.nb = h.nb - P.low;
+  P.nf = h.nf;
+  P.kind = h.kind;
+  P.parity0 = h.parity0;
+  P.fx = -h.fx_sum;
+  P.has_base = h.has_base;
+  P.n_codes = (int64_t)(h.total_codes >> P.low);
+  P.n_threads = n_threads;
+  P.align = range_align(P.n_codes, n_threads, P.nb);
+  P.scale = h.scale;
+  P.fixed_digit = (h.fixed_mode >= 0) ? 1 : 0;
+  P.group = 1;
+  for (int i = 0; i < P.nd; ++i) P.mult[i] = h.mult[i + P.low];
+}
+
+// Threads for each of a launch's sweeps (all of one sweep_class).
+static void split_threads(const std::vector<HostSweep>& sweeps, int64_t resident, std::vector<int64_t>& nthr) {
+  const int low = sweeps[0].layout == kRowsQuad ? 2 : 0;
+  std::vector<uint64_t> codes(sweeps.size());
+  for (size_t p = 0; p < sweeps.size(); ++p) codes[p] = sweeps[p].total_codes >> low;
+  partition_threads(codes, resident, nthr, kMinCodesPerThread >> low);
 }
 
 // A list of sweeps that share one factor count, uploaded and ready to launch.
@@ -110,58 +134,42 @@ static int sweeps_prepare(Context* cx, const std::vector<HostSweep>& sweeps, boo
   B.nf = sweeps[0].nf;
   B.minors = minors;
   B.nd_max = nd_max;
-  // Float pairs only for Glynn-kind sweeps: the Ryser form's alternating sum cancels
-  // far more (its FP64 error is already ~1e-10 at n = 20), and float pairs would
-  // leave theboss's tolerance.
-  bool glynn = true;
-  for (const HostSweep& h : sweeps) glynn = glynn && h.kind == kGlynn;
-  B.ff = glynn && (minors ? (g_minors_arith == 0 && minors_ff_available(B.nf))
-                          : (g_perm_arith == 0 && perm_ff_available(B.nf)));
+  // Float pairs (planned as plain rows) only for Glynn-kind sweeps: the Ryser form's
+  // alternating sum cancels far more (its FP64 error is already ~1e-10 at n = 20),
+  // and float pairs would leave theboss's tolerance.
+  B.ff = sweeps[0].layout == kRowsPlain;
+  const bool quad = sweeps[0].layout == kRowsQuad;
   const SweepOp op = minors ? SweepOp::kMinors : (B.ff ? SweepOp::kPermFF : SweepOp::kPerm);
-  std::vector<uint64_t> codes(n);
   B.codes = 0.0;
+  int rows = 1;  // all-minors: rows of minors per thread
   for (int p = 0; p < n; ++p) {
-    codes[p] = sweeps[p].total_codes;
-    B.codes += (double)codes[p];
+    B.codes += (double)sweeps[p].total_codes;
+    rows = std::max(rows, sweeps[p].nd + (sweeps[p].fixed_mode >= 0 ? 1 : 0));
   }
-  int rows = 1;  // all-minors: shared-memory rows of minors per thread
-  for (int p = 0; p < n; ++p) rows = std::max(rows, sweeps[p].nd + (sweeps[p].fixed_mode >= 0 ? 1 : 0));
   std::vector<int64_t> nthr;
-  partition_threads(codes,
-                    minors ? sweep_resident_minors(B.nf, rows, cx->sm_count, B.ff)
-                           : sweep_resident_threads(B.nf, op, cx->sm_count),
-                    nthr);
+  split_threads(sweeps,
+                quad     ? quad_resident_walkers(B.nf, rows, minors, cx->sm_count)
+                : minors ? sweep_resident_minors(B.nf, rows, cx->sm_count, B.ff)
+                         : sweep_resident_threads(B.nf, op, cx->sm_count),
+                nthr);
   std::vector<SweepProblem> probs(n);
   int64_t pool_n = 0, threads = 0, parts = 0;
   for (int p = 0; p < n; ++p) {
     const HostSweep& h = sweeps[p];
     SweepProblem& P = probs[p];
-    memset(&P, 0, sizeof(P));
-    P.nd = h.nd;
-    P.nb = h.nb;
-    P.nf = h.nf;
-    P.kind = h.kind;
-    P.parity0 = h.parity0;
-    P.fx = -h.fx_sum;
-    P.has_base = h.has_base;
+    describe_sweep(h, nthr[p], P);
     P.out_idx = p;
-    P.align = range_align((int64_t)h.total_codes, nthr[p], h.nb);
-    P.n_codes = (int64_t)h.total_codes;
     P.thread_begin = threads;
-    P.n_threads = nthr[p];
     P.mat_off = pool_n;
     pool_n += (int64_t)h.D.size();
     P.base_off = pool_n;
     pool_n += (int64_t)h.base.size();
     P.part_off = parts;
-    P.scale = h.scale;
     if (B.ff) {  // float-pair rows of the binary digits, then the factors' biases
       P.ff_off = pool_n;
       pool_n += (int64_t)h.nb * h.nf + (h.nf + 3) / 4;
       P.scale = std::ldexp(h.scale, h.ff_exp);
     }
-    P.fixed_digit = (h.fixed_mode >= 0) ? 1 : 0;
-    for (int i = 0; i < h.nd; ++i) P.mult[i] = h.mult[i];
     threads += nthr[p];
     parts += nthr[p] * (minors ? h.nd + P.fixed_digit : 1);
   }
@@ -181,11 +189,9 @@ static int sweeps_prepare(Context* cx, const std::vector<HostSweep>& sweeps, boo
   longlong2* hp = (longlong2*)(h + o_pool);
   for (int p = 0; p < n; ++p) {
     const HostSweep& hs = sweeps[p];
+    std::copy(hs.D.begin(), hs.D.end(), hp + probs[p].mat_off);
     std::copy(hs.base.begin(), hs.base.end(), hp + probs[p].base_off);
-    if (!B.ff) {
-      pack_rows(hs.D, hp + probs[p].mat_off);
-    } else {
-      std::copy(hs.D.begin(), hs.D.end(), hp + probs[p].mat_off);
+    if (B.ff) {
       float4* df = reinterpret_cast<float4*>(hp + probs[p].ff_off);
       for (int d = 0; d < hs.nb; ++d)
         for (int f = 0; f < hs.nf; ++f) {
@@ -208,6 +214,7 @@ static int sweeps_prepare(Context* cx, const std::vector<HostSweep>& sweeps, boo
   B.L.partials = (double2*)cx->partials.ptr;
   B.L.grid = (int)((threads + 127) / 128);
   B.L.rows = rows;
+  B.L.quad = quad;
   return kOk;
 }
 
@@ -272,13 +279,12 @@ static Side make_side(const int32_t* occ, int len) {
 }
 
 // Fixed-point fraction bits for sums bounded by `bound` (|s| <= bound): the
-// integer sums stay below 2^61.
-static int choose_fx(double bound) {
+// integer sums stay below 2^bits (with room for the entries' roundings).
+static int choose_fx(double bound, int bits) {
   if (!(bound > 0.0) || !std::isfinite(bound)) return 56;
   int ex = 0;
-  std::frexp(bound, &ex);  // bound < 2^ex
-  int fx = 61 - ex;
-  return std::max(-1000, std::min(fx, 1000));
+  std::frexp(bound * (1.0 + 0x1p-40), &ex);  // bound < 2^ex
+  return std::max(-1000, std::min(bits - ex, 1000));
 }
 
 // v * 2^fx rounded to the nearest integer (ties to even); |v * 2^fx| < 2^62.
@@ -289,15 +295,75 @@ static inline long long to_fixed(double v, double scale) {
   return (long long)x;
 }
 
+// FP64 by default (theboss computes in float64); float pairs on request.
+int g_minors_arith = 1;
+int g_perm_arith = 1;
+
+static longlong2 packed(Cx64 v) { return longlong2{pack_row(v.re), pack_row(v.im)}; }
+static longlong2 plain(Cx64 v) { return longlong2{v.re, v.im}; }
+static Cx64 times(Cx64 v, long long k) { return Cx64{v.re * k, v.im * k}; }
+
+// The rows, base and constants of boss_quad.cuh.  u[a * nf + f]: every digit's
+// fixed-point u (binary digits first, the held one at `drop`).
+static void fill_quad(HostSweep& hs, const Side& dig, int drop, bool glynn, const std::vector<Cx64>& u) {
+  const int nf = hs.nf, slots = quad_slots(nf), W = 4 * slots, nd_all = (int)dig.modes.size(), ndo = hs.nd - 2;
+  const Cx64 zero{0, 0};
+  hs.D.assign((size_t)ndo * W, longlong2{0, 0});
+  hs.base.assign((size_t)W + 2 * slots, longlong2{0, 0});
+  longlong2* consts = hs.base.data() + W;
+  for (int g = 0; g < slots; ++g) {
+    const bool unit = 2 * g + 1 >= nf;  // an odd last factor's partner, the constant 1
+    auto U = [&](int a, int k) { return k && unit ? zero : u[(size_t)a * nf + 2 * g + k]; };
+    const Cx64 f0 = U(0, 0), f1 = U(1, 0), g0 = U(0, 1), g1 = U(1, 1);
+    Cx64 of = zero, og = zero, ep = zero, em = zero;
+    int row = 0;
+    for (int a = 2; a < nd_all; ++a) {
+      const Cx64 uf = U(a, 0), ug = U(a, 1);
+      Cx64 rp, rm;
+      quad_row(uf, ug, f0, f1, g0, g1, rp, rm);
+      if (a != drop) {
+        longlong2* r = &hs.D[(size_t)(row++) * W + 4 * g];
+        r[0] = packed(uf);
+        r[1] = packed(ug);
+        r[2] = packed(rp);
+        r[3] = packed(rm);
+      }
+      of = cx_add(of, times(uf, dig.mult[a]));
+      og = cx_add(og, times(ug, dig.mult[a]));
+      ep = cx_add(ep, times(rp, dig.mult[a]));
+      em = cx_add(em, times(rm, dig.mult[a]));
+    }
+    if (!glynn) {  // Ryser: no base, and r = (1 - d) / 2 leaves -(u0 + u1)
+      of = cx_sub(zero, cx_add(f0, f1));
+      og = cx_sub(zero, cx_add(g0, g1));
+      quad_row(of, og, f0, f1, g0, g1, ep, em);
+    }
+    if (unit) {
+      og = Cx64{kQuadOne, 0};
+      quad_row(zero, og, f0, f1, zero, zero, ep, em);
+    }
+    longlong2* b = &hs.base[4 * g];
+    b[0] = plain(of);
+    b[1] = plain(og);
+    b[2] = plain(ep);
+    b[3] = plain(em);
+    Cx64 cp, cm;
+    quad_const(f0, f1, g0, g1, cp, cm);
+    consts[2 * g] = plain(cp);
+    consts[2 * g + 1] = plain(cm);
+  }
+  if (nf & 1) hs.fx_sum += 62;
+}
+
 // Fills a sweep that iterates `dig` and multiplies over the particles of `col`
 // (a mode occupied p times gives p factors).  entry(a, l) is the matrix element
 // between digit mode a and product mode l.  Every factor f has its own fixed-point
-// scale 2^fx_f, chosen so that its largest possible sum fills 61 bits (a shared
-// scale would leave the factors of small rows with fewer significant bits);
-// shared_fx: one scale for all of them.
+// scale 2^fx_f, chosen so that its largest possible sum fills the bits (a shared
+// scale would leave the factors of small rows with fewer significant bits); the
+// gradients share one.
 template <class F>
-static int fill_sweep(HostSweep& hs, const Side& dig, const Side& col, int kind, bool halve, bool shared_fx,
-                      F entry) {
+static int fill_sweep(HostSweep& hs, const Side& dig, const Side& col, int kind, bool halve, PlanFor plan, bool ff,
+                      int quad_min, F entry) {
   int drop = -1;
   if (halve && dig.nb > 0) drop = dig.nb - 1;  // a binary digit fixed at r = 0
   hs.kind = kind;
@@ -327,11 +393,16 @@ static int fill_sweep(HostSweep& hs, const Side& dig, const Side& col, int kind,
     hs.total_codes *= b;
     ++a_out;
   }
+  const bool glynn = kind == kGlynn;
+  hs.layout = (plan == kPlanGrad || (ff && glynn && plan == kPlanAny)) ? kRowsPlain
+              : (plan != kPlanTemplated && hs.nb >= 2 && hs.nf >= quad_min)   ? kRowsQuad
+                                                                       : kRowsPacked;
   // |row sum| <= sum_a mult_a * max component of the entries (of one factor, or of all)
+  const int nf = hs.nf, nd_all = (int)dig.modes.size();
   double bound[kMaxFactors] = {}, shared = 0.0;
-  for (size_t a = 0; a < dig.modes.size(); ++a) {
+  for (int a = 0; a < nd_all; ++a) {
     double mx = 0.0;
-    for (int f = 0; f < hs.nf; ++f) {
+    for (int f = 0; f < nf; ++f) {
       const double2 z = entry(dig.modes[a], fmode[f]);
       const double c = std::max(std::fabs(z.x), std::fabs(z.y));
       bound[f] += dig.mult[a] * c;
@@ -339,44 +410,54 @@ static int fill_sweep(HostSweep& hs, const Side& dig, const Side& col, int kind,
     }
     shared += dig.mult[a] * mx;
   }
-  hs.fx = choose_fx(shared);
-  hs.D.resize((size_t)hs.nd * hs.nf);
-  hs.has_base = (kind == kGlynn);
-  if (hs.has_base) hs.base.assign(hs.nf, longlong2{0, 0});
-  hs.fbias.assign(hs.nf, 189);
-  hs.ff_exp = 0;
+  const bool old_rows = hs.layout == kRowsPlain;
+  const int bits = old_rows ? 61 : 62;  // plain rows hold D = -2 u, which needs the bit
+  hs.fx = choose_fx(shared, bits);
   hs.fx_sum = 0;
-  const long long fsign = (kind == kGlynn) ? -2 : 1;  // Glynn: s = base - 2 sum r U
-  for (int f = 0; f < hs.nf; ++f) {
-    const int fx = shared_fx ? hs.fx : choose_fx(bound[f]);
-    const double scale = std::ldexp(1.0, fx);
-    long long re = 0, im = 0;
+  hs.ff_exp = 0;
+  hs.fbias.assign(nf, 189);
+  std::vector<Cx64> u((size_t)nd_all * nf);
+  for (int f = 0; f < nf; ++f) {
+    const int fx = plan == kPlanGrad ? hs.fx : choose_fx(bound[f], bits);
+    const double scale = std::ldexp(glynn || old_rows ? 1.0 : -0.5, fx);  // Ryser's u = -U / 2
     unsigned long long bx = 0, by = 0;
-    a_out = 0;
-    for (size_t a = 0; a < dig.modes.size(); ++a) {
+    for (int a = 0; a < nd_all; ++a) {
       const double2 z = entry(dig.modes[a], fmode[f]);
       const long long x = to_fixed(z.x, scale), y = to_fixed(z.y, scale);
-      re += (long long)dig.mult[a] * x;
-      im += (long long)dig.mult[a] * y;
+      u[(size_t)a * nf + f] = Cx64{x, y};
       bx += (unsigned long long)dig.mult[a] * (unsigned long long)std::llabs(x);
       by += (unsigned long long)dig.mult[a] * (unsigned long long)std::llabs(y);
-      if ((int)a != drop) hs.D[(size_t)(a_out++) * hs.nf + f] = longlong2{fsign * x, fsign * y};
     }
-    if (hs.has_base) hs.base[f] = longlong2{re, im};
     const unsigned long long b = std::max(bx, by);
     const int p = b ? 63 - __builtin_clzll(b) : 0;
     hs.fbias[f] = 189 - p;
     hs.ff_exp += p + 1 - fx;
     hs.fx_sum += fx;
   }
-  hs.scale = hs.has_base ? std::ldexp(1.0, -dig.n) * (drop >= 0 ? 2.0 : 1.0) : 1.0;
-  hs.parity0 = hs.has_base ? 0 : (dig.n & 1);
+  hs.scale = glynn ? std::ldexp(1.0, -dig.n) * (drop >= 0 ? 2.0 : 1.0) : 1.0;
+  hs.parity0 = glynn ? 0 : (dig.n & 1);
+  hs.has_base = glynn || !old_rows;
+  if (hs.layout == kRowsQuad) {
+    fill_quad(hs, dig, drop, glynn, u);
+    return kOk;
+  }
+  hs.D.resize((size_t)hs.nd * nf);
+  if (hs.has_base) hs.base.assign(nf, longlong2{0, 0});
+  a_out = 0;
+  for (int a = 0; a < nd_all; ++a) {
+    for (int f = 0; f < nf; ++f) {
+      const Cx64 v = u[(size_t)a * nf + f];
+      if (a != drop)
+        hs.D[(size_t)a_out * nf + f] = !old_rows ? packed(v) : glynn ? longlong2{-2 * v.re, -2 * v.im} : plain(v);
+      if (glynn) {
+        hs.base[f].x += (long long)dig.mult[a] * v.re;
+        hs.base[f].y += (long long)dig.mult[a] * v.im;
+      }
+    }
+    if (a != drop) ++a_out;
+  }
   return kOk;
 }
-
-// FP64 by default (theboss computes in float64); float pairs on request.
-int g_minors_arith = 1;
-int g_perm_arith = 1;
 
 void host_fx_to_ff(long long x, int fbias, float& hi, float& lo) {
   const unsigned long long sgn = (unsigned long long)(x >> 63);
@@ -411,8 +492,9 @@ void host_fx_to_ff(long long x, int fbias, float& hi, float& lo) {
 // One permanent request.  Returns kOk and either fills `hs` (needs_sweep = true)
 // or sets `value` directly for the edge cases theboss special-cases.
 int plan_permanent(const double* U, int m, const int32_t* S, const int32_t* T, int len, int variant,
-                          HostSweep& hs, bool& needs_sweep, double2& value, bool shared_fx) {
+                          HostSweep& hs, bool& needs_sweep, double2& value, PlanFor plan) {
   needs_sweep = false;
+  const bool ff = g_perm_arith == 0;  // float pairs: every factor count has the kernel (kFFPermMaxFactors)
   if (len > m || len < 0) {  // bs_permanent_calculator_base.py:61-72
     set_error("state length exceeds matrix dimension");
     return kErrSize;
@@ -437,7 +519,7 @@ int plan_permanent(const double* U, int m, const int32_t* S, const int32_t* T, i
         return kOk;
       }
       const bool ch = (variant == BOSS_CHIN_HUH);
-      const int st = fill_sweep(hs, in, out, ch ? kGlynn : kRyser, ch && in.n == out.n, shared_fx, entry_in_out);
+      const int st = fill_sweep(hs, in, out, ch ? kGlynn : kRyser, ch && in.n == out.n, plan, ff, kQuadMinFactors, entry_in_out);
       if (st) return st;
       needs_sweep = true;
       return kOk;
@@ -461,10 +543,10 @@ int plan_permanent(const double* U, int m, const int32_t* S, const int32_t* T, i
       const uint64_t co = out.nb ? out.codes / 2 : out.codes;
       int st;
       bool outs = co < ci;
-      st = outs ? fill_sweep(hs, out, in, kGlynn, true, shared_fx, entry_out_in) : fill_sweep(hs, in, out, kGlynn, true, shared_fx, entry_in_out);
+      st = outs ? fill_sweep(hs, out, in, kGlynn, true, plan, ff, kQuadMinFactors, entry_out_in) : fill_sweep(hs, in, out, kGlynn, true, plan, ff, kQuadMinFactors, entry_in_out);
       if (st == kErrLimit) {  // try the other orientation
         outs = !outs;
-        st = outs ? fill_sweep(hs, out, in, kGlynn, true, shared_fx, entry_out_in) : fill_sweep(hs, in, out, kGlynn, true, shared_fx, entry_in_out);
+        st = outs ? fill_sweep(hs, out, in, kGlynn, true, plan, ff, kQuadMinFactors, entry_out_in) : fill_sweep(hs, in, out, kGlynn, true, plan, ff, kQuadMinFactors, entry_in_out);
       }
       if (st) return st;
       hs.digits_are_outputs = outs;
@@ -544,7 +626,8 @@ static int plan_minors(const double* U, int m, const int32_t* S, const int32_t* 
   // from one sweep, one single-occupied digit held at r = 0); the kernel
   // accumulates half of each, hence the factor 2.
   auto entry = [&](int i_mode, int j_mode) { return U_at(U, m, j_mode, i_mode); };
-  const int st = fill_sweep(hs, in, out, kGlynn, true, false, entry);
+  const int st = fill_sweep(hs, in, out, kGlynn, true, kPlanAny, g_minors_arith == 0 && out.n <= kFFMaxFactors,
+                            kQuadMinMinorFactors, entry);
   if (st) return st;
   hs.scale *= 2.0;
   needs_sweep = true;
@@ -588,8 +671,8 @@ int boss_perm_batch(const double* matrix, int32_t m, const int32_t* input_states
     return kErrArg;
   }
   std::lock_guard<std::mutex> lk(g_api_mutex);
-  std::vector<HostSweep> by_nf[kMaxFactors + 1];
-  std::vector<int> which[kMaxFactors + 1];
+  std::vector<HostSweep> by_class[kSweepClasses];
+  std::vector<int> which[kSweepClasses];
   std::vector<int> small[kSmallPermMax + 1];  // one GPU thread per permanent, no planning
   bool any = false, any_small = false;
   if (variant < BOSS_RYSER || variant > BOSS_CLASSIC) {
@@ -619,8 +702,9 @@ int boss_perm_batch(const double* matrix, int32_t m, const int32_t* input_states
     const int st = plan_permanent(matrix, m, Sk, Tk, len, variant, hs, need, v);
     if (st) return st;
     if (need) {
-      which[hs.nf].push_back(k);
-      by_nf[hs.nf].push_back(std::move(hs));
+      const int c = sweep_class(hs);
+      which[c].push_back(k);
+      by_class[c].push_back(std::move(hs));
       any = true;
     } else {
       results[2 * k] = v.x;
@@ -634,14 +718,14 @@ int boss_perm_batch(const double* matrix, int32_t m, const int32_t* input_states
   if (any_small && (st = small_perm_batch(cx, matrix, m, len, input_states, output_states, small,
                                           (double2*)results)))
     return st;
-  for (int nf = 1; nf <= kMaxFactors; ++nf) {
-    if (by_nf[nf].empty()) continue;
-    std::vector<double2> out(by_nf[nf].size());
-    st = run_sweeps(cx, by_nf[nf], false, 1, out.data());
+  for (int c = 0; c < kSweepClasses; ++c) {
+    if (by_class[c].empty()) continue;
+    std::vector<double2> out(by_class[c].size());
+    st = run_sweeps(cx, by_class[c], false, 1, out.data());
     if (st) return st;
     for (size_t a = 0; a < out.size(); ++a) {
-      results[2 * which[nf][a]] = out[a].x;
-      results[2 * which[nf][a] + 1] = out[a].y;
+      results[2 * which[c][a]] = out[a].x;
+      results[2 * which[c][a] + 1] = out[a].y;
     }
   }
   return kOk;
@@ -659,8 +743,8 @@ int boss_submatrices_batch(const double* matrix, int32_t m, const int32_t* input
     return kErrArg;
   }
   std::lock_guard<std::mutex> lk(g_api_mutex);
-  std::vector<HostSweep> by_nf[kMaxFactors + 1];
-  std::vector<int> which[kMaxFactors + 1];
+  std::vector<HostSweep> by_class[kSweepClasses];
+  std::vector<int> which[kSweepClasses];
   double2* res = (double2*)results;
   bool any = false;
   for (int k = 0; k < count; ++k) {
@@ -670,8 +754,9 @@ int boss_submatrices_batch(const double* matrix, int32_t m, const int32_t* input
                                need, res + (size_t)k * len);
     if (st) return st;
     if (need) {
-      which[hs.nf].push_back(k);
-      by_nf[hs.nf].push_back(std::move(hs));
+      const int c = sweep_class(hs);
+      which[c].push_back(k);
+      by_class[c].push_back(std::move(hs));
       any = true;
     }
   }
@@ -680,14 +765,14 @@ int boss_submatrices_batch(const double* matrix, int32_t m, const int32_t* input
   Context* cx = context(&st);
   if (!cx) return st;
   const int nd_max = kMaxMinorDigits;
-  for (int nf = 1; nf <= kMaxFactors; ++nf) {
-    if (by_nf[nf].empty()) continue;
-    std::vector<double2> out(by_nf[nf].size() * nd_max);
-    st = run_sweeps(cx, by_nf[nf], true, nd_max, out.data());
+  for (int c = 0; c < kSweepClasses; ++c) {
+    if (by_class[c].empty()) continue;
+    std::vector<double2> out(by_class[c].size() * nd_max);
+    st = run_sweeps(cx, by_class[c], true, nd_max, out.data());
     if (st) return st;
-    for (size_t a = 0; a < by_nf[nf].size(); ++a) {
-      const HostSweep& hs = by_nf[nf][a];
-      double2* row = res + (size_t)which[nf][a] * len;
+    for (size_t a = 0; a < by_class[c].size(); ++a) {
+      const HostSweep& hs = by_class[c][a];
+      double2* row = res + (size_t)which[c][a] * len;
       for (int d = 0; d < hs.nd; ++d) {  // the sweep gives S_i minor_i
         const double2 v = out[a * nd_max + d];
         row[hs.digit_mode[d]] = make_double2(v.x / hs.mult[d], v.y / hs.mult[d]);
@@ -717,7 +802,7 @@ int boss_perm_grad_batch(const double* matrix, int32_t m, const int32_t* input_s
     double2 v = make_double2(0.0, 0.0);
     const int32_t* S = input_states + (size_t)k * len;
     const int32_t* T = output_states + (size_t)k * len;
-    int st = plan_permanent(matrix, m, S, T, len, BOSS_GLYNN, hs, need, v, true);
+    int st = plan_permanent(matrix, m, S, T, len, BOSS_GLYNN, hs, need, v, kPlanGrad);
     if (st) return st;
     if (!need) {  // no particles: perm = 1, gradient 0
       P2[k] = v;
@@ -854,13 +939,14 @@ int boss_perm_bench(const double* matrix, int32_t m, const int32_t* input_states
   }
   std::lock_guard<std::mutex> lk(g_api_mutex);
   std::vector<HostSweep> sweeps;
+  PlanFor plan = kPlanAny;
   double flops = 0.0;
   for (int k = 0; k < count; ++k) {
     HostSweep hs;
     bool need = false;
     double2 v;
     const int st = plan_permanent(matrix, m, input_states + (size_t)k * len, output_states + (size_t)k * len, len,
-                                  variant, hs, need, v);
+                                  variant, hs, need, v, plan);
     if (st) return st;
     if (!need) {
       set_error("benchmark permanents must need a sweep");
@@ -869,6 +955,13 @@ int boss_perm_bench(const double* matrix, int32_t m, const int32_t* input_states
     if (!sweeps.empty() && hs.nf != sweeps[0].nf) {
       set_error("benchmark permanents must share one product size");
       return kErrArg;
+    }
+    if (!sweeps.empty() && hs.layout != sweeps[0].layout && plan == kPlanAny) {  // one kernel for all: start over
+      plan = kPlanTemplated;
+      sweeps.clear();
+      flops = 0.0;
+      k = -1;
+      continue;
     }
     // per code: nf complex adds, nf - 1 complex products, one signed complex add
     flops += (double)hs.total_codes * (8.0 * hs.nf - 4.0);
@@ -1010,7 +1103,7 @@ __global__ void noalloc_scatter_kernel(const int32_t* __restrict__ idx, const do
 
 // One product-size group of a request: its sweeps' layout in the scratch.
 struct NoAllocGroup {
-  int nf = 0;
+  int cls = 0;  // sweep_class
   std::vector<int64_t> nthr;
   int64_t threads = 0;
   size_t o_pool = 0, o_part = 0, bytes = 0;
@@ -1035,38 +1128,52 @@ extern "C" int boss_perm_batch_noalloc(const double* matrix, int32_t m, const in
   cudaStream_t s = (cudaStream_t)stream;
   double2* out = (double2*)results_device;
   // (1) Plan every permanent and lay out every scratch image; reject the request
-  // before anything is queued if one image exceeds the scratch.
-  std::vector<HostSweep> by_nf[kMaxFactors + 1];
-  std::vector<int> which[kMaxFactors + 1];
+  // before anything is queued if one image exceeds the scratch.  The quad kernel's
+  // rows take twice the templated kernels': a request too large for them is planned
+  // again for those.
+  std::vector<HostSweep> by_class[kSweepClasses];
+  std::vector<int> which[kSweepClasses];
   std::vector<int32_t> direct_idx;
   std::vector<double2> direct_val;
+  std::vector<NoAllocGroup> groups;
+  size_t o_dval = 0, direct_bytes = 0, need_bytes = 0;
+  for (PlanFor plan : {kPlanFP64, kPlanTemplated}) {
+  for (int c = 0; c < kSweepClasses; ++c) {
+    by_class[c].clear();
+    which[c].clear();
+  }
+  direct_idx.clear();
+  direct_val.clear();
+  groups.clear();
   for (int k = 0; k < count; ++k) {
     HostSweep hs;
     bool need = false;
     double2 v = make_double2(0.0, 0.0);
     st = plan_permanent(matrix, m, input_states + (size_t)k * len, output_states + (size_t)k * len, len, variant, hs,
-                        need, v);
+                        need, v, plan);
     if (st) return st;
     if (need) {
-      which[hs.nf].push_back(k);
-      by_nf[hs.nf].push_back(std::move(hs));
+      const int c = sweep_class(hs);
+      which[c].push_back(k);
+      by_class[c].push_back(std::move(hs));
     } else {  // a permanent theboss defines without a sweep (empty states)
       direct_idx.push_back(k);
       direct_val.push_back(v);
     }
   }
-  const size_t o_dval = align_up(sizeof(int32_t) * direct_idx.size(), 256);
-  const size_t direct_bytes = o_dval + sizeof(double2) * direct_val.size();
-  std::vector<NoAllocGroup> groups;
-  for (int nf = 1; nf <= kMaxFactors; ++nf) {
-    const std::vector<HostSweep>& sw = by_nf[nf];
+  o_dval = align_up(sizeof(int32_t) * direct_idx.size(), 256);
+  direct_bytes = o_dval + sizeof(double2) * direct_val.size();
+  for (int c = 0; c < kSweepClasses; ++c) {
+    const std::vector<HostSweep>& sw = by_class[c];
     const int n = (int)sw.size();
     if (n == 0) continue;
     NoAllocGroup G;
-    G.nf = nf;
-    std::vector<uint64_t> codes(n);
-    for (int p = 0; p < n; ++p) codes[p] = sw[p].total_codes;
-    partition_threads(codes, sweep_resident_threads(nf, SweepOp::kPerm, dev->sm_count), G.nthr);
+    G.cls = c;
+    const int nf = sw[0].nf;
+    split_threads(sw,
+                  sw[0].layout == kRowsQuad ? quad_resident_walkers(nf, 0, false, dev->sm_count)
+                                            : sweep_resident_threads(nf, SweepOp::kPerm, dev->sm_count),
+                  G.nthr);
     int64_t pool_n = 0;
     for (int p = 0; p < n; ++p) {
       pool_n += (int64_t)(sw[p].D.size() + sw[p].base.size());
@@ -1077,8 +1184,10 @@ extern "C" int boss_perm_batch_noalloc(const double* matrix, int32_t m, const in
     G.bytes = G.o_part + sizeof(double2) * (size_t)G.threads;
     groups.push_back(std::move(G));
   }
-  size_t need_bytes = direct_bytes;
+  need_bytes = direct_bytes;
   for (const NoAllocGroup& G : groups) need_bytes = std::max(need_bytes, G.bytes);
+  if (need_bytes <= kNoAllocScratchBytes) break;
+  }
   if (need_bytes > kNoAllocScratchBytes) {
     set_error("request needs " + std::to_string(need_bytes) + " bytes of scratch; the allocation-free entry "
               "point has " + std::to_string(kNoAllocScratchBytes) + " (split the batch)");
@@ -1098,8 +1207,8 @@ extern "C" int boss_perm_batch_noalloc(const double* matrix, int32_t m, const in
   // (3) One sweep launch per product size; each image reuses the scratch from its
   // start (stream order keeps it behind the previous image's kernels).
   for (const NoAllocGroup& G : groups) {
-    const int nf = G.nf;
-    const std::vector<HostSweep>& sw = by_nf[nf];
+    const std::vector<HostSweep>& sw = by_class[G.cls];
+    const int nf = sw[0].nf;
     const int n = (int)sw.size();
     if ((st = noalloc_staging_wait())) return st;
     SweepProblem* hp = (SweepProblem*)g_noalloc_staging;
@@ -1108,28 +1217,16 @@ extern "C" int boss_perm_batch_noalloc(const double* matrix, int32_t m, const in
     for (int p = 0; p < n; ++p) {
       const HostSweep& h = sw[p];
       SweepProblem& P = hp[p];
-      memset(&P, 0, sizeof(P));
-      P.nd = h.nd;
-      P.nb = h.nb;
-      P.nf = h.nf;
-      P.kind = h.kind;
-      P.parity0 = h.parity0;
-      P.fx = -h.fx_sum;
-      P.align = range_align((int64_t)h.total_codes, G.nthr[p], h.nb);
-      P.has_base = h.has_base;
-      P.out_idx = which[nf][p];  // the reduction writes straight into the caller's buffer
-      P.n_codes = (int64_t)h.total_codes;
+      describe_sweep(h, G.nthr[p], P);
+      P.out_idx = which[G.cls][p];  // the reduction writes straight into the caller's buffer
       P.thread_begin = thread_at;
-      P.n_threads = G.nthr[p];
       P.mat_off = pool_at;
-      pack_rows(h.D, hpool + pool_at);
+      std::copy(h.D.begin(), h.D.end(), hpool + pool_at);
       pool_at += (int64_t)h.D.size();
       P.base_off = pool_at;
       std::copy(h.base.begin(), h.base.end(), hpool + pool_at);
       pool_at += (int64_t)h.base.size();
       P.part_off = thread_at;
-      P.scale = h.scale;
-      for (int i = 0; i < h.nd; ++i) P.mult[i] = h.mult[i];
       thread_at += G.nthr[p];
     }
     if ((st = noalloc_stage(dev, G.o_part, s))) return st;
@@ -1140,6 +1237,7 @@ extern "C" int boss_perm_batch_noalloc(const double* matrix, int32_t m, const in
     L.total_threads = G.threads;
     L.partials = (double2*)(dev->scratch + G.o_part);
     L.grid = (int)((G.threads + 127) / 128);
+    L.quad = sw[0].layout == kRowsQuad;
     if ((e = launch_sweep(nf, SweepOp::kPerm, L, s)) != cudaSuccess) return fail_cuda(e, "sweep launch");
     if ((e = launch_perm_reduce(L.probs, n, L.partials, out, s)) != cudaSuccess) return fail_cuda(e, "reduce launch");
   }

@@ -359,8 +359,8 @@ static int group_large(Context* cx, const double* matrix, int m, int n, int l, c
   const int K = (int)LI.occ.size();
   const int O = (int)outs.size();
   std::vector<double> terms((size_t)K * O, 0.0);
-  std::vector<HostSweep> by_nf[kMaxFactors + 1];
-  std::vector<size_t> which[kMaxFactors + 1];
+  std::vector<HostSweep> by_class[kSweepClasses];
+  std::vector<size_t> which[kSweepClasses];
   for (int k = 0; k < K; ++k)
     for (int o = 0; o < O; ++o) {
       HostSweep hs;
@@ -370,18 +370,19 @@ static int group_large(Context* cx, const double* matrix, int m, int n, int l, c
       if (st) return st;
       const size_t t = (size_t)k * O + o;
       if (need) {
-        which[hs.nf].push_back(t);
-        by_nf[hs.nf].push_back(std::move(hs));
+        const int c = sweep_class(hs);
+        which[c].push_back(t);
+        by_class[c].push_back(std::move(hs));
       } else {
         terms[t] = v.x * v.x + v.y * v.y;
       }
     }
-  for (int nf = 1; nf <= kMaxFactors; ++nf) {
-    if (by_nf[nf].empty()) continue;
-    std::vector<double2> res(by_nf[nf].size());
-    const int st = run_sweeps(cx, by_nf[nf], false, 1, res.data());
+  for (int c = 0; c < kSweepClasses; ++c) {
+    if (by_class[c].empty()) continue;
+    std::vector<double2> res(by_class[c].size());
+    const int st = run_sweeps(cx, by_class[c], false, 1, res.data());
     if (st) return st;
-    for (size_t a = 0; a < res.size(); ++a) terms[which[nf][a]] = fma(res[a].x, res[a].x, res[a].y * res[a].y);
+    for (size_t a = 0; a < res.size(); ++a) terms[which[c][a]] = fma(res[a].x, res[a].x, res[a].y * res[a].y);
   }
   double div[kDistMaxDiv];
   for (int k = 0; k < K; ++k) {

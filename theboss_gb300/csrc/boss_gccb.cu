@@ -41,6 +41,7 @@
 
 #include "../../include/boss.h"
 #include "boss_internal.h"
+#include "boss_quad.cuh"
 
 namespace boss {
 
@@ -677,6 +678,7 @@ struct FinalizeArgs {
                                 // strides of partials (part_off) and rows (pool_off)
   int next_group;               // uniform next level: threads per summed group of minors
   int cur_ff;                   // this level's sweep ran on float pairs: its partials are float4
+  int next_quad;                // the next level runs four codes per step (boss_quad.cuh)
   int next_ff;                  // the next level's sweep runs on float pairs (float-pair rows, biases)
   int* err;                     // err[0]: a pmf could not be normalised; err[1]: draws decided by the
                                 // exact sequential rule because a cdf step lay within the error window
@@ -830,7 +832,7 @@ __global__ void __launch_bounds__(128) gccb_partials_reduce_kernel(const SweepPr
   __shared__ double sx[128], sy[128];
   const int j = blockIdx.x, d = blockIdx.y;
   const SweepProblem& P = probs[j];
-  const int nd = P.nd + P.fixed_digit;
+  const int nd = P.nd + P.low + P.fixed_digit;
   if (d >= nd) return;
   const int64_t parts = P.n_threads / P.group;
   double x = 0.0, y = 0.0;
@@ -912,7 +914,7 @@ __global__ void __launch_bounds__(kFinWarps * 32, 8) gccb_finalize_kernel(Finali
     nd = 1;
   } else {
     const SweepProblem& P = a.probs_cur[j];
-    nd = P.nd + P.fixed_digit;  // the held (halved) digit's minor is the last row
+    nd = P.nd + P.low + P.fixed_digit;  // the held (halved) digit's minor is the last row
     const int64_t parts = P.n_threads / P.group;
     if (a.cur_ff) {
       // float-pair partials: summed as float pairs in a fixed order, scaled by the
@@ -1496,68 +1498,133 @@ __global__ void __launch_bounds__(kFinWarps * 32, 8) gccb_finalize_kernel(Finali
     ls.pool_off = (int64_t)j * a.next_uni.pool_off;
     ls.align = a.next_uni.align;
   }
-  // rows: -2 U[out][in] for the sweep's digits; base sums: sum_i S_i U[out][i]
-  // over every input mode (all signs +1 at r = 0), exact in fixed point
+  // The rows and base sums (sum_i S_i U[out][i] over every input mode: all signs +1
+  // at r = 0), exact in fixed point: the layout of boss_quad.cuh, or u = U packed
+  // for the templated FP64 kernels, or D = -2 U for the float pairs.
   longlong2* D = a.pool_next + ls.pool_off;
-  #pragma unroll 8  // independent gathers in flight
-  for (int e = lane; e < nds * nf; e += 32) {
-    const int d = e / nf, f = e - d * nf;
-    const longlong2 u = Ufxs[(size_t)fm_s[w][f] * m + dm_s[w][d]];
-    D[e] = a.next_ff ? make_longlong2(-2 * u.x, -2 * u.y) : make_longlong2(pack_row(-2 * u.x), pack_row(-2 * u.y));
-  }
-  longlong2* B = D + (size_t)nds * nf;
-  // Float-pair sweeps: factor f is scaled by 2^-(p_f + 1), 2^p_f <= its bound
-  // max(sum_d mult_d |Re U|, sum_d mult_d |Im U|) < 2^(p_f + 1) (fixed-point units),
-  // so |s_f| < 1 in that scale; fx_to_ff takes the bias 189 - p_f.
-  float4* DF = reinterpret_cast<float4*>(B + nf);
-  int* fbias = reinterpret_cast<int*>(DF + (size_t)(nb - held) * nf);
-  int esum = 0;   // sum_f (p_f + 1)
+  int esum = 0;   // float pairs: sum_f (p_f + 1)
   int fxsum = 0;  // sum_f fx_f
-  for (int f = lane; f < nf; f += 32) {
-    long long bx = 0, by = 0;
-    unsigned long long ax = 0, ay = 0;
-    #pragma unroll 8  // independent gathers in flight
-    for (int d = 0; d < nd; ++d) {
-      const longlong2 u = Ufxs[(size_t)fm_s[w][f] * m + dm_s[w][d]];
-      bx += (long long)mult_s[w][d] * u.x;
-      by += (long long)mult_s[w][d] * u.y;
-      ax += (unsigned long long)mult_s[w][d] * (unsigned long long)(u.x < 0 ? -u.x : u.x);
-      ay += (unsigned long long)mult_s[w][d] * (unsigned long long)(u.y < 0 ? -u.y : u.y);
+  const int low = a.next_quad ? 2 : 0;
+  int64_t base_off;  // from the start of the sweep's rows
+  auto entry = [&](int f, int d) -> Cx64 {
+    const longlong2 u = Ufxs[(size_t)fm_s[w][f] * m + dm_s[w][d]];
+    return cx(u.x, u.y);
+  };
+  if (a.next_quad) {
+    const int slots = quad_slots(nf), W = 4 * slots, ndo = nds - 2;
+    base_off = (int64_t)ndo * W;
+    longlong2* B = D + base_off;
+    longlong2* consts = B + W;
+    // an odd last factor's partner is the constant 1: its entries are zero
+    auto second = [&](int g, int d) -> Cx64 { return 2 * g + 1 < nf ? entry(2 * g + 1, d) : cx(0, 0); };
+    for (int e = lane; e < ndo * slots; e += 32) {
+      const int d = e / slots, g = e - d * slots;
+      const Cx64 uf = entry(2 * g, d + 2), ug = second(g, d + 2);
+      Cx64 ep, em;
+      quad_row(uf, ug, entry(2 * g, 0), entry(2 * g, 1), second(g, 0), second(g, 1), ep, em);
+      longlong2* r = D + (size_t)d * W + 4 * g;
+      r[0] = make_longlong2(pack_row(uf.re), pack_row(uf.im));
+      r[1] = make_longlong2(pack_row(ug.re), pack_row(ug.im));
+      r[2] = make_longlong2(pack_row(ep.re), pack_row(ep.im));
+      r[3] = make_longlong2(pack_row(em.re), pack_row(em.im));
     }
-    B[f] = make_longlong2(bx, by);
-    fxsum += rowfx[fm_s[w][f]];
+    __syncwarp();  // the rows just written by other lanes
+    for (int f = lane; f < nf; f += 32) {  // the factors' outer sums
+      Cx64 o = cx(0, 0);
+#pragma unroll 4
+      for (int d = 2; d < nd; ++d) {
+        const Cx64 u = entry(f, d);
+        const long long mu = mult_s[w][d];
+        o = cx(o.re + mu * u.re, o.im + mu * u.im);
+      }
+      B[4 * (f >> 1) + (f & 1)] = make_longlong2(o.re, o.im);
+      fxsum += rowfx[fm_s[w][f]];
+    }
+    for (int g = lane; g < slots; g += 32) {  // the pairs' E+-: the rows' coefficients and the held digit's
+      const Cx64 f0 = entry(2 * g, 0), f1 = entry(2 * g, 1), g0 = second(g, 0), g1 = second(g, 1);
+      Cx64 ep = cx(0, 0), em = cx(0, 0);
+      if (2 * g + 1 >= nf) {
+        B[4 * g + 1] = make_longlong2(kQuadOne, 0);
+        quad_row(cx(0, 0), cx(kQuadOne, 0), f0, f1, cx(0, 0), cx(0, 0), ep, em);
+        fxsum += 62;
+      } else {
+        if (held) quad_row(entry(2 * g, nds), second(g, nds), f0, f1, g0, g1, ep, em);
+#pragma unroll 4
+        for (int d = 0; d < ndo; ++d) {
+          const longlong2 p = D[(size_t)d * W + 4 * g + 2], q = D[(size_t)d * W + 4 * g + 3];
+          const long long mu = mult_s[w][d + 2];
+          ep = cx(ep.re + mu * unpack_row(p.x), ep.im + mu * unpack_row(p.y));
+          em = cx(em.re + mu * unpack_row(q.x), em.im + mu * unpack_row(q.y));
+        }
+      }
+      B[4 * g + 2] = make_longlong2(ep.re, ep.im);
+      B[4 * g + 3] = make_longlong2(em.re, em.im);
+      Cx64 cp, cm;
+      quad_const(f0, f1, g0, g1, cp, cm);
+      consts[2 * g] = make_longlong2(cp.re, cp.im);
+      consts[2 * g + 1] = make_longlong2(cm.re, cm.im);
+    }
+  } else {
+    base_off = (int64_t)nds * nf;
+#pragma unroll 8  // independent gathers in flight
+    for (int e = lane; e < nds * nf; e += 32) {
+      const int d = e / nf, f = e - d * nf;
+      const Cx64 u = entry(f, d);
+      D[e] = a.next_ff ? make_longlong2(-2 * u.re, -2 * u.im) : make_longlong2(pack_row(u.re), pack_row(u.im));
+    }
+    longlong2* B = D + base_off;
+    // Float-pair sweeps: factor f is scaled by 2^-(p_f + 1), 2^p_f <= its bound
+    // max(sum_d mult_d |Re U|, sum_d mult_d |Im U|) < 2^(p_f + 1) (fixed-point units),
+    // so |s_f| < 1 in that scale; fx_to_ff takes the bias 189 - p_f.
+    float4* DF = reinterpret_cast<float4*>(B + nf);
+    int* fbias = reinterpret_cast<int*>(DF + (size_t)(nb - held) * nf);
+    for (int f = lane; f < nf; f += 32) {
+      long long bx = 0, by = 0;
+      unsigned long long ax = 0, ay = 0;
+#pragma unroll 8  // independent gathers in flight
+      for (int d = 0; d < nd; ++d) {
+        const Cx64 u = entry(f, d);
+        bx += (long long)mult_s[w][d] * u.re;
+        by += (long long)mult_s[w][d] * u.im;
+        ax += (unsigned long long)mult_s[w][d] * (unsigned long long)(u.re < 0 ? -u.re : u.re);
+        ay += (unsigned long long)mult_s[w][d] * (unsigned long long)(u.im < 0 ? -u.im : u.im);
+      }
+      B[f] = make_longlong2(bx, by);
+      fxsum += rowfx[fm_s[w][f]];
+      if (a.next_ff) {
+        const unsigned long long bnd = ax > ay ? ax : ay;
+        const int p = bnd ? 63 - __clzll((long long)bnd) : 0;
+        fbias[f] = 189 - p;
+        esum += p + 1;
+      }
+    }
     if (a.next_ff) {
-      const unsigned long long bnd = ax > ay ? ax : ay;
-      const int p = bnd ? 63 - __clzll((long long)bnd) : 0;
-      fbias[f] = 189 - p;
-      esum += p + 1;
+#pragma unroll
+      for (int off = 16; off > 0; off >>= 1) esum += __shfl_xor_sync(0xffffffffu, esum, off);
+      __syncwarp();  // fbias written by the other lanes
+#pragma unroll 8  // independent gathers in flight
+      for (int e = lane; e < (nb - held) * nf; e += 32) {
+        const int d = e / nf, f = e - d * nf;
+        const Cx64 u = entry(f, d);
+        float4 v;
+        fx_to_ff(-2 * u.re, fbias[f], v.x, v.y);
+        fx_to_ff(-2 * u.im, fbias[f], v.z, v.w);
+        DF[e] = v;
+      }
     }
   }
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) fxsum += __shfl_xor_sync(0xffffffffu, fxsum, off);
-  if (a.next_ff) {
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) esum += __shfl_xor_sync(0xffffffffu, esum, off);
-    __syncwarp();  // fbias written by the other lanes
-    #pragma unroll 8  // independent gathers in flight
-    for (int e = lane; e < (nb - held) * nf; e += 32) {
-      const int d = e / nf, f = e - d * nf;
-      const longlong2 u = Ufxs[(size_t)fm_s[w][f] * m + dm_s[w][d]];
-      float4 v;
-      fx_to_ff(-2 * u.x, fbias[f], v.x, v.y);
-      fx_to_ff(-2 * u.y, fbias[f], v.z, v.w);
-      DF[e] = v;
-    }
-  }
   SweepProblem& P = a.probs_next[j];
-  P.mult[lane] = (lane < nd) ? mult_s[w][lane] : 0;
+  P.mult[lane] = (lane + low < nd) ? mult_s[w][lane + low] : 0;
   P.mult[lane + 32] = 0;
   a.dmode_next[(size_t)j * 32 + lane] = (lane < nd) ? dm_s[w][lane] : 0;
   if (lane == 0) {
     // S_i minor_i = 2^-(k-1) (halved) or 2^-k (not) times the Glynn sum, k = nf + 1
     // input particles; the kernel accumulates half of it.
-    P.nd = nds;
-    P.nb = nb - held;
+    P.nd = nds - low;
+    P.nb = nb - held - low;
+    P.low = low;
     P.nf = nf;
     P.kind = kGlynn;
     P.parity0 = 0;
@@ -1569,7 +1636,7 @@ __global__ void __launch_bounds__(kFinWarps * 32, 8) gccb_finalize_kernel(Finali
     P.thread_begin = ls.thread_begin;
     P.n_threads = ls.n_threads;
     P.mat_off = ls.pool_off;
-    P.base_off = ls.pool_off + (int64_t)nds * nf;
+    P.base_off = ls.pool_off + base_off;
     P.part_off = ls.part_off;
     // float pairs: the factors' scales 2^(p_f + 1 - fx_f) multiply the product
     P.ff_off = a.next_ff ? ls.pool_off + (int64_t)(nds + 1) * nf : 0;
@@ -1654,7 +1721,7 @@ __global__ void transpose_matrices_kernel(const double2* __restrict__ U, void* _
 
 // One warp per row o of a matrix (n_mats x m rows): the row's fixed-point scale,
 // the largest 2^rowfx for which its possible sums, sum_i w_i max(|Re U[o][i]|,
-// |Im U[o][i]|) over the input's particles, stay below 2^61, and the row in it.
+// |Im U[o][i]|) over the input's particles, stay below 2^bits, and the row in it.
 // weight: each mode's particle count at most (one matrix for all samples); else
 // the sample's own particles (pmode row of its draws, `order` as everywhere).
 __global__ void __launch_bounds__(128) fixed_rows_kernel(const double2* __restrict__ U, longlong2* __restrict__ out,
@@ -1662,7 +1729,7 @@ __global__ void __launch_bounds__(128) fixed_rows_kernel(const double2* __restri
                                                          const uint8_t* __restrict__ weight,
                                                          const int32_t* __restrict__ order,
                                                          const uint8_t* __restrict__ pmode,
-                                                         const uint8_t* __restrict__ npart, int n) {
+                                                         const uint8_t* __restrict__ npart, int n, int bits) {
   const int64_t r = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (r >= rows) return;
@@ -1689,7 +1756,7 @@ __global__ void __launch_bounds__(128) fixed_rows_kernel(const double2* __restri
   }
   bound = warp_sum(bound) * (1.0 + 0x1p-40);  // the sums' own rounding
   int fx = 56;
-  if (bound > 0.0 && bound < 1.7e308) fx = max(-1000, min(60 - ilogb(bound), 1000));  // bound < 2^(ilogb + 1)
+  if (bound > 0.0 && bound < 1.7e308) fx = max(-1000, min(bits - 1 - ilogb(bound), 1000));  // bound < 2^(ilogb + 1)
   if (lane == 0) rowfx[r] = fx;
   for (int i = lane; i < m; i += 32) {
     const double2 v = row[i];
@@ -1848,6 +1915,7 @@ static int gccb_prepare(Context* cx, const double* matrix, int n_mats, int m, Dr
   // count by (occ_a + 2) / (occ_a + 1).
   std::vector<std::vector<uint64_t>> lvl_codes(Lmax + 2);
   std::vector<std::vector<int>> lvl_nd(Lmax + 2);
+  std::vector<int> lvl_singles(Lmax + 2, 0);  // binned: the fewest single-occupied modes of a sample's input there
   std::vector<char> ffl(Lmax + 2, 0);  // level k's sweep runs on float pairs
   // FP64 (the default): FP64 sweeps and an FP64 pmf; float pairs where the
   // float-pair sweep exists for the level's factor count, and a float-pair pmf
@@ -1869,6 +1937,7 @@ static int gccb_prepare(Context* cx, const double* matrix, int n_mats, int m, Dr
     for (int k = 2; k <= Lmax; ++k) {
       lvl_codes[k].resize(A[k]);
       lvl_nd[k].resize(A[k]);
+      lvl_singles[k] = 256;
     }
     std::vector<uint8_t> occ(m, 0);
     for (int jj = 0; jj < A[1]; ++jj) {
@@ -1885,6 +1954,7 @@ static int gccb_prepare(Context* cx, const double* matrix, int n_mats, int m, Dr
           const uint64_t cg = singles > 0 ? c / 2 : c;  // Glynn form: one single digit held
           lvl_codes[k][jj] = cg;
           lvl_nd[k][jj] = nd;
+          lvl_singles[k] = std::min(lvl_singles[k], singles);
           // flops per code of the all-minors sweep: (k-1) complex adds, (k-2) complex
           // products, one sign, k/2 real-weighted adds = 9k - 12; theboss's Ryser
           // form sweeps c codes, the Glynn form cg
@@ -1896,6 +1966,10 @@ static int gccb_prepare(Context* cx, const double* matrix, int n_mats, int m, Dr
       for (int k = 0; k < L[s]; ++k) occ[D.modes[(size_t)s * n + k]] = 0;
     }
   }
+  // Levels that run four codes per step: FP64 sweeps of two factors at least whose
+  // every sample has two binary digits besides the held one.
+  std::vector<char> quad(Lmax + 2, 0);
+  for (int k = 3; k <= Lmax; ++k) quad[k] = !ffl[k] && k - 1 >= kQuadMinMinorFactors && (!D.binned || lvl_singles[k] >= 3);
   std::vector<char> uniform(Lmax + 2, 0);
   std::vector<LevelSample> uni_lvl(Lmax + 2);
   std::vector<int> grp(Lmax + 2, 1);
@@ -1906,10 +1980,16 @@ static int gccb_prepare(Context* cx, const double* matrix, int n_mats, int m, Dr
     const std::vector<uint64_t>& codes = lvl_codes[k];
     const std::vector<int>& ndv = lvl_nd[k];
     // k input particles: at most k distinct modes, so at most k rows of minors per thread
-    const int64_t resident = sweep_resident_minors(k - 1, std::min(k, kMaxMinorDigits), cx->sm_count, ffl[k]);
+    const int rows_k = std::min(k, kMaxMinorDigits);
+    const int64_t resident = quad[k] ? quad_resident_walkers(k - 1, rows_k, true, cx->sm_count)
+                                     : sweep_resident_minors(k - 1, rows_k, cx->sm_count, ffl[k]);
+    const int low = quad[k] ? 2 : 0;  // codes in steps of four
+    const int block = quad[k] ? kQuadWalkers : 128;  // walkers or threads per block
     // pool per sample: rows of D and the base sums; float pairs add the float-pair
     // rows of the binary digits and the factors' biases
-    auto pool_units = [&](int nd_) { return (int64_t)(ffl[k] ? 2 * nd_ + 2 : nd_ + 1) * (k - 1); };
+    auto pool_units = [&](int nd_) -> int64_t {
+      return quad[k] ? quad_pool(nd_ - 3, k - 1) : (int64_t)(ffl[k] ? 2 * nd_ + 2 : nd_ + 1) * (k - 1);
+    };
     bool same = true;
     uint64_t code0 = 1ull << (k - 1);
     int nd0 = k;
@@ -1919,20 +1999,21 @@ static int gccb_prepare(Context* cx, const double* matrix, int n_mats, int m, Dr
       for (int jj = 1; jj < Ak && same; ++jj) same = (codes[jj] == code0 && ndv[jj] == nd0);
     }
     if (same) {  // one small descriptor instead of a per-sample table
+      code0 >>= low;
       const double total = (double)code0 * Ak;
-      const double want = std::max<double>(Ak, std::min<double>((double)resident, total / kMinCodesPerThread));
+      const double want = std::max<double>(Ak, std::min<double>((double)resident, total / (kMinCodesPerThread >> low)));
       int64_t tps = std::max<int64_t>(1, std::min<int64_t>((int64_t)code0, (int64_t)(want / Ak)));
       const LevelTune lt = level_tune(f64, k, Ak);
       if (lt.shift > 0) tps = std::min<int64_t>((int64_t)code0, tps << lt.shift);
       if (lt.shift < 0) tps = std::max<int64_t>(1, tps >> -lt.shift);
       // Each aligned group of G threads of a sample sums its minors inside the sweep:
-      // the largest G (up to a block of 128, when the launch's threads then fill
+      // the largest G (up to a whole block, when the launch's threads then fill
       // whole blocks) that costs at most 2% of the sample's threads.
-      int G = 128;
+      int G = block;
       if (lt.gmax > 0) G = std::min(G, lt.gmax);
       auto ok = [&](int g) {
         if (!(tps >= g && (double)(tps / g * g) >= 0.98 * (double)tps)) return false;
-        return g <= 32 || ((tps / g * g) * (int64_t)Ak) % 128 == 0;
+        return g <= (quad[k] ? 8 : 32) || ((tps / g * g) * (int64_t)Ak) % block == 0;
       };
       while (G > 1 && !ok(G)) G >>= 1;
       tps = tps / G * G;
@@ -1957,14 +2038,16 @@ static int gccb_prepare(Context* cx, const double* matrix, int n_mats, int m, Dr
     {
       const LevelTune lt = level_tune(f64, k, Ak);
       const int64_t res = lt.shift >= 0 ? resident << lt.shift : std::max<int64_t>(1, resident >> -lt.shift);
-      partition_threads(codes, res, nthr);
+      std::vector<uint64_t> steps(codes);
+      for (uint64_t& c : steps) c >>= low;
+      partition_threads(steps, res, nthr, kMinCodesPerThread >> low);
     }
     auto& t = tab[k];
     t.resize(Ak);
     int64_t threads = 0, parts = 0, pool = 0;
     for (int jj = 0; jj < Ak; ++jj) {
       LevelSample ls;
-      ls.n_codes = (int64_t)codes[jj];
+      ls.n_codes = (int64_t)(codes[jj] >> low);
       ls.thread_begin = threads;
       ls.n_threads = nthr[jj];
       ls.part_off = parts;
@@ -2058,7 +2141,8 @@ static int gccb_prepare(Context* cx, const double* matrix, int n_mats, int m, Dr
     const int64_t rows = (int64_t)m * n_mats;
     fixed_rows_kernel<<<(unsigned)((rows + 3) / 4), 128, 0, s>>>(
         (const double2*)(d + o_U), dUfx, drowfx, m, rows, n_mats > 1 ? nullptr : (const uint8_t*)(d + o_cap),
-        (const int32_t*)(d + o_ord), (const uint8_t*)(d + o_pm), (const uint8_t*)(d + o_np), n);
+        (const int32_t*)(d + o_ord), (const uint8_t*)(d + o_pm), (const uint8_t*)(d + o_np), n,
+        f64 ? 62 : 61);  // the float pairs' D = -2 U needs the bit
     if ((e = cudaGetLastError()) != cudaSuccess) return fail_cuda(e, "fixed-point matrices");
     const int64_t cnt2 = (int64_t)mm * n_mats;
     transpose_matrices_kernel<<<(unsigned)((cnt2 + 255) / 256), 256, 0, s>>>((const double2*)(d + o_U), dUt, dUabs,
@@ -2090,6 +2174,7 @@ static int gccb_prepare(Context* cx, const double* matrix, int n_mats, int m, Dr
       SL.partials = partials;
       SL.grid = (int)((lvl_threads[k] + 127) / 128);
       SL.rows = std::min(k, kMaxMinorDigits);
+      SL.quad = quad[k] != 0;
       SL.uniform_threads = uniform[k] ? uni_lvl[k].n_threads : 0;
       if (timing == 1) le = cudaEventRecordWithFlags(R.ev[2 * (k - 2)], s, cudaEventRecordExternal);
       if (timing == 2) le = cudaEventRecordWithFlags(R.ev[2 * (k - 1)], s, cudaEventRecordExternal);
@@ -2137,6 +2222,7 @@ static int gccb_prepare(Context* cx, const double* matrix, int n_mats, int m, Dr
     fa.next_tab = (k < Lmax && !uniform[k + 1]) ? (const LevelSample*)(d + o_tab[k + 1]) : nullptr;
     fa.next_uni = (k < Lmax) ? uni_lvl[k + 1] : LevelSample{};
     fa.next_group = (k < Lmax) ? grp[k + 1] : 1;
+    fa.next_quad = (k < Lmax) ? quad[k + 1] : 0;
     fa.next_ff = (k < Lmax) ? ffl[k + 1] : 0;
     fa.cur_ff = (k >= 2) ? ffl[k] : 0;
     fa.err = R.derr;

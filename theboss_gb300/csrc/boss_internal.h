@@ -23,6 +23,7 @@ struct SweepLaunch {
   double2* partials2 = nullptr;  // gradients: per-warp permanent partials
   int grid = 1;
   int rows = 32;  // all-minors: shared-memory rows of minors per thread (nd + held digit, at most 32)
+  bool quad = false;  // permanents, all-minors in FP64: the four-codes-per-step kernels (boss_quad.cuh)
   int64_t uniform_threads = 0;  // all-minors: > 0 when every sweep has this many threads and sweep p
                                 // starts at thread p * uniform_threads (no search for the sweep)
 };
@@ -34,6 +35,11 @@ int64_t sweep_resident_threads(int nf, SweepOp op, int sm_count);
 // Resident threads of the all-minors kernel (FP64, or the float-pair one) with
 // `rows` rows of minors per thread.
 int64_t sweep_resident_minors(int nf, int rows, int sm_count, bool ff = false);
+// The same for the four-codes-per-step kernels (boss_quad.cu; rows matter to the
+// all-minors kernel only).
+cudaError_t prepare_quad_kernels();
+int64_t quad_resident_walkers(int nf, int rows, bool minors, int sm_count);
+cudaError_t launch_quad_sweep(int nf, bool minors, const SweepLaunch& L, cudaStream_t st);
 // Whether the float-pair all-minors / single-permanent kernel exists for nf factors.
 bool minors_ff_available(int nf);
 bool perm_ff_available(int nf);
@@ -47,8 +53,11 @@ cudaError_t launch_minors_reduce(const SweepProblem* probs, int n_probs, const d
 
 // Splits `n_codes` codes over at most `resident` threads, proportionally, at
 // least one thread per sweep and at least kMinCodesPerThread codes per thread.
+constexpr int kFFMaxFactors = 24;      // float-pair all-minors: above this the sums exhaust the registers
+constexpr int kFFPermMaxFactors = 32;  // float-pair permanents
 constexpr int64_t kMinCodesPerThread = 8;
-void partition_threads(const std::vector<uint64_t>& n_codes, int64_t resident, std::vector<int64_t>& n_threads);
+void partition_threads(const std::vector<uint64_t>& n_codes, int64_t resident, std::vector<int64_t>& n_threads,
+                       int64_t min_codes = kMinCodesPerThread);
 // log2 of the codes every range of a sweep starts at a multiple of: the largest
 // (at most 6, at most the nb binary digits) that makes the longest range at most
 // 1/32 longer than an even split.  Lanes of a warp then flip the same low digit
@@ -58,7 +67,22 @@ int range_align(int64_t n_codes, int64_t n_threads, int nb);
 // ---------------------------------------------------------------------------
 // Host-side sweep description.
 // ---------------------------------------------------------------------------
+// Factors from which a sweep with two binary digits takes four codes per step
+// (boss_quad.cuh) instead of the templated kernel.  Permanents: always (64
+// permanents: n = 12 18 against 20 us, n = 16 86 against 109, n = 18 354 against 400,
+// n = 24 24.0 against 33.5 ms).  All-minors: from 14 (the sampler's levels of 10^4
+// samples, n = 20: 13 factors 186 against 197 us but its rows cost the finalize 8 us
+// more to plan; 12 factors 197 against 200, 11 factors 199 against 172, 14 factors
+// 125 against 135).
+constexpr int kQuadMinFactors = 2;
+constexpr int kQuadMinMinorFactors = 14;
+enum RowLayout : int {
+  kRowsPlain = 0,   // D (float pairs, gradients)
+  kRowsPacked = 1,  // u = -D / 2 packed: the templated FP64 kernels
+  kRowsQuad = 2     // boss_quad.cuh: two binary digits and two factors at least
+};
 struct HostSweep {
+  int layout = kRowsPlain;
   int kind = kRyser;
   int parity0 = 0;
   int nd = 0, nb = 0, nf = 0;
@@ -66,8 +90,8 @@ struct HostSweep {
   int fx = 56;                 // fraction bits shared by all factors (gradients)
   int fx_sum = 0;              // sum of the factors' own fraction bits (permanents, all-minors)
   uint8_t mult[kMaxDigits] = {};
-  std::vector<longlong2> D;     // nd x nf
-  std::vector<longlong2> base;  // nf (has_base)
+  std::vector<longlong2> D;     // nd x nf; kRowsQuad: (nd - 2) x quad_width(nf)
+  std::vector<longlong2> base;  // nf (has_base); kRowsQuad: base and constants
   double scale = 1.0;
   uint64_t total_codes = 1;
   int digit_mode[kMaxDigits] = {};  // digit -> mode (all-minors results)
@@ -123,7 +147,7 @@ Context* context(int* status);
 int ensure(DeviceBuffer& b, size_t bytes);
 int ensure_pinned(Context* cx, size_t bytes);
 
-// Uploads a list of sweeps (all with the same factor count), launches the sweep
+// Uploads a list of sweeps (all of one sweep_class), launches the sweep
 // and the reduction, copies the results back.  results: one complex per sweep
 // (perms) or nd_max complex per sweep (all-minors).
 int run_sweeps(Context* cx, const std::vector<HostSweep>& sweeps, bool minors, int nd_max, double2* results_host);
@@ -138,8 +162,15 @@ int small_perm_batch(Context* cx, const double* matrix, int m, int len, const in
 // One permanent request (theboss's variant semantics).  Returns kOk and either
 // fills `hs` (needs_sweep = true) or sets `value` for the edge cases theboss
 // special-cases.
-// shared_fx: one scale for all factors (the gradient sweeps) instead of one each.
+// What the sweep is planned for: any kernel, float pairs where they are chosen; the
+// templated FP64 kernels only; FP64 always (the allocation-free entry point); the
+// gradient kernel (one fixed-point scale for all factors).
+enum PlanFor : int { kPlanAny = 0, kPlanTemplated = 1, kPlanFP64 = 2, kPlanGrad = 3 };
 int plan_permanent(const double* U, int m, const int32_t* S, const int32_t* T, int len, int variant, HostSweep& hs,
-                   bool& needs_sweep, double2& value, bool shared_fx = false);
+                   bool& needs_sweep, double2& value, PlanFor plan = kPlanAny);
+
+// Sweeps of one launch share the factor count and the kernel: class 2 nf + quad.
+constexpr int kSweepClasses = 2 * (kMaxFactors + 1);
+inline int sweep_class(const HostSweep& h) { return 2 * h.nf + (h.layout == kRowsQuad ? 1 : 0); }
 
 }  // namespace boss

@@ -34,7 +34,9 @@ cudaError_t prepare_sweep_kernels() {
     return e;
   if ((e = sweep_nf_c_prepare(g_perm_occ + 17, &g_minors_occ[17][0], &g_minors_ff_occ[17][0], g_perm_ff_occ + 17)))
     return e;
-  return sweep_nf_d_prepare(g_perm_occ + 25, &g_minors_occ[25][0], &g_minors_ff_occ[25][0], g_perm_ff_occ + 25);
+  if ((e = sweep_nf_d_prepare(g_perm_occ + 25, &g_minors_occ[25][0], &g_minors_ff_occ[25][0], g_perm_ff_occ + 25)))
+    return e;
+  return prepare_quad_kernels();
 }
 
 bool perm_ff_available(int nf) { return nf >= 1 && nf <= kMaxFactors && g_perm_ff_occ[nf] > 0; }
@@ -70,6 +72,7 @@ int64_t sweep_resident_threads(int nf, SweepOp op, int sm_count) {
 
 cudaError_t launch_sweep(int nf, SweepOp op, const SweepLaunch& L, cudaStream_t st) {
   if (L.total_threads <= 0) return cudaSuccess;
+  if (L.quad) return launch_quad_sweep(nf, op == SweepOp::kMinors, L, st);
   if (nf >= 1 && nf <= 8) return sweep_nf_a_launch(nf, op, L, st);
   if (nf <= 16) return sweep_nf_b_launch(nf, op, L, st);
   if (nf <= 24) return sweep_nf_c_launch(nf, op, L, st);
@@ -77,13 +80,14 @@ cudaError_t launch_sweep(int nf, SweepOp op, const SweepLaunch& L, cudaStream_t 
   return cudaErrorInvalidValue;
 }
 
-void partition_threads(const std::vector<uint64_t>& n_codes, int64_t resident, std::vector<int64_t>& n_threads) {
+void partition_threads(const std::vector<uint64_t>& n_codes, int64_t resident, std::vector<int64_t>& n_threads,
+                       int64_t min_codes) {
   const size_t n = n_codes.size();
   n_threads.assign(n, 1);
   long double total = 0;
   for (uint64_t c : n_codes) total += (long double)c;
   if (total <= 0) return;
-  long double want = std::min<long double>((long double)resident, total / (long double)kMinCodesPerThread);
+  long double want = std::min<long double>((long double)resident, total / (long double)min_codes);
   want = std::max<long double>(want, (long double)n);
   for (size_t p = 0; p < n; ++p) {
     long double t = want * (long double)n_codes[p] / total;
@@ -143,7 +147,7 @@ __global__ void minors_reduce_kernel(const SweepProblem* __restrict__ probs, con
                                      double2* __restrict__ out, int nd_max, int ff) {
   __shared__ double sr[256], si[256];
   const SweepProblem& P = probs[blockIdx.x];
-  const int nd = P.nd + P.fixed_digit;  // the held digit's row last
+  const int nd = P.nd + P.low + P.fixed_digit;  // the held digit's row last
   for (int j = 0; j < nd; ++j) {
     double ar = 0.0, ai = 0.0;
     for (int64_t q = threadIdx.x; q < P.n_threads; q += blockDim.x) {

@@ -1,0 +1,401 @@
+// boss_quad.cu -- four codes per step over pairs of factors (boss_quad.cuh): the
+// sweeps with two binary digits and enough factors (kQuadMinFactors,
+// kQuadMinMinorFactors).  The templated kernels of boss_sweep_kernels.cuh take the
+// others.
+//
+// Measured (64 permanents, input-side digits): n = 20 1.41 ms, n = 24 24.0 ms, n = 28
+// 486 ms, against 1.71, 33.5 and about 640 ms with the templated kernel; the
+// benchmark's output-side batches n = 28 104 ms against 154.  45 instructions per
+// factor and code (58 there); the FMA pipe 61 % busy, the ALU pipe 51 %, the rest
+// dispatch and fixed-latency stalls at 16 warps per SM, which more warps do not
+// lessen.
+#include <algorithm>
+
+#include "boss_internal.h"
+#include "boss_quad.cuh"
+
+namespace boss {
+
+// Blocks of 128 per SM the kernels are compiled for: the state is 16 registers per
+// four slots.  One block more or fewer at any size is no faster (64 permanents at
+// n = 20: 4 blocks 1.41 ms, 3 blocks 1.47; n = 28: 3 or 4 blocks 104 ms).
+constexpr int quad_blocks(int slots) { return slots <= 4 ? 5 : slots <= 12 ? 4 : 3; }
+
+// A lane's slots are 4 i + (lane & 3) of its walker, i = 0 .. ceil(S / 4) - 1, their
+// state in registers (lanes past the last slot repeat it, so that no lane
+// branches).  Shared memory, 16-byte entries: two buffers for the slots' four
+// values on their way to the chains' lanes, value v of thread t at
+// [v * kQuadXStride + t] (the odd stride puts a walker's four readers in different
+// banks).
+constexpr int kQuadXStride = kQuadBlock + 1;
+constexpr int kQuadX = 4 * kQuadXStride;
+template <int S>
+struct QuadState {
+  static constexpr int kRounds = (S + 3) / 4;
+  Cx64 v[kRounds][4];  // o_f o_g E+ E-
+  __device__ __forceinline__ static int slot(int i) {
+    const int s = 4 * i + (int)(threadIdx.x & 3);
+    return 4 * i + 4 <= S ? s : min(s, S - 1);
+  }
+};
+
+// The walk over the outer digits: the reflected mixed-radix Gray code changes one
+// digit by one per step, so the state moves by one row and is decoded only once.
+struct QuadWalk {
+  uint64_t g;      // the binary digits
+  uint32_t parity; // sign parity
+  double w;        // binomial weight of the multi-valued digits
+  uint8_t r[kMaxDigits];  // their values (entries nb .. nd - 1; local memory)
+};
+
+// The walk at outer code t, and this lane's state.
+template <int S>
+__device__ __forceinline__ void quad_decode(const SweepProblem& P, const longlong2* __restrict__ rows,
+                                            const longlong2* __restrict__ base, uint64_t t, QuadState<S>& st, QuadWalk& k) {
+  constexpr int W = 4 * S;
+  const int nb = P.nb;
+  k.g = (t ^ (t >> 1));
+  if (nb < 64) k.g &= (1ull << nb) - 1ull;
+  k.parity = (uint32_t)P.parity0 ^ ((uint32_t)__popcll((long long)k.g) & 1u);
+  k.w = 1.0;
+  uint64_t th = t >> nb;
+  for (int i = nb; i < P.nd; ++i) {
+    const uint32_t mu = P.mult[i];
+    const uint64_t b = (uint64_t)mu + 1ull, q = th / b;
+    const uint32_t dgt = (uint32_t)(th - q * b);
+    th = q;
+    const uint32_t r = (q & 1ull) ? (mu - dgt) : dgt;
+    k.r[i] = (uint8_t)r;
+    k.parity ^= r & 1u;
+    if (r) k.w *= binom_small((int)mu, (int)r);
+  }
+#pragma unroll
+  for (int i = 0; i < QuadState<S>::kRounds; ++i)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const longlong2 b = base[4 * QuadState<S>::slot(i) + c];
+      st.v[i][c] = cx(b.x, b.y);
+    }
+  auto add = [&](int d, int sg) {
+    const longlong2* row = rows + (int64_t)d * W;
+#pragma unroll
+    for (int i = 0; i < QuadState<S>::kRounds; ++i)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const longlong2 x = __ldg(row + 4 * QuadState<S>::slot(i) + c);
+        st.v[i][c] = cx(add_packed(st.v[i][c].re, x.x, sg), add_packed(st.v[i][c].im, x.y, sg));
+      }
+  };
+  for (uint64_t bits = k.g; bits; bits &= bits - 1ull) add(__ffsll((long long)bits) - 1, -2);
+  for (int d = nb; d < P.nd; ++d)
+    if (k.r[d]) add(d, -2 * (int)k.r[d]);
+}
+
+// The step to outer code t: the digit that moves, and by how much (+-1).
+__device__ __forceinline__ int quad_next(const SweepProblem& P, uint64_t t, QuadWalk& k, int& dr) {
+  const int nb = P.nb;
+  int i = __ffsll((long long)t) - 1;
+  k.parity ^= 1u;
+  if (i < nb) {
+    dr = ((k.g >> i) & 1ull) ? -1 : 1;
+    k.g ^= 1ull << i;
+    return i;
+  }
+  uint64_t th = t >> nb, q;
+  uint32_t mu, dgt;
+  for (i = nb;; ++i) {  // the lowest digit whose plain value is not back at zero
+    mu = P.mult[i];
+    q = th / (mu + 1ull);
+    dgt = (uint32_t)(th - q * (mu + 1ull));
+    if (dgt || i + 1 >= P.nd) break;
+    th = q;
+  }
+  const int r = (int)((q & 1ull) ? (mu - dgt) : dgt), before = k.r[i];
+  dr = r - before;
+  k.r[i] = (uint8_t)r;
+  // C(mu, r) from C(mu, before), exact while the weight is below 2^53
+  k.w = dr > 0 ? k.w * (double)(mu - (uint32_t)before) / (double)r : k.w * (double)before / (double)(mu - (uint32_t)r);
+  return i;
+}
+
+// Moves the state by sg times a row (sg = 0: as it is) and multiplies this lane's
+// code over S slots: the product is (re + i im) 2^e.  Every lane of the warp calls
+// it.  The next round's slots are prepared beside the chains of the one before.
+template <int S>
+__device__ __forceinline__ void quad_eval(QuadState<S>& st, longlong2* xbuf, const longlong2* __restrict__ row, int sg,
+                                          const longlong2* __restrict__ consts, int e0, long long& re, long long& im,
+                                          int& e) {
+  constexpr int kRounds = (S + 3) / 4;
+  const int kk = threadIdx.x & 3;
+  longlong2* mine = xbuf + threadIdx.x;
+  const longlong2* from = xbuf + kk * kQuadXStride + (threadIdx.x & ~3);
+  int ls = 0, ps = 0;  // leading bits: of this lane's slots, of its chain
+  auto prepare = [&](int i) {
+    const int s = QuadState<S>::slot(i);
+    const longlong2 cp = __ldg(consts + 2 * s), cm = __ldg(consts + 2 * s + 1);
+    Cx64(&v)[4] = st.v[i];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const longlong2 d = __ldg(row + 4 * s + c);
+      v[c] = cx(add_packed(v[c].re, d.x, sg), add_packed(v[c].im, d.y, sg));
+    }
+    Cx64 q[4];
+    const int l = quad_pair(v[0], v[1], v[2], v[3], cx(cp.x, cp.y), cx(cm.x, cm.y), q);
+    ls += (4 * i + 4 <= S || 4 * i + kk < S) ? l : 0;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) mine[(i & 1) * kQuadX + c * kQuadXStride] = make_longlong2(q[c].re, q[c].im);
+  };
+  prepare(0);
+  __syncwarp();
+#pragma unroll
+  for (int i = 0; i < kRounds; ++i) {
+    if (i + 1 < kRounds) prepare(i + 1);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      if (4 * i + j >= S) break;
+      const longlong2 q = from[(i & 1) * kQuadX + j];
+      ps += (i + j == 0) ? quad_chain_first(re, im, q.x, q.y) : quad_chain(re, im, q.x, q.y);
+    }
+    __syncwarp();
+  }
+  ls += __shfl_xor_sync(0xffffffffu, ls, 1);
+  ls += __shfl_xor_sync(0xffffffffu, ls, 2);
+  e = quad_exponent(e0, ls, S) + ps;
+}
+
+// This lane's walker and its range; lanes past the launch's last walker take the
+// last one's problem with an empty range, so that whole warps stay together.
+struct QuadRange {
+  int64_t q;       // the walker within its sweep
+  int64_t a, len;  // its outer codes
+  int64_t most;    // the longest range in the warp
+  bool live;
+};
+__device__ __forceinline__ QuadRange quad_range(const SweepProblem& P, int64_t walker, bool live) {
+  QuadRange r;
+  r.live = live;
+  r.q = walker - P.thread_begin;
+  thread_range_aligned(P, r.q, P.align, r.a, r.len);
+  if (!live) r.len = 0;
+  r.most = r.len;
+#pragma unroll
+  for (int o = 16; o >= 4; o >>= 1) {
+    const int64_t x = __shfl_xor_sync(0xffffffffu, r.most, o);
+    r.most = x > r.most ? x : r.most;
+  }
+  return r;
+}
+
+// One permanent per sweep problem; every walker writes one complex partial.
+template <int S>
+__global__ void __launch_bounds__(kQuadBlock, quad_blocks(S)) perm_quad_kernel(const SweepProblem* __restrict__ probs,
+                                                                        int n_probs,
+                                                                        const longlong2* __restrict__ pool,
+                                                                        int64_t total_walkers,
+                                                                        double2* __restrict__ partials) {
+  extern __shared__ longlong2 quad_smem[];
+  const int64_t at = (int64_t)blockIdx.x * kQuadWalkers + (threadIdx.x >> 2);
+  const bool live = at < total_walkers;
+  const int64_t walker = live ? at : total_walkers - 1;
+  const SweepProblem& P = probs[find_problem(probs, n_probs, walker)];
+  const QuadRange R = quad_range(P, walker, live);
+  constexpr int W = 4 * S;
+  const longlong2* rows = pool + P.mat_off;
+  const longlong2* base = pool + P.base_off;
+  QuadState<S> st;
+  QuadWalk k;
+  quad_decode<S>(P, rows, base, (uint64_t)(R.len > 0 ? R.a : 0), st, k);
+  // sign of this lane's code: + for (+,+) and (-,-), - for the mixed ones
+  const uint32_t mixed = (threadIdx.x >> 1) & 1u;
+  double ar = 0.0, ai = 0.0;
+  const longlong2* row = base;
+  int sg = 0;
+  for (int64_t it = 0; it < R.most; ++it) {
+    if (it > 0 && it < R.len) {
+      int dr;
+      row = rows + (int64_t)quad_next(P, (uint64_t)(R.a + it), k, dr) * W;
+      sg = -2 * dr;
+    }
+    if (it >= R.len) sg = 0;
+    long long re, im;
+    int e;
+    quad_eval<S>(st, quad_smem, row, sg, base + W, P.fx, re, im, e);
+    const double w = it < R.len ? xor_sign(k.w, (k.parity ^ mixed) << 31) : 0.0;
+    ar = fma(w, bf_to_double(re, e), ar);
+    ai = fma(w, bf_to_double(im, e), ai);
+  }
+#pragma unroll
+  for (int o = 1; o < 4; o <<= 1) {  // the walker's four codes, in a fixed order
+    ar += __shfl_xor_sync(0xffffffffu, ar, o);
+    ai += __shfl_xor_sync(0xffffffffu, ai, o);
+  }
+  if (live && (threadIdx.x & 3) == 0) partials[P.part_off + R.q] = make_double2(ar, ai);
+}
+
+// All-minors in Glynn form (see minors_walk): half of every minor, row order low
+// digits, outer digits, held digit.  A lane's code has fixed low digits, so the low
+// digits' minors are +- its total; an outer digit's weight w_j = mult_j - 2 r_j
+// changes by -+2 when the digit moves, so its row then takes +-R, R the lane's
+// running total of signed and weighted products, and w_j R / 2 when the total is
+// closed (every 2^16 steps and at the end).
+template <int S>
+__global__ void __launch_bounds__(kQuadBlock, quad_blocks(S)) minors_quad_kernel(const SweepProblem* __restrict__ probs,
+                                                                          int n_probs,
+                                                                          const longlong2* __restrict__ pool,
+                                                                          int64_t total_walkers,
+                                                                          double2* __restrict__ partials,
+                                                                          int64_t uniform_walkers) {
+  extern __shared__ longlong2 quad_smem[];
+  const int64_t at = (int64_t)blockIdx.x * kQuadWalkers + (threadIdx.x >> 2);
+  const bool live = at < total_walkers;
+  const int64_t walker = live ? at : total_walkers - 1;
+  const SweepProblem& P =
+      probs[uniform_walkers > 0 ? (int)(walker / uniform_walkers) : find_problem(probs, n_probs, walker)];
+  const QuadRange R = quad_range(P, walker, live);
+  constexpr int W = 4 * S;
+  const int ndo = P.nd, nb = P.nb;
+  const longlong2* rows = pool + P.mat_off;
+  const longlong2* base = pool + P.base_off;
+  QuadState<S> st;
+  double2 M[kMaxMinorDigits];  // outer digits' rows (local memory: row i is touched when digit i moves)
+  for (int j = 0; j < ndo; ++j) M[j] = make_double2(0.0, 0.0);
+  double hr = 0.0, hi = 0.0;   // half of the lane's total
+  QuadWalk k;
+  quad_decode<S>(P, rows, base, (uint64_t)(R.len > 0 ? R.a : 0), st, k);
+  const uint32_t mixed = (threadIdx.x >> 1) & 1u;
+  double Rr = 0.0, Ri = 0.0;  // since the last settle
+  auto settle = [&]() {
+    const double wr = 0.5 * Rr, wi = 0.5 * Ri;
+    for (int j = 0; j < ndo; ++j) {
+      const double f = j < nb ? (((k.g >> j) & 1ull) ? -1.0 : 1.0) : (double)P.mult[j] - 2.0 * (double)k.r[j];
+      M[j].x = fma(wr, f, M[j].x);
+      M[j].y = fma(wi, f, M[j].y);
+    }
+    hr += wr;
+    hi += wi;
+    Rr = Ri = 0.0;
+  };
+  const longlong2* row = base;
+  int sg = 0;
+  for (int64_t it = 0; it < R.most; ++it) {
+    if (it > 0 && it < R.len) {
+      if ((it & ((1ll << kSegLog) - 1ll)) == 0) settle();
+      int dr;
+      const int i = quad_next(P, (uint64_t)(R.a + it), k, dr);
+      const uint32_t neg = (uint32_t)dr & 0x80000000u;  // the digit goes down: -R
+      double2 m = M[i];
+      m.x += xor_sign(Rr, neg);
+      m.y += xor_sign(Ri, neg);
+      M[i] = m;
+      row = rows + (int64_t)i * W;
+      sg = -2 * dr;
+    }
+    if (it >= R.len) sg = 0;
+    long long re, im;
+    int e;
+    quad_eval<S>(st, quad_smem, row, sg, base + W, P.fx, re, im, e);
+    const double w = it < R.len ? xor_sign(k.w, (k.parity ^ mixed) << 31) : 0.0;
+    Rr = fma(w, bf_to_double(re, e), Rr);
+    Ri = fma(w, bf_to_double(im, e), Ri);
+  }
+  settle();
+  // Each aligned group of G walkers (4 G lanes) sums its rows through the block's
+  // shared memory (every warp done with its buffers): component c of row j of thread t at
+  // smem[(2 j + c) * kQuadBlock + t].  The group's lanes take the components in turn,
+  // each in a fixed, staggered order (fewer bank conflicts).
+  const int nd = ndo + 2 + P.fixed_digit, G = max(P.group, 1), GL = 4 * G;
+  double* ms = reinterpret_cast<double*>(quad_smem);
+  __syncthreads();  // the rows lie across other warps' buffers
+  {
+    const int kk = threadIdx.x & 3;
+    const uint32_t n0 = (kk == 1 || kk == 3) ? 0x80000000u : 0u;  // d0 = -1
+    const uint32_t n1 = (kk == 1 || kk == 2) ? 0x80000000u : 0u;  // d1 = -1
+    double* o = ms + threadIdx.x;
+    o[0] = xor_sign(hr, n0);
+    o[kQuadBlock] = xor_sign(hi, n0);
+    o[2 * kQuadBlock] = xor_sign(hr, n1);
+    o[3 * kQuadBlock] = xor_sign(hi, n1);
+    for (int j = 0; j < ndo; ++j) {
+      const double2 m = M[j];
+      o[(4 + 2 * j) * kQuadBlock] = m.x;
+      o[(5 + 2 * j) * kQuadBlock] = m.y;
+    }
+    if (P.fixed_digit) {
+      o[(4 + 2 * ndo) * kQuadBlock] = hr;
+      o[(5 + 2 * ndo) * kQuadBlock] = hi;
+    }
+  }
+  if (GL > 32) __syncthreads(); else __syncwarp();  // a group's rows are its own columns
+  const int gl = threadIdx.x & (GL - 1);
+  const double* grp = ms + (threadIdx.x - gl);
+  double* out = reinterpret_cast<double*>(partials + P.part_off + (R.q / G) * nd);
+  for (int c = gl; c < 2 * nd; c += GL) {
+    const double* col = grp + c * kQuadBlock;
+    double s = 0.0;
+    for (int i = 0; i < GL; ++i) s += col[(i + gl) & (GL - 1)];
+    if (live) out[c] = s;
+  }
+}
+
+static size_t quad_smem_bytes(int slots, int rows) {
+  const int rounds = (slots + 3) / 4;
+  return sizeof(longlong2) *
+         (size_t)std::max((rounds > 1 ? 2 : 1) * kQuadX, rows * kQuadBlock);
+}
+
+constexpr int kQuadMaxSlots = (kMaxFactors + 1) / 2;
+using PermQuad = void (*)(const SweepProblem*, int, const longlong2*, int64_t, double2*);
+using MinorsQuad = void (*)(const SweepProblem*, int, const longlong2*, int64_t, double2*, int64_t);
+static const PermQuad kPermQuad[kQuadMaxSlots + 1] = {
+    nullptr,           perm_quad_kernel<1>,  perm_quad_kernel<2>,  perm_quad_kernel<3>,  perm_quad_kernel<4>,
+    perm_quad_kernel<5>,  perm_quad_kernel<6>,  perm_quad_kernel<7>,  perm_quad_kernel<8>,  perm_quad_kernel<9>,
+    perm_quad_kernel<10>, perm_quad_kernel<11>, perm_quad_kernel<12>, perm_quad_kernel<13>, perm_quad_kernel<14>,
+    perm_quad_kernel<15>, perm_quad_kernel<16>};
+static const MinorsQuad kMinorsQuad[kQuadMaxSlots + 1] = {
+    nullptr,           minors_quad_kernel<1>,  minors_quad_kernel<2>,  minors_quad_kernel<3>,  minors_quad_kernel<4>,
+    minors_quad_kernel<5>,  minors_quad_kernel<6>,  minors_quad_kernel<7>,  minors_quad_kernel<8>,  minors_quad_kernel<9>,
+    minors_quad_kernel<10>, minors_quad_kernel<11>, minors_quad_kernel<12>, minors_quad_kernel<13>, minors_quad_kernel<14>,
+    minors_quad_kernel<15>, minors_quad_kernel<16>};
+
+static int g_quad_occ[2][kQuadMaxSlots + 1][kMaxMinorDigits + 1];
+
+cudaError_t prepare_quad_kernels() {
+  cudaError_t e;
+  for (int s = 1; s <= kQuadMaxSlots; ++s) {
+    const int most = (int)quad_smem_bytes(s, kMaxMinorDigits);
+    if ((e = cudaFuncSetAttribute(kPermQuad[s], cudaFuncAttributeMaxDynamicSharedMemorySize, most))) return e;
+    if ((e = cudaFuncSetAttribute(kMinorsQuad[s], cudaFuncAttributeMaxDynamicSharedMemorySize, most))) return e;
+    for (int rows = 0; rows <= kMaxMinorDigits; ++rows) {
+      int* occ[2] = {&g_quad_occ[0][s][rows], &g_quad_occ[1][s][rows]};
+      const size_t b = quad_smem_bytes(s, rows);
+      if (rows > 0 && b == quad_smem_bytes(s, rows - 1)) {  // the same block as before
+        *occ[0] = occ[0][-1];
+        *occ[1] = occ[1][-1];
+        continue;
+      }
+      if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ[0], kPermQuad[s], kQuadBlock, b))) return e;
+      if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ[1], kMinorsQuad[s], kQuadBlock, b))) return e;
+    }
+  }
+  return cudaSuccess;
+}
+
+int64_t quad_resident_walkers(int nf, int rows, bool minors, int sm_count) {
+  if (nf < 2 || nf > kMaxFactors) return kQuadWalkers;
+  rows = minors ? std::min(std::max(rows, 0), kMaxMinorDigits) : 0;
+  return (int64_t)std::max(1, g_quad_occ[minors ? 1 : 0][quad_slots(nf)][rows]) * sm_count * kQuadWalkers;
+}
+
+cudaError_t launch_quad_sweep(int nf, bool minors, const SweepLaunch& L, cudaStream_t st) {
+  const unsigned grid = (unsigned)((L.total_threads + kQuadWalkers - 1) / kQuadWalkers);
+  const int s = quad_slots(nf);
+  if (minors)
+    kMinorsQuad[s]<<<grid, kQuadBlock, quad_smem_bytes(s, L.rows), st>>>(L.probs, L.n_probs, L.pool, L.total_threads,
+                                                                         L.partials, L.uniform_threads);
+  else
+    kPermQuad[s]<<<grid, kQuadBlock, quad_smem_bytes(s, 0), st>>>(L.probs, L.n_probs, L.pool, L.total_threads,
+                                                                  L.partials);
+  return cudaGetLastError();
+}
+
+}  // namespace boss

@@ -47,7 +47,7 @@ enum SweepKind : int32_t { kRyser = 0, kGlynn = 1 };
 // One sweep (a permanent or an all-minors problem).  Plain old data in device
 // memory; built by the host planner or by the sampler's device-side planner.
 struct SweepProblem {
-  int32_t nd;        // digits, binary ones first
+  int32_t nd;        // digits walked, binary ones first (without the `low` ones)
   int32_t nb;        // leading binary digits
   int32_t nf;        // product factors
   int32_t kind;      // SweepKind
@@ -56,12 +56,13 @@ struct SweepProblem {
                      // its own scale 2^fx_f); gradients: the fraction bits shared by all factors
   int32_t has_base;  // base sums present
   int32_t out_idx;   // result index
-  int64_t n_codes;       // codes in the sweep
+  int64_t n_codes;       // codes in the sweep (low = 2: steps of four codes)
   int64_t thread_begin;  // first global thread of this sweep
   int64_t n_threads;     // threads working on it
-  int64_t mat_off;   // D: nd x nf fixed-point complex (longlong2), row-major
+  int64_t mat_off;   // rows, nd x nf fixed-point complex (longlong2): D, or -D / 2 packed (pack_row) for the FP64
+                     // permanent and all-minors sweeps; low = 2: the layout of boss_quad.cuh
   int64_t base_off;  // nf fixed-point complex
-  int64_t part_off;  // partials: n_threads complex (perms) or n_threads x (nd + fixed_digit) (all-minors)
+  int64_t part_off;  // partials: n_threads complex (perms) or n_threads x (nd + low + fixed_digit) (all-minors)
   int64_t ff_off;    // float-pair all-minors only: nb x nf rows of D as float pairs (float4: re hi, re lo,
                      // im hi, im lo, each factor in its own scale), then nf int32 exponent biases
   double scale;      // final real scale
@@ -71,16 +72,20 @@ struct SweepProblem {
                      // (n_threads / group) x nd; n_threads and thread_begin are multiples of it, and
                      // every sweep of the launch has the same
   int32_t align;     // permanents, all-minors: ranges start at multiples of 2^align codes (range_align)
+  int32_t low;       // 2: two more binary digits, all four of whose values are taken at every step (boss_quad.cuh)
   uint8_t mult[kMaxDigits];
 };
 
-// A row entry of D for the integer-pipe sweeps (permanents, all-minors): the
+// A row entry of the integer-pipe sweeps (permanents, all-minors): u = -D / 2, the
 // 64-bit value hi 2^32 + lo with lo taken as a SIGNED word (hi carries its sign
-// bit), so that adding sg times it (sg = +-1) is one 32 x 32 + 64-bit multiply-add
-// and one 32-bit one per component, on the FMA pipe, instead of two exclusive-ors
-// and two carry-linked adds on the ALU pipe, which bounds these sweeps.
+// bit), so that adding sg times it (sg = +-2 for a flip, -2 r for a digit's value)
+// is one 32 x 32 + 64-bit multiply-add and one 32-bit one per component, without
+// exclusive-ors for the sign.
 __host__ __device__ __forceinline__ long long pack_row(long long v) {
   return (long long)((unsigned long long)v + (((unsigned long long)v & 0x80000000ull) << 1));
+}
+__host__ __device__ __forceinline__ long long unpack_row(long long v) {
+  return (long long)((unsigned long long)v - (((unsigned long long)v & 0x80000000ull) << 1));
 }
 
 // ---------------------------------------------------------------------------
@@ -157,8 +162,7 @@ __host__ __device__ __forceinline__ long long mad_wide(int a, int b, long long c
 #endif
 }
 
-// acc + sg * d for a packed row component d (pack_row): one 32 x 32 + 64-bit and
-// one 32-bit multiply-add.  sg is a small integer (+-1, or a digit's value).
+// acc + sg * d for a packed row component d (pack_row), sg a small integer.
 __device__ __forceinline__ long long add_packed(long long acc, long long d, int sg) {
   const int lo = (int)(unsigned)(unsigned long long)d, hi = (int)((unsigned long long)d >> 32);
   const unsigned long long t = (unsigned long long)mad_wide(lo, sg, acc);
@@ -198,8 +202,8 @@ __device__ __forceinline__ void decode_code(const SweepProblem& P, const longlon
     for (int f = 0; f < NF; ++f) {
       if (f > 0 && (f & 7) == 0) load_fence();
       const longlong2 d = row[f];
-      sr[f] = kPacked ? add_packed(sr[f], d.x, 1) : sr[f] + d.x;
-      si[f] = kPacked ? add_packed(si[f], d.y, 1) : si[f] + d.y;
+      sr[f] = kPacked ? add_packed(sr[f], d.x, -2) : sr[f] + d.x;
+      si[f] = kPacked ? add_packed(si[f], d.y, -2) : si[f] + d.y;
     }
   }
   uint64_t th = t >> P.nb;
@@ -217,8 +221,8 @@ __device__ __forceinline__ void decode_code(const SweepProblem& P, const longlon
 #pragma unroll
       for (int f = 0; f < NF; ++f) {
         const longlong2 d = row[f];
-        sr[f] = kPacked ? add_packed(sr[f], d.x, (int)r) : sr[f] + (long long)r * d.x;
-        si[f] = kPacked ? add_packed(si[f], d.y, (int)r) : si[f] + (long long)r * d.y;
+        sr[f] = kPacked ? add_packed(sr[f], d.x, -2 * (int)r) : sr[f] + (long long)r * d.x;
+        si[f] = kPacked ? add_packed(si[f], d.y, -2 * (int)r) : si[f] + (long long)r * d.y;
       }
     }
   }
@@ -245,7 +249,7 @@ template <int NF>
 __device__ __forceinline__ void flip_packed(const longlong2* __restrict__ D, int i, uint32_t bit, long long (&sr)[NF],
                                             long long (&si)[NF]) {
   const longlong2* row = D + (size_t)i * NF;
-  const int sg = 1 - 2 * (int)bit;
+  const int sg = 4 * (int)bit - 2;  // r 0 -> 1 adds D = -2 u
 #pragma unroll
   for (int f = 0; f < NF; ++f) {
     if (f > 0 && (f & 7) == 0) load_fence();
@@ -306,8 +310,8 @@ __host__ __device__ __forceinline__ I128 sub128(I128 x, I128 y) {
 //     a unit, is dropped), then one normalising shift.  Of two normal values
 //     |product| >= 2^122 before the >> 64, off by less than 2 units a component:
 //     relative error below 2^-56.5 of the product's magnitude;
-//   * bf_mul with a fixed-point factor as it is (|re|, |im| < 2^61, its own scale
-//     2^fx_f such that its largest possible sum has 61 bits): the same absolute
+//   * bf_mul_high with a fixed-point factor as it is (|re|, |im| < 2^62, its own scale
+//     2^fx_f such that its largest possible sum has 62 bits): the same absolute
 //     error, under 2^-58 of (the first value's magnitude times that largest
 //     sum), so a factor that happens to be small costs nothing extra to scale;
 //   * bf_to_double: one rounding to FP64 (2^-53) at the end.
@@ -315,11 +319,10 @@ __host__ __device__ __forceinline__ I128 sub128(I128 x, I128 y) {
 // of these products is more accurate than the FP64 chain it replaces (64
 // permanents at n = 28: 9.9e-14 from 64-bit values against 1.5e-13 with the last
 // 8 factors multiplied in FP64).
-// Measured, 64 permanents (input-side digits, 2^(n-1) codes each): n = 20 1.71 ms,
-// n = 24 33.5 ms, against 2.08 and 39.3 ms with the limb products left to the
-// compiler and 3.5 and 62 ms with exact 128-bit leaves and 8 FP64 products.
-// Bound by the FMA pipe (a 32 x 32 + 64-bit multiply-add holds it for 4 cycles a
-// warp, 66 % busy) and dependent latency at 3 warps per scheduler.
+// Measured, 64 permanents (input-side digits, 2^(n-1) codes each) with the templated
+// kernel: n = 20 1.71 ms, n = 24 33.5 ms (2.08 and 39.3 ms with the limb products left
+// to the compiler).  Bound by the FMA pipe (a 32 x 32 + 64-bit multiply-add holds it
+// for 4 cycles a warp, 66 % busy) and dependent latency at 3 warps per scheduler.
 // ---------------------------------------------------------------------------
 struct BFloat {
   long long re, im;

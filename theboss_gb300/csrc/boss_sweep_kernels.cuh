@@ -245,7 +245,6 @@ __global__ void __launch_bounds__(128, kMinorsMinBlocks<NF>) minors_sweep_kernel
 //     float-pair rows of D.  The drift between two resynchronisations is a few
 //     units of 2^-47 of the rows per code in between.
 // ---------------------------------------------------------------------------
-constexpr int kFFMaxFactors = 24;  // above this the float-pair sums exhaust the registers
 // Codes between two resynchronisations of the float-pair sums with the exact
 // ones: the all-minors sweeps 32 (measured at n = 20, 10^4 samples: 8 -> 16 -> 32
 // -> 64 gave 1.72, 1.55, 1.47, 1.43 ms per step, and max error against
@@ -510,7 +509,6 @@ __global__ void __launch_bounds__(128, kFFMinBlocks<NF>) minors_sweep_ff_kernel(
 // one launch (each thread walking ~64x more codes than a lone permanent) n = 30
 // measured 5.9e-10 against double-double.
 // Each thread writes its partial as a float pair (float4) in the factors' scales.
-constexpr int kFFPermMaxFactors = 32;
 constexpr uint64_t kFFPermFold = 64;
 template <int NF>
 constexpr int kFFPermMinBlocks = NF <= 12 ? 4 : (NF <= 20 ? 3 : 2);
