@@ -99,21 +99,137 @@ __device__ __forceinline__ double glynn_abs2(const double2* __restrict__ U, int 
   return fma(p.x, p.x, p.y * p.y);
 }
 
-// Small permanents, one thread each: perm(U[T_k, S_k]) from the occupation rows
-// (len entries, uint8) of equally many (L) input and output particles.
-template <int L>
-__global__ void __launch_bounds__(128) small_perm_kernel(const double2* __restrict__ U, int m, int len,
-                                                         const uint8_t* __restrict__ S, const uint8_t* __restrict__ T,
-                                                         int64_t count, double2* __restrict__ out) {
-  const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= count) return;
-  int row[L], col[L];
-  int a = 0, b = 0;
-  for (int i = 0; i < len; ++i) {
-    for (int c = T[k * len + i]; c > 0 && a < L; --c) row[a++] = i;
-    for (int c = S[k * len + i]; c > 0 && b < L; --c) col[b++] = i;
+// A row's fixed-point scale for sums of at most `terms` of its entries: the fraction
+// bits that keep them below 2^62, or kNoScale where that cannot be done (a
+// non-finite entry, or sizes near the ends of the exponent range): such rows are
+// summed in FP64.
+constexpr int kNoScale = 1 << 30;
+__host__ __device__ inline int row_fraction_bits(double largest, int terms) {
+  if (largest == 0.0) return 56;
+  if (!(largest < 1e270 && largest > 1e-270)) return kNoScale;
+  return 61 - ilogb(largest * terms);  // largest * terms < 2^(ilogb + 1)
+}
+
+// One warp per row of U: its scale, and its entries in it, packed (pack_row).
+__global__ void __launch_bounds__(128) small_fixed_kernel(const double2* __restrict__ U, int m, int terms,
+                                                          longlong2* __restrict__ out, int32_t* __restrict__ rowfx) {
+  const int r = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (r >= m) return;
+  const double2* row = U + (size_t)r * m;
+  double mx = 0.0;
+  bool fine = true;
+  for (int i = lane; i < m; i += 32) {
+    const double x = fmax(fabs(row[i].x), fabs(row[i].y));
+    fine = fine && isfinite(row[i].x) && isfinite(row[i].y);
+    mx = fmax(mx, x);
   }
-  out[k] = glynn_small<L>(U, m, row, col);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  fine = __all_sync(0xffffffffu, fine);
+  const int fx = fine ? row_fraction_bits(mx, terms) : kNoScale;
+  if (lane == 0) rowfx[r] = fx;
+  for (int i = lane; i < m && fx != kNoScale; i += 32)
+    out[(size_t)r * m + i] = make_longlong2(pack_row(__double2ll_rn(ldexp(row[i].x, fx))),
+                                            pack_row(__double2ll_rn(ldexp(row[i].y, fx))));
+}
+
+// Small permanents: perm of the L x L matrix with rows rows[k][a] and columns
+// cols[k][b] of A (row stride ld, fixed point, packed).  2^lg lanes per permanent,
+// each over 2^(L - 1 - lg) sign vectors: the last lg columns' signs are the lane's
+// bits, the others walk in Gray order, column 0 stays +.  The products run on the
+// integer pipe (accumulate_product_bf), so a code costs ~45 instructions per factor
+// where FP64 ones hold its pipe for 4 * 64 clocks, and a single permanent has all
+// lanes of a block instead of one thread's chain of dependent FP64 products
+// (n = 8: 248 -> 40 us a call, planning and synchronisation included).  e0: minus the rows' fraction bits if given, else
+// rowfx by row; a permanent with a row that has no scale is summed in FP64 from U by
+// its first lane.
+template <int L>
+__global__ void __launch_bounds__(128) small_perm_kernel(const longlong2* __restrict__ A, int ld, int64_t stride,
+                                                         const uint16_t* __restrict__ rows,
+                                                         const uint16_t* __restrict__ cols,
+                                                         const int32_t* __restrict__ rowfx,
+                                                         const int32_t* __restrict__ e0s,
+                                                         const double2* __restrict__ U, int64_t count, int lg,
+                                                         double2* __restrict__ out) {
+  __shared__ double2 part[4];
+  const int64_t gid = (int64_t)blockIdx.x * 128 + threadIdx.x;
+  const int64_t at = gid >> lg;
+  const int64_t k = at < count ? at : count - 1;
+  const uint32_t mine = (uint32_t)gid & ((1u << lg) - 1u);
+  const uint16_t* ck = cols + k * L;
+  const longlong2* Ak = A + k * stride;
+  int row[L];
+  int e0 = e0s ? e0s[k] : 0;
+  bool fp64 = false;
+#pragma unroll
+  for (int a = 0; a < L; ++a) {
+    row[a] = rows[k * L + a];
+    if (!e0s) {
+      const int fx = rowfx[row[a]];
+      fp64 = fp64 || fx == kNoScale;
+      e0 -= fx;
+    }
+  }
+  double ar = 0.0, ai = 0.0;
+  if (fp64) {
+    if (mine == 0) {
+      int col[L];
+#pragma unroll
+      for (int b = 0; b < L; ++b) col[b] = ck[b];
+      const double2 p = glynn_small<L>(U, ld, row, col);
+      ar = p.x;
+      ai = p.y;
+    }
+  } else {
+    long long sr[L], si[L];
+#pragma unroll
+    for (int a = 0; a < L; ++a) sr[a] = si[a] = 0;
+    const int low = L - lg;  // columns low .. L - 1 have the lane's signs
+    for (int b = 0; b < L; ++b) {
+      const int sg = (b >= low && ((mine >> (b - low)) & 1u)) ? -1 : 1;
+      const int c = ck[b];
+#pragma unroll
+      for (int a = 0; a < L; ++a) {
+        const longlong2 u = Ak[(size_t)row[a] * ld + c];
+        sr[a] = add_packed(sr[a], u.x, sg);
+        si[a] = add_packed(si[a], u.y, sg);
+      }
+    }
+    uint32_t neg = 0, parity = __popc(mine) & 1;
+    const uint32_t codes = 1u << (low - 1);
+    for (uint32_t t = 0;;) {
+      accumulate_product_bf<L>(sr, si, e0, parity << 31, ar, ai);
+      if (++t >= codes) break;
+      const int b = __ffs(t);  // column 1 + ctz(t)
+      const int sg = ((neg >> b) & 1u) ? 2 : -2;
+      neg ^= 1u << b;
+      parity ^= 1u;
+      const int c = ck[b];
+#pragma unroll
+      for (int a = 0; a < L; ++a) {
+        const longlong2 u = Ak[(size_t)row[a] * ld + c];
+        sr[a] = add_packed(sr[a], u.x, sg);
+        si[a] = add_packed(si[a], u.y, sg);
+      }
+    }
+    const double s = 1.0 / (double)(1u << (L - 1));
+    ar *= s;
+    ai *= s;
+  }
+  for (int o = 1; o < (1 << min(lg, 5)); o <<= 1) {  // the permanent's lanes, in a fixed order
+    ar += __shfl_xor_sync(0xffffffffu, ar, o);
+    ai += __shfl_xor_sync(0xffffffffu, ai, o);
+  }
+  if (lg > 5) {  // 2 or 4 whole warps per permanent
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = make_double2(ar, ai);
+    __syncthreads();
+    if (mine == 0)
+      for (int w = 1; w < (1 << (lg - 5)); ++w) {
+        ar += part[(threadIdx.x >> 5) + w].x;
+        ai += part[(threadIdx.x >> 5) + w].y;
+      }
+  }
+  if (mine == 0 && at < count) out[k] = make_double2(ar, ai);
 }
 
 // One thread per (lossy input k, outcome o); the layout [k][o] lets the outcome
@@ -415,74 +531,186 @@ static int group_large(Context* cx, const double* matrix, int m, int n, int l, c
   return kOk;
 }
 
+struct SmallLaunch {
+  const longlong2* A;
+  int ld;
+  int64_t stride;  // between the permanents' own matrices (0: one for all)
+  const uint16_t *rows, *cols;  // L per permanent
+  const int32_t *rowfx, *e0;
+  const double2* U;
+  int64_t count;
+  double2* out;
+};
+
 template <int L>
-static cudaError_t launch_small(const double2* U, int m, int len, const uint8_t* S, const uint8_t* T, int64_t count,
-                                double2* out, cudaStream_t s) {
-  small_perm_kernel<L><<<(unsigned)((count + 127) / 128), 128, 0, s>>>(U, m, len, S, T, count, out);
+static cudaError_t launch_small(const SmallLaunch& s, int sm_count, cudaStream_t st) {
+  // lanes per permanent: as many as keep the launch below a few blocks per SM, at
+  // most a block and at least one sign vector each
+  int lg = 0;
+  while (lg < 7 && lg < L - 1 && (s.count << (lg + 1)) <= (int64_t)sm_count * 256) ++lg;
+  const int64_t threads = s.count << lg;
+  small_perm_kernel<L><<<(unsigned)((threads + 127) / 128), 128, 0, st>>>(s.A, s.ld, s.stride, s.rows, s.cols, s.rowfx,
+                                                                          s.e0, s.U, s.count, lg, s.out);
   return cudaGetLastError();
 }
 
-static cudaError_t launch_small_l(int l, const double2* U, int m, int len, const uint8_t* S, const uint8_t* T,
-                                  int64_t count, double2* out, cudaStream_t s) {
+static cudaError_t launch_small_l(int l, const SmallLaunch& a, int sms, cudaStream_t s) {
   switch (l) {
-    case 1: return launch_small<1>(U, m, len, S, T, count, out, s);
-    case 2: return launch_small<2>(U, m, len, S, T, count, out, s);
-    case 3: return launch_small<3>(U, m, len, S, T, count, out, s);
-    case 4: return launch_small<4>(U, m, len, S, T, count, out, s);
-    case 5: return launch_small<5>(U, m, len, S, T, count, out, s);
-    case 6: return launch_small<6>(U, m, len, S, T, count, out, s);
-    case 7: return launch_small<7>(U, m, len, S, T, count, out, s);
-    case 8: return launch_small<8>(U, m, len, S, T, count, out, s);
-    case 9: return launch_small<9>(U, m, len, S, T, count, out, s);
-    case 10: return launch_small<10>(U, m, len, S, T, count, out, s);
+    case 1: return launch_small<1>(a, sms, s);
+    case 2: return launch_small<2>(a, sms, s);
+    case 3: return launch_small<3>(a, sms, s);
+    case 4: return launch_small<4>(a, sms, s);
+    case 5: return launch_small<5>(a, sms, s);
+    case 6: return launch_small<6>(a, sms, s);
+    case 7: return launch_small<7>(a, sms, s);
+    case 8: return launch_small<8>(a, sms, s);
+    case 9: return launch_small<9>(a, sms, s);
+    case 10: return launch_small<10>(a, sms, s);
     default: return cudaErrorInvalidValue;
   }
+}
+
+static void particle_modes(const int32_t* occ, int len, uint16_t* out) {
+  int p = 0;
+  for (int i = 0; i < len; ++i)
+    for (int c = 0; c < occ[i]; ++c) out[p++] = (uint16_t)i;
+}
+
+static size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
+
+// A few permanents: each one's matrix is gathered and scaled on the host (L^2
+// entries), and the kernel reads it from, and writes its result to, page-locked
+// host memory: one launch and one synchronisation, no copies.  done = false: a row
+// has no fixed-point scale, nothing was launched.
+constexpr int64_t kFewPerms = 16;
+
+static int small_perm_few(Context* cx, const double* matrix, int m, int len, const int32_t* S, const int32_t* T,
+                          const std::vector<int>* by_l, int64_t total, double2* results, bool& done) {
+  constexpr int L = kSmallPermMax;
+  done = false;
+  const size_t o_rows = align256(sizeof(longlong2) * L * L * (size_t)total);
+  const size_t o_cols = o_rows + align256(sizeof(uint16_t) * (size_t)total * L);
+  const size_t o_e0 = o_cols + align256(sizeof(uint16_t) * (size_t)total * L);
+  const size_t o_out = o_e0 + align256(sizeof(int32_t) * (size_t)total);
+  int st;
+  if ((st = ensure_pinned(cx, o_out + sizeof(double2) * (size_t)total))) return st;
+  char* h = (char*)cx->pinned;
+  uint16_t* hr = (uint16_t*)(h + o_rows);
+  uint16_t* hc = (uint16_t*)(h + o_cols);
+  size_t at = 0;  // rows and columns, l per permanent
+  int64_t q = 0;
+  for (int l = 1; l <= L; ++l)
+    for (int k : by_l[l]) {
+      uint16_t r[L], c[L];
+      particle_modes(T + (size_t)k * len, len, r);
+      particle_modes(S + (size_t)k * len, len, c);
+      longlong2* M = (longlong2*)(h) + q * L * L;
+      int e0 = 0;
+      for (int a = 0; a < l; ++a) {
+        double mx = 0.0;
+        bool fine = true;
+        const double* row = matrix + 2 * (size_t)r[a] * m;
+        for (int b = 0; b < l; ++b) {
+          const double x = row[2 * c[b]], y = row[2 * c[b] + 1];
+          fine = fine && std::isfinite(x) && std::isfinite(y);
+          mx = std::max(mx, std::max(std::fabs(x), std::fabs(y)));
+        }
+        const int fx = fine ? row_fraction_bits(mx, l) : kNoScale;
+        if (fx == kNoScale) return kOk;
+        const double scale = std::ldexp(1.0, fx);
+        for (int b = 0; b < l; ++b)
+          M[a * L + b] = longlong2{pack_row(std::llrint(row[2 * c[b]] * scale)),
+                                   pack_row(std::llrint(row[2 * c[b] + 1] * scale))};
+        e0 -= fx;
+        hr[at + a] = hc[at + a] = (uint16_t)a;
+      }
+      ((int32_t*)(h + o_e0))[q++] = e0;
+      at += l;
+    }
+  at = 0;
+  q = 0;
+  for (int l = 1; l <= L; ++l) {
+    const int64_t c = (int64_t)by_l[l].size();
+    if (!c) continue;
+    const SmallLaunch s{(longlong2*)h + q * L * L, L, L * L, hr + at, hc + at, nullptr, (int32_t*)(h + o_e0) + q, nullptr,
+                        c, (double2*)(h + o_out) + q};
+    const cudaError_t e = launch_small_l(l, s, cx->sm_count, cx->stream);
+    if (e != cudaSuccess) return fail_cuda(e, "small permanents");
+    at += (size_t)c * l;
+    q += c;
+  }
+  const cudaError_t e = cudaStreamSynchronize(cx->stream);
+  if (e != cudaSuccess) return fail_cuda(e, "small permanents");
+  const double2* out = (const double2*)(h + o_out);
+  q = 0;
+  for (int l = 1; l <= L; ++l)
+    for (int k : by_l[l]) results[k] = out[q++];
+  done = true;
+  return kOk;
 }
 
 int small_perm_batch(Context* cx, const double* matrix, int m, int len, const int32_t* S, const int32_t* T,
                      const std::vector<int>* by_l, double2* results) {
   int64_t total = 0;
-  for (int l = 1; l <= kSmallPermMax; ++l) total += (int64_t)by_l[l].size();
+  int most = 0;
+  size_t particles = 0;
+  for (int l = 1; l <= kSmallPermMax; ++l)
+    if (!by_l[l].empty()) {
+      total += (int64_t)by_l[l].size();
+      particles += (size_t)l * by_l[l].size();
+      most = l;
+    }
   if (total == 0) return kOk;
-  auto al = [](size_t x) { return (x + 255) & ~(size_t)255; };
-  const size_t o_U = 0, o_S = al(sizeof(double2) * (size_t)m * m), o_T = o_S + al((size_t)total * len);
-  const size_t o_out = o_T + al((size_t)total * len), arena = o_out + sizeof(double2) * (size_t)total;
   int st;
-  if ((st = ensure(cx->dist[3], arena))) return st;
-  if ((st = ensure_pinned(cx, arena))) return st;
+  if (total <= kFewPerms) {
+    bool done = false;
+    if ((st = small_perm_few(cx, matrix, m, len, S, T, by_l, total, results, done)) || done) return st;
+  }
+  // U | rows | columns up; results down; U in fixed point and its scales on the device
+  const size_t mm = (size_t)m * m;
+  const size_t o_rows = align256(sizeof(double2) * mm), o_cols = o_rows + align256(sizeof(uint16_t) * particles);
+  const size_t in_bytes = o_cols + align256(sizeof(uint16_t) * particles);
+  const size_t o_fx = in_bytes + align256(sizeof(double2) * (size_t)total);
+  const size_t o_rowfx = o_fx + align256(sizeof(longlong2) * mm);
+  if ((st = ensure(cx->dist[3], o_rowfx + sizeof(int32_t) * (size_t)m))) return st;
+  if ((st = ensure_pinned(cx, o_fx))) return st;
   char* h = (char*)cx->pinned;
-  memcpy(h + o_U, matrix, sizeof(double2) * (size_t)m * m);
-  uint8_t* hS = (uint8_t*)(h + o_S);
-  uint8_t* hT = (uint8_t*)(h + o_T);
-  int64_t at = 0;
+  memcpy(h, matrix, sizeof(double2) * mm);
+  uint16_t* hr = (uint16_t*)(h + o_rows);
+  uint16_t* hc = (uint16_t*)(h + o_cols);
+  size_t at = 0;
   for (int l = 1; l <= kSmallPermMax; ++l)
     for (int k : by_l[l]) {
-      for (int i = 0; i < len; ++i) {
-        hS[at * len + i] = (uint8_t)S[(size_t)k * len + i];
-        hT[at * len + i] = (uint8_t)T[(size_t)k * len + i];
-      }
-      ++at;
+      particle_modes(T + (size_t)k * len, len, hr + at);
+      particle_modes(S + (size_t)k * len, len, hc + at);
+      at += l;
     }
   char* d = (char*)cx->dist[3].ptr;
   cudaStream_t s = cx->stream;
-  cudaError_t e = cudaMemcpyAsync(d, h, o_out, cudaMemcpyHostToDevice, s);
+  cudaError_t e = cudaMemcpyAsync(d, h, in_bytes, cudaMemcpyHostToDevice, s);
   if (e != cudaSuccess) return fail_cuda(e, "H2D small permanents");
+  small_fixed_kernel<<<(unsigned)((m + 3) / 4), 128, 0, s>>>((const double2*)d, m, most, (longlong2*)(d + o_fx),
+                                                             (int32_t*)(d + o_rowfx));
+  if ((e = cudaGetLastError()) != cudaSuccess) return fail_cuda(e, "small permanents");
   at = 0;
+  int64_t q = 0;
   for (int l = 1; l <= kSmallPermMax; ++l) {
     const int64_t c = (int64_t)by_l[l].size();
     if (!c) continue;
-    e = launch_small_l(l, (const double2*)(d + o_U), m, len, (const uint8_t*)(d + o_S) + at * len,
-                       (const uint8_t*)(d + o_T) + at * len, c, (double2*)(d + o_out) + at, s);
-    if (e != cudaSuccess) return fail_cuda(e, "small permanents");
-    at += c;
+    const SmallLaunch a{(const longlong2*)(d + o_fx), m, 0, (const uint16_t*)(d + o_rows) + at,
+                        (const uint16_t*)(d + o_cols) + at, (const int32_t*)(d + o_rowfx), nullptr, (const double2*)d, c,
+                        (double2*)(d + in_bytes) + q};
+    if ((e = launch_small_l(l, a, cx->sm_count, s)) != cudaSuccess) return fail_cuda(e, "small permanents");
+    at += (size_t)c * l;
+    q += c;
   }
-  e = cudaMemcpyAsync(h + o_out, d + o_out, sizeof(double2) * (size_t)total, cudaMemcpyDeviceToHost, s);
+  e = cudaMemcpyAsync(h + in_bytes, d + in_bytes, sizeof(double2) * (size_t)total, cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) return fail_cuda(e, "small permanents");
-  const double2* hr = (const double2*)(h + o_out);
-  at = 0;
+  const double2* out = (const double2*)(h + in_bytes);
+  q = 0;
   for (int l = 1; l <= kSmallPermMax; ++l)
-    for (int k : by_l[l]) results[k] = hr[at++];
+    for (int k : by_l[l]) results[k] = out[q++];
   return kOk;
 }
 

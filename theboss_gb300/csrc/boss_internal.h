@@ -48,8 +48,9 @@ cudaError_t launch_perm_reduce(const SweepProblem* probs, int n_probs, const dou
                                cudaStream_t st, bool ff = false);
 cudaError_t launch_grad_reduce(const SweepProblem* probs, int n_probs, const double2* gpart, const double2* ppart,
                                double2* grad_out, double2* perm_out, int row_stride, cudaStream_t st);
-cudaError_t launch_minors_reduce(const SweepProblem* probs, int n_probs, const double2* partials, double2* out,
-                                 int nd_max, cudaStream_t st, bool ff = false);
+// rows: the most digits (held one included) of a sweep.
+cudaError_t launch_minors_reduce(const SweepProblem* probs, int n_probs, int rows, const double2* partials,
+                                 double2* out, int nd_max, cudaStream_t st, bool ff = false);
 
 // Splits `n_codes` codes over at most `resident` threads, proportionally, at
 // least one thread per sweep and at least kMinCodesPerThread codes per thread.
@@ -152,8 +153,8 @@ int ensure_pinned(Context* cx, size_t bytes);
 // (perms) or nd_max complex per sweep (all-minors).
 int run_sweeps(Context* cx, const std::vector<HostSweep>& sweeps, bool minors, int nd_max, double2* results_host);
 
-// Permanents of at most kSmallPermMax particles, one GPU thread each (Glynn's
-// formula in registers, no sweep planning): by_l[l] lists the requests k with
+// Permanents of at most kSmallPermMax particles, 1 to 128 GPU threads each (Glynn's
+// formula in registers, no sweep planning; m <= 65536): by_l[l] lists the requests k with
 // l = sum(S_k) = sum(T_k) particles; S, T are the callers' occupation rows.
 constexpr int kSmallPermMax = 10;
 int small_perm_batch(Context* cx, const double* matrix, int m, int len, const int32_t* S, const int32_t* T,

@@ -109,14 +109,16 @@ int range_align(int64_t n_codes, int64_t n_threads, int nb) {
   return c;
 }
 
-// One block per sweep: fixed-order sum of its threads' partials.
+// One block per sweep: fixed-order sum of its groups' partials.
 // ff: the partials are float pairs (float4), as the float-pair sweep writes them.
 __global__ void perm_reduce_kernel(const SweepProblem* __restrict__ probs, const double2* __restrict__ partials,
                                    double2* __restrict__ out, int ff) {
   __shared__ double sr[256], si[256];
   const SweepProblem& P = probs[blockIdx.x];
   double ar = 0.0, ai = 0.0;
-  for (int64_t i = threadIdx.x; i < P.n_threads; i += blockDim.x) {
+  const int64_t parts = P.n_threads / P.group;
+#pragma unroll 4  // independent loads in flight
+  for (int64_t i = threadIdx.x; i < parts; i += blockDim.x) {
     double2 v;
     if (ff) {
       const float4 f = reinterpret_cast<const float4*>(partials)[P.part_off + i];
@@ -140,40 +142,41 @@ __global__ void perm_reduce_kernel(const SweepProblem* __restrict__ probs, const
   if (threadIdx.x == 0) out[P.out_idx] = make_double2(sr[0] * P.scale, si[0] * P.scale);
 }
 
-// One block per all-minors sweep; digit by digit, a fixed-order tree sum over the
-// threads' partials.
+// One block per all-minors sweep and digit: a fixed-order tree sum over the
+// groups' partials.
 // ff: the partials are float pairs (float4), as the float-pair sweep writes them.
-__global__ void minors_reduce_kernel(const SweepProblem* __restrict__ probs, const double2* __restrict__ partials,
-                                     double2* __restrict__ out, int nd_max, int ff) {
-  __shared__ double sr[256], si[256];
+__global__ void __launch_bounds__(128) minors_reduce_kernel(const SweepProblem* __restrict__ probs,
+                                                            const double2* __restrict__ partials,
+                                                            double2* __restrict__ out, int nd_max, int ff) {
+  __shared__ double sr[128], si[128];
   const SweepProblem& P = probs[blockIdx.x];
-  const int nd = P.nd + P.low + P.fixed_digit;  // the held digit's row last
-  for (int j = 0; j < nd; ++j) {
-    double ar = 0.0, ai = 0.0;
-    for (int64_t q = threadIdx.x; q < P.n_threads; q += blockDim.x) {
-      double2 v;
-      if (ff) {
-        const float4 f = reinterpret_cast<const float4*>(partials)[P.part_off + q * nd + j];
-        v = make_double2(ff_to_double(f.x, f.y), ff_to_double(f.z, f.w));
-      } else {
-        v = partials[P.part_off + q * nd + j];
-      }
-      ar += v.x;
-      ai += v.y;
+  const int nd = P.nd + P.low + P.fixed_digit, j = blockIdx.y;  // the held digit's row last
+  if (j >= nd) return;
+  const int64_t parts = P.n_threads / P.group;
+  double ar = 0.0, ai = 0.0;
+#pragma unroll 4  // independent loads in flight
+  for (int64_t q = threadIdx.x; q < parts; q += 128) {
+    double2 v;
+    if (ff) {
+      const float4 f = reinterpret_cast<const float4*>(partials)[P.part_off + q * nd + j];
+      v = make_double2(ff_to_double(f.x, f.y), ff_to_double(f.z, f.w));
+    } else {
+      v = partials[P.part_off + q * nd + j];
     }
-    sr[threadIdx.x] = ar;
-    si[threadIdx.x] = ai;
-    __syncthreads();
-    for (int s = blockDim.x >> 1; s > 0; s >>= 1) {
-      if ((int)threadIdx.x < s) {
-        sr[threadIdx.x] += sr[threadIdx.x + s];
-        si[threadIdx.x] += si[threadIdx.x + s];
-      }
-      __syncthreads();
+    ar += v.x;
+    ai += v.y;
+  }
+  sr[threadIdx.x] = ar;
+  si[threadIdx.x] = ai;
+  __syncthreads();
+  for (int s = 64; s > 0; s >>= 1) {
+    if ((int)threadIdx.x < s) {
+      sr[threadIdx.x] += sr[threadIdx.x + s];
+      si[threadIdx.x] += si[threadIdx.x + s];
     }
-    if (threadIdx.x == 0) out[(size_t)P.out_idx * nd_max + j] = make_double2(sr[0] * P.scale, si[0] * P.scale);
     __syncthreads();
   }
+  if (threadIdx.x == 0) out[(size_t)P.out_idx * nd_max + j] = make_double2(sr[0] * P.scale, si[0] * P.scale);
 }
 
 // One block per gradient sweep: every (digit, factor) entry of the per-warp
@@ -228,10 +231,10 @@ cudaError_t launch_perm_reduce(const SweepProblem* probs, int n_probs, const dou
   return cudaGetLastError();
 }
 
-cudaError_t launch_minors_reduce(const SweepProblem* probs, int n_probs, const double2* partials, double2* out,
-                                 int nd_max, cudaStream_t st, bool ff) {
+cudaError_t launch_minors_reduce(const SweepProblem* probs, int n_probs, int rows, const double2* partials,
+                                 double2* out, int nd_max, cudaStream_t st, bool ff) {
   if (n_probs <= 0) return cudaSuccess;
-  minors_reduce_kernel<<<n_probs, 256, 0, st>>>(probs, partials, out, nd_max, ff ? 1 : 0);
+  minors_reduce_kernel<<<dim3((unsigned)n_probs, (unsigned)rows), 128, 0, st>>>(probs, partials, out, nd_max, ff ? 1 : 0);
   return cudaGetLastError();
 }
 

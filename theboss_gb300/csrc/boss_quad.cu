@@ -186,7 +186,7 @@ __device__ __forceinline__ QuadRange quad_range(const SweepProblem& P, int64_t w
   return r;
 }
 
-// One permanent per sweep problem; every walker writes one complex partial.
+// One permanent per sweep problem; every group of walkers writes one complex partial.
 template <int S>
 __global__ void __launch_bounds__(kQuadBlock, quad_blocks(S)) perm_quad_kernel(const SweepProblem* __restrict__ probs,
                                                                         int n_probs,
@@ -224,12 +224,12 @@ __global__ void __launch_bounds__(kQuadBlock, quad_blocks(S)) perm_quad_kernel(c
     ar = fma(w, bf_to_double(re, e), ar);
     ai = fma(w, bf_to_double(im, e), ai);
   }
-#pragma unroll
-  for (int o = 1; o < 4; o <<= 1) {  // the walker's four codes, in a fixed order
+  const int G = P.group;  // 1, 2, 4 or 8 walkers (one warp at most), the same for the whole launch
+  for (int o = 1; o < 4 * G; o <<= 1) {  // the walkers' codes, in a fixed order
     ar += __shfl_xor_sync(0xffffffffu, ar, o);
     ai += __shfl_xor_sync(0xffffffffu, ai, o);
   }
-  if (live && (threadIdx.x & 3) == 0) partials[P.part_off + R.q] = make_double2(ar, ai);
+  if (live && (threadIdx.x & (4 * G - 1)) == 0) partials[P.part_off + R.q / G] = make_double2(ar, ai);
 }
 
 // All-minors in Glynn form (see minors_walk): half of every minor, row order low

@@ -67,10 +67,11 @@ struct SweepProblem {
                      // im hi, im lo, each factor in its own scale), then nf int32 exponent biases
   double scale;      // final real scale
   int32_t fixed_digit;  // gradients, all-minors: a binary digit held at r = 0 (Glynn halving) adds a weight-1 row
-  int32_t group;     // all-minors: each aligned group of `group` threads (1, 2, 4, .., 128; above 32 only when the
-                     // launch's threads fill whole blocks) sums its minors, so the partials are
-                     // (n_threads / group) x nd; n_threads and thread_begin are multiples of it, and
-                     // every sweep of the launch has the same
+  int32_t group;     // each aligned group of `group` threads (all-minors: 1, 2, 4, .., 128; above 32 only when the
+                     // launch's threads fill whole blocks; low = 2: walkers, permanents up to 8, all-minors up
+                     // to 32; the templated permanents 1) sums its partials, so there are n_threads / group of
+                     // them; n_threads and thread_begin are multiples of it, and every sweep of the launch has
+                     // the same
   int32_t align;     // permanents, all-minors: ranges start at multiples of 2^align codes (range_align)
   int32_t low;       // 2: two more binary digits, all four of whose values are taken at every step (boss_quad.cuh)
   uint8_t mult[kMaxDigits];
