@@ -365,12 +365,34 @@ static void fill_quad(HostSweep& hs, const Side& dig, int drop, bool glynn, cons
   if (nf & 1) hs.fx_sum += 62;
 }
 
+// The rows, base and fraction bits of boss_grad.cu (Glynn kind).
+static void fill_grad(HostSweep& hs, const Side& dig, int drop, const std::vector<Cx64>& u, const int* fxs) {
+  const int nf = hs.nf, F = grad_factors(nf), nd_all = (int)dig.modes.size();
+  hs.D.assign((size_t)hs.nd * F, longlong2{0, 0});
+  hs.base.assign((size_t)F + F / 4, longlong2{0, 0});
+  int32_t* bits = (int32_t*)(hs.base.data() + F);
+  for (int f = 0; f < F; ++f) {
+    bits[f] = f < nf ? fxs[f] : 61;
+    if (f >= nf) hs.base[f] = longlong2{1ll << 61, 0};  // padding: the constant 1
+  }
+  int row = 0;
+  for (int a = 0; a < nd_all; ++a) {
+    for (int f = 0; f < nf; ++f) {
+      const Cx64 v = u[(size_t)a * nf + f];
+      if (a != drop) hs.D[(size_t)row * F + f] = packed(v);
+      hs.base[f].x += (long long)dig.mult[a] * v.re;
+      hs.base[f].y += (long long)dig.mult[a] * v.im;
+    }
+    if (a != drop) ++row;
+  }
+  hs.fx_sum += 61 * (F - nf);
+}
+
 // Fills a sweep that iterates `dig` and multiplies over the particles of `col`
 // (a mode occupied p times gives p factors).  entry(a, l) is the matrix element
 // between digit mode a and product mode l.  Every factor f has its own fixed-point
 // scale 2^fx_f, chosen so that its largest possible sum fills the bits (a shared
-// scale would leave the factors of small rows with fewer significant bits); the
-// gradients share one.
+// scale would leave the factors of small rows with fewer significant bits).
 template <class F>
 static int fill_sweep(HostSweep& hs, const Side& dig, const Side& col, int kind, bool halve, PlanFor plan, bool ff,
                       int quad_min, F entry) {
@@ -404,31 +426,28 @@ static int fill_sweep(HostSweep& hs, const Side& dig, const Side& col, int kind,
     ++a_out;
   }
   const bool glynn = kind == kGlynn;
-  hs.layout = (plan == kPlanGrad || (ff && glynn && plan == kPlanAny)) ? kRowsPlain
+  hs.layout = plan == kPlanGrad                                         ? kRowsGrad
+              : (ff && glynn && plan == kPlanAny)                       ? kRowsPlain
               : (plan != kPlanTemplated && hs.nb >= 2 && hs.nf >= quad_min)   ? kRowsQuad
                                                                        : kRowsPacked;
-  // |row sum| <= sum_a mult_a * max component of the entries (of one factor, or of all)
+  // |row sum| <= sum_a mult_a * max component of the entries
   const int nf = hs.nf, nd_all = (int)dig.modes.size();
-  double bound[kMaxFactors] = {}, shared = 0.0;
-  for (int a = 0; a < nd_all; ++a) {
-    double mx = 0.0;
+  double bound[kMaxFactors] = {};
+  for (int a = 0; a < nd_all; ++a)
     for (int f = 0; f < nf; ++f) {
       const double2 z = entry(dig.modes[a], fmode[f]);
-      const double c = std::max(std::fabs(z.x), std::fabs(z.y));
-      bound[f] += dig.mult[a] * c;
-      mx = std::max(mx, c);
+      bound[f] += dig.mult[a] * std::max(std::fabs(z.x), std::fabs(z.y));
     }
-    shared += dig.mult[a] * mx;
-  }
   const bool old_rows = hs.layout == kRowsPlain;
   const int bits = old_rows ? 61 : 62;  // plain rows hold D = -2 u, which needs the bit
-  hs.fx = choose_fx(shared, bits);
   hs.fx_sum = 0;
   hs.ff_exp = 0;
   hs.fbias.assign(nf, 189);
+  int fxs[kMaxFactors];
   std::vector<Cx64> u((size_t)nd_all * nf);
   for (int f = 0; f < nf; ++f) {
-    const int fx = plan == kPlanGrad ? hs.fx : choose_fx(bound[f], bits);
+    const int fx = choose_fx(bound[f], bits);
+    fxs[f] = fx;
     const double scale = std::ldexp(glynn || old_rows ? 1.0 : -0.5, fx);  // Ryser's u = -U / 2
     unsigned long long bx = 0, by = 0;
     for (int a = 0; a < nd_all; ++a) {
@@ -449,6 +468,10 @@ static int fill_sweep(HostSweep& hs, const Side& dig, const Side& col, int kind,
   hs.has_base = glynn || !old_rows;
   if (hs.layout == kRowsQuad) {
     fill_quad(hs, dig, drop, glynn, u);
+    return kOk;
+  }
+  if (hs.layout == kRowsGrad) {
+    fill_grad(hs, dig, drop, u, fxs);
     return kOk;
   }
   hs.D.resize((size_t)hs.nd * nf);
@@ -834,51 +857,32 @@ int boss_perm_grad_batch(const double* matrix, int32_t m, const int32_t* input_s
     const std::vector<HostSweep>& sw = by_nf[nf];
     const int n = (int)sw.size();
     if (n == 0) continue;
-    // at least 32 codes per thread (each thread also writes a (nd+1) x nf slice)
-    std::vector<uint64_t> codes(n);
+    // walkers in proportion to the codes, at least 32 codes each (a walker also leaves
+    // a (nd + 1) x nf slice), whole warps of 8, one wave of resident warps
     double total = 0.0;
-    for (int p = 0; p < n; ++p) {
-      codes[p] = sw[p].total_codes;
-      total += (double)codes[p];
-    }
-    const int64_t resident = sweep_resident_threads(nf, SweepOp::kGrad, cx->sm_count);
-    const int64_t want = std::max<int64_t>(n, std::min<int64_t>(resident, (int64_t)(total / 32.0)));
-    // whole groups of 32 threads per sweep (the gradient slices interleave by lane),
-    // rounded down so the launch stays within one wave of resident threads
-    std::vector<int64_t> nthr(n);
-    for (int p = 0; p < n; ++p) {
-      const int64_t t = (int64_t)std::floor(want * (double)codes[p] / total);
-      nthr[p] = std::max<int64_t>(32, t / 32 * 32);
-    }
+    for (const HostSweep& h : sw) total += (double)h.total_codes;
+    const int64_t resident = grad_resident_walkers(nf, cx->sm_count);
+    const double want = std::max<double>(n, std::min<double>((double)resident, total / 32.0));
+    const int F = grad_factors(nf);
     std::vector<SweepProblem> probs(n);
-    int64_t pool_n = 0, threads = 0, gparts = 0;
-    int row = 0;
-    for (int p = 0; p < n; ++p) row = std::max(row, (sw[p].nd + 1) * nf);
+    int64_t pool_n = 0, walkers = 0, gparts = 0;
+    int row = 0;  // entries of the largest sweep's gradient
     for (int p = 0; p < n; ++p) {
       const HostSweep& h = sw[p];
       SweepProblem& Pp = probs[p];
-      memset(&Pp, 0, sizeof(Pp));
-      Pp.nd = h.nd;
-      Pp.nb = h.nb;
-      Pp.nf = h.nf;
-      Pp.kind = h.kind;
-      Pp.parity0 = h.parity0;
-      Pp.fx = h.fx;
-      Pp.has_base = h.has_base;
+      const int64_t share = (int64_t)std::floor(want * (double)h.total_codes / total);
+      describe_sweep(h, std::max<int64_t>(8, share / 8 * 8), 1, Pp);
       Pp.out_idx = p;
-      Pp.n_codes = (int64_t)h.total_codes;
-      Pp.thread_begin = threads;
-      Pp.n_threads = nthr[p];
+      Pp.thread_begin = walkers;
       Pp.mat_off = pool_n;
       pool_n += (int64_t)h.D.size();
       Pp.base_off = pool_n;
       pool_n += (int64_t)h.base.size();
-      Pp.fixed_digit = (h.fixed_mode >= 0) ? 1 : 0;
       Pp.part_off = gparts;
-      Pp.scale = h.scale;
-      for (int i = 0; i < h.nd; ++i) Pp.mult[i] = h.mult[i];
-      threads += nthr[p];
-      gparts += nthr[p] * (int64_t)(h.nd + Pp.fixed_digit) * nf;  // nthr is a multiple of 32
+      const int rows = h.nd + Pp.fixed_digit;
+      row = std::max(row, rows * F);
+      walkers += Pp.n_threads;
+      gparts += Pp.n_threads / 8 * grad_slice(rows, nf);
     }
     size_t off = 0;
     const size_t o_probs = off; off = align_up(off + sizeof(SweepProblem) * n, 256);
@@ -887,7 +891,7 @@ int boss_perm_grad_batch(const double* matrix, int32_t m, const int32_t* input_s
     const size_t out_g = (size_t)n * row, out_p = (size_t)n;
     if ((st = ensure(cx->plans, arena_bytes))) return st;
     if ((st = ensure(cx->gpart, sizeof(double2) * std::max<int64_t>(gparts, 1)))) return st;
-    if ((st = ensure(cx->pperm, sizeof(double2) * std::max<int64_t>(threads, 1)))) return st;
+    if ((st = ensure(cx->pperm, sizeof(double2) * std::max<int64_t>(walkers / 8, 1)))) return st;
     if ((st = ensure(cx->out, sizeof(double2) * (out_g + out_p)))) return st;
     if ((st = ensure_pinned(cx, std::max(arena_bytes, sizeof(double2) * (out_g + out_p))))) return st;
     char* h = (char*)cx->pinned;
@@ -900,18 +904,13 @@ int boss_perm_grad_batch(const double* matrix, int32_t m, const int32_t* input_s
     char* d = (char*)cx->plans.ptr;
     cudaError_t e = cudaMemcpyAsync(d, h, arena_bytes, cudaMemcpyHostToDevice, cx->stream);
     if (e != cudaSuccess) return fail_cuda(e, "H2D gradient sweeps");
-    SweepLaunch L;
-    L.probs = (const SweepProblem*)(d + o_probs);
-    L.n_probs = n;
-    L.pool = (const longlong2*)(d + o_pool);
-    L.total_threads = threads;
-    L.partials = (double2*)cx->gpart.ptr;
-    L.partials2 = (double2*)cx->pperm.ptr;
-    L.grid = (int)((threads + 63) / 64);
-    if ((e = launch_sweep(nf, SweepOp::kGrad, L, cx->stream)) != cudaSuccess) return fail_cuda(e, "gradient sweep");
-    double2* dout = (double2*)cx->out.ptr;
-    if ((e = launch_grad_reduce(L.probs, n, L.partials, L.partials2, dout, dout + out_g, row, cx->stream)) !=
+    const SweepProblem* dp = (const SweepProblem*)(d + o_probs);
+    double2 *gpart = (double2*)cx->gpart.ptr, *ppart = (double2*)cx->pperm.ptr;
+    if ((e = launch_grad_sweep(nf, dp, n, (const longlong2*)(d + o_pool), walkers, gpart, ppart, cx->stream)) !=
         cudaSuccess)
+      return fail_cuda(e, "gradient sweep");
+    double2* dout = (double2*)cx->out.ptr;
+    if ((e = launch_grad_reduce(nf, dp, n, gpart, ppart, dout, dout + out_g, row, cx->stream)) != cudaSuccess)
       return fail_cuda(e, "gradient reduce");
     e = cudaMemcpyAsync(cx->pinned, dout, sizeof(double2) * (out_g + out_p), cudaMemcpyDeviceToHost, cx->stream);
     if (e != cudaSuccess) return fail_cuda(e, "D2H gradients");
@@ -930,7 +929,7 @@ int boss_perm_grad_batch(const double* matrix, int32_t m, const int32_t* input_s
           const int fmode = hs.factor_mode[f];
           const int j = hs.digits_are_outputs ? bmode : fmode;  // output mode
           const int i = hs.digits_are_outputs ? fmode : bmode;  // input mode
-          const double2 v = hg[(size_t)p * row + (size_t)b * nf + f];
+          const double2 v = hg[(size_t)p * row + (size_t)b * F + f];
           gk[(size_t)j * len + i].x += v.x;
           gk[(size_t)j * len + i].y += v.y;
         }

@@ -11,7 +11,7 @@
 
 namespace boss {
 
-enum class SweepOp { kPerm = 0, kMinors = 1, kGrad = 2, kMinorsFF = 3, kPermFF = 4 };  // FF: float pairs
+enum class SweepOp { kPerm = 0, kMinors = 1, kMinorsFF = 2, kPermFF = 3 };  // FF: float pairs
 
 // Everything one sweep launch needs (device pointers).
 struct SweepLaunch {
@@ -20,7 +20,6 @@ struct SweepLaunch {
   const longlong2* pool = nullptr;
   int64_t total_threads = 0;
   double2* partials = nullptr;
-  double2* partials2 = nullptr;  // gradients: per-warp permanent partials
   int grid = 1;
   int rows = 32;  // all-minors: shared-memory rows of minors per thread (nd + held digit, at most 32)
   bool quad = false;  // permanents, all-minors in FP64: the four-codes-per-step kernels (boss_quad.cuh)
@@ -40,14 +39,25 @@ int64_t sweep_resident_minors(int nf, int rows, int sm_count, bool ff = false);
 cudaError_t prepare_quad_kernels();
 int64_t quad_resident_walkers(int nf, int rows, bool minors, int sm_count);
 cudaError_t launch_quad_sweep(int nf, bool minors, const SweepLaunch& L, cudaStream_t st);
+// Gradient sweeps (boss_grad.cu) of nf factors: walkers resident at once; the sweep
+// (grad_slice entries of gpart per warp of 8 walkers, one of ppart) and the
+// reduction (grad_out: per sweep row_stride entries, digit by digit, factor by
+// factor with the factor count padded to a multiple of 4).
+cudaError_t prepare_grad_kernels();
+int64_t grad_resident_walkers(int nf, int sm_count);
+inline int grad_factors(int nf) { return (nf + 3) / 4 * 4; }
+inline int64_t grad_slice(int rows, int nf) { return (int64_t)rows * grad_factors(nf) * 8; }
+cudaError_t launch_grad_sweep(int nf, const SweepProblem* probs, int n_probs, const longlong2* pool, int64_t walkers,
+                              double2* gpart, double2* ppart, cudaStream_t st);
+cudaError_t launch_grad_reduce(int nf, const SweepProblem* probs, int n_probs, const double2* gpart,
+                               const double2* ppart, double2* grad_out, double2* perm_out, int row_stride,
+                               cudaStream_t st);
 // Whether the float-pair all-minors / single-permanent kernel exists for nf factors.
 bool minors_ff_available(int nf);
 bool perm_ff_available(int nf);
 cudaError_t launch_sweep(int nf, SweepOp op, const SweepLaunch& L, cudaStream_t st);
 cudaError_t launch_perm_reduce(const SweepProblem* probs, int n_probs, const double2* partials, double2* out,
                                cudaStream_t st, bool ff = false);
-cudaError_t launch_grad_reduce(const SweepProblem* probs, int n_probs, const double2* gpart, const double2* ppart,
-                               double2* grad_out, double2* perm_out, int row_stride, cudaStream_t st);
 // rows: the most digits (held one included) of a sweep.
 cudaError_t launch_minors_reduce(const SweepProblem* probs, int n_probs, int rows, const double2* partials,
                                  double2* out, int nd_max, cudaStream_t st, bool ff = false);
@@ -78,9 +88,10 @@ int range_align(int64_t n_codes, int64_t n_threads, int nb);
 constexpr int kQuadMinFactors = 2;
 constexpr int kQuadMinMinorFactors = 14;
 enum RowLayout : int {
-  kRowsPlain = 0,   // D (float pairs, gradients)
+  kRowsPlain = 0,   // D (float pairs)
   kRowsPacked = 1,  // u = -D / 2 packed: the templated FP64 kernels
-  kRowsQuad = 2     // boss_quad.cuh: two binary digits and two factors at least
+  kRowsQuad = 2,    // boss_quad.cuh: two binary digits and two factors at least
+  kRowsGrad = 3     // boss_grad.cu
 };
 struct HostSweep {
   int layout = kRowsPlain;
@@ -88,7 +99,6 @@ struct HostSweep {
   int parity0 = 0;
   int nd = 0, nb = 0, nf = 0;
   int has_base = 0;
-  int fx = 56;                 // fraction bits shared by all factors (gradients)
   int fx_sum = 0;              // sum of the factors' own fraction bits (permanents, all-minors)
   uint8_t mult[kMaxDigits] = {};
   std::vector<longlong2> D;     // nd x nf; kRowsQuad: (nd - 2) x quad_width(nf)
@@ -165,7 +175,7 @@ int small_perm_batch(Context* cx, const double* matrix, int m, int len, const in
 // special-cases.
 // What the sweep is planned for: any kernel, float pairs where they are chosen; the
 // templated FP64 kernels only; FP64 always (the allocation-free entry point); the
-// gradient kernel (one fixed-point scale for all factors).
+// gradient kernel.
 enum PlanFor : int { kPlanAny = 0, kPlanTemplated = 1, kPlanFP64 = 2, kPlanGrad = 3 };
 int plan_permanent(const double* U, int m, const int32_t* S, const int32_t* T, int len, int variant, HostSweep& hs,
                    bool& needs_sweep, double2& value, PlanFor plan = kPlanAny);

@@ -39,36 +39,13 @@ struct QuadState {
   }
 };
 
-// The walk over the outer digits: the reflected mixed-radix Gray code changes one
-// digit by one per step, so the state moves by one row and is decoded only once.
-struct QuadWalk {
-  uint64_t g;      // the binary digits
-  uint32_t parity; // sign parity
-  double w;        // binomial weight of the multi-valued digits
-  uint8_t r[kMaxDigits];  // their values (entries nb .. nd - 1; local memory)
-};
-
 // The walk at outer code t, and this lane's state.
 template <int S>
 __device__ __forceinline__ void quad_decode(const SweepProblem& P, const longlong2* __restrict__ rows,
                                             const longlong2* __restrict__ base, uint64_t t, QuadState<S>& st, QuadWalk& k) {
   constexpr int W = 4 * S;
   const int nb = P.nb;
-  k.g = (t ^ (t >> 1));
-  if (nb < 64) k.g &= (1ull << nb) - 1ull;
-  k.parity = (uint32_t)P.parity0 ^ ((uint32_t)__popcll((long long)k.g) & 1u);
-  k.w = 1.0;
-  uint64_t th = t >> nb;
-  for (int i = nb; i < P.nd; ++i) {
-    const uint32_t mu = P.mult[i];
-    const uint64_t b = (uint64_t)mu + 1ull, q = th / b;
-    const uint32_t dgt = (uint32_t)(th - q * b);
-    th = q;
-    const uint32_t r = (q & 1ull) ? (mu - dgt) : dgt;
-    k.r[i] = (uint8_t)r;
-    k.parity ^= r & 1u;
-    if (r) k.w *= binom_small((int)mu, (int)r);
-  }
+  quad_walk_at(P, t, k);
 #pragma unroll
   for (int i = 0; i < QuadState<S>::kRounds; ++i)
 #pragma unroll
@@ -89,33 +66,6 @@ __device__ __forceinline__ void quad_decode(const SweepProblem& P, const longlon
   for (uint64_t bits = k.g; bits; bits &= bits - 1ull) add(__ffsll((long long)bits) - 1, -2);
   for (int d = nb; d < P.nd; ++d)
     if (k.r[d]) add(d, -2 * (int)k.r[d]);
-}
-
-// The step to outer code t: the digit that moves, and by how much (+-1).
-__device__ __forceinline__ int quad_next(const SweepProblem& P, uint64_t t, QuadWalk& k, int& dr) {
-  const int nb = P.nb;
-  int i = __ffsll((long long)t) - 1;
-  k.parity ^= 1u;
-  if (i < nb) {
-    dr = ((k.g >> i) & 1ull) ? -1 : 1;
-    k.g ^= 1ull << i;
-    return i;
-  }
-  uint64_t th = t >> nb, q;
-  uint32_t mu, dgt;
-  for (i = nb;; ++i) {  // the lowest digit whose plain value is not back at zero
-    mu = P.mult[i];
-    q = th / (mu + 1ull);
-    dgt = (uint32_t)(th - q * (mu + 1ull));
-    if (dgt || i + 1 >= P.nd) break;
-    th = q;
-  }
-  const int r = (int)((q & 1ull) ? (mu - dgt) : dgt), before = k.r[i];
-  dr = r - before;
-  k.r[i] = (uint8_t)r;
-  // C(mu, r) from C(mu, before), exact while the weight is below 2^53
-  k.w = dr > 0 ? k.w * (double)(mu - (uint32_t)before) / (double)r : k.w * (double)before / (double)(mu - (uint32_t)r);
-  return i;
 }
 
 // Moves the state by sg times a row (sg = 0: as it is) and multiplies this lane's
@@ -161,29 +111,6 @@ __device__ __forceinline__ void quad_eval(QuadState<S>& st, longlong2* xbuf, con
   ls += __shfl_xor_sync(0xffffffffu, ls, 1);
   ls += __shfl_xor_sync(0xffffffffu, ls, 2);
   e = quad_exponent(e0, ls, S) + ps;
-}
-
-// This lane's walker and its range; lanes past the launch's last walker take the
-// last one's problem with an empty range, so that whole warps stay together.
-struct QuadRange {
-  int64_t q;       // the walker within its sweep
-  int64_t a, len;  // its outer codes
-  int64_t most;    // the longest range in the warp
-  bool live;
-};
-__device__ __forceinline__ QuadRange quad_range(const SweepProblem& P, int64_t walker, bool live) {
-  QuadRange r;
-  r.live = live;
-  r.q = walker - P.thread_begin;
-  thread_range_aligned(P, r.q, P.align, r.a, r.len);
-  if (!live) r.len = 0;
-  r.most = r.len;
-#pragma unroll
-  for (int o = 16; o >= 4; o >>= 1) {
-    const int64_t x = __shfl_xor_sync(0xffffffffu, r.most, o);
-    r.most = x > r.most ? x : r.most;
-  }
-  return r;
 }
 
 // One permanent per sweep problem; every group of walkers writes one complex partial.

@@ -23,8 +23,6 @@
 //   * the products are formed in block floating point on the integer pipe (62-bit
 //     mantissas, accumulate_product_bf), rounded to FP64 once per code;
 //   * sign flips are integer XORs on the sign bit.
-// (The gradient sweep multiplies on the FP64 pipe, its factors converted with
-// integer instructions, fx_to_double.)
 //
 // Work split: the codes of a sweep are cut into one contiguous range per thread
 // (lengths differ by at most one), each thread decodes its start code in closed
@@ -52,8 +50,7 @@ struct SweepProblem {
   int32_t nf;        // product factors
   int32_t kind;      // SweepKind
   int32_t parity0;   // sign parity of the r = 0 code
-  int32_t fx;        // permanents, all-minors: minus the sum of the factors' fraction bits (every factor has
-                     // its own scale 2^fx_f); gradients: the fraction bits shared by all factors
+  int32_t fx;        // minus the sum of the factors' fraction bits (every factor has its own scale 2^fx_f)
   int32_t has_base;  // base sums present
   int32_t out_idx;   // result index
   int64_t n_codes;       // codes in the sweep (low = 2: steps of four codes)
@@ -94,22 +91,6 @@ __host__ __device__ __forceinline__ long long unpack_row(long long v) {
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ double xor_sign(double x, uint32_t neg_mask) {
   return __hiloint2double(__double2hiint(x) ^ (int)neg_mask, __double2loint(x));
-}
-
-// x * 2^-fx as a double, rounded to nearest (ties away from zero), using integer
-// instructions only.  bias_exp = 1023 + 63 - fx.  Requires the result to be a
-// normal double or zero.
-__device__ __forceinline__ double fx_to_double(long long x, int bias_exp) {
-  const unsigned long long sgn = (unsigned long long)(x >> 63);
-  const unsigned long long ax = ((unsigned long long)x ^ sgn) - sgn;
-  const int lz = __clzll((long long)ax);
-  const unsigned long long y = ax << (lz & 63);
-  const unsigned long long yr = y + 0x400ull;
-  const unsigned long long carry = (yr < y) ? 1ull : 0ull;
-  const unsigned long long mant = (yr >> 11) & 0xFFFFFFFFFFFFFull;
-  const unsigned long long e = (unsigned long long)(bias_exp - lz) + carry;
-  const unsigned long long bits = (sgn << 63) | (e << 52) | mant;
-  return __longlong_as_double(ax ? (long long)bits : 0ll);
 }
 
 // Compiler-only barrier: keeps the scheduler from hoisting all of a row's loads
@@ -229,23 +210,7 @@ __device__ __forceinline__ void decode_code(const SweepProblem& P, const longlon
   }
 }
 
-// Binary digit i moves from `bit` to 1 - bit: sums +/-= D_i.
-template <int NF>
-__device__ __forceinline__ void flip_binary(const longlong2* __restrict__ D, int i, uint32_t bit, long long (&sr)[NF],
-                                            long long (&si)[NF]) {
-  const longlong2* row = D + (size_t)i * NF;
-  const long long sgn = bit ? -1ll : 0ll;  // -x = (x ^ -1) + 1: one three-input add per word
-  const long long one = (long long)bit;
-#pragma unroll
-  for (int f = 0; f < NF; ++f) {
-    if (f > 0 && (f & 7) == 0) load_fence();
-    const longlong2 d = row[f];
-    sr[f] = sr[f] + (d.x ^ sgn) + one;
-    si[f] = si[f] + (d.y ^ sgn) + one;
-  }
-}
-
-// The same with packed rows.
+// Binary digit i moves from `bit` to 1 - bit: sums +/-= D_i (packed rows).
 template <int NF>
 __device__ __forceinline__ void flip_packed(const longlong2* __restrict__ D, int i, uint32_t bit, long long (&sr)[NF],
                                             long long (&si)[NF]) {
