@@ -9,12 +9,11 @@
 //     p(T) = [ sum_S' |perm(U[T, S'])|^2 / prod_i S'_i! * mult(S') ] / l! / C(n, l) * l! / prod_i T_i!
 // with mult(S') = prod_i C(S_i, S_i - S'_i); theboss evaluates one outcome at a
 // time (the uniform-loss calculator maps outcomes over a process pool,
-// bs_exact_distribution_with_uniform_losses.py:62-71).  Here every (lossy input,
-// outcome) pair of a particle count l is one GPU thread:
-//   * lossy_pair_kernel<L> (L = l <= kDistMaxL): the Glynn permanent of the L x L
-//     matrix (rows: the outcome's particles, columns: the lossy input's particles)
-//     over the 2^(L-1) sign vectors with the first column's sign fixed, in
-//     registers, then |perm|^2, theboss's divisions and the multiplicity;
+// bs_exact_distribution_with_uniform_losses.py:62-71).  Here, for every particle
+// count l <= kDistMaxL:
+//   * lossy_table_kernel: the row sums of every (lossy input, sign vector);
+//   * lossy_walk_kernel: the Glynn permanents of every (lossy input, outcome) from
+//     them, then |perm|^2, theboss's divisions and the multiplicity;
 //   * lossy_outcome_kernel: per outcome, the sum over lossy inputs in theboss's
 //     order and the normalisation, with theboss's operation order.
 // Larger l goes through the sweep engine (one Glynn sweep per pair, many threads
@@ -27,6 +26,7 @@
 #include <cmath>
 #include <mutex>
 #include <string>
+#include <type_traits>
 #include <unordered_map>
 #include <vector>
 
@@ -90,13 +90,6 @@ __device__ __forceinline__ double2 glynn_small(const double2* __restrict__ U, in
   }
   const double s = ldexp(1.0, -(L - 1));
   return make_double2(accr * s, acci * s);
-}
-
-template <int L>
-__device__ __forceinline__ double glynn_abs2(const double2* __restrict__ U, int m, const int (&row)[L],
-                                            const int (&col)[L]) {
-  const double2 p = glynn_small<L>(U, m, row, col);
-  return fma(p.x, p.x, p.y * p.y);
 }
 
 // A row's fixed-point scale for sums of at most `terms` of its entries: the fraction
@@ -232,34 +225,177 @@ __global__ void __launch_bounds__(128) small_perm_kernel(const longlong2* __rest
   if (mine == 0 && at < count) out[k] = make_double2(ar, ai);
 }
 
-// One thread per (lossy input k, outcome o); the layout [k][o] lets the outcome
-// kernel read coalesced.
+// ---------------------------------------------------------------------------
+// All (lossy input, outcome) permanents of one particle count L.
+//
+// For a lossy input and a sign vector d (first sign +) the row sums V[o] =
+// sum_b d_b U[o][col b] depend on the output mode o only, so they are tabulated, and
+// an outcome's product over its particles' modes (in mode order) shares its leading
+// factors with the outcome before it: outcomes in lexicographic order need 1 to 2
+// products each instead of L - 1 products and L row updates.  A lane takes one
+// (input, sign vector), a warp 32 of them (several sign vectors of one input from
+// L = 6 on, several inputs below), and walks a chunk of outcomes with the partial
+// products in registers: the same control flow in every lane.
+// Bound by the FP64 pipe (4 instructions per product, 2 per outcome for the sum over
+// the lanes).  8 photons in 16 modes, all 735,471 outcomes: 16.5 -> 4.4 ms, FP64 pipe
+// 85 % busy, against one thread per (input, outcome) walking all sign vectors.
+// ---------------------------------------------------------------------------
+constexpr int kWalkChunk = 128;  // outcomes per warp at most (a multiple of 8)
+
+// Every outcome's particles in mode order (bytes 0 .. L - 1) and how many leading
+// ones it shares with the outcome before it (byte 15).
+__global__ void lossy_rows_kernel(const uint8_t* __restrict__ occ, int m, int64_t O, uint4* __restrict__ rows) {
+  const int64_t o = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (o >= O) return;
+  uint32_t w[4] = {0, 0, 0, 0};
+  const uint8_t* t = occ + o * m;
+  const uint8_t* before = o > 0 ? t - m : nullptr;
+  int a = 0, same = 0;
+  bool equal = before != nullptr;
+  for (int i = 0; i < m; ++i) {
+    const int c = t[i];
+    if (equal) {
+      same += min(c, (int)before[i]);
+      equal = c == before[i];
+    }
+    for (int k = 0; k < c && a < 15; ++k, ++a) w[a >> 2] |= (uint32_t)i << (8 * (a & 3));
+  }
+  w[3] |= (uint32_t)same << 24;
+  rows[o] = make_uint4(w[0], w[1], w[2], w[3]);
+}
+
+// V[(combo / 32 * m + row) * 32 + combo % 32], combo = input * 2^(L-1) + sign vector.
+__global__ void lossy_table_kernel(const double2* __restrict__ U, int m, int L, const uint8_t* __restrict__ cols,
+                                   int K, int64_t combos, double2* __restrict__ V) {
+  const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= combos * m) return;
+  const int64_t combo = e / ((int64_t)32 * m) * 32 + (e & 31);
+  const int row = (int)((e >> 5) % m);
+  const int64_t k = combo >> (L - 1);
+  double x = 0.0, y = 0.0;
+  if (k < K) {
+    const uint32_t d = (uint32_t)combo & ((1u << (L - 1)) - 1u);
+    for (int b = 0; b < L; ++b) {
+      const double2 u = U[(size_t)row * m + cols[k * L + b]];
+      const bool neg = b > 0 && ((d >> (b - 1)) & 1u);
+      x += neg ? -u.x : u.x;
+      y += neg ? -u.y : u.y;
+    }
+  }
+  V[e] = make_double2(x, y);
+}
+
+// One warp per (group of 32 combos of equal input or of several inputs, chunk of
+// outcomes); from L = 6 on a group is one input and its 2^(L-6) blocks of 32 sign
+// vectors are walked one after the other.
 template <int L>
-__global__ void __launch_bounds__(128) lossy_pair_kernel(const double2* __restrict__ U, int m,
-                                                         const uint8_t* __restrict__ in_cols,  // [K][L]
+__global__ void __launch_bounds__(128) lossy_walk_kernel(const double2* __restrict__ V, int m,
+                                                         const uint4* __restrict__ rows, int64_t O, int K, int groups,
                                                          const double* __restrict__ in_div,    // [K][kDistMaxDiv]
                                                          const int* __restrict__ in_ndiv,      // [K]
                                                          const double* __restrict__ in_mult,   // [K]
-                                                         int K, const uint8_t* __restrict__ out_occ,  // [O][m]
-                                                         int64_t O, double* __restrict__ terms) {     // [K][O]
-  const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= (int64_t)K * O) return;
-  const int k = (int)(idx / O);
-  const int64_t o = idx - (int64_t)k * O;
-  int row[L], col[L];
+                                                         int chunk, double* __restrict__ terms) {  // [K][O]
+  constexpr int kBlocks = L >= 6 ? 1 << (L - 6) : 1;  // blocks of 32 sign vectors per input
+  constexpr int kLanes = L >= 6 ? 32 : 1 << (L - 1);  // lanes of one input
+  __shared__ double2 buf_s[4][8 * 33];
+  __shared__ double2 acc_s[4][kWalkChunk];
+  const int wp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int64_t chunks = (O + chunk - 1) / chunk;
+  const int64_t task = (int64_t)blockIdx.x * 4 + wp;
+  if (task >= chunks * groups) return;  // whole warps
+  const int g = (int)(task / chunks);
+  const int64_t o0 = (task - (int64_t)g * chunks) * chunk;
+  const int n = (int)min((int64_t)chunk, O - o0);
+  double2* buf = buf_s[wp];
+  double2* acc = acc_s[wp];
+  const double scale = 1.0 / (double)(1u << (L - 1));
+  auto term = [&](double2 p, int k) {
+    const double re = p.x * scale, im = p.y * scale;
+    double v = fma(re, re, im * im);
+    // bs_distribution_calculator_with_fixed_losses.py:137-142, same operation order
+    const int nd = in_ndiv[k];
+    for (int d = 0; d < nd; ++d) v /= in_div[(size_t)k * kDistMaxDiv + d];
+    return v * in_mult[k];
+  };
+  for (int j = 0; j < kBlocks; ++j) {
+    const int64_t block = L >= 6 ? (int64_t)g * kBlocks + j : g;
+    const double2* Vg = V + block * 32 * m + lane;
+    const uint32_t d = L >= 6 ? (uint32_t)(j * 32 + lane) : (uint32_t)(lane & (kLanes - 1));
+    const uint32_t neg = (__popc(d) & 1) << 31;
+    double2 P[L];
+    for (int q = 0; q < n; ++q) {
+      const uint4 r = __ldg(rows + o0 + q);
+      const uint32_t w[4] = {r.x, r.y, r.z, r.w};
+      const int c = q > 0 ? (int)(r.w >> 24) : 0;
+      auto step = [&](auto index) {
+        constexpr int a = decltype(index)::value;
+        if constexpr (a < L) {
+          const double2 v = __ldg(Vg + (size_t)((w[a >> 2] >> (8 * (a & 3))) & 255u) * 32);
+          if constexpr (a == 0) {
+            P[0] = make_double2(xor_sign(v.x, neg), xor_sign(v.y, neg));
+          } else {
+            const double2 p = P[a - 1];
+            P[a] = make_double2(fma(p.x, v.x, -(p.y * v.y)), fma(p.x, v.y, p.y * v.x));
+          }
+        }
+      };
+      // a jump into the chain, not a condition per step: predicated-off FP64
+      // instructions would hold the pipe all the same
+      switch (c) {
+        case 0: step(std::integral_constant<int, 0>{}); [[fallthrough]];
+        case 1: step(std::integral_constant<int, 1>{}); [[fallthrough]];
+        case 2: step(std::integral_constant<int, 2>{}); [[fallthrough]];
+        case 3: step(std::integral_constant<int, 3>{}); [[fallthrough]];
+        case 4: step(std::integral_constant<int, 4>{}); [[fallthrough]];
+        case 5: step(std::integral_constant<int, 5>{}); [[fallthrough]];
+        case 6: step(std::integral_constant<int, 6>{}); [[fallthrough]];
+        case 7: step(std::integral_constant<int, 7>{}); [[fallthrough]];
+        case 8: step(std::integral_constant<int, 8>{}); [[fallthrough]];
+        case 9: step(std::integral_constant<int, 9>{}); break;
+        default: break;
+      }
+      double2 x = P[L - 1];
+      if constexpr (L < 6) {
 #pragma unroll
-  for (int a = 0; a < L; ++a) col[a] = in_cols[(size_t)k * L + a];
-  {  // the outcome's particles, in mode order
-    const uint8_t* occ = out_occ + o * m;
-    int a = 0;
-    for (int i = 0; i < m && a < L; ++i)
-      for (int c = occ[i]; c > 0 && a < L; --c) row[a++] = i;
+        for (int o = 1; o < kLanes; o <<= 1) {
+          x.x += __shfl_xor_sync(0xffffffffu, x.x, o);
+          x.y += __shfl_xor_sync(0xffffffffu, x.y, o);
+        }
+        const int k = g * (32 / kLanes) + lane / kLanes;
+        if ((lane & (kLanes - 1)) == 0 && k < K) terms[(size_t)k * O + o0 + q] = term(x, k);
+      } else {
+        // eight outcomes at a time: four lanes add up eight combos each of one outcome
+        buf[(q & 7) * 33 + lane] = x;
+        if ((q & 7) == 7 || q + 1 == n) {
+          __syncwarp();
+          const int oo = lane >> 2, part = lane & 3, at = (q & ~7) + oo;
+          double2 s = make_double2(0.0, 0.0);
+          if (at < n) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              const double2 v = buf[oo * 33 + part * 8 + i];
+              s.x += v.x;
+              s.y += v.y;
+            }
+          }
+#pragma unroll
+          for (int o = 1; o < 4; o <<= 1) {
+            s.x += __shfl_xor_sync(0xffffffffu, s.x, o);
+            s.y += __shfl_xor_sync(0xffffffffu, s.y, o);
+          }
+          if (part == 0 && at < n) {
+            if (j > 0) s = make_double2(s.x + acc[at].x, s.y + acc[at].y);
+            acc[at] = s;
+          }
+          __syncwarp();
+        }
+      }
+    }
   }
-  double v = glynn_abs2<L>(U, m, row, col);
-  // bs_distribution_calculator_with_fixed_losses.py:137-142, same operation order
-  const int nd = in_ndiv[k];
-  for (int d = 0; d < nd; ++d) v /= in_div[(size_t)k * kDistMaxDiv + d];
-  terms[idx] = v * in_mult[k];
+  if constexpr (L >= 6) {
+    __syncwarp();
+    for (int q = lane; q < n; q += 32) terms[(size_t)g * O + o0 + q] = term(acc[q], g);
+  }
 }
 
 __global__ void lossy_outcome_kernel(const double* __restrict__ terms, int K, int64_t O, int m,
@@ -283,6 +419,8 @@ __global__ void lossy_outcome_kernel(const double* __restrict__ terms, int K, in
 // ---------------------------------------------------------------------------
 // Host side
 // ---------------------------------------------------------------------------
+static size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
+
 static double factorial_d(int k) {  // exact up to 20!, then the nearest double of the product
   if (k <= 20) {
     uint64_t f = 1;
@@ -368,75 +506,99 @@ static void particle_list(const int32_t* occ, int m, uint8_t* out) {
 }
 
 template <int L>
-static cudaError_t launch_pairs(const double2* U, int m, const uint8_t* cols, const double* div, const int* ndiv,
-                                const double* mult, int K, const uint8_t* rows, int64_t O, double* terms,
-                                cudaStream_t s) {
-  const int64_t n = (int64_t)K * O;
-  lossy_pair_kernel<L><<<(unsigned)((n + 127) / 128), 128, 0, s>>>(U, m, cols, div, ndiv, mult, K, rows, O, terms);
+static cudaError_t launch_walk(const double2* V, int m, const uint4* rows, int64_t O, int K, int groups,
+                               const double* div, const int* ndiv, const double* mult, double* terms,
+                               int sm_count, cudaStream_t s) {
+  // chunks of outcomes that leave about 16 warps per SM: a walk is serial (a chunk of
+  // 128 takes 80 us), so a few outcomes are spread over more warps
+  const int64_t want = O * groups / ((int64_t)sm_count * 16);
+  const int chunk = (int)std::min<int64_t>(kWalkChunk, std::max<int64_t>(8, want / 8 * 8));
+  const int64_t tasks = (O + chunk - 1) / chunk * groups;
+  lossy_walk_kernel<L><<<(unsigned)((tasks + 3) / 4), 128, 0, s>>>(V, m, rows, O, K, groups, div, ndiv, mult,
+                                                                chunk, terms);
   return cudaGetLastError();
 }
 
-static cudaError_t launch_pairs_l(int l, const double2* U, int m, const uint8_t* cols, const double* div,
-                                  const int* ndiv, const double* mult, int K, const uint8_t* rows, int64_t O,
-                                  double* terms, cudaStream_t s) {
+static cudaError_t launch_walk_l(int l, const double2* V, int m, const uint4* rows, int64_t O, int K, int groups,
+                                 const double* div, const int* ndiv, const double* mult, double* terms,
+                                 int sms, cudaStream_t s) {
   switch (l) {
-    case 1: return launch_pairs<1>(U, m, cols, div, ndiv, mult, K, rows, O, terms, s);
-    case 2: return launch_pairs<2>(U, m, cols, div, ndiv, mult, K, rows, O, terms, s);
-    case 3: return launch_pairs<3>(U, m, cols, div, ndiv, mult, K, rows, O, terms, s);
-    case 4: return launch_pairs<4>(U, m, cols, div, ndiv, mult, K, rows, O, terms, s);
-    case 5: return launch_pairs<5>(U, m, cols, div, ndiv, mult, K, rows, O, terms, s);
-    case 6: return launch_pairs<6>(U, m, cols, div, ndiv, mult, K, rows, O, terms, s);
-    case 7: return launch_pairs<7>(U, m, cols, div, ndiv, mult, K, rows, O, terms, s);
-    case 8: return launch_pairs<8>(U, m, cols, div, ndiv, mult, K, rows, O, terms, s);
-    case 9: return launch_pairs<9>(U, m, cols, div, ndiv, mult, K, rows, O, terms, s);
-    case 10: return launch_pairs<10>(U, m, cols, div, ndiv, mult, K, rows, O, terms, s);
+    case 1: return launch_walk<1>(V, m, rows, O, K, groups, div, ndiv, mult, terms, sms, s);
+    case 2: return launch_walk<2>(V, m, rows, O, K, groups, div, ndiv, mult, terms, sms, s);
+    case 3: return launch_walk<3>(V, m, rows, O, K, groups, div, ndiv, mult, terms, sms, s);
+    case 4: return launch_walk<4>(V, m, rows, O, K, groups, div, ndiv, mult, terms, sms, s);
+    case 5: return launch_walk<5>(V, m, rows, O, K, groups, div, ndiv, mult, terms, sms, s);
+    case 6: return launch_walk<6>(V, m, rows, O, K, groups, div, ndiv, mult, terms, sms, s);
+    case 7: return launch_walk<7>(V, m, rows, O, K, groups, div, ndiv, mult, terms, sms, s);
+    case 8: return launch_walk<8>(V, m, rows, O, K, groups, div, ndiv, mult, terms, sms, s);
+    case 9: return launch_walk<9>(V, m, rows, O, K, groups, div, ndiv, mult, terms, sms, s);
+    case 10: return launch_walk<10>(V, m, rows, O, K, groups, div, ndiv, mult, terms, sms, s);
     default: return cudaErrorInvalidValue;
   }
 }
 
-// All outcomes of one particle count l (1 <= l <= kDistMaxL) on the per-thread path.
-static int group_small(Context* cx, const double* matrix, int m, int n, int l, const LossyInputs& LI,
-                       const std::vector<const int32_t*>& outs, double* prob_out, const std::vector<int>& where,
-                       float* kernel_ms) {
-  const int K = (int)LI.occ.size();
-  const int64_t O = (int64_t)outs.size();
-  auto al = [](size_t x) { return (x + 255) & ~(size_t)255; };
+// The outcomes of the particle counts 1 <= l <= kDistMaxL, grouped: count l's rows
+// are first[l] .. first[l] + size[l] - 1 of `occ` (uint8, m per row) and its
+// probabilities go to the same places of `prob` (both on the device).
+struct SmallGroups {
+  const uint8_t* occ;
+  double* prob;
+  int64_t first[kDistMaxL + 1], size[kDistMaxL + 1];
+};
+
+constexpr int64_t kTableBytes = (int64_t)64 << 20;  // the row-sum table of one launch
+
+// Tables and kernels of all groups, queued on the library's stream.
+static int queue_small_groups(Context* cx, const double* matrix, int m, int n, const int32_t* initial_state,
+                              const SmallGroups& G, float* kernel_ms) {
+  std::vector<LossyInputs> LI(kDistMaxL + 1);
   size_t off = 0;
-  const size_t o_U = off; off = al(off + sizeof(double2) * (size_t)m * m);
-  const size_t o_fact = off; off = al(off + sizeof(double) * 256);
-  const size_t o_cols = off; off = al(off + (size_t)K * l);
-  const size_t o_div = off; off = al(off + sizeof(double) * (size_t)K * kDistMaxDiv);
-  const size_t o_ndiv = off; off = al(off + sizeof(int) * (size_t)K);
-  const size_t o_mult = off; off = al(off + sizeof(double) * (size_t)K);
-  const size_t o_occ = off; off = al(off + (size_t)O * m);
-  const size_t arena = off;
+  const size_t o_U = off; off = align256(off + sizeof(double2) * (size_t)m * m);
+  const size_t o_fact = off; off = align256(off + sizeof(double) * 256);
+  size_t o_cols[kDistMaxL + 1], o_div[kDistMaxL + 1], o_ndiv[kDistMaxL + 1], o_mult[kDistMaxL + 1];
+  int64_t most_terms = 1, most_O = 1, most_V = 1;
   int st;
-  if ((st = ensure(cx->dist[0], arena))) return st;
-  if ((st = ensure(cx->dist[1], sizeof(double) * (size_t)K * O))) return st;  // terms
-  if ((st = ensure(cx->dist[2], sizeof(double) * (size_t)O))) return st;      // probabilities
-  if ((st = ensure_pinned(cx, std::max(arena, sizeof(double) * (size_t)O)))) return st;
+  for (int l = 1; l <= kDistMaxL; ++l) {
+    if (!G.size[l]) continue;
+    if ((st = lossy_inputs(initial_state, m, l, LI[l]))) return st;
+    const int64_t K = (int64_t)LI[l].occ.size();
+    o_cols[l] = off; off = align256(off + (size_t)K * l);
+    o_div[l] = off; off = align256(off + sizeof(double) * (size_t)K * kDistMaxDiv);
+    o_ndiv[l] = off; off = align256(off + sizeof(int) * (size_t)K);
+    o_mult[l] = off; off = align256(off + sizeof(double) * (size_t)K);
+    most_terms = std::max(most_terms, K * G.size[l]);
+    most_O = std::max(most_O, G.size[l]);
+    const int64_t combos = ((K << (l - 1)) + 31) / 32 * 32;
+    most_V = std::max(most_V, std::min(combos * m, std::max<int64_t>(kTableBytes / 16, (int64_t)m << l) + 32 * m));
+  }
+  if ((st = ensure(cx->dist[0], off))) return st;
+  if ((st = ensure(cx->dist[1], sizeof(double) * (size_t)most_terms))) return st;
+  if ((st = ensure(cx->gpart, sizeof(uint4) * (size_t)most_O + sizeof(double2) * (size_t)most_V + 256))) return st;
+  if ((st = ensure_pinned(cx, off))) return st;
   char* h = (char*)cx->pinned;
   memcpy(h + o_U, matrix, sizeof(double2) * (size_t)m * m);
   double* hf = (double*)(h + o_fact);
   for (int k = 0; k < 256; ++k) hf[k] = factorial_d(k);
-  for (int k = 0; k < K; ++k) {
-    particle_list(LI.occ[k].data(), m, (uint8_t*)(h + o_cols) + (size_t)k * l);
-    const int nd = divisors(LI.occ[k].data(), m, (double*)(h + o_div) + (size_t)k * kDistMaxDiv);
-    if (nd < 0) {
-      set_error("too many multiply occupied modes in a lossy input");
-      return kErrLimit;
+  for (int l = 1; l <= kDistMaxL; ++l) {
+    if (!G.size[l]) continue;
+    const int K = (int)LI[l].occ.size();
+    for (int k = 0; k < K; ++k) {
+      particle_list(LI[l].occ[k].data(), m, (uint8_t*)(h + o_cols[l]) + (size_t)k * l);
+      const int nd = divisors(LI[l].occ[k].data(), m, (double*)(h + o_div[l]) + (size_t)k * kDistMaxDiv);
+      if (nd < 0) {
+        set_error("too many multiply occupied modes in a lossy input");
+        return kErrLimit;
+      }
+      ((int*)(h + o_ndiv[l]))[k] = nd;
+      ((double*)(h + o_mult[l]))[k] = LI[l].mult[k];
     }
-    ((int*)(h + o_ndiv))[k] = nd;
-    ((double*)(h + o_mult))[k] = LI.mult[k];
   }
-  uint8_t* hocc = (uint8_t*)(h + o_occ);
-  for (int64_t o = 0; o < O; ++o)
-    for (int i = 0; i < m; ++i) hocc[(size_t)o * m + i] = (uint8_t)outs[o][i];
   char* d = (char*)cx->dist[0].ptr;
   double* terms = (double*)cx->dist[1].ptr;
-  double* prob = (double*)cx->dist[2].ptr;
+  uint4* rows = (uint4*)cx->gpart.ptr;
+  double2* V = (double2*)((char*)cx->gpart.ptr + align256(sizeof(uint4) * (size_t)most_O));
   cudaStream_t s = cx->stream;
-  cudaError_t e = cudaMemcpyAsync(d, h, arena, cudaMemcpyHostToDevice, s);
+  cudaError_t e = cudaMemcpyAsync(d, h, off, cudaMemcpyHostToDevice, s);
   if (e != cudaSuccess) return fail_cuda(e, "H2D distribution tables");
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   if (kernel_ms) {
@@ -444,28 +606,41 @@ static int group_small(Context* cx, const double* matrix, int m, int n, int l, c
     cudaEventCreate(&e1);
     cudaEventRecord(e0, s);
   }
-  e = launch_pairs_l(l, (const double2*)(d + o_U), m, (const uint8_t*)(d + o_cols), (const double*)(d + o_div),
-                     (const int*)(d + o_ndiv), (const double*)(d + o_mult), K, (const uint8_t*)(d + o_occ), O,
-                     terms, s);
-  if (e != cudaSuccess) return fail_cuda(e, "lossy pair kernel");
-  lossy_outcome_kernel<<<(unsigned)((O + 127) / 128), 128, 0, s>>>(terms, K, O, m, (const uint8_t*)(d + o_occ),
-                                                                   (const double*)(d + o_fact), factorial_d(l),
-                                                                   binom_d(n, l), prob);
-  if ((e = cudaGetLastError()) != cudaSuccess) return fail_cuda(e, "lossy outcome kernel");
-  if (kernel_ms) cudaEventRecord(e1, s);
-  e = cudaMemcpyAsync(h, prob, sizeof(double) * (size_t)O, cudaMemcpyDeviceToHost, s);
-  if (e != cudaSuccess) return fail_cuda(e, "D2H probabilities");
-  if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return fail_cuda(e, "distribution kernels");
+  for (int l = 1; l <= kDistMaxL && e == cudaSuccess; ++l) {
+    const int64_t O = G.size[l];
+    if (!O) continue;
+    const int K = (int)LI[l].occ.size();
+    const uint8_t* occ = G.occ + G.first[l] * m;
+    lossy_rows_kernel<<<(unsigned)((O + 127) / 128), 128, 0, s>>>(occ, m, O, rows);
+    // inputs in chunks whose table stays below kTableBytes (whole warps of combos)
+    const int per_warp = l >= 6 ? 1 : 32 >> (l - 1);  // inputs per group of combos
+    const int64_t each = (int64_t)m * 16 << (l >= 6 ? l - 1 : 5);  // table bytes of a group
+    const int64_t step = std::max<int64_t>(1, kTableBytes / each) * per_warp;
+    for (int64_t k0 = 0; k0 < K && e == cudaSuccess; k0 += step) {
+      const int kn = (int)std::min<int64_t>(step, K - k0);
+      const int groups = (kn + per_warp - 1) / per_warp;
+      const int64_t combos = l >= 6 ? (int64_t)kn << (l - 1) : (int64_t)groups * 32;
+      const uint8_t* cols = (const uint8_t*)(d + o_cols[l]) + k0 * l;
+      lossy_table_kernel<<<(unsigned)((combos * m + 127) / 128), 128, 0, s>>>((const double2*)(d + o_U), m, l, cols, kn,
+                                                                             combos, V);
+      e = launch_walk_l(l, V, m, rows, O, kn, groups, (const double*)(d + o_div[l]) + k0 * kDistMaxDiv,
+                        (const int*)(d + o_ndiv[l]) + k0, (const double*)(d + o_mult[l]) + k0, terms + k0 * O, cx->sm_count, s);
+    }
+    lossy_outcome_kernel<<<(unsigned)((O + 127) / 128), 128, 0, s>>>(terms, K, O, m, occ, (const double*)(d + o_fact),
+                                                                     factorial_d(l), binom_d(n, l),
+                                                                     G.prob + G.first[l]);
+    if (e == cudaSuccess) e = cudaGetLastError();
+  }
   if (kernel_ms) {
+    cudaEventRecord(e1, s);
+    if (e == cudaSuccess) e = cudaEventSynchronize(e1);
     float ms = 0.f;
     cudaEventElapsedTime(&ms, e0, e1);
     *kernel_ms += ms;
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
   }
-  const double* hp = (const double*)h;
-  for (int64_t o = 0; o < O; ++o) prob_out[where[o]] = hp[o];
-  return kOk;
+  return e == cudaSuccess ? kOk : fail_cuda(e, "distribution kernels");
 }
 
 // Larger l: one Glynn sweep per (lossy input, outcome) on the sweep engine, the
@@ -575,8 +750,6 @@ static void particle_modes(const int32_t* occ, int len, uint16_t* out) {
   for (int i = 0; i < len; ++i)
     for (int c = 0; c < occ[i]; ++c) out[p++] = (uint16_t)i;
 }
-
-static size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 // A few permanents: each one's matrix is gathered and scaled on the host (L^2
 // entries), and the kernel reads it from, and writes its result to, page-locked
@@ -714,6 +887,23 @@ int small_perm_batch(Context* cx, const double* matrix, int m, int len, const in
   return kOk;
 }
 
+// Page-locked staging of the outcomes and their probabilities, apart from the
+// context's buffer, which holds the tables.  Grow-only, like the context's.
+static DeviceBuffer g_outcome_staging;
+static int ensure_outcome_staging(size_t bytes) {
+  DeviceBuffer& b = g_outcome_staging;
+  if (bytes <= b.bytes) return kOk;
+  if (b.ptr) cudaFreeHost(b.ptr);
+  b = DeviceBuffer{};
+  const cudaError_t e = cudaMallocHost(&b.ptr, bytes);
+  if (e != cudaSuccess) {
+    b.ptr = nullptr;
+    return fail_cuda(e, "cudaMallocHost");
+  }
+  b.bytes = bytes;
+  return kOk;
+}
+
 }  // namespace boss
 
 using namespace boss;
@@ -744,40 +934,112 @@ int boss_lossy_probabilities(const double* matrix, int32_t m, const int32_t* ini
   }
   if (kernel_ms) *kernel_ms = 0.f;
   std::lock_guard<std::mutex> lk(g_api_mutex);
-  // group the outcomes by particle count
-  std::vector<std::vector<const int32_t*>> by_l(n + 1);
-  std::vector<std::vector<int>> where(n + 1);
-  for (int o = 0; o < count; ++o) {
-    const int32_t* T = outcomes + (size_t)o * m;
-    int l = 0;
-    for (int i = 0; i < m; ++i) {
-      if (T[i] < 0 || T[i] > 255) {
-        set_error("occupations must be in [0, 255]");
-        return kErrArg;
+  // (1) every outcome's particle count, by slices on the host's threads
+  const int T = count < 20000 ? 1 : 8;
+  std::vector<uint8_t> ls(count);
+  std::vector<std::vector<int64_t>> tally(T, std::vector<int64_t>(n + 1, 0));
+  std::vector<int> bad(T, 0);  // 1: an occupation out of range, 2: too many particles (the first of the slice)
+  host_parallel(T, [&](int t) {
+    const int64_t lo = (int64_t)count * t / T, hi = (int64_t)count * (t + 1) / T;
+    for (int64_t o = lo; o < hi; ++o) {
+      const int32_t* x = outcomes + o * m;
+      int32_t l = 0;
+      uint32_t out = 0;
+      for (int i = 0; i < m; ++i) {
+        l += x[i] & 255;
+        out |= (uint32_t)x[i] & ~255u;
       }
-      l += T[i];
+      if (out || l > n) {
+        bad[t] = out ? 1 : 2;
+        return;
+      }
+      ls[o] = (uint8_t)l;
+      ++tally[t][l];
     }
-    if (l > n) {
-      set_error("an outcome holds more particles than the initial state");
+  });
+  for (int t = 0; t < T; ++t)
+    if (bad[t]) {
+      set_error(bad[t] == 1 ? "occupations must be in [0, 255]" : "an outcome holds more particles than the initial state");
       return kErrArg;
     }
-    if (l == 0) {  // the empty lossy input: perm = 1, every factor 1
-      probabilities[o] = 1.0;
-      continue;
-    }
-    by_l[l].push_back(T);
-    where[l].push_back(o);
+  std::vector<int64_t> size(n + 1, 0);
+  for (int t = 0; t < T; ++t)
+    for (int l = 0; l <= n; ++l) size[l] += tally[t][l];
+  // (2) the counts up to kDistMaxL: rows grouped by count in page-locked memory, one
+  // copy up, all kernels, one copy down
+  SmallGroups G{};
+  std::vector<int64_t> first(n + 1, 0);
+  int64_t total = 0;
+  for (int l = 1; l <= std::min(n, kDistMaxL); ++l) {
+    first[l] = total;
+    G.first[l] = total;
+    G.size[l] = size[l];
+    total += size[l];
   }
-  int st;
+  // where slice t's outcomes of count l start among the grouped rows
+  std::vector<std::vector<int64_t>> start(T, std::vector<int64_t>(n + 1, 0));
+  for (int l = 1; l <= n; ++l)
+    for (int64_t t = 0, at = first[l]; t < T; ++t) {
+      start[t][l] = at;
+      at += tally[t][l];
+    }
+  int st = kOk;
   Context* cx = nullptr;
-  for (int l = 1; l <= n; ++l) {
-    if (by_l[l].empty()) continue;
+  if (total > 0) {
+    if (!(cx = context(&st))) return st;
+    const size_t o_prob = align256((size_t)total * m);
+    if ((st = ensure(cx->dist[2], o_prob + sizeof(double) * (size_t)total))) return st;
+    if ((st = ensure_outcome_staging(o_prob + sizeof(double) * (size_t)total))) return st;
+    uint8_t* h = (uint8_t*)g_outcome_staging.ptr;
+    host_parallel(T, [&](int t) {
+      std::vector<int64_t> at = start[t];
+      const int64_t lo = (int64_t)count * t / T, hi = (int64_t)count * (t + 1) / T;
+      for (int64_t o = lo; o < hi; ++o) {
+        const int l = ls[o];
+        if (l == 0 || l > kDistMaxL) continue;
+        const int32_t* x = outcomes + o * m;
+        uint8_t* y = h + at[l]++ * m;
+        for (int i = 0; i < m; ++i) y[i] = (uint8_t)x[i];
+      }
+    });
+    uint8_t* d = (uint8_t*)cx->dist[2].ptr;
+    G.occ = d;
+    G.prob = (double*)(d + o_prob);
+    cudaError_t e = cudaMemcpyAsync(d, h, (size_t)total * m, cudaMemcpyHostToDevice, cx->stream);
+    if (e != cudaSuccess) return fail_cuda(e, "H2D outcomes");
+    if ((st = queue_small_groups(cx, matrix, m, n, initial_state, G, kernel_ms))) {
+      cudaStreamSynchronize(cx->stream);  // nothing queued may outlive the call's staging
+      return st;
+    }
+    e = cudaMemcpyAsync(h + o_prob, G.prob, sizeof(double) * (size_t)total, cudaMemcpyDeviceToHost, cx->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(cx->stream);
+    if (e != cudaSuccess) return fail_cuda(e, "distribution kernels");
+    const double* hp = (const double*)(h + o_prob);
+    host_parallel(T, [&](int t) {
+      std::vector<int64_t> at = start[t];
+      const int64_t lo = (int64_t)count * t / T, hi = (int64_t)count * (t + 1) / T;
+      for (int64_t o = lo; o < hi; ++o)
+        if (ls[o] && ls[o] <= kDistMaxL) probabilities[o] = hp[at[ls[o]]++];
+    });
+  }
+  // (3) no particle: the empty lossy input, perm = 1, every factor 1; larger counts
+  // through the sweep engine
+  if (size[0])
+    for (int64_t o = 0; o < count; ++o)
+      if (!ls[o]) probabilities[o] = 1.0;
+  for (int l = kDistMaxL + 1; l <= n; ++l) {
+    if (!size[l]) continue;
     if (!cx && !(cx = context(&st))) return st;
+    std::vector<const int32_t*> outs;
+    std::vector<int> where;
+    for (int o = 0; o < count; ++o)
+      if (ls[o] == l) {
+        outs.push_back(outcomes + (size_t)o * m);
+        where.push_back(o);
+      }
     LossyInputs LI;
     if ((st = lossy_inputs(initial_state, m, l, LI))) return st;
-    st = (l <= kDistMaxL) ? group_small(cx, matrix, m, n, l, LI, by_l[l], probabilities, where[l], kernel_ms)
-                          : group_large(cx, matrix, m, n, l, LI, by_l[l], probabilities, where[l]);
-    if (st) return st;
+    if ((st = group_large(cx, matrix, m, n, l, LI, outs, probabilities, where))) return st;
   }
   return kOk;
 }

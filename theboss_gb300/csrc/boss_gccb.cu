@@ -267,6 +267,13 @@ class HostPool {
   int T_ = 0, pending_ = 0, nthreads_ = 0;
 };
 
+void host_parallel(int threads, const std::function<void(int)>& fn) {
+  if (threads <= 1)
+    fn(0);
+  else
+    HostPool::get().run(threads, fn);
+}
+
 // The generator's output words from its current state on, with the key of every
 // kKeyStride-th block generated, so that the state after any number of words can
 // be set (by re-twisting at most kKeyStride - 1 blocks).  The storage is the

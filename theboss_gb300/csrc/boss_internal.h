@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <functional>
 #include <string>
 #include <vector>
 
@@ -142,6 +143,10 @@ struct DeviceBuffer {
   void* ptr = nullptr;
   size_t bytes = 0;
 };
+// Runs fn(0 .. threads - 1) on the library's host threads (fn(0) on the caller) and
+// returns when all have finished.
+void host_parallel(int threads, const std::function<void(int)>& fn);
+
 struct Context {
   bool ready = false;
   int device = 0;
