@@ -127,6 +127,34 @@ static int split_threads(const std::vector<HostSweep>& sweeps, int64_t resident,
   return G;
 }
 
+static size_t rows_of(const HostSweep& h) { return h.on_device ? h.D_size : h.D.size(); }
+static size_t base_of(const HostSweep& h) { return h.on_device ? h.base_size : h.base.size(); }
+
+// Whether a call's sweeps have their rows made on the GPU: from four permanents on,
+// while the matrix is a small upload (64 permanents at n = 16: 340 -> 150 us a call; a
+// single one is planned on the host in the time of the extra launch).
+static bool plan_on_device(int m, int count) { return count >= 4 && m <= 512; }
+
+static void describe_plan(const HostSweep& h, int64_t mat_off, int64_t base_off, PlanItem& I) {
+  I.layout = h.layout;
+  I.nd = h.nd;
+  I.nd_all = h.nd + (h.fixed_mode >= 0 ? 1 : 0);
+  I.nf = h.nf;
+  I.glynn = h.kind == kGlynn ? 1 : 0;
+  I.digits_are_outputs = h.digits_are_outputs ? 1 : 0;
+  I.mat_off = mat_off;
+  I.base_off = base_off;
+  for (int a = 0; a < h.nd; ++a) {
+    I.digit[a] = (uint16_t)h.digit_mode[a];
+    I.mult[a] = h.mult[a];
+  }
+  if (h.fixed_mode >= 0) {
+    I.digit[h.nd] = (uint16_t)h.fixed_mode;
+    I.mult[h.nd] = 1;
+  }
+  for (int f = 0; f < h.nf; ++f) I.factor[f] = (uint16_t)h.factor_mode[f];
+}
+
 // A list of sweeps that share one factor count, uploaded and ready to launch.
 struct SweepBatch {
   int n = 0, nf = 0;
@@ -138,7 +166,8 @@ struct SweepBatch {
   double codes = 0.0;  // codes swept per launch
 };
 
-static int sweeps_prepare(Context* cx, const std::vector<HostSweep>& sweeps, bool minors, int nd_max, SweepBatch& B) {
+static int sweeps_prepare(Context* cx, const std::vector<HostSweep>& sweeps, bool minors, int nd_max, SweepBatch& B,
+                          const double* matrix = nullptr, int m = 0) {
   const int n = (int)sweeps.size();
   B.n = n;
   B.nf = sweeps[0].nf;
@@ -171,9 +200,9 @@ static int sweeps_prepare(Context* cx, const std::vector<HostSweep>& sweeps, boo
     P.out_idx = p;
     P.thread_begin = threads;
     P.mat_off = pool_n;
-    pool_n += (int64_t)h.D.size();
+    pool_n += (int64_t)rows_of(h);
     P.base_off = pool_n;
-    pool_n += (int64_t)h.base.size();
+    pool_n += (int64_t)base_of(h);
     P.part_off = parts;
     if (B.ff) {  // float-pair rows of the binary digits, then the factors' biases
       P.ff_off = pool_n;
@@ -183,21 +212,31 @@ static int sweeps_prepare(Context* cx, const std::vector<HostSweep>& sweeps, boo
     threads += nthr[p];
     parts += nthr[p] / G * (minors ? h.nd + P.fixed_digit : 1);
   }
-  // arena: problems | pool
+  // arena: problems | matrix and plan items (rows made on the device) | pool; `up` bytes
+  // of it come from the host
+  const bool device_rows = sweeps[0].on_device;  // all of a call's sweeps of a class alike
   size_t off = 0;
   const size_t o_probs = off; off = align_up(off + sizeof(SweepProblem) * n, 256);
+  const size_t o_U = off; off = align_up(off + (device_rows ? sizeof(double2) * (size_t)m * m : 0), 256);
+  const size_t o_items = off; off = align_up(off + (device_rows ? sizeof(PlanItem) * n : 0), 256);
   const size_t o_pool = off; off = align_up(off + sizeof(longlong2) * std::max<int64_t>(pool_n, 1), 256);
-  const size_t arena_bytes = off;
+  const size_t arena_bytes = off, up = device_rows ? o_pool : arena_bytes;
   B.out_elems = (size_t)n * (minors ? nd_max : 1);
   int st;
   if ((st = ensure(cx->plans, arena_bytes))) return st;
   if ((st = ensure(cx->partials, sizeof(double2) * std::max<int64_t>(parts, 1)))) return st;
   if ((st = ensure(cx->out, sizeof(double2) * B.out_elems))) return st;
-  if ((st = ensure_pinned(cx, std::max(arena_bytes, sizeof(double2) * B.out_elems)))) return st;
+  if ((st = ensure_pinned(cx, std::max(up, sizeof(double2) * B.out_elems)))) return st;
   char* h = (char*)cx->pinned;
   memcpy(h + o_probs, probs.data(), sizeof(SweepProblem) * n);
   longlong2* hp = (longlong2*)(h + o_pool);
-  for (int p = 0; p < n; ++p) {
+  int max_entries = 0;
+  if (device_rows) memcpy(h + o_U, matrix, sizeof(double2) * (size_t)m * m);
+  for (int p = 0; p < n && device_rows; ++p) {
+    describe_plan(sweeps[p], probs[p].mat_off, probs[p].base_off, ((PlanItem*)(h + o_items))[p]);
+    max_entries = std::max(max_entries, (sweeps[p].nd + 1) * B.nf);
+  }
+  for (int p = 0; p < n && !device_rows; ++p) {
     const HostSweep& hs = sweeps[p];
     std::copy(hs.D.begin(), hs.D.end(), hp + probs[p].mat_off);
     std::copy(hs.base.begin(), hs.base.end(), hp + probs[p].base_off);
@@ -215,8 +254,13 @@ static int sweeps_prepare(Context* cx, const std::vector<HostSweep>& sweeps, boo
     }
   }
   char* d = (char*)cx->plans.ptr;
-  cudaError_t e = cudaMemcpyAsync(d, h, arena_bytes, cudaMemcpyHostToDevice, cx->stream);
+  cudaError_t e = cudaMemcpyAsync(d, h, up, cudaMemcpyHostToDevice, cx->stream);
   if (e != cudaSuccess) return fail_cuda(e, "H2D sweeps");
+  if (device_rows) {
+    e = launch_plan_rows((const PlanItem*)(d + o_items), n, (const double2*)(d + o_U), m, max_entries,
+                         (longlong2*)(d + o_pool), (SweepProblem*)(d + o_probs), cx->stream);
+    if (e != cudaSuccess) return fail_cuda(e, "sweep rows");
+  }
   B.L.probs = (const SweepProblem*)(d + o_probs);
   B.L.n_probs = n;
   B.L.pool = (const longlong2*)(d + o_pool);
@@ -248,10 +292,11 @@ static int sweeps_collect(Context* cx, const SweepBatch& B, double2* results_hos
   return kOk;
 }
 
-int run_sweeps(Context* cx, const std::vector<HostSweep>& sweeps, bool minors, int nd_max, double2* results_host) {
+int run_sweeps(Context* cx, const std::vector<HostSweep>& sweeps, bool minors, int nd_max, double2* results_host,
+               const double* matrix, int m) {
   if (sweeps.empty()) return kOk;
   SweepBatch B;
-  int st = sweeps_prepare(cx, sweeps, minors, nd_max, B);
+  int st = sweeps_prepare(cx, sweeps, minors, nd_max, B, matrix, m);
   if (st) return st;
   if ((st = sweeps_launch(cx, B))) return st;
   return sweeps_collect(cx, B, results_host);
@@ -395,7 +440,7 @@ static void fill_grad(HostSweep& hs, const Side& dig, int drop, const std::vecto
 // scale would leave the factors of small rows with fewer significant bits).
 template <class F>
 static int fill_sweep(HostSweep& hs, const Side& dig, const Side& col, int kind, bool halve, PlanFor plan, bool ff,
-                      int quad_min, F entry) {
+                      int quad_min, bool on_device, F entry) {
   int drop = -1;
   if (halve && dig.nb > 0) drop = dig.nb - 1;  // a binary digit fixed at r = 0
   hs.kind = kind;
@@ -430,6 +475,16 @@ static int fill_sweep(HostSweep& hs, const Side& dig, const Side& col, int kind,
               : (ff && glynn && plan == kPlanAny)                       ? kRowsPlain
               : (plan != kPlanTemplated && hs.nb >= 2 && hs.nf >= quad_min)   ? kRowsQuad
                                                                        : kRowsPacked;
+  hs.scale = glynn ? std::ldexp(1.0, -dig.n) * (drop >= 0 ? 2.0 : 1.0) : 1.0;
+  hs.parity0 = glynn ? 0 : (dig.n & 1);
+  hs.has_base = glynn || hs.layout != kRowsPlain;
+  hs.on_device = on_device && (hs.layout == kRowsQuad || hs.layout == kRowsGrad);
+  if (hs.on_device) {
+    const int Fg = grad_factors(hs.nf), W = quad_width(hs.nf);
+    hs.D_size = hs.layout == kRowsGrad ? (size_t)hs.nd * Fg : (size_t)(hs.nd - 2) * W;
+    hs.base_size = hs.layout == kRowsGrad ? (size_t)Fg + Fg / 4 : (size_t)W + W / 2;
+    return kOk;
+  }
   // |row sum| <= sum_a mult_a * max component of the entries
   const int nf = hs.nf, nd_all = (int)dig.modes.size();
   double bound[kMaxFactors] = {};
@@ -463,9 +518,6 @@ static int fill_sweep(HostSweep& hs, const Side& dig, const Side& col, int kind,
     hs.ff_exp += p + 1 - fx;
     hs.fx_sum += fx;
   }
-  hs.scale = glynn ? std::ldexp(1.0, -dig.n) * (drop >= 0 ? 2.0 : 1.0) : 1.0;
-  hs.parity0 = glynn ? 0 : (dig.n & 1);
-  hs.has_base = glynn || !old_rows;
   if (hs.layout == kRowsQuad) {
     fill_quad(hs, dig, drop, glynn, u);
     return kOk;
@@ -525,7 +577,8 @@ void host_fx_to_ff(long long x, int fbias, float& hi, float& lo) {
 // One permanent request.  Returns kOk and either fills `hs` (needs_sweep = true)
 // or sets `value` directly for the edge cases theboss special-cases.
 int plan_permanent(const double* U, int m, const int32_t* S, const int32_t* T, int len, int variant,
-                          HostSweep& hs, bool& needs_sweep, double2& value, PlanFor plan) {
+                          HostSweep& hs, bool& needs_sweep, double2& value, PlanFor plan,
+                          bool on_device) {
   needs_sweep = false;
   const bool ff = g_perm_arith == 0;  // float pairs: every factor count has the kernel (kFFPermMaxFactors)
   if (len > m || len < 0) {  // bs_permanent_calculator_base.py:61-72
@@ -552,7 +605,7 @@ int plan_permanent(const double* U, int m, const int32_t* S, const int32_t* T, i
         return kOk;
       }
       const bool ch = (variant == BOSS_CHIN_HUH);
-      const int st = fill_sweep(hs, in, out, ch ? kGlynn : kRyser, ch && in.n == out.n, plan, ff, kQuadMinFactors, entry_in_out);
+      const int st = fill_sweep(hs, in, out, ch ? kGlynn : kRyser, ch && in.n == out.n, plan, ff, kQuadMinFactors, on_device, entry_in_out);
       if (st) return st;
       needs_sweep = true;
       return kOk;
@@ -576,10 +629,10 @@ int plan_permanent(const double* U, int m, const int32_t* S, const int32_t* T, i
       const uint64_t co = out.nb ? out.codes / 2 : out.codes;
       int st;
       bool outs = co < ci;
-      st = outs ? fill_sweep(hs, out, in, kGlynn, true, plan, ff, kQuadMinFactors, entry_out_in) : fill_sweep(hs, in, out, kGlynn, true, plan, ff, kQuadMinFactors, entry_in_out);
+      st = outs ? fill_sweep(hs, out, in, kGlynn, true, plan, ff, kQuadMinFactors, on_device, entry_out_in) : fill_sweep(hs, in, out, kGlynn, true, plan, ff, kQuadMinFactors, on_device, entry_in_out);
       if (st == kErrLimit) {  // try the other orientation
         outs = !outs;
-        st = outs ? fill_sweep(hs, out, in, kGlynn, true, plan, ff, kQuadMinFactors, entry_out_in) : fill_sweep(hs, in, out, kGlynn, true, plan, ff, kQuadMinFactors, entry_in_out);
+        st = outs ? fill_sweep(hs, out, in, kGlynn, true, plan, ff, kQuadMinFactors, on_device, entry_out_in) : fill_sweep(hs, in, out, kGlynn, true, plan, ff, kQuadMinFactors, on_device, entry_in_out);
       }
       if (st) return st;
       hs.digits_are_outputs = outs;
@@ -660,7 +713,7 @@ static int plan_minors(const double* U, int m, const int32_t* S, const int32_t* 
   // accumulates half of each, hence the factor 2.
   auto entry = [&](int i_mode, int j_mode) { return U_at(U, m, j_mode, i_mode); };
   const int st = fill_sweep(hs, in, out, kGlynn, true, kPlanAny, g_minors_arith == 0 && out.n <= kFFMaxFactors,
-                            kQuadMinMinorFactors, entry);
+                            kQuadMinMinorFactors, false, entry);
   if (st) return st;
   hs.scale *= 2.0;
   needs_sweep = true;
@@ -732,7 +785,7 @@ int boss_perm_batch(const double* matrix, int32_t m, const int32_t* input_states
     HostSweep hs;
     bool need = false;
     double2 v = make_double2(0.0, 0.0);
-    const int st = plan_permanent(matrix, m, Sk, Tk, len, variant, hs, need, v);
+    const int st = plan_permanent(matrix, m, Sk, Tk, len, variant, hs, need, v, kPlanAny, plan_on_device(m, count));
     if (st) return st;
     if (need) {
       const int c = sweep_class(hs);
@@ -754,7 +807,7 @@ int boss_perm_batch(const double* matrix, int32_t m, const int32_t* input_states
   for (int c = 0; c < kSweepClasses; ++c) {
     if (by_class[c].empty()) continue;
     std::vector<double2> out(by_class[c].size());
-    st = run_sweeps(cx, by_class[c], false, 1, out.data());
+    st = run_sweeps(cx, by_class[c], false, 1, out.data(), matrix, m);
     if (st) return st;
     for (size_t a = 0; a < out.size(); ++a) {
       results[2 * which[c][a]] = out[a].x;
@@ -835,7 +888,7 @@ int boss_perm_grad_batch(const double* matrix, int32_t m, const int32_t* input_s
     double2 v = make_double2(0.0, 0.0);
     const int32_t* S = input_states + (size_t)k * len;
     const int32_t* T = output_states + (size_t)k * len;
-    int st = plan_permanent(matrix, m, S, T, len, BOSS_GLYNN, hs, need, v, kPlanGrad);
+    int st = plan_permanent(matrix, m, S, T, len, BOSS_GLYNN, hs, need, v, kPlanGrad, plan_on_device(m, count));
     if (st) return st;
     if (!need) {  // no particles: perm = 1, gradient 0
       P2[k] = v;
@@ -875,9 +928,9 @@ int boss_perm_grad_batch(const double* matrix, int32_t m, const int32_t* input_s
       Pp.out_idx = p;
       Pp.thread_begin = walkers;
       Pp.mat_off = pool_n;
-      pool_n += (int64_t)h.D.size();
+      pool_n += (int64_t)rows_of(h);
       Pp.base_off = pool_n;
-      pool_n += (int64_t)h.base.size();
+      pool_n += (int64_t)base_of(h);
       Pp.part_off = gparts;
       const int rows = h.nd + Pp.fixed_digit;
       row = std::max(row, rows * F);
@@ -886,24 +939,39 @@ int boss_perm_grad_batch(const double* matrix, int32_t m, const int32_t* input_s
     }
     size_t off = 0;
     const size_t o_probs = off; off = align_up(off + sizeof(SweepProblem) * n, 256);
+    const bool device_rows = sw[0].on_device;
+    const size_t o_U = off; off = align_up(off + (device_rows ? sizeof(double2) * (size_t)m * m : 0), 256);
+    const size_t o_items = off; off = align_up(off + (device_rows ? sizeof(PlanItem) * n : 0), 256);
     const size_t o_pool = off; off = align_up(off + sizeof(longlong2) * std::max<int64_t>(pool_n, 1), 256);
-    const size_t arena_bytes = off;
+    const size_t arena_bytes = off, up = device_rows ? o_pool : arena_bytes;
     const size_t out_g = (size_t)n * row, out_p = (size_t)n;
     if ((st = ensure(cx->plans, arena_bytes))) return st;
     if ((st = ensure(cx->gpart, sizeof(double2) * std::max<int64_t>(gparts, 1)))) return st;
     if ((st = ensure(cx->pperm, sizeof(double2) * std::max<int64_t>(walkers / 8, 1)))) return st;
     if ((st = ensure(cx->out, sizeof(double2) * (out_g + out_p)))) return st;
-    if ((st = ensure_pinned(cx, std::max(arena_bytes, sizeof(double2) * (out_g + out_p))))) return st;
+    if ((st = ensure_pinned(cx, std::max(up, sizeof(double2) * (out_g + out_p))))) return st;
     char* h = (char*)cx->pinned;
     memcpy(h + o_probs, probs.data(), sizeof(SweepProblem) * n);
     longlong2* hp = (longlong2*)(h + o_pool);
+    int max_entries = 0;
+    if (device_rows) memcpy(h + o_U, matrix, sizeof(double2) * (size_t)m * m);
     for (int p = 0; p < n; ++p) {
+      if (device_rows) {
+        describe_plan(sw[p], probs[p].mat_off, probs[p].base_off, ((PlanItem*)(h + o_items))[p]);
+        max_entries = std::max(max_entries, (sw[p].nd + 1) * nf);
+        continue;
+      }
       std::copy(sw[p].D.begin(), sw[p].D.end(), hp + probs[p].mat_off);
       std::copy(sw[p].base.begin(), sw[p].base.end(), hp + probs[p].base_off);
     }
     char* d = (char*)cx->plans.ptr;
-    cudaError_t e = cudaMemcpyAsync(d, h, arena_bytes, cudaMemcpyHostToDevice, cx->stream);
+    cudaError_t e = cudaMemcpyAsync(d, h, up, cudaMemcpyHostToDevice, cx->stream);
     if (e != cudaSuccess) return fail_cuda(e, "H2D gradient sweeps");
+    if (device_rows) {
+      e = launch_plan_rows((const PlanItem*)(d + o_items), n, (const double2*)(d + o_U), m, max_entries,
+                           (longlong2*)(d + o_pool), (SweepProblem*)(d + o_probs), cx->stream);
+      if (e != cudaSuccess) return fail_cuda(e, "gradient rows");
+    }
     const SweepProblem* dp = (const SweepProblem*)(d + o_probs);
     double2 *gpart = (double2*)cx->gpart.ptr, *ppart = (double2*)cx->pperm.ptr;
     if ((e = launch_grad_sweep(nf, dp, n, (const longlong2*)(d + o_pool), walkers, gpart, ppart, cx->stream)) !=

@@ -2052,6 +2052,7 @@ static int gccb_prepare(Context* cx, const double* matrix, int n_mats, int m, Dr
     auto& t = tab[k];
     t.resize(Ak);
     int64_t threads = 0, parts = 0, pool = 0;
+    struct { int64_t codes, threads, align; } seen[8] = {};  // few code counts: their alignments, remembered
     for (int jj = 0; jj < Ak; ++jj) {
       LevelSample ls;
       ls.n_codes = (int64_t)(codes[jj] >> low);
@@ -2059,7 +2060,10 @@ static int gccb_prepare(Context* cx, const double* matrix, int n_mats, int m, Dr
       ls.n_threads = nthr[jj];
       ls.part_off = parts;
       ls.pool_off = pool;
-      ls.align = range_align(ls.n_codes, ls.n_threads, k);
+      auto& a = seen[(ls.n_codes ^ (ls.n_codes >> 3)) & 7];
+      if (a.codes != ls.n_codes || a.threads != ls.n_threads)
+        a = {ls.n_codes, ls.n_threads, range_align(ls.n_codes, ls.n_threads, k)};
+      ls.align = a.align;
       threads += nthr[jj];
       parts += nthr[jj] * ndv[jj];
       pool += pool_units(ndv[jj]);

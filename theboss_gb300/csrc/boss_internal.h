@@ -46,7 +46,7 @@ cudaError_t launch_quad_sweep(int nf, bool minors, const SweepLaunch& L, cudaStr
 // factor with the factor count padded to a multiple of 4).
 cudaError_t prepare_grad_kernels();
 int64_t grad_resident_walkers(int nf, int sm_count);
-inline int grad_factors(int nf) { return (nf + 3) / 4 * 4; }
+__host__ __device__ inline int grad_factors(int nf) { return (nf + 3) / 4 * 4; }
 inline int64_t grad_slice(int rows, int nf) { return (int64_t)rows * grad_factors(nf) * 8; }
 cudaError_t launch_grad_sweep(int nf, const SweepProblem* probs, int n_probs, const longlong2* pool, int64_t walkers,
                               double2* gpart, double2* ppart, cudaStream_t st);
@@ -96,6 +96,8 @@ enum RowLayout : int {
 };
 struct HostSweep {
   int layout = kRowsPlain;
+  bool on_device = false;  // D and base are made by boss_plan.cu (D_size, base_size entries)
+  size_t D_size = 0, base_size = 0;
   int kind = kRyser;
   int parity0 = 0;
   int nd = 0, nb = 0, nf = 0;
@@ -115,6 +117,18 @@ struct HostSweep {
   std::vector<int> fbias;
   int ff_exp = 0;  // sum_f (p_f + 1 - fx_f): the float-pair products' scale
 };
+
+// What boss_plan.cu needs to make one sweep's rows on the GPU.
+struct PlanItem {
+  int32_t layout, nd, nd_all, nf;  // nd_all: with the held digit, last
+  int32_t glynn, digits_are_outputs;
+  int64_t mat_off, base_off;       // its rows and base in the pool
+  uint16_t digit[kMaxDigits + 1], factor[kMaxFactors];
+  uint8_t mult[kMaxDigits + 1];
+};
+// max_entries: the most digits x factors of an item (at most 65 x 32: 33 KB of shared memory).
+cudaError_t launch_plan_rows(const PlanItem* items, int n, const double2* U, int m, int max_entries, longlong2* pool,
+                             SweepProblem* probs, cudaStream_t st);
 
 // Arithmetic of the all-minors sweeps (boss_minors_arithmetic): 0 float pairs
 // where the kernel exists for the factor count, 1 FP64.
@@ -166,7 +180,8 @@ int ensure_pinned(Context* cx, size_t bytes);
 // Uploads a list of sweeps (all of one sweep_class), launches the sweep
 // and the reduction, copies the results back.  results: one complex per sweep
 // (perms) or nd_max complex per sweep (all-minors).
-int run_sweeps(Context* cx, const std::vector<HostSweep>& sweeps, bool minors, int nd_max, double2* results_host);
+int run_sweeps(Context* cx, const std::vector<HostSweep>& sweeps, bool minors, int nd_max, double2* results_host,
+               const double* matrix = nullptr, int m = 0);  // the matrix of sweeps whose rows the device makes
 
 // Permanents of at most kSmallPermMax particles, 1 to 128 GPU threads each (Glynn's
 // formula in registers, no sweep planning; m <= 65536): by_l[l] lists the requests k with
@@ -183,7 +198,7 @@ int small_perm_batch(Context* cx, const double* matrix, int m, int len, const in
 // gradient kernel.
 enum PlanFor : int { kPlanAny = 0, kPlanTemplated = 1, kPlanFP64 = 2, kPlanGrad = 3 };
 int plan_permanent(const double* U, int m, const int32_t* S, const int32_t* T, int len, int variant, HostSweep& hs,
-                   bool& needs_sweep, double2& value, PlanFor plan = kPlanAny);
+                   bool& needs_sweep, double2& value, PlanFor plan = kPlanAny, bool on_device = false);
 
 // Sweeps of one launch share the factor count and the kernel: class 2 nf + quad.
 constexpr int kSweepClasses = 2 * (kMaxFactors + 1);
