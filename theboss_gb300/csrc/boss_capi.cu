@@ -113,13 +113,16 @@ static void describe_sweep(const HostSweep& h, int64_t n_threads, int group, Swe
 // aligned groups that sum their partials in the sweep (returned: the group's size):
 // the largest that costs no sweep more than 2 % of its threads, so that the
 // reduction reads that many times fewer rows (one k = 21 all-minors sweep: 21 rows of
-// 39 k partials, 0.36 ms in the reduction without groups).
-static int split_threads(const std::vector<HostSweep>& sweeps, int64_t resident, bool minors,
+// 39 k partials, 0.36 ms in the reduction without groups).  sm_count = 0: launches that
+// leave SMs idle are not spread over them (fewer partials).
+static int split_threads(const std::vector<HostSweep>& sweeps, int64_t resident, bool minors, int sm_count,
                          std::vector<int64_t>& nthr) {
   const int low = sweeps[0].layout == kRowsQuad ? 2 : 0;
   std::vector<uint64_t> codes(sweeps.size());
-  for (size_t p = 0; p < sweeps.size(); ++p) codes[p] = sweeps[p].total_codes >> low;
-  partition_threads(codes, resident, nthr, kMinCodesPerThread >> low);
+  double total = 0.0;
+  for (size_t p = 0; p < sweeps.size(); ++p) total += (double)(codes[p] = sweeps[p].total_codes >> low);
+  partition_threads(codes, resident, nthr,
+                    min_codes_per_thread(total, kMinCodesPerThread >> low, 1, low ? kQuadWalkers : 128, sm_count));
   int G = minors ? 32 : low ? 8 : 1;  // what the kernels can sum
   for (int64_t t : nthr)
     while (G > 1 && (double)(t / G * G) < 0.98 * (double)t) G >>= 1;
@@ -190,7 +193,7 @@ static int sweeps_prepare(Context* cx, const std::vector<HostSweep>& sweeps, boo
                               quad     ? quad_resident_walkers(B.nf, rows, minors, cx->sm_count)
                               : minors ? sweep_resident_minors(B.nf, rows, cx->sm_count, B.ff)
                                        : sweep_resident_threads(B.nf, op, cx->sm_count),
-                              minors, nthr);
+                              minors, cx->sm_count, nthr);
   std::vector<SweepProblem> probs(n);
   int64_t pool_n = 0, threads = 0, parts = 0;
   for (int p = 0; p < n; ++p) {
@@ -1215,7 +1218,9 @@ extern "C" int boss_perm_batch_noalloc(const double* matrix, int32_t m, const in
   std::vector<double2> direct_val;
   std::vector<NoAllocGroup> groups;
   size_t o_dval = 0, direct_bytes = 0, need_bytes = 0;
-  for (PlanFor plan : {kPlanFP64, kPlanTemplated}) {
+  // So is, before that, one whose partials are too many with few codes a thread.
+  const struct { PlanFor plan; int spread; } attempts[] = {{kPlanFP64, dev->sm_count}, {kPlanFP64, 0}, {kPlanTemplated, 0}};
+  for (const auto& at : attempts) {
   for (int c = 0; c < kSweepClasses; ++c) {
     by_class[c].clear();
     which[c].clear();
@@ -1228,7 +1233,7 @@ extern "C" int boss_perm_batch_noalloc(const double* matrix, int32_t m, const in
     bool need = false;
     double2 v = make_double2(0.0, 0.0);
     st = plan_permanent(matrix, m, input_states + (size_t)k * len, output_states + (size_t)k * len, len, variant, hs,
-                        need, v, plan);
+                        need, v, at.plan);
     if (st) return st;
     if (need) {
       const int c = sweep_class(hs);
@@ -1251,7 +1256,7 @@ extern "C" int boss_perm_batch_noalloc(const double* matrix, int32_t m, const in
     G.group = split_threads(sw,
                             sw[0].layout == kRowsQuad ? quad_resident_walkers(nf, 0, false, dev->sm_count)
                                                       : sweep_resident_threads(nf, SweepOp::kPerm, dev->sm_count),
-                            false, G.nthr);
+                            false, at.spread, G.nthr);
     int64_t pool_n = 0;
     for (int p = 0; p < n; ++p) {
       pool_n += (int64_t)(sw[p].D.size() + sw[p].base.size());

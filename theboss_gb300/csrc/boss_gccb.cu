@@ -2008,7 +2008,7 @@ static int gccb_prepare(Context* cx, const double* matrix, int n_mats, int m, Dr
     if (same) {  // one small descriptor instead of a per-sample table
       code0 >>= low;
       const double total = (double)code0 * Ak;
-      const double want = std::max<double>(Ak, std::min<double>((double)resident, total / (kMinCodesPerThread >> low)));
+      const double want = std::max<double>(Ak, std::min<double>((double)resident, total / min_codes_per_thread(total, kMinCodesPerThread >> low, 1, block, cx->sm_count)));
       int64_t tps = std::max<int64_t>(1, std::min<int64_t>((int64_t)code0, (int64_t)(want / Ak)));
       const LevelTune lt = level_tune(f64, k, Ak);
       if (lt.shift > 0) tps = std::min<int64_t>((int64_t)code0, tps << lt.shift);
@@ -2046,8 +2046,9 @@ static int gccb_prepare(Context* cx, const double* matrix, int n_mats, int m, Dr
       const LevelTune lt = level_tune(f64, k, Ak);
       const int64_t res = lt.shift >= 0 ? resident << lt.shift : std::max<int64_t>(1, resident >> -lt.shift);
       std::vector<uint64_t> steps(codes);
-      for (uint64_t& c : steps) c >>= low;
-      partition_threads(steps, res, nthr, kMinCodesPerThread >> low);
+      double total = 0.0;
+      for (uint64_t& c : steps) total += (double)(c >>= low);
+      partition_threads(steps, res, nthr, min_codes_per_thread(total, kMinCodesPerThread >> low, 1, block, cx->sm_count));
     }
     auto& t = tab[k];
     t.resize(Ak);

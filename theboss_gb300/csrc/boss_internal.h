@@ -64,12 +64,23 @@ cudaError_t launch_minors_reduce(const SweepProblem* probs, int n_probs, int row
                                  double2* out, int nd_max, cudaStream_t st, bool ff = false);
 
 // Splits `n_codes` codes over at most `resident` threads, proportionally, at
-// least one thread per sweep and at least kMinCodesPerThread codes per thread.
+// least one thread per sweep and at least min_codes codes per thread.
 constexpr int kFFMaxFactors = 24;      // float-pair all-minors: above this the sums exhaust the registers
 constexpr int kFFPermMaxFactors = 32;  // float-pair permanents
 constexpr int64_t kMinCodesPerThread = 8;
 void partition_threads(const std::vector<uint64_t>& n_codes, int64_t resident, std::vector<int64_t>& n_threads,
                        int64_t min_codes = kMinCodesPerThread);
+// The fewest codes (steps of four for the quad kernels) a thread takes in a launch of
+// `codes`: `most` amortise a thread's first sums and its row of partials while the GPU
+// is full, but below one block of `block` threads or walkers per SM the launch lasts as
+// long as one thread's chain, so it halves down to `least`.  16 samples of 8 photons,
+// two input modes doubly occupied: 15 kernels of 254 us in all with 8 codes a thread,
+// 148 with one; one k = 10 all-minors call: 53 and 40 us.
+inline int64_t min_codes_per_thread(double codes, int64_t most, int64_t least, int block, int sm_count) {
+  int64_t c = most;
+  while (c > least && codes < (double)c * block * sm_count) c >>= 1;
+  return c;
+}
 // log2 of the codes every range of a sweep starts at a multiple of: the largest
 // (at most 6, at most the nb binary digits) that makes the longest range at most
 // 1/32 longer than an even split.  Lanes of a warp then flip the same low digit
