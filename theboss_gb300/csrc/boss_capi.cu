@@ -914,11 +914,13 @@ int boss_perm_grad_batch(const double* matrix, int32_t m, const int32_t* input_s
     const int n = (int)sw.size();
     if (n == 0) continue;
     // walkers in proportion to the codes, at least 32 codes each (a walker also leaves
-    // a (nd + 1) x nf slice), whole warps of 8, one wave of resident warps
+    // a (nd + 1) x nf slice; 4 where that leaves SMs idle: one gradient at n = 14 takes
+    // 134 us with 32, 70 with 4), whole warps of 8, one wave of resident warps
     double total = 0.0;
     for (const HostSweep& h : sw) total += (double)h.total_codes;
     const int64_t resident = grad_resident_walkers(nf, cx->sm_count);
-    const double want = std::max<double>(n, std::min<double>((double)resident, total / 32.0));
+    const int64_t least = min_codes_per_thread(total, 32, 4, kQuadWalkers, cx->sm_count);
+    const double want = std::max<double>(n, std::min<double>((double)resident, total / (double)least));
     const int F = grad_factors(nf);
     std::vector<SweepProblem> probs(n);
     int64_t pool_n = 0, walkers = 0, gparts = 0;
@@ -949,7 +951,9 @@ int boss_perm_grad_batch(const double* matrix, int32_t m, const int32_t* input_s
     const size_t arena_bytes = off, up = device_rows ? o_pool : arena_bytes;
     const size_t out_g = (size_t)n * row, out_p = (size_t)n;
     if ((st = ensure(cx->plans, arena_bytes))) return st;
-    if ((st = ensure(cx->gpart, sizeof(double2) * std::max<int64_t>(gparts, 1)))) return st;
+    const int parts = grad_reduce_parts(walkers, n, row, cx->sm_count);
+    const int64_t mid = parts > 1 ? (int64_t)n * parts * (row + 1) : 0;
+    if ((st = ensure(cx->gpart, sizeof(double2) * std::max<int64_t>(gparts + mid, 1)))) return st;
     if ((st = ensure(cx->pperm, sizeof(double2) * std::max<int64_t>(walkers / 8, 1)))) return st;
     if ((st = ensure(cx->out, sizeof(double2) * (out_g + out_p)))) return st;
     if ((st = ensure_pinned(cx, std::max(up, sizeof(double2) * (out_g + out_p))))) return st;
@@ -981,7 +985,8 @@ int boss_perm_grad_batch(const double* matrix, int32_t m, const int32_t* input_s
         cudaSuccess)
       return fail_cuda(e, "gradient sweep");
     double2* dout = (double2*)cx->out.ptr;
-    if ((e = launch_grad_reduce(nf, dp, n, gpart, ppart, dout, dout + out_g, row, cx->stream)) != cudaSuccess)
+    if ((e = launch_grad_reduce(nf, dp, n, gpart, ppart, gpart + gparts, parts, dout, dout + out_g, row,
+                                cx->stream)) != cudaSuccess)
       return fail_cuda(e, "gradient reduce");
     e = cudaMemcpyAsync(cx->pinned, dout, sizeof(double2) * (out_g + out_p), cudaMemcpyDeviceToHost, cx->stream);
     if (e != cudaSuccess) return fail_cuda(e, "D2H gradients");

@@ -165,8 +165,12 @@ __global__ void __launch_bounds__(128, M <= 3 ? 5 : M <= 5 ? 4 : 3) grad_sweep_k
   if (live && lane == 0) ppart[walker >> 3] = make_double2(pr, pi);
 }
 
-// Sums of the warps' slices: block (sweep, 64 entries), entry e = (row * M + i) * 4 +
-// lane & 3 by four threads, each a quarter of the walkers in order, then the four.
+// Sums of the warps' slices: block (sweep, 64 entries, part z of the walkers), entry
+// e = (row * M + i) * 4 + lane & 3 by four threads, each every fourth walker of the
+// part in order, then the four.  Bound by reading the slices; few sweeps fill the GPU
+// only if a sweep's walkers are split over blocks (one gradient at n = 18: 312 us with
+// one part, 154 with 51, of which most is the sweep).  One part writes the gradients and permanents, several
+// write gridDim.z rows of row_stride + 1 sums a sweep (the permanent's last) to grad_out.
 __global__ void __launch_bounds__(256) grad_reduce_kernel(const SweepProblem* __restrict__ probs,
                                                           const double2* __restrict__ gpart,
                                                           const double2* __restrict__ ppart,
@@ -174,14 +178,28 @@ __global__ void __launch_bounds__(256) grad_reduce_kernel(const SweepProblem* __
                                                           double2* __restrict__ perm_out, int row_stride, int F) {
   __shared__ double2 sum[256];
   const SweepProblem& P = probs[blockIdx.x];
-  const int ne = (P.nd + P.fixed_digit) * F, M = F >> 2;
+  const int ne = (P.nd + P.fixed_digit) * F;
   const int64_t warps = P.n_threads >> 3, slice = (int64_t)ne * 8;
+  const int parts = (int)gridDim.z;
+  const int64_t w0 = warps * blockIdx.z / parts, w1 = warps * (blockIdx.z + 1) / parts;
+  double2* g_out;
+  double2* p_out;
+  double scale;
+  if (parts == 1) {
+    g_out = grad_out + (size_t)P.out_idx * row_stride;
+    p_out = perm_out + P.out_idx;
+    scale = P.scale;
+  } else {
+    g_out = grad_out + ((size_t)blockIdx.x * parts + blockIdx.z) * (row_stride + 1);
+    p_out = g_out + row_stride;
+    scale = 1.0;
+  }
   const int part = threadIdx.x >> 6, e = blockIdx.y * 64 + (threadIdx.x & 63);
   double ar = 0.0, ai = 0.0;
   if (e < ne) {
     const double2* g = gpart + P.part_off + (int64_t)(e >> 2) * 32 + (e & 3);
 #pragma unroll 8  // independent loads in flight
-    for (int64_t q = part; q < warps * 8; q += 4) {
+    for (int64_t q = 8 * w0 + part; q < 8 * w1; q += 4) {
       const double2 v = g[(q >> 3) * slice + 4 * (q & 7)];
       ar += v.x;
       ai += v.y;
@@ -194,13 +212,12 @@ __global__ void __launch_bounds__(256) grad_reduce_kernel(const SweepProblem* __
       ar += sum[threadIdx.x + 64 * p].x;
       ai += sum[threadIdx.x + 64 * p].y;
     }
-    const int row = e / F, r = e - row * F;  // r = 4 i + lane: the factor
-    grad_out[(size_t)P.out_idx * row_stride + (size_t)row * F + r] = make_double2(ar * P.scale, ai * P.scale);
+    g_out[e] = make_double2(ar * scale, ai * scale);  // e = row F + 4 i + lane: the factor
   }
   if (blockIdx.y == 0) {
     __syncthreads();
     ar = ai = 0.0;
-    for (int64_t q = threadIdx.x; q < warps; q += 256) {
+    for (int64_t q = w0 + threadIdx.x; q < w1; q += 256) {
       const double2 v = ppart[(P.thread_begin >> 3) + q];
       ar += v.x;
       ai += v.y;
@@ -214,8 +231,28 @@ __global__ void __launch_bounds__(256) grad_reduce_kernel(const SweepProblem* __
       }
       __syncthreads();
     }
-    if (threadIdx.x == 0) perm_out[P.out_idx] = make_double2(sum[0].x * P.scale, sum[0].y * P.scale);
+    if (threadIdx.x == 0) *p_out = make_double2(sum[0].x * scale, sum[0].y * scale);
   }
+}
+
+// The parts' sums: one thread per entry (the permanent's last), the parts in order.
+__global__ void __launch_bounds__(128) grad_parts_kernel(const SweepProblem* __restrict__ probs,
+                                                         const double2* __restrict__ mid, int parts,
+                                                         double2* __restrict__ grad_out,
+                                                         double2* __restrict__ perm_out, int row_stride, int F) {
+  const SweepProblem& P = probs[blockIdx.x];
+  const int e = blockIdx.y * 128 + threadIdx.x, ne = (P.nd + P.fixed_digit) * F;
+  if (e > row_stride || (e >= ne && e < row_stride)) return;
+  const double2* v = mid + (size_t)blockIdx.x * parts * (row_stride + 1) + e;
+  double ar = 0.0, ai = 0.0;
+#pragma unroll 8  // independent loads in flight
+  for (int z = 0; z < parts; ++z) {
+    const double2 x = v[(size_t)z * (row_stride + 1)];
+    ar += x.x;
+    ai += x.y;
+  }
+  double2* o = e == row_stride ? perm_out + P.out_idx : grad_out + (size_t)P.out_idx * row_stride + e;
+  *o = make_double2(ar * P.scale, ai * P.scale);
 }
 
 constexpr int kGradMaxM = kMaxFactors / 4;
@@ -252,12 +289,21 @@ cudaError_t launch_grad_sweep(int nf, const SweepProblem* probs, int n_probs, co
   return cudaGetLastError();
 }
 
+int grad_reduce_parts(int64_t walkers, int n_probs, int row_stride, int sm_count) {
+  const int64_t blocks = (int64_t)n_probs * ((row_stride + 63) / 64);
+  const int64_t fill = (2 * sm_count + blocks - 1) / blocks;
+  return (int)std::max<int64_t>(1, std::min<int64_t>(fill, walkers / n_probs / 128));
+}
+
 cudaError_t launch_grad_reduce(int nf, const SweepProblem* probs, int n_probs, const double2* gpart,
-                               const double2* ppart, double2* grad_out, double2* perm_out, int row_stride,
-                               cudaStream_t st) {
+                               const double2* ppart, double2* mid, int parts, double2* grad_out, double2* perm_out,
+                               int row_stride, cudaStream_t st) {
   if (n_probs <= 0) return cudaSuccess;
-  grad_reduce_kernel<<<dim3((unsigned)n_probs, (unsigned)((row_stride + 63) / 64)), 256, 0, st>>>(
-      probs, gpart, ppart, grad_out, perm_out, row_stride, grad_factors(nf));
+  grad_reduce_kernel<<<dim3((unsigned)n_probs, (unsigned)((row_stride + 63) / 64), (unsigned)parts), 256, 0, st>>>(
+      probs, gpart, ppart, parts > 1 ? mid : grad_out, perm_out, row_stride, grad_factors(nf));
+  if (parts > 1)
+    grad_parts_kernel<<<dim3((unsigned)n_probs, (unsigned)(row_stride / 128 + 1)), 128, 0, st>>>(
+        probs, mid, parts, grad_out, perm_out, row_stride, grad_factors(nf));
   return cudaGetLastError();
 }
 

@@ -50,9 +50,12 @@ __host__ __device__ inline int grad_factors(int nf) { return (nf + 3) / 4 * 4; }
 inline int64_t grad_slice(int rows, int nf) { return (int64_t)rows * grad_factors(nf) * 8; }
 cudaError_t launch_grad_sweep(int nf, const SweepProblem* probs, int n_probs, const longlong2* pool, int64_t walkers,
                               double2* gpart, double2* ppart, cudaStream_t st);
+// parts of the walkers that blocks of their own sum, into parts * (row_stride + 1)
+// entries of mid per sweep: few sweeps leave SMs idle otherwise.
+int grad_reduce_parts(int64_t walkers, int n_probs, int row_stride, int sm_count);
 cudaError_t launch_grad_reduce(int nf, const SweepProblem* probs, int n_probs, const double2* gpart,
-                               const double2* ppart, double2* grad_out, double2* perm_out, int row_stride,
-                               cudaStream_t st);
+                               const double2* ppart, double2* mid, int parts, double2* grad_out, double2* perm_out,
+                               int row_stride, cudaStream_t st);
 // Whether the float-pair all-minors / single-permanent kernel exists for nf factors.
 bool minors_ff_available(int nf);
 bool perm_ff_available(int nf);
