@@ -42,6 +42,7 @@
 #include "../../include/boss.h"
 #include "boss_internal.h"
 #include "boss_quad.cuh"
+#include "boss_sweep_kernels.cuh"
 
 namespace boss {
 
@@ -862,216 +863,83 @@ __global__ void __launch_bounds__(128) gccb_partials_reduce_kernel(const SweepPr
   if (threadIdx.x == 0) out[(size_t)j * 32 + d] = make_double2(sx[0], sy[0]);
 }
 
-// kF64: the minors, the Laplace step, |.|^2 and the pmf are FP64 (the default);
-// otherwise float pairs on the FP32 pipe (the opt-in float-pair arithmetic).
-template <bool kF64>
-__global__ void __launch_bounds__(kFinWarps * 32, 8) gccb_finalize_kernel(FinalizeArgs a) {
-  __shared__ double2 sub_s[kFinWarps][32];
-  __shared__ float4 subf_s[kFinWarps][32];
-  __shared__ uint8_t dm_s[kFinWarps][32];
-  __shared__ uint8_t mult_s[kFinWarps][32];
-  __shared__ uint8_t fm_s[kFinWarps][32];
-  __shared__ double pmf_s[kFinWarps][256];
-  __shared__ float cn_s[kFinWarps][32];  // |c_d|_1 2^-Ec (the pmf error bound)
-  __shared__ int4 climb_s[kFinWarps][32];  // FP64 pmf: the minors as 27-bit limbs (re lo, re hi, im lo, im hi)
-  __shared__ int2 cnb_s[kFinWarps][32];    // and -Im as limbs
-  __shared__ uint8_t srow_s[kFinWarps][256];  // the sample's input and output occupations, kept here
-  __shared__ uint8_t trow_s[kFinWarps][256];  // while the kernel updates them (written through to S, T)
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int j = blockIdx.x * kFinWarps + w;
-  if (j >= a.A) return;
+// A warp's working set in shared memory.
+struct FinShared {
+  double2 sub[32];
+  float4 subf[32];
+  int4 climb[32];  // FP64 pmf: the minors as 27-bit limbs (re lo, re hi, im lo, im hi)
+  int2 cnb[32];    // and -Im as limbs
+  double pmf[256];
+  float cn[32];  // |c_d|_1 2^-Ec (the pmf error bound)
+  uint8_t dm[32], mult[32], fm[32];
+  uint8_t srow[256];  // the sample's input and output occupations, kept here
+  uint8_t trow[256];  // while the kernel updates them (written through to S, T)
+};
+
+// A sample's bookkeeping: what a lane holds of it.
+struct FinSample {
+  size_t drow;    // the row of its replayed draws
+  int idxv, pmv;  // lane's randint result and particle mode
+  uint32_t remw;  // particles not yet popped (one word per lane 0..7)
+};
+
+// The digits and factors of a sample's next sweep (their modes in FinShared).
+struct FinDigits {
+  int nb, nf, nd, held;  // binary digits, factors, digits; held: a binary digit is held at r = 0 (and comes last)
+};
+
+__device__ __forceinline__ FinSample fin_load(const FinalizeArgs& a, int k, int j, FinShared& sh, int lane) {
   const int m = a.m;
-  const longlong2* Ufxs = a.Ufx + (size_t)j * a.mstride;  // the sample's fixed-point matrix
-  const int32_t* rowfx = a.rowfx + (a.mstride ? (size_t)j * m : 0);
-  uint8_t* S = a.S + (size_t)j * m;
-  uint8_t* T = a.T + (size_t)j * m;
+  const uint8_t* S = a.S + (size_t)j * m;
+  const uint8_t* T = a.T + (size_t)j * m;
   // Everything the particle bookkeeping needs, loaded up front (independent
   // loads, in flight during the sums below): the occupations, the sample's
   // randint results and particle modes (one per lane; at most 32 particles), and
   // its set of particles not yet popped (one word per lane 0..7).
-  const size_t drow = (size_t)a.order[j] * a.n;  // this sample's replayed draws
+  FinSample me;
+  me.drow = (size_t)a.order[j] * a.n;
   for (int i = lane; i < m; i += 32) {
-    srow_s[w][i] = S[i];
-    trow_s[w][i] = T[i];
+    sh.srow[i] = S[i];
+    sh.trow[i] = T[i];
   }
-  const int idxv = (lane < a.n) ? (int)a.idx[drow + lane] : 0;
-  const int pmv = (lane < a.n) ? (int)a.pmode[drow + lane] : 0;
-  uint32_t remw = 0;
-  if (a.k == 1) {
+  me.idxv = (lane < a.n) ? (int)a.idx[me.drow + lane] : 0;
+  me.pmv = (lane < a.n) ? (int)a.pmode[me.drow + lane] : 0;
+  me.remw = 0;
+  if (k == 1) {
     const int np = a.npart[a.order[j]];
     const int lo = lane * 32;
-    if (lane < 8) remw = (np >= lo + 32) ? 0xffffffffu : (np > lo ? ((1u << (np - lo)) - 1u) : 0u);
+    if (lane < 8) me.remw = (np >= lo + 32) ? 0xffffffffu : (np > lo ? ((1u << (np - lo)) - 1u) : 0u);
   } else if (lane < 8) {
-    remw = a.rem[(size_t)j * 8 + lane];
+    me.remw = a.rem[(size_t)j * 8 + lane];
   }
   __syncwarp();
-  int nd;
-  if (a.k == 1) {
-    // one particle: the minors are the input occupations themselves
-    // (bs_submatrices_permanent_calculator_base.py:157-158)
-    const int mode = __shfl_sync(0xffffffffu, pmv, pop_particle_warp(remw, __shfl_sync(0xffffffffu, idxv, 0), lane));
-    if (lane == 0) {
-      srow_s[w][mode] = 1;
-      S[mode] = 1;
-      subf_s[w][0] = make_float4(1.0f, 0.0f, 0.0f, 0.0f);
-      sub_s[w][0] = make_double2(1.0, 0.0);
-      dm_s[w][0] = (uint8_t)mode;
-      mult_s[w][0] = 1;
-    }
-    nd = 1;
-  } else {
-    const SweepProblem& P = a.probs_cur[j];
-    nd = P.nd + P.low + P.fixed_digit;  // the held (halved) digit's minor is the last row
-    const int64_t parts = P.n_threads / P.group;
-    if (a.cur_ff) {
-      // float-pair partials: summed as float pairs in a fixed order, scaled by the
-      // problem's power of two, exactly in float when that power is a normal float
-      // (always, for factors of comparable size); otherwise in FP64 below
-      const float4* fp = reinterpret_cast<const float4*>(a.partials) + P.part_off;
-      const int sc_exp = (int)((__double_as_longlong(P.scale) >> 52) & 0x7FF) - 1023;
-      const bool sc_float = sc_exp >= -126 && sc_exp <= 127;
-      const float sc = sc_float ? __double2float_rn(P.scale) : 1.0f;
-      if (parts <= 64) {
-        if (lane < nd) {
-          float rh = 0.0f, rl = 0.0f, ih = 0.0f, il = 0.0f;
-#pragma unroll 8
-          for (int64_t q = 0; q < parts; ++q) {  // unrolled: 8 loads in flight
-            const float4 v = fp[q * nd + lane];
-            ff_acc(rh, rl, 1.0f, v.x, v.y);
-            ff_acc(ih, il, 1.0f, v.z, v.w);
-          }
-          subf_s[w][lane] = make_float4(rh * sc, rl * sc, ih * sc, il * sc);
-        }
-      } else {
-        for (int d = 0; d < nd; ++d) {
-          float rh = 0.0f, rl = 0.0f, ih = 0.0f, il = 0.0f;
-          for (int64_t q = lane; q < parts; q += 32) {
-            const float4 v = fp[q * nd + d];
-            ff_acc(rh, rl, 1.0f, v.x, v.y);
-            ff_acc(ih, il, 1.0f, v.z, v.w);
-          }
-#pragma unroll
-          for (int off = 16; off > 0; off >>= 1) {  // fixed butterfly order
-            const float orh = __shfl_xor_sync(0xffffffffu, rh, off), orl = __shfl_xor_sync(0xffffffffu, rl, off);
-            const float oih = __shfl_xor_sync(0xffffffffu, ih, off), oil = __shfl_xor_sync(0xffffffffu, il, off);
-            ff_acc(rh, rl, 1.0f, orh, orl);
-            ff_acc(ih, il, 1.0f, oih, oil);
-          }
-          if (lane == d) subf_s[w][d] = make_float4(rh * sc, rl * sc, ih * sc, il * sc);
-        }
-      }
-    } else if (a.reduced) {  // summed by gccb_partials_reduce_kernel
-      if (lane < nd) {
-        const double2 v = a.reduced[(size_t)j * 32 + lane];
-        sub_s[w][lane] = make_double2(v.x * P.scale, v.y * P.scale);
-      }
-    } else {
-      // FP64 partials (parts x nd), summed in a fixed order.  Every FP64
-      // instruction holds the pipe for a whole warp however few lanes are active,
-      // so the lanes are spread over the partials: either gc <= 32 / nd groups of
-      // nd lanes (lane g * nd + d sums rows g, g + gc, .. of digit d, then lane d
-      // adds up the gc group sums; gc = 1 is one lane per digit), or, with many
-      // partials, all 32 lanes stripe over each digit's rows and a butterfly sums
-      // them; whichever issues fewer FP64 instructions.
-      int gc = 1;
-      int64_t cost_groups = 2 * (parts - 1);  // each group's first row is a copy, not an add
-      for (int g2 = 2; g2 * nd <= 32 && g2 <= parts; ++g2) {
-        const int64_t c = 2 * ((parts + g2 - 1) / g2 - 1) + 2 * (g2 - 1);
-        if (c < cost_groups) {
-          cost_groups = c;
-          gc = g2;
-        }
-      }
-      const int64_t cost_stripes = (int64_t)nd * (2 * ((parts + 31) / 32) + 10);
-      if (cost_groups <= cost_stripes) {
-        const int g = lane / nd, d = lane - g * nd;
-        double sx = 0.0, sy = 0.0;
-        if (g < gc && parts >= 8 * gc) {
-          // long sums (the top levels, where one warp has the SM's FP64 unit to
-          // itself): four interleaved chains, rows g + (4 i + c) gc in chain c,
-          // combined in a fixed order, a quarter of one chain's latency
-          double x0 = 0.0, y0 = 0.0, x1 = 0.0, y1 = 0.0, x2 = 0.0, y2 = 0.0, x3 = 0.0, y3 = 0.0;
-          int64_t q = g;
-#pragma unroll 4
-          for (; q + 3 * gc < parts; q += 4 * gc) {
-            const double2 v0 = a.partials[P.part_off + q * nd + d];
-            const double2 v1 = a.partials[P.part_off + (q + gc) * nd + d];
-            const double2 v2 = a.partials[P.part_off + (q + 2 * gc) * nd + d];
-            const double2 v3 = a.partials[P.part_off + (q + 3 * gc) * nd + d];
-            x0 += v0.x;
-            y0 += v0.y;
-            x1 += v1.x;
-            y1 += v1.y;
-            x2 += v2.x;
-            y2 += v2.y;
-            x3 += v3.x;
-            y3 += v3.y;
-          }
-          for (; q < parts; q += gc) {
-            const double2 v = a.partials[P.part_off + q * nd + d];
-            x0 += v.x;
-            y0 += v.y;
-          }
-          sx = (x0 + x1) + (x2 + x3);
-          sy = (y0 + y1) + (y2 + y3);
-        } else if (g < gc) {  // gc <= parts: every group has a first row
-          const double2 v0 = a.partials[P.part_off + (int64_t)g * nd + d];
-          sx = v0.x;
-          sy = v0.y;
-#pragma unroll 8
-          for (int64_t q = g + gc; q < parts; q += gc) {
-            const double2 v = a.partials[P.part_off + q * nd + d];
-            sx += v.x;
-            sy += v.y;
-          }
-        }
-        sub_s[w][lane] = make_double2(sx, sy);
-        __syncwarp();
-        if (lane < nd) {
-          double tx = sx, ty = sy;  // group 0 is this lane's own sum
-          for (int gg = 1; gg < gc; ++gg) {
-            const double2 v = sub_s[w][gg * nd + lane];
-            tx += v.x;
-            ty += v.y;
-          }
-          sx = tx * P.scale;
-          sy = ty * P.scale;
-        }
-        __syncwarp();
-        if (lane < nd) sub_s[w][lane] = make_double2(sx, sy);
-      } else {  // many partials: the lanes stripe over them, then a fixed-order warp
-                // sum; two digits at a time (independent chains in flight)
-        for (int d = 0; d < nd; d += 2) {
-          const int d1 = (d + 1 < nd) ? d + 1 : d;  // an odd last digit is summed twice, stored once
-          double sx = 0.0, sy = 0.0, tx = 0.0, ty = 0.0;
-#pragma unroll 4
-          for (int64_t q = lane; q < parts; q += 32) {
-            const double2 v = a.partials[P.part_off + q * nd + d];
-            const double2 u = a.partials[P.part_off + q * nd + d1];
-            sx += v.x;
-            sy += v.y;
-            tx += u.x;
-            ty += u.y;
-          }
-#pragma unroll
-          for (int o = 16; o > 0; o >>= 1) {  // warp_sum's butterfly, the four sums interleaved
-            sx += __shfl_xor_sync(0xffffffffu, sx, o);
-            sy += __shfl_xor_sync(0xffffffffu, sy, o);
-            tx += __shfl_xor_sync(0xffffffffu, tx, o);
-            ty += __shfl_xor_sync(0xffffffffu, ty, o);
-          }
-          if (lane == d) sub_s[w][d] = make_double2(sx * P.scale, sy * P.scale);
-          if (lane == d1 && d1 != d) sub_s[w][d1] = make_double2(tx * P.scale, ty * P.scale);
-        }
-      }
-    }
-    if (lane < nd) {
-      dm_s[w][lane] = a.dmode_cur[(size_t)j * 32 + lane];
-      mult_s[w][lane] = P.mult[lane];
-    }
+  return me;
+}
+
+// One particle: the minors are the input occupations themselves
+// (bs_submatrices_permanent_calculator_base.py:157-158).
+__device__ __forceinline__ void fin_first(const FinalizeArgs& a, int j, FinSample& me, FinShared& sh, int lane) {
+  uint8_t* S = a.S + (size_t)j * a.m;
+  const int mode = __shfl_sync(0xffffffffu, me.pmv, pop_particle_warp(me.remw, __shfl_sync(0xffffffffu, me.idxv, 0), lane));
+  if (lane == 0) {
+    sh.srow[mode] = 1;
+    S[mode] = 1;
+    sh.subf[0] = make_float4(1.0f, 0.0f, 0.0f, 0.0f);
+    sh.sub[0] = make_double2(1.0, 0.0);
+    sh.dm[0] = (uint8_t)mode;
+    sh.mult[0] = 1;
   }
   __syncwarp();
-  const double uu = a.uni[drow + (a.k - 1)];
+}
+
+// Level k's draw of an output mode from the nd minors in sh (FP64: sub, float pairs:
+// subf), kF64: the Laplace step, |.|^2 and the pmf in FP64 (the default); otherwise
+// float pairs on the FP32 pipe (the opt-in float-pair arithmetic).
+template <bool kF64>
+__device__ __forceinline__ void fin_draw(const FinalizeArgs& a, int k, int j, int nd, double uu, FinShared& sh,
+                                         int lane) {
+  const int m = a.m;
+  uint8_t* T = a.T + (size_t)j * m;
   const int K = (m + 31) >> 5;  // contiguous outputs per lane in the cdf scan
   const int o0 = lane * K;
   const int full = m & ~31;
@@ -1108,12 +976,12 @@ __global__ void __launch_bounds__(kFinWarps * 32, 8) gccb_finalize_kernel(Finali
     // than its FP64 pipe; only |.|^2 (2 DFMA per output) stays on the FP64 pipe.
     const int4* UL = a.Ulimb + (size_t)j * a.mstride;
     const float* UA = a.Uabs + (size_t)j * a.mstride;
-    double* pmf = pmf_s[w];
+    double* pmf = sh.pmf;
     // the bound's scale: 2^-Ec, 2^Ec <= max_d |c_d|_1 < 2^(Ec + 1)
     double c1 = 0.0;
     double2 cv = make_double2(0.0, 0.0);
     if (lane < nd) {
-      cv = sub_s[w][lane];
+      cv = sh.sub[lane];
       c1 = fabs(cv.x) + fabs(cv.y);
     }
     const unsigned long long cb = warp_max_u64((unsigned long long)__double_as_longlong(c1));
@@ -1122,13 +990,13 @@ __global__ void __launch_bounds__(kFinWarps * 32, 8) gccb_finalize_kernel(Finali
     float cn = 0.0f;
     if (lane < nd) {
       cn = __double2float_ru(c1 * sc);  // in [0, 2)
-      cn_s[w][lane] = cn;
+      sh.cn[lane] = cn;
       // c * 2^(52 - Ec) (exact: a power of two; every component < 2^53), rounded
       const double s52 = sc * 4503599627370496.0;  // 2^52
       const long long A = __double2ll_rn(cv.x * s52), B = __double2ll_rn(cv.y * s52);
       const long long NB = -B;
-      climb_s[w][lane] = make_int4((int)(A & 0x7FFFFFF), (int)(A >> 27), (int)(B & 0x7FFFFFF), (int)(B >> 27));
-      cnb_s[w][lane] = make_int2((int)(NB & 0x7FFFFFF), (int)(NB >> 27));
+      sh.climb[lane] = make_int4((int)(A & 0x7FFFFFF), (int)(A >> 27), (int)(B & 0x7FFFFFF), (int)(B >> 27));
+      sh.cnb[lane] = make_int2((int)(NB & 0x7FFFFFF), (int)(NB >> 27));
     }
     const float csum = warp_sum_f(cn);  // sum_d |c_d|_1 2^-Ec
     __syncwarp();
@@ -1145,9 +1013,9 @@ __global__ void __launch_bounds__(kFinWarps * 32, 8) gccb_finalize_kernel(Finali
       float ao = 0.0f, bo = 0.0f;
 #pragma unroll 8  // independent gathers in flight
       for (int d = 0; d < nd; ++d) {
-        const int4 c = climb_s[w][d];  // a0 a1 b0 b1
-        const int2 nb = cnb_s[w][d];   // (-b)0 (-b)1
-        const int e = dm_s[w][d] * m + o;
+        const int4 c = sh.climb[d];  // a0 a1 b0 b1
+        const int2 nb = sh.cnb[d];   // (-b)0 (-b)1
+        const int e = sh.dm[d] * m + o;
         const int4 u = UL[e];          // x0 x1 y0 y1
         const float ua = UA[e];
         r2 += (long long)c.y * u.y + (long long)nb.y * u.w;
@@ -1156,7 +1024,7 @@ __global__ void __launch_bounds__(kFinWarps * 32, 8) gccb_finalize_kernel(Finali
         i2 += (long long)c.y * u.w + (long long)c.w * u.y;
         i1 += (long long)c.y * u.z + (long long)c.x * u.w + (long long)c.w * u.x + (long long)c.z * u.y;
         i0 += (long long)c.x * u.z + (long long)c.z * u.x;
-        ao = fmaf(cn_s[w][d], ua, ao);
+        ao = fmaf(sh.cn[d], ua, ao);
         bo += ua;
       }
       const double pr = limbs_to_double(r2, r1, r0, pexp);
@@ -1175,9 +1043,9 @@ __global__ void __launch_bounds__(kFinWarps * 32, 8) gccb_finalize_kernel(Finali
       if (oi < r) {
 #pragma unroll 4
         for (int d = c0; d < nd; d += s) {
-          const int4 c = climb_s[w][d];
-          const int2 nb = cnb_s[w][d];
-          const int e = dm_s[w][d] * m + full + oi;
+          const int4 c = sh.climb[d];
+          const int2 nb = sh.cnb[d];
+          const int e = sh.dm[d] * m + full + oi;
           const int4 u = UL[e];
           const float ua = UA[e];
           r2 += (long long)c.y * u.y + (long long)nb.y * u.w;
@@ -1186,7 +1054,7 @@ __global__ void __launch_bounds__(kFinWarps * 32, 8) gccb_finalize_kernel(Finali
           i2 += (long long)c.y * u.w + (long long)c.w * u.y;
           i1 += (long long)c.y * u.z + (long long)c.x * u.w + (long long)c.w * u.x + (long long)c.z * u.y;
           i0 += (long long)c.x * u.z + (long long)c.z * u.x;
-          ao = fmaf(cn_s[w][d], ua, ao);
+          ao = fmaf(sh.cn[d], ua, ao);
           bo += ua;
         }
       }
@@ -1259,36 +1127,36 @@ __global__ void __launch_bounds__(kFinWarps * 32, 8) gccb_finalize_kernel(Finali
     }
   } else {
     // ---- float pairs on the FP32 pipe (opt-in) ----
-    if (a.k > 1 && a.cur_ff && lane < nd) {  // a scale beyond the float range: apply it in FP64
+    if (k > 1 && a.cur_ff && lane < nd) {  // a scale beyond the float range: apply it in FP64
       const SweepProblem& P = a.probs_cur[j];
       const int sc_exp = (int)((__double_as_longlong(P.scale) >> 52) & 0x7FF) - 1023;
       if (!(sc_exp >= -126 && sc_exp <= 127)) {
-        const float4 u = subf_s[w][lane];
+        const float4 u = sh.subf[lane];
         float4 f;
         double_to_ff(ff_to_double(u.x, u.y) * P.scale, f.x, f.y);
         double_to_ff(ff_to_double(u.z, u.w) * P.scale, f.z, f.w);
-        subf_s[w][lane] = f;
+        sh.subf[lane] = f;
       }
     }
-    if (a.k > 1 && !a.cur_ff && lane < nd) {  // FP64 minors to float pairs
-      const double2 v = sub_s[w][lane];
+    if (k > 1 && !a.cur_ff && lane < nd) {  // FP64 minors to float pairs
+      const double2 v = sh.sub[lane];
       float4 f;
       double_to_ff(v.x, f.x, f.y);
       double_to_ff(v.y, f.z, f.w);
-      subf_s[w][lane] = f;
+      sh.subf[lane] = f;
     }
     __syncwarp();
     // the bound's scale: 2^-Ec, 2^Ec <= max_d |c_d|_1 < 2^(Ec + 1)
     float c1 = 0.0f;
     if (lane < nd) {
-      const float4 c = subf_s[w][lane];
+      const float4 c = sh.subf[lane];
       c1 = fabsf(c.x) + fabsf(c.z);
     }
     unsigned cbits = __float_as_uint(c1);
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) cbits = max(cbits, __shfl_xor_sync(0xffffffffu, cbits, off));
     const int Ec = (int)(cbits >> 23) - 127;
-    if (lane < nd) cn_s[w][lane] = scale_pow2f(c1, -Ec) * 1.0000002f;  // in [0, 2); the lo parts
+    if (lane < nd) sh.cn[lane] = scale_pow2f(c1, -Ec) * 1.0000002f;  // in [0, 2); the lo parts
     __syncwarp();
     const float eps2 = 2.0f * kMinorsErrFF;
     const float gam = 9.094947e-13f;  // 2^-40: the compensated dot products
@@ -1297,20 +1165,20 @@ __global__ void __launch_bounds__(kFinWarps * 32, 8) gccb_finalize_kernel(Finali
     // (stored in the warp's pmf row, float2 per output).
     const float4* UT = a.Uff + (size_t)j * a.mstride;
     const float* UA = a.Uabs + (size_t)j * a.mstride;
-    float2* pf = reinterpret_cast<float2*>(pmf_s[w]);
+    float2* pf = reinterpret_cast<float2*>(sh.pmf);
     for (int o = lane; o < full; o += 32) {
       float sr = 0.0f, cr = 0.0f, si = 0.0f, ci = 0.0f, ao = 0.0f, bo = 0.0f;
 #pragma unroll 4  // independent gathers in flight
       for (int d = 0; d < nd; ++d) {
-        const float4 c = subf_s[w][d];
-        const int e = dm_s[w][d] * m + o;
+        const float4 c = sh.subf[d];
+        const int e = sh.dm[d] * m + o;
         const float4 u = UT[e];
         const float ua = UA[e];
         ff_dot_acc(sr, cr, 1.0f, c.x, c.y, u.x, u.y);
         ff_dot_acc(sr, cr, -1.0f, c.z, c.w, u.z, u.w);
         ff_dot_acc(si, ci, 1.0f, c.x, c.y, u.z, u.w);
         ff_dot_acc(si, ci, 1.0f, c.z, c.w, u.x, u.y);
-        ao = fmaf(cn_s[w][d], ua, ao);
+        ao = fmaf(sh.cn[d], ua, ao);
         bo += ua;
       }
       pf[o] = ff_abs2(sr, cr, si, ci);
@@ -1326,15 +1194,15 @@ __global__ void __launch_bounds__(kFinWarps * 32, 8) gccb_finalize_kernel(Finali
       if (oi < r) {
 #pragma unroll 4  // independent gathers in flight
         for (int d = c0; d < nd; d += s) {
-          const float4 c = subf_s[w][d];
-          const int e = dm_s[w][d] * m + full + oi;
+          const float4 c = sh.subf[d];
+          const int e = sh.dm[d] * m + full + oi;
           const float4 u = UT[e];
           const float ua = UA[e];
           ff_dot_acc(sr, cr, 1.0f, c.x, c.y, u.x, u.y);
           ff_dot_acc(sr, cr, -1.0f, c.z, c.w, u.z, u.w);
           ff_dot_acc(si, ci, 1.0f, c.x, c.y, u.z, u.w);
           ff_dot_acc(si, ci, 1.0f, c.z, c.w, u.x, u.y);
-          ao = fmaf(cn_s[w][d], ua, ao);
+          ao = fmaf(sh.cn[d], ua, ao);
           bo += ua;
         }
       }
@@ -1388,7 +1256,7 @@ __global__ void __launch_bounds__(kFinWarps * 32, 8) gccb_finalize_kernel(Finali
       if (__any_sync(0xffffffffu, near)) {
         for (int o = lane; o < m; o += 32) {  // the pmf as doubles, in place (same 8-byte slots)
           const float2 v = pf[o];
-          pmf_s[w][o] = ff_to_double(v.x, v.y);
+          sh.pmf[o] = ff_to_double(v.x, v.y);
         }
       }
     }
@@ -1399,83 +1267,86 @@ __global__ void __launch_bounds__(kFinWarps * 32, 8) gccb_finalize_kernel(Finali
     __syncwarp();
     double total = 0.0;
     if (lane == 0)
-      for (int o = 0; o < m; ++o) total += pmf_s[w][o];
+      for (int o = 0; o < m; ++o) total += sh.pmf[o];
     total = __shfl_sync(0xffffffffu, total, 0);
-    for (int o = lane; o < m; o += 32) pmf_s[w][o] = pmf_s[w][o] / total;
+    for (int o = lane; o < m; o += 32) sh.pmf[o] = sh.pmf[o] / total;
     __syncwarp();
     if (lane == 0) {
       double acc = 0.0;
       for (int o = 0; o < m; ++o) {
-        acc += pmf_s[w][o];
-        pmf_s[w][o] = acc;
+        acc += sh.pmf[o];
+        sh.pmf[o] = acc;
       }
       atomicAdd(a.err + 1, 1);
     }
     __syncwarp();
-    const double last = pmf_s[w][m - 1];
+    const double last = sh.pmf[m - 1];
     int cnt2 = 0;
-    for (int o = lane; o < m; o += 32) cnt2 += (pmf_s[w][o] / last <= uu) ? 1 : 0;
+    for (int o = lane; o < m; o += 32) cnt2 += (sh.pmf[o] / last <= uu) ? 1 : 0;
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) cnt2 += __shfl_xor_sync(0xffffffffu, cnt2, off);
     idx = cnt2 < m ? cnt2 : m - 1;
   }
   if (lane == 0) {
-    const uint8_t tv = (uint8_t)(trow_s[w][idx] + 1);
-    trow_s[w][idx] = tv;
+    const uint8_t tv = (uint8_t)(sh.trow[idx] + 1);
+    sh.trow[idx] = tv;
     T[idx] = tv;
   }
   __syncwarp();
-  if (j >= a.A_next) return;
+}
 
-  // ---- the all-minors sweep of level k + 1 ----
+// The particle that enters at level k + 1, and that sweep's digits and factors.
+__device__ __forceinline__ FinDigits fin_digits(const FinalizeArgs& a, int k, int j, FinSample& me, FinShared& sh,
+                                                int lane) {
+  const int m = a.m;
+  uint8_t* S = a.S + (size_t)j * m;
   {
-    const int mode = __shfl_sync(0xffffffffu, pmv, pop_particle_warp(remw, __shfl_sync(0xffffffffu, idxv, a.k), lane));
+    const int mode = __shfl_sync(0xffffffffu, me.pmv, pop_particle_warp(me.remw, __shfl_sync(0xffffffffu, me.idxv, k), lane));
     if (lane == 0) {
-      const uint8_t sv = (uint8_t)(srow_s[w][mode] + 1);
-      srow_s[w][mode] = sv;
+      const uint8_t sv = (uint8_t)(sh.srow[mode] + 1);
+      sh.srow[mode] = sv;
       S[mode] = sv;
     }
-    if (lane < 8) a.rem[(size_t)j * 8 + lane] = remw;
   }
   __syncwarp();
   int nb = 0, nmul = 0, nf = 0;
   for (int base = 0; base < m; base += 32) {
     const int mode = base + lane;
-    const int sv = (mode < m) ? srow_s[w][mode] : 0;
+    const int sv = (mode < m) ? sh.srow[mode] : 0;
     const unsigned b1 = __ballot_sync(0xffffffffu, sv == 1);
     if (sv == 1) {
       const int pos = nb + __popc(b1 & ((1u << lane) - 1u));
-      dm_s[w][pos] = (uint8_t)mode;
-      mult_s[w][pos] = 1;
+      sh.dm[pos] = (uint8_t)mode;
+      sh.mult[pos] = 1;
     }
     nb += __popc(b1);
   }
   for (int base = 0; base < m; base += 32) {
     const int mode = base + lane;
-    const int sv = (mode < m) ? srow_s[w][mode] : 0;
+    const int sv = (mode < m) ? sh.srow[mode] : 0;
     const unsigned bm = __ballot_sync(0xffffffffu, sv > 1);
     if (sv > 1) {
       const int pos = nb + nmul + __popc(bm & ((1u << lane) - 1u));
-      dm_s[w][pos] = (uint8_t)mode;
-      mult_s[w][pos] = (uint8_t)sv;
+      sh.dm[pos] = (uint8_t)mode;
+      sh.mult[pos] = (uint8_t)sv;
     }
     nmul += __popc(bm);
   }
   // factors: every output particle (a mode occupied p times gives p factors)
   for (int base = 0; base < m; base += 32) {
     const int mode = base + lane;
-    const int tv = (mode < m) ? trow_s[w][mode] : 0;
+    const int tv = (mode < m) ? sh.trow[mode] : 0;
     int incl = tv;
 #pragma unroll
     for (int off = 1; off < 32; off <<= 1) {
       const int y = __shfl_up_sync(0xffffffffu, incl, off);
       if (lane >= off) incl += y;
     }
-    for (int q = 0; q < tv; ++q) fm_s[w][nf + incl - tv + q] = (uint8_t)mode;
+    for (int q = 0; q < tv; ++q) sh.fm[nf + incl - tv + q] = (uint8_t)mode;
     nf += __shfl_sync(0xffffffffu, incl, 31);
   }
   __syncwarp();
-  nd = nb + nmul;
+  const int nd = nb + nmul;
   // Glynn form: hold the last binary digit at r = 0 (halving); it moves to the
   // end of the digit list, where its minor row is.
   const int held = (nb > 0) ? 1 : 0;
@@ -1483,16 +1354,25 @@ __global__ void __launch_bounds__(kFinWarps * 32, 8) gccb_finalize_kernel(Finali
     const int src = (lane + 1 < nd) ? lane + 1 : nb - 1;  // rotate entries nb-1 .. nd-1 left by one
     uint8_t dmv = 0, muv = 0;
     if (lane >= nb - 1 && lane < nd) {
-      dmv = dm_s[w][src];
-      muv = mult_s[w][src];
+      dmv = sh.dm[src];
+      muv = sh.mult[src];
     }
     __syncwarp();
     if (lane >= nb - 1 && lane < nd) {
-      dm_s[w][lane] = dmv;
-      mult_s[w][lane] = muv;
+      sh.dm[lane] = dmv;
+      sh.mult[lane] = muv;
     }
     __syncwarp();
   }
+  return {nb, nf, nd, held};
+}
+
+// Writes the next level's sweep: its rows, base sums and descriptor.
+__device__ __forceinline__ void fin_rows(const FinalizeArgs& a, int j, const FinDigits& dg, const FinShared& sh,
+                                         int lane) {
+  const int m = a.m, nb = dg.nb, nf = dg.nf, nd = dg.nd, held = dg.held;
+  const longlong2* Ufxs = a.Ufx + (size_t)j * a.mstride;  // the sample's fixed-point matrix
+  const int32_t* rowfx = a.rowfx + (a.mstride ? (size_t)j * m : 0);
   const int nds = nd - held;  // digits of the sweep
   LevelSample ls;
   if (a.next_tab) {
@@ -1514,7 +1394,7 @@ __global__ void __launch_bounds__(kFinWarps * 32, 8) gccb_finalize_kernel(Finali
   const int low = a.next_quad ? 2 : 0;
   int64_t base_off;  // from the start of the sweep's rows
   auto entry = [&](int f, int d) -> Cx64 {
-    const longlong2 u = Ufxs[(size_t)fm_s[w][f] * m + dm_s[w][d]];
+    const longlong2 u = Ufxs[(size_t)sh.fm[f] * m + sh.dm[d]];
     return cx(u.x, u.y);
   };
   if (a.next_quad) {
@@ -1541,11 +1421,11 @@ __global__ void __launch_bounds__(kFinWarps * 32, 8) gccb_finalize_kernel(Finali
 #pragma unroll 4
       for (int d = 2; d < nd; ++d) {
         const Cx64 u = entry(f, d);
-        const long long mu = mult_s[w][d];
+        const long long mu = sh.mult[d];
         o = cx(o.re + mu * u.re, o.im + mu * u.im);
       }
       B[4 * (f >> 1) + (f & 1)] = make_longlong2(o.re, o.im);
-      fxsum += rowfx[fm_s[w][f]];
+      fxsum += rowfx[sh.fm[f]];
     }
     for (int g = lane; g < slots; g += 32) {  // the pairs' E+-: the rows' coefficients and the held digit's
       const Cx64 f0 = entry(2 * g, 0), f1 = entry(2 * g, 1), g0 = second(g, 0), g1 = second(g, 1);
@@ -1559,7 +1439,7 @@ __global__ void __launch_bounds__(kFinWarps * 32, 8) gccb_finalize_kernel(Finali
 #pragma unroll 4
         for (int d = 0; d < ndo; ++d) {
           const longlong2 p = D[(size_t)d * W + 4 * g + 2], q = D[(size_t)d * W + 4 * g + 3];
-          const long long mu = mult_s[w][d + 2];
+          const long long mu = sh.mult[d + 2];
           ep = cx(ep.re + mu * unpack_row(p.x), ep.im + mu * unpack_row(p.y));
           em = cx(em.re + mu * unpack_row(q.x), em.im + mu * unpack_row(q.y));
         }
@@ -1591,13 +1471,13 @@ __global__ void __launch_bounds__(kFinWarps * 32, 8) gccb_finalize_kernel(Finali
 #pragma unroll 8  // independent gathers in flight
       for (int d = 0; d < nd; ++d) {
         const Cx64 u = entry(f, d);
-        bx += (long long)mult_s[w][d] * u.re;
-        by += (long long)mult_s[w][d] * u.im;
-        ax += (unsigned long long)mult_s[w][d] * (unsigned long long)(u.re < 0 ? -u.re : u.re);
-        ay += (unsigned long long)mult_s[w][d] * (unsigned long long)(u.im < 0 ? -u.im : u.im);
+        bx += (long long)sh.mult[d] * u.re;
+        by += (long long)sh.mult[d] * u.im;
+        ax += (unsigned long long)sh.mult[d] * (unsigned long long)(u.re < 0 ? -u.re : u.re);
+        ay += (unsigned long long)sh.mult[d] * (unsigned long long)(u.im < 0 ? -u.im : u.im);
       }
       B[f] = make_longlong2(bx, by);
-      fxsum += rowfx[fm_s[w][f]];
+      fxsum += rowfx[sh.fm[f]];
       if (a.next_ff) {
         const unsigned long long bnd = ax > ay ? ax : ay;
         const int p = bnd ? 63 - __clzll((long long)bnd) : 0;
@@ -1623,9 +1503,9 @@ __global__ void __launch_bounds__(kFinWarps * 32, 8) gccb_finalize_kernel(Finali
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) fxsum += __shfl_xor_sync(0xffffffffu, fxsum, off);
   SweepProblem& P = a.probs_next[j];
-  P.mult[lane] = (lane + low < nd) ? mult_s[w][lane + low] : 0;
+  P.mult[lane] = (lane + low < nd) ? sh.mult[lane + low] : 0;
   P.mult[lane + 32] = 0;
-  a.dmode_next[(size_t)j * 32 + lane] = (lane < nd) ? dm_s[w][lane] : 0;
+  a.dmode_next[(size_t)j * 32 + lane] = (lane < nd) ? sh.dm[lane] : 0;
   if (lane == 0) {
     // S_i minor_i = 2^-(k-1) (halved) or 2^-k (not) times the Glynn sum, k = nf + 1
     // input particles; the kernel accumulates half of it.
@@ -1654,6 +1534,304 @@ __global__ void __launch_bounds__(kFinWarps * 32, 8) gccb_finalize_kernel(Finali
   }
 }
 
+// Level k's minors from its sweep's partials, into sh; returns their count.
+__device__ __forceinline__ int fin_sums(const FinalizeArgs& a, int j, FinShared& sh, int lane) {
+  int nd;
+  const SweepProblem& P = a.probs_cur[j];
+  nd = P.nd + P.low + P.fixed_digit;  // the held (halved) digit's minor is the last row
+  const int64_t parts = P.n_threads / P.group;
+  if (a.cur_ff) {
+    // float-pair partials: summed as float pairs in a fixed order, scaled by the
+    // problem's power of two, exactly in float when that power is a normal float
+    // (always, for factors of comparable size); otherwise in FP64 below
+    const float4* fp = reinterpret_cast<const float4*>(a.partials) + P.part_off;
+    const int sc_exp = (int)((__double_as_longlong(P.scale) >> 52) & 0x7FF) - 1023;
+    const bool sc_float = sc_exp >= -126 && sc_exp <= 127;
+    const float sc = sc_float ? __double2float_rn(P.scale) : 1.0f;
+    if (parts <= 64) {
+      if (lane < nd) {
+        float rh = 0.0f, rl = 0.0f, ih = 0.0f, il = 0.0f;
+#pragma unroll 8
+        for (int64_t q = 0; q < parts; ++q) {  // unrolled: 8 loads in flight
+          const float4 v = fp[q * nd + lane];
+          ff_acc(rh, rl, 1.0f, v.x, v.y);
+          ff_acc(ih, il, 1.0f, v.z, v.w);
+        }
+        sh.subf[lane] = make_float4(rh * sc, rl * sc, ih * sc, il * sc);
+      }
+    } else {
+      for (int d = 0; d < nd; ++d) {
+        float rh = 0.0f, rl = 0.0f, ih = 0.0f, il = 0.0f;
+        for (int64_t q = lane; q < parts; q += 32) {
+          const float4 v = fp[q * nd + d];
+          ff_acc(rh, rl, 1.0f, v.x, v.y);
+          ff_acc(ih, il, 1.0f, v.z, v.w);
+        }
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) {  // fixed butterfly order
+          const float orh = __shfl_xor_sync(0xffffffffu, rh, off), orl = __shfl_xor_sync(0xffffffffu, rl, off);
+          const float oih = __shfl_xor_sync(0xffffffffu, ih, off), oil = __shfl_xor_sync(0xffffffffu, il, off);
+          ff_acc(rh, rl, 1.0f, orh, orl);
+          ff_acc(ih, il, 1.0f, oih, oil);
+        }
+        if (lane == d) sh.subf[d] = make_float4(rh * sc, rl * sc, ih * sc, il * sc);
+      }
+    }
+  } else if (a.reduced) {  // summed by gccb_partials_reduce_kernel
+    if (lane < nd) {
+      const double2 v = a.reduced[(size_t)j * 32 + lane];
+      sh.sub[lane] = make_double2(v.x * P.scale, v.y * P.scale);
+    }
+  } else {
+    // FP64 partials (parts x nd), summed in a fixed order.  Every FP64
+    // instruction holds the pipe for a whole warp however few lanes are active,
+    // so the lanes are spread over the partials: either gc <= 32 / nd groups of
+    // nd lanes (lane g * nd + d sums rows g, g + gc, .. of digit d, then lane d
+    // adds up the gc group sums; gc = 1 is one lane per digit), or, with many
+    // partials, all 32 lanes stripe over each digit's rows and a butterfly sums
+    // them; whichever issues fewer FP64 instructions.
+    int gc = 1;
+    int64_t cost_groups = 2 * (parts - 1);  // each group's first row is a copy, not an add
+    for (int g2 = 2; g2 * nd <= 32 && g2 <= parts; ++g2) {
+      const int64_t c = 2 * ((parts + g2 - 1) / g2 - 1) + 2 * (g2 - 1);
+      if (c < cost_groups) {
+        cost_groups = c;
+        gc = g2;
+      }
+    }
+    const int64_t cost_stripes = (int64_t)nd * (2 * ((parts + 31) / 32) + 10);
+    if (cost_groups <= cost_stripes) {
+      const int g = lane / nd, d = lane - g * nd;
+      double sx = 0.0, sy = 0.0;
+      if (g < gc && parts >= 8 * gc) {
+        // long sums (the top levels, where one warp has the SM's FP64 unit to
+        // itself): four interleaved chains, rows g + (4 i + c) gc in chain c,
+        // combined in a fixed order, a quarter of one chain's latency
+        double x0 = 0.0, y0 = 0.0, x1 = 0.0, y1 = 0.0, x2 = 0.0, y2 = 0.0, x3 = 0.0, y3 = 0.0;
+        int64_t q = g;
+#pragma unroll 4
+        for (; q + 3 * gc < parts; q += 4 * gc) {
+          const double2 v0 = a.partials[P.part_off + q * nd + d];
+          const double2 v1 = a.partials[P.part_off + (q + gc) * nd + d];
+          const double2 v2 = a.partials[P.part_off + (q + 2 * gc) * nd + d];
+          const double2 v3 = a.partials[P.part_off + (q + 3 * gc) * nd + d];
+          x0 += v0.x;
+          y0 += v0.y;
+          x1 += v1.x;
+          y1 += v1.y;
+          x2 += v2.x;
+          y2 += v2.y;
+          x3 += v3.x;
+          y3 += v3.y;
+        }
+        for (; q < parts; q += gc) {
+          const double2 v = a.partials[P.part_off + q * nd + d];
+          x0 += v.x;
+          y0 += v.y;
+        }
+        sx = (x0 + x1) + (x2 + x3);
+        sy = (y0 + y1) + (y2 + y3);
+      } else if (g < gc) {  // gc <= parts: every group has a first row
+        const double2 v0 = a.partials[P.part_off + (int64_t)g * nd + d];
+        sx = v0.x;
+        sy = v0.y;
+#pragma unroll 8
+        for (int64_t q = g + gc; q < parts; q += gc) {
+          const double2 v = a.partials[P.part_off + q * nd + d];
+          sx += v.x;
+          sy += v.y;
+        }
+      }
+      sh.sub[lane] = make_double2(sx, sy);
+      __syncwarp();
+      if (lane < nd) {
+        double tx = sx, ty = sy;  // group 0 is this lane's own sum
+        for (int gg = 1; gg < gc; ++gg) {
+          const double2 v = sh.sub[gg * nd + lane];
+          tx += v.x;
+          ty += v.y;
+        }
+        sx = tx * P.scale;
+        sy = ty * P.scale;
+      }
+      __syncwarp();
+      if (lane < nd) sh.sub[lane] = make_double2(sx, sy);
+    } else {  // many partials: the lanes stripe over them, then a fixed-order warp
+              // sum; two digits at a time (independent chains in flight)
+      for (int d = 0; d < nd; d += 2) {
+        const int d1 = (d + 1 < nd) ? d + 1 : d;  // an odd last digit is summed twice, stored once
+        double sx = 0.0, sy = 0.0, tx = 0.0, ty = 0.0;
+#pragma unroll 4
+        for (int64_t q = lane; q < parts; q += 32) {
+          const double2 v = a.partials[P.part_off + q * nd + d];
+          const double2 u = a.partials[P.part_off + q * nd + d1];
+          sx += v.x;
+          sy += v.y;
+          tx += u.x;
+          ty += u.y;
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {  // warp_sum's butterfly, the four sums interleaved
+          sx += __shfl_xor_sync(0xffffffffu, sx, o);
+          sy += __shfl_xor_sync(0xffffffffu, sy, o);
+          tx += __shfl_xor_sync(0xffffffffu, tx, o);
+          ty += __shfl_xor_sync(0xffffffffu, ty, o);
+        }
+        if (lane == d) sh.sub[d] = make_double2(sx * P.scale, sy * P.scale);
+        if (lane == d1 && d1 != d) sh.sub[d1] = make_double2(tx * P.scale, ty * P.scale);
+      }
+    }
+  }
+  if (lane < nd) {
+    sh.dm[lane] = a.dmode_cur[(size_t)j * 32 + lane];
+    sh.mult[lane] = P.mult[lane];
+  }
+  __syncwarp();
+  return nd;
+}
+
+// One level of every sample, one warp each.
+template <bool kF64>
+__global__ void __launch_bounds__(kFinWarps * 32, 8) gccb_finalize_kernel(FinalizeArgs a) {
+  __shared__ FinShared sh_s[kFinWarps];
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int j = blockIdx.x * kFinWarps + w;
+  if (j >= a.A) return;
+  FinShared& sh = sh_s[w];
+  // Everything the particle bookkeeping needs is loaded up front (independent loads,
+  // in flight during the sums below).
+  FinSample me = fin_load(a, a.k, j, sh, lane);
+  int nd = 1;
+  if (a.k == 1)
+    fin_first(a, j, me, sh, lane);
+  else
+    nd = fin_sums(a, j, sh, lane);
+  const double uu = a.uni[me.drow + (a.k - 1)];
+  fin_draw<kF64>(a, a.k, j, nd, uu, sh, lane);
+  if (j >= a.A_next) return;
+  const FinDigits dg = fin_digits(a, a.k, j, me, sh, lane);
+  if (lane < 8) a.rem[(size_t)j * 8 + lane] = me.remw;
+  fin_rows(a, j, dg, sh, lane);
+}
+
+// Levels 1..levels of every sample in one launch: a warp keeps its sample's sweep in
+// shared memory and runs it over its lanes (at most 2^(kHeadLevels - 1) codes), then
+// draws, level after level.  As launches of their own these levels are latency: a sweep
+// of 10 us and a finalize of 8 whatever the samples, two launches each.
+constexpr int kHeadLevels = 8;
+constexpr int kHeadStride = 36;  // lanes' minors, 16 bytes each: four lanes of two rows read different banks
+struct HeadArgs {
+  int levels;
+  int A[kHeadLevels + 2];  // samples with at least k particles
+};
+struct HeadShared {
+  FinShared f;
+  double2 M[kHeadLevels * kHeadStride];
+  longlong2 D[(kHeadLevels - 1) * (kHeadLevels - 1)], B[kHeadLevels - 1];
+  SweepProblem P;
+};
+
+template <int NF>
+__device__ __forceinline__ void head_walk(int nf, HeadShared& sh, int lane) {
+  if constexpr (NF < kHeadLevels) {
+    if (nf == NF)
+      minors_walk<NF, kHeadStride>(sh.P, sh.D, sh.B, lane, sh.M + lane);
+    else
+      head_walk<NF + 1>(nf, sh, lane);
+  }
+}
+
+// The sweep of the digits and factors in sh.f: S_i minor_i into sh.f.sub (as fin_rows
+// lays a sweep out for the templated kernels, and fin_sums adds it up).
+__device__ __forceinline__ void head_sweep(const FinalizeArgs& a, int j, const FinDigits& dg, HeadShared& sh,
+                                           int lane) {
+  const int m = a.m, nf = dg.nf, nd = dg.nd, nds = nd - dg.held;
+  const longlong2* U = a.Ufx + (size_t)j * a.mstride;
+  const int32_t* rowfx = a.rowfx + (a.mstride ? (size_t)j * m : 0);
+  for (int e = lane; e < nds * nf; e += 32) {
+    const int d = e / nf, f = e - d * nf;
+    const longlong2 u = U[(size_t)sh.f.fm[f] * m + sh.f.dm[d]];
+    sh.D[e] = make_longlong2(pack_row(u.x), pack_row(u.y));
+  }
+  int fxsum = 0;
+  if (lane < nf) {
+    long long bx = 0, by = 0;
+#pragma unroll 8  // independent gathers in flight
+    for (int d = 0; d < nd; ++d) {
+      const longlong2 u = U[(size_t)sh.f.fm[lane] * m + sh.f.dm[d]];
+      bx += (long long)sh.f.mult[d] * u.x;
+      by += (long long)sh.f.mult[d] * u.y;
+    }
+    sh.B[lane] = make_longlong2(bx, by);
+    fxsum = rowfx[sh.f.fm[lane]];
+  }
+  fxsum = __reduce_add_sync(0xffffffffu, fxsum);
+  int codes = 1;
+  for (int d = 0; d < nds; ++d) codes *= sh.f.mult[d] + 1;
+  const int walkers = codes < 32 ? codes : 32;
+  sh.P.mult[lane] = lane < nd ? sh.f.mult[lane] : 0;
+  if (lane == 0) {
+    sh.P.nd = nds;
+    sh.P.nb = dg.nb - dg.held;
+    sh.P.parity0 = 0;
+    sh.P.fx = -fxsum;
+    sh.P.has_base = 1;
+    sh.P.n_codes = codes;
+    sh.P.n_threads = walkers;
+    sh.P.align = 0;
+    sh.P.fixed_digit = dg.held;
+  }
+  __syncwarp();
+  head_walk<1>(nf, sh, lane);
+  __syncwarp();
+  // gs lanes a digit, each every gs-th walker in order, then a butterfly
+  int gs = 32;
+  while (gs * nd > 32) gs >>= 1;
+  const int d = lane / gs, g = lane & (gs - 1);
+  double x = 0.0, y = 0.0;
+  if (d < nd)
+    for (int i = g; i < walkers; i += gs) {
+      const double2 v = sh.M[d * kHeadStride + i];
+      x += v.x;
+      y += v.y;
+    }
+  for (int off = gs >> 1; off > 0; off >>= 1) {
+    x += __shfl_xor_sync(0xffffffffu, x, off);
+    y += __shfl_xor_sync(0xffffffffu, y, off);
+  }
+  if (d < nd && g == 0) {
+    const double scale = ldexp(1.0, dg.held ? -(nf - 1) : -nf);
+    sh.f.sub[d] = make_double2(x * scale, y * scale);
+  }
+  __syncwarp();
+}
+
+__global__ void __launch_bounds__(kFinWarps * 32, 4) gccb_head_kernel(FinalizeArgs a, HeadArgs h) {
+  extern __shared__ HeadShared head_smem[];
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int j = blockIdx.x * kFinWarps + w;
+  if (j >= h.A[1]) return;
+  HeadShared& sh = head_smem[w];
+  FinSample me = fin_load(a, 1, j, sh.f, lane);
+  fin_first(a, j, me, sh.f, lane);
+  int nd = 1;
+  for (int k = 1;; ++k) {
+    fin_draw<true>(a, k, j, nd, a.uni[me.drow + (k - 1)], sh.f, lane);
+    if (j >= h.A[k + 1]) return;
+    const FinDigits dg = fin_digits(a, k, j, me, sh.f, lane);
+    if (k == h.levels) {
+      if (lane < 8) a.rem[(size_t)j * 8 + lane] = me.remw;
+      fin_rows(a, j, dg, sh.f, lane);
+      return;
+    }
+    nd = dg.nd;
+    head_sweep(a, j, dg, sh, lane);
+  }
+}
+
+// Levels of a run that gccb_head_kernel takes (its sweeps and draws are FP64).
+static int head_levels(bool f64, int Lmax) { return f64 ? std::min(Lmax, kHeadLevels) : 0; }
+
 // ---------------------------------------------------------------------------
 // Host orchestration: prepare (schedule, upload, capture) / launch / collect.
 // ---------------------------------------------------------------------------
@@ -1669,7 +1847,8 @@ struct GccbRun {
   double ref_flops = 0.0;    // the same count over theboss's Ryser-form codes
   double ff_inst = 0.0;      // FP32 instructions of the float-pair sweeps (model count per code)
   bool f64 = true;           // FP64 sweeps and pmf (false: float pairs)
-  std::vector<cudaEvent_t> ev;  // 2 per sweep level when timing
+  std::vector<cudaEvent_t> ev;  // 2 per level from ev_first on when timing
+  int ev_first = 0;
 };
 // Draws decided by the exact sequential rule (a cdf step within the error window
 // of the uniform), summed over the sampler's calls until read (boss_gccb_near_ties).
@@ -1872,7 +2051,8 @@ static inline cudaStream_t slot_stream(Context* cx, int slot) { return slot ? cx
 // matrices: n_mats complex m x m matrices, U[out][in]; one for every sample
 // (n_mats == 1) or one per sample (n_mats == number of samples).
 // timing: 0 none; 1 an event pair around every sweep launch; 2 an event pair
-// around every level (its sweep and its finalize).
+// around every level (its sweep and its finalize); either way one pair around
+// gccb_head_kernel.
 static int gccb_prepare(Context* cx, const double* matrix, int n_mats, int m, Draws& D, int timing, GccbRun& R,
                         int slot = 0) {
   const int N = (int)D.L.size();
@@ -1928,6 +2108,7 @@ static int gccb_prepare(Context* cx, const double* matrix, int n_mats, int m, Dr
   // float-pair sweep exists for the level's factor count, and a float-pair pmf
   const bool f64 = (g_minors_arith != 0);
   R.f64 = f64;
+  const int head = head_levels(f64, Lmax);  // levels 1..head need no layout
   for (int k = 2; k <= Lmax; ++k) ffl[k] = (!f64 && minors_ff_available(k - 1)) ? 1 : 0;
   // FP32 instructions per code of a float-pair sweep with nf = k - 1 factors
   auto ff_per_code = [&](int k) { return ffl[k] ? 47.5625 * (k - 1) : 0.0; };
@@ -1982,7 +2163,7 @@ static int gccb_prepare(Context* cx, const double* matrix, int n_mats, int m, Dr
   std::vector<int> grp(Lmax + 2, 1);
   std::vector<char> red(Lmax + 2, 0);  // level k's partial rows summed by gccb_partials_reduce_kernel
   int64_t max_red = 0;                 // samples of the largest such level
-  for (int k = 2; k <= Lmax; ++k) {
+  for (int k = std::max(2, head + 1); k <= Lmax; ++k) {
     const int Ak = A[k];
     const std::vector<uint64_t>& codes = lvl_codes[k];
     const std::vector<int>& ndv = lvl_nd[k];
@@ -2163,7 +2344,8 @@ static int gccb_prepare(Context* cx, const double* matrix, int n_mats, int m, Dr
   }
   destroy_events(R);
   if (timing) {
-    R.ev.resize(2 * (size_t)std::max(timing == 2 ? Lmax : Lmax - 1, 0));
+    R.ev_first = std::max(head, timing == 2 ? 1 : 2);
+    R.ev.resize(2 * (size_t)std::max(Lmax - R.ev_first + 1, 0));
     for (auto& ev : R.ev)
       if ((e = cudaEventCreate(&ev)) != cudaSuccess) return fail_cuda(e, "event create");
   }
@@ -2175,9 +2357,14 @@ static int gccb_prepare(Context* cx, const double* matrix, int n_mats, int m, Dr
   R.kernels = 0;
   R.sweeps = 0;
   cudaError_t le = cudaMemsetAsync(dS, 0, (size_t)N * m * 2, s);
-  for (int k = 1; k <= Lmax && le == cudaSuccess; ++k) {
+  // level k's first and last event, where it has them
+  auto event = [&](int k, int last) {
+    if (!R.ev.empty() && k >= R.ev_first && le == cudaSuccess)
+      le = cudaEventRecordWithFlags(R.ev[2 * (k - R.ev_first) + last], s, cudaEventRecordExternal);
+  };
+  for (int k = std::max(head, 1); k <= Lmax && le == cudaSuccess; ++k) {
     const int cur = k & 1, nxt = (k + 1) & 1;
-    if (k >= 2) {
+    if (k > head && k >= 2) {
       SweepLaunch SL;
       SL.probs = probs[cur];
       SL.n_probs = A[k];
@@ -2188,11 +2375,9 @@ static int gccb_prepare(Context* cx, const double* matrix, int n_mats, int m, Dr
       SL.rows = std::min(k, kMaxMinorDigits);
       SL.quad = quad[k] != 0;
       SL.uniform_threads = uniform[k] ? uni_lvl[k].n_threads : 0;
-      if (timing == 1) le = cudaEventRecordWithFlags(R.ev[2 * (k - 2)], s, cudaEventRecordExternal);
-      if (timing == 2) le = cudaEventRecordWithFlags(R.ev[2 * (k - 1)], s, cudaEventRecordExternal);
+      event(k, 0);
       if (le == cudaSuccess) le = launch_sweep(k - 1, ffl[k] ? SweepOp::kMinorsFF : SweepOp::kMinors, SL, s);
-      if (timing == 1 && le == cudaSuccess)
-        le = cudaEventRecordWithFlags(R.ev[2 * (k - 2) + 1], s, cudaEventRecordExternal);
+      if (timing == 1) event(k, 1);
       if (le != cudaSuccess) break;
       ++R.kernels;
       ++R.sweeps;
@@ -2238,15 +2423,20 @@ static int gccb_prepare(Context* cx, const double* matrix, int n_mats, int m, Dr
     fa.next_ff = (k < Lmax) ? ffl[k + 1] : 0;
     fa.cur_ff = (k >= 2) ? ffl[k] : 0;
     fa.err = R.derr;
-    if (timing == 2 && k == 1) le = cudaEventRecordWithFlags(R.ev[0], s, cudaEventRecordExternal);
+    if (k == head || k == 1) event(k, 0);
     if (le != cudaSuccess) break;
-    if (f64)
+    if (k == head) {
+      HeadArgs ha = {};
+      ha.levels = head;
+      for (int l = 1; l <= head; ++l) ha.A[l] = A[l];
+      ha.A[head + 1] = fa.A_next;
+      gccb_head_kernel<<<(A[1] + kFinWarps - 1) / kFinWarps, kFinWarps * 32, kFinWarps * sizeof(HeadShared), s>>>(fa, ha);
+    } else if (f64)
       gccb_finalize_kernel<true><<<(A[k] + kFinWarps - 1) / kFinWarps, kFinWarps * 32, 0, s>>>(fa);
     else
       gccb_finalize_kernel<false><<<(A[k] + kFinWarps - 1) / kFinWarps, kFinWarps * 32, 0, s>>>(fa);
     le = cudaGetLastError();
-    if (timing == 2 && le == cudaSuccess)
-      le = cudaEventRecordWithFlags(R.ev[2 * (k - 1) + 1], s, cudaEventRecordExternal);
+    if (timing == 2 || k == head) event(k, 1);
     ++R.kernels;
   }
   e = cudaStreamEndCapture(s, &graph);
@@ -2454,7 +2644,8 @@ static int tune_levels(Context* cx, const double* matrix, int m, Draws& D, int r
   GccbRun R;
   int st = gccb_prepare(cx, matrix, 1, m, D, 2, R);
   if (st) return st;
-  lvl_ms.assign(R.Lmax + 2, 1e30);
+  lvl_ms.assign(R.Lmax + 2, 0.0);
+  for (int k = R.ev_first; k <= R.Lmax; ++k) lvl_ms[k] = 1e30;
   for (int it = 0; it <= reps && !st; ++it) {
     if ((st = gccb_launch(cx))) break;
     const cudaError_t e = cudaStreamSynchronize(cx->stream);
@@ -2462,9 +2653,9 @@ static int tune_levels(Context* cx, const double* matrix, int m, Draws& D, int r
       st = fail_cuda(e, "autotune");
       break;
     }
-    for (int k = 1; it > 0 && k <= R.Lmax; ++k) {
+    for (int k = R.ev_first; it > 0 && k <= R.Lmax; ++k) {
       float x = 0.f;
-      if (cudaEventElapsedTime(&x, R.ev[2 * (k - 1)], R.ev[2 * (k - 1) + 1]) == cudaSuccess)
+      if (cudaEventElapsedTime(&x, R.ev[2 * (k - R.ev_first)], R.ev[2 * (k - R.ev_first) + 1]) == cudaSuccess)
         lvl_ms[k] = std::min(lvl_ms[k], (double)x);
       else
         cudaGetLastError();
@@ -2525,6 +2716,7 @@ static int gccb_autotune_locked(Context* cx, const double* matrix, int m, const 
   const int Lmax = (int)A.size() - 2;
   if (Lmax < 1) return kOk;
   const bool f64 = (g_minors_arith != 0);
+  const int tuned = std::max(2, head_levels(f64, Lmax) + 1);  // levels with a shape of their own from here
   struct ForceGuard {
     ~ForceGuard() {
       g_tune_force = nullptr;
@@ -2543,7 +2735,7 @@ static int gccb_autotune_locked(Context* cx, const double* matrix, int m, const 
     const LevelTune c{sh, 0};
     g_tune_force = &c;
     if ((st = tune_levels(cx, matrix, m, D, reps, ms))) return st;
-    for (int k = 2; k <= Lmax; ++k)
+    for (int k = tuned; k <= Lmax; ++k)
       if (ms[k] < 0.97 * best_ms[k]) {
         best_ms[k] = ms[k];
         best[k] = c;
@@ -2554,7 +2746,7 @@ static int gccb_autotune_locked(Context* cx, const double* matrix, int m, const 
     g_tune_force_level.assign(Lmax + 1, LevelTune{});
     for (int k = 2; k <= Lmax; ++k) g_tune_force_level[k] = LevelTune{best[k].shift, gm};
     if ((st = tune_levels(cx, matrix, m, D, reps, ms))) return st;
-    for (int k = 2; k <= Lmax; ++k)
+    for (int k = tuned; k <= Lmax; ++k)
       if (ms[k] < 0.97 * best_ms[k]) {
         best_ms[k] = ms[k];
         best[k].gmax = gm;
