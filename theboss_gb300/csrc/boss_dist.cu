@@ -103,27 +103,61 @@ __host__ __device__ inline int row_fraction_bits(double largest, int terms) {
   return 61 - ilogb(largest * terms);  // largest * terms < 2^(ilogb + 1)
 }
 
-// One warp per row of U: its scale, and its entries in it, packed (pack_row).
-__global__ void __launch_bounds__(128) small_fixed_kernel(const double2* __restrict__ U, int m, int terms,
-                                                          longlong2* __restrict__ out, int32_t* __restrict__ rowfx) {
-  const int r = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-  if (r >= m) return;
+// The permanents of a batch by particle count: count l has permanents first[l] to
+// first[l + 1] - 1 and, l modes each, entries at[l] on of the rows and columns.
+struct SmallClasses {
+  int64_t first[kSmallPermMax + 2], at[kSmallPermMax + 2];
+};
+
+// One warp per row of U: its scale, and its entries in it, packed (pack_row); then one
+// per permanent and side: the modes of its particles, from len occupations.  U and
+// the occupations are in page-locked host memory, and every one is read once.
+__global__ void __launch_bounds__(128) small_prepare_kernel(const double2* __restrict__ U, int m, int terms,
+                                                            longlong2* __restrict__ out, int32_t* __restrict__ rowfx,
+                                                            const uint8_t* __restrict__ T,
+                                                            const uint8_t* __restrict__ S, int len, SmallClasses c,
+                                                            uint16_t* __restrict__ rows, uint16_t* __restrict__ cols) {
+  const int64_t r = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  if (r >= m) {
+    const int64_t k = (r - m) >> 1;
+    if (k >= c.first[kSmallPermMax + 1]) return;
+    int l = 1;
+    while (k >= c.first[l + 1]) ++l;
+    const uint8_t* occ = (((r - m) & 1) ? S : T) + k * len;
+    uint16_t* to = (((r - m) & 1) ? cols : rows) + c.at[l] + (k - c.first[l]) * l;
+    int done = 0;
+    for (int base = 0; base < len && done < l; base += 32) {
+      const int v = base + lane < len ? occ[base + lane] : 0;
+      int incl = v;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
+      }
+      for (int q = 0; q < v; ++q) to[done + incl - v + q] = (uint16_t)(base + lane);
+      done += __shfl_sync(0xffffffffu, incl, 31);
+    }
+    return;
+  }
   const double2* row = U + (size_t)r * m;
   double mx = 0.0;
   bool fine = true;
   for (int i = lane; i < m; i += 32) {
-    const double x = fmax(fabs(row[i].x), fabs(row[i].y));
-    fine = fine && isfinite(row[i].x) && isfinite(row[i].y);
-    mx = fmax(mx, x);
+    const double2 v = row[i];
+    fine = fine && isfinite(v.x) && isfinite(v.y);
+    mx = fmax(mx, fmax(fabs(v.x), fabs(v.y)));
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
   fine = __all_sync(0xffffffffu, fine);
   const int fx = fine ? row_fraction_bits(mx, terms) : kNoScale;
   if (lane == 0) rowfx[r] = fx;
-  for (int i = lane; i < m && fx != kNoScale; i += 32)
-    out[(size_t)r * m + i] = make_longlong2(pack_row(__double2ll_rn(ldexp(row[i].x, fx))),
-                                            pack_row(__double2ll_rn(ldexp(row[i].y, fx))));
+  for (int i = lane; i < m && fx != kNoScale; i += 32) {
+    const double2 v = row[i];
+    out[(size_t)r * m + i] =
+        make_longlong2(pack_row(__double2ll_rn(ldexp(v.x, fx))), pack_row(__double2ll_rn(ldexp(v.y, fx))));
+  }
 }
 
 // Small permanents: perm of the L x L matrix with rows rows[k][a] and columns
@@ -822,6 +856,10 @@ static int small_perm_few(Context* cx, const double* matrix, int m, int len, con
   return kOk;
 }
 
+static void bytes_of(const int32_t* x, size_t n, uint8_t* out) {  // occupations: at most 255
+  for (size_t i = 0; i < n; ++i) out[i] = (uint8_t)x[i];
+}
+
 int small_perm_batch(Context* cx, const double* matrix, int m, int len, const int32_t* S, const int32_t* T,
                      const std::vector<int>* by_l, double2* results) {
   int64_t total = 0;
@@ -839,48 +877,51 @@ int small_perm_batch(Context* cx, const double* matrix, int m, int len, const in
     bool done = false;
     if ((st = small_perm_few(cx, matrix, m, len, S, T, by_l, total, results, done)) || done) return st;
   }
-  // U | rows | columns up; results down; U in fixed point and its scales on the device
-  const size_t mm = (size_t)m * m;
-  const size_t o_rows = align256(sizeof(double2) * mm), o_cols = o_rows + align256(sizeof(uint16_t) * particles);
-  const size_t in_bytes = o_cols + align256(sizeof(uint16_t) * particles);
-  const size_t o_fx = in_bytes + align256(sizeof(double2) * (size_t)total);
-  const size_t o_rowfx = o_fx + align256(sizeof(longlong2) * mm);
-  if ((st = ensure(cx->dist[3], o_rowfx + sizeof(int32_t) * (size_t)m))) return st;
-  if ((st = ensure_pinned(cx, o_fx))) return st;
+  // Page-locked: U, the occupations (grouped by particle count) and the results, which
+  // the kernels read and write there; on the device: U in fixed point, its scales and
+  // the particles' modes.  Making the modes here took longer than the permanents
+  // (4000 of 5 particles in 64 modes: 0.69 ms a call, 0.31 when the GPU decodes them).
+  const size_t mm = (size_t)m * m, occ = (size_t)len;  // a byte each
+  const size_t o_T = align256(sizeof(double2) * mm), o_S = o_T + align256(occ * total);
+  const size_t o_out = o_S + align256(occ * total);
+  const size_t o_rowfx = align256(sizeof(longlong2) * mm), o_rows = o_rowfx + align256(sizeof(int32_t) * (size_t)m);
+  const size_t o_cols = o_rows + align256(sizeof(uint16_t) * particles);
+  if ((st = ensure(cx->dist[3], o_cols + sizeof(uint16_t) * particles))) return st;
+  if ((st = ensure_pinned(cx, o_out + sizeof(double2) * (size_t)total))) return st;
   char* h = (char*)cx->pinned;
   memcpy(h, matrix, sizeof(double2) * mm);
-  uint16_t* hr = (uint16_t*)(h + o_rows);
-  uint16_t* hc = (uint16_t*)(h + o_cols);
-  size_t at = 0;
-  for (int l = 1; l <= kSmallPermMax; ++l)
-    for (int k : by_l[l]) {
-      particle_modes(T + (size_t)k * len, len, hr + at);
-      particle_modes(S + (size_t)k * len, len, hc + at);
-      at += l;
+  SmallClasses c = {};
+  int64_t q = 0, at = 0;
+  for (int l = 1; l <= kSmallPermMax; ++l) {
+    c.first[l] = q;
+    c.at[l] = at;
+    const std::vector<int>& ks = by_l[l];
+    for (size_t i = 0, e; i < ks.size(); i = e) {  // neighbours in the batch in one go
+      for (e = i + 1; e < ks.size() && ks[e] == ks[e - 1] + 1;) ++e;
+      bytes_of(T + (size_t)ks[i] * len, occ * (e - i), (uint8_t*)h + o_T + q * occ);
+      bytes_of(S + (size_t)ks[i] * len, occ * (e - i), (uint8_t*)h + o_S + q * occ);
+      q += e - i;
     }
+    at += (int64_t)l * (int64_t)ks.size();
+  }
+  c.first[kSmallPermMax + 1] = q;
   char* d = (char*)cx->dist[3].ptr;
   cudaStream_t s = cx->stream;
-  cudaError_t e = cudaMemcpyAsync(d, h, in_bytes, cudaMemcpyHostToDevice, s);
-  if (e != cudaSuccess) return fail_cuda(e, "H2D small permanents");
-  small_fixed_kernel<<<(unsigned)((m + 3) / 4), 128, 0, s>>>((const double2*)d, m, most, (longlong2*)(d + o_fx),
-                                                             (int32_t*)(d + o_rowfx));
-  if ((e = cudaGetLastError()) != cudaSuccess) return fail_cuda(e, "small permanents");
-  at = 0;
-  int64_t q = 0;
-  for (int l = 1; l <= kSmallPermMax; ++l) {
-    const int64_t c = (int64_t)by_l[l].size();
-    if (!c) continue;
-    const SmallLaunch a{(const longlong2*)(d + o_fx), m, 0, (const uint16_t*)(d + o_rows) + at,
-                        (const uint16_t*)(d + o_cols) + at, (const int32_t*)(d + o_rowfx), nullptr, (const double2*)d, c,
-                        (double2*)(d + in_bytes) + q};
-    if ((e = launch_small_l(l, a, cx->sm_count, s)) != cudaSuccess) return fail_cuda(e, "small permanents");
-    at += (size_t)c * l;
-    q += c;
-  }
-  e = cudaMemcpyAsync(h + in_bytes, d + in_bytes, sizeof(double2) * (size_t)total, cudaMemcpyDeviceToHost, s);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  small_prepare_kernel<<<(unsigned)((m + 2 * total + 3) / 4), 128, 0, s>>>(
+      (const double2*)h, m, most, (longlong2*)d, (int32_t*)(d + o_rowfx), (const uint8_t*)(h + o_T),
+      (const uint8_t*)(h + o_S), len, c, (uint16_t*)(d + o_rows), (uint16_t*)(d + o_cols));
+  cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return fail_cuda(e, "small permanents");
-  const double2* out = (const double2*)(h + in_bytes);
+  for (int l = 1; l <= kSmallPermMax; ++l) {
+    if (by_l[l].empty()) continue;
+    const SmallLaunch a{(const longlong2*)d, m, 0, (const uint16_t*)(d + o_rows) + c.at[l],
+                        (const uint16_t*)(d + o_cols) + c.at[l], (const int32_t*)(d + o_rowfx), nullptr,
+                        (const double2*)h, (int64_t)by_l[l].size(), (double2*)(h + o_out) + c.first[l]};
+    if ((e = launch_small_l(l, a, cx->sm_count, s)) != cudaSuccess) break;
+  }
+  const cudaError_t w = cudaStreamSynchronize(s);
+  if (e != cudaSuccess || w != cudaSuccess) return fail_cuda(e != cudaSuccess ? e : w, "small permanents");
+  const double2* out = (const double2*)(h + o_out);
   q = 0;
   for (int l = 1; l <= kSmallPermMax; ++l)
     for (int k : by_l[l]) results[k] = out[q++];
