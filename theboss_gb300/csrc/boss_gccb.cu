@@ -684,7 +684,7 @@ struct FinalizeArgs {
   const LevelSample* next_tab;  // A_next entries, or null when the next level is uniform
   LevelSample next_uni;         // uniform next level: n_codes, threads per sample and the per-sample
                                 // strides of partials (part_off) and rows (pool_off)
-  int next_group;               // uniform next level: threads per summed group of minors
+  int next_group;               // the next level's threads per summed group of minors
   int cur_ff;                   // this level's sweep ran on float pairs: its partials are float4
   int next_quad;                // the next level runs four codes per step (boss_quad.cuh)
   int next_ff;                  // the next level's sweep runs on float pairs (float-pair rows, biases)
@@ -1530,7 +1530,7 @@ __device__ __forceinline__ void fin_rows(const FinalizeArgs& a, int j, const Fin
     const int e2 = (held ? -(nf - 1) : -nf) + (a.next_ff ? esum - fxsum : 0);
     P.scale = (e2 >= -1022 && e2 <= 1023) ? __longlong_as_double((long long)(e2 + 1023) << 52) : ldexp(1.0, e2);
     P.fixed_digit = held;
-    P.group = a.next_tab ? 1 : a.next_group;
+    P.group = a.next_group;
   }
 }
 
@@ -2231,6 +2231,12 @@ static int gccb_prepare(Context* cx, const double* matrix, int n_mats, int m, Dr
       for (uint64_t& c : steps) total += (double)(c >>= low);
       partition_threads(steps, res, nthr, min_codes_per_thread(total, kMinCodesPerThread >> low, 1, block, cx->sm_count));
     }
+    // groups of threads that sum their minors inside the sweep, as for uniform levels,
+    // where that costs no sample more than 2% of its threads
+    int G = quad[k] ? 8 : 32;
+    for (int64_t v : nthr)
+      while (G > 1 && (double)(v / G * G) < 0.98 * (double)v) G >>= 1;
+    grp[k] = G;
     auto& t = tab[k];
     t.resize(Ak);
     int64_t threads = 0, parts = 0, pool = 0;
@@ -2239,17 +2245,21 @@ static int gccb_prepare(Context* cx, const double* matrix, int n_mats, int m, Dr
       LevelSample ls;
       ls.n_codes = (int64_t)(codes[jj] >> low);
       ls.thread_begin = threads;
-      ls.n_threads = nthr[jj];
+      ls.n_threads = nthr[jj] / G * G;
       ls.part_off = parts;
       ls.pool_off = pool;
       auto& a = seen[(ls.n_codes ^ (ls.n_codes >> 3)) & 7];
       if (a.codes != ls.n_codes || a.threads != ls.n_threads)
         a = {ls.n_codes, ls.n_threads, range_align(ls.n_codes, ls.n_threads, k)};
       ls.align = a.align;
-      threads += nthr[jj];
-      parts += nthr[jj] * ndv[jj];
+      threads += ls.n_threads;
+      parts += ls.n_threads / G * ndv[jj];
       pool += pool_units(ndv[jj]);
       t[jj] = ls;
+    }
+    if (!ffl[k] && threads / G >= (int64_t)kReduceMinParts * Ak && Ak <= kReduceMaxSamples && k <= 32) {
+      red[k] = 1;
+      max_red = std::max<int64_t>(max_red, Ak);
     }
     lvl_threads[k] = threads;
     lvl_parts[k] = parts;
