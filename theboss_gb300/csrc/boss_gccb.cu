@@ -672,7 +672,7 @@ struct FinalizeArgs {
   const uint8_t* pmode;   // [input-order sample][n] particle -> input mode
   const uint8_t* npart;   // [input-order sample] input particles
   int64_t mstride;        // elements between the samples' matrices (0: one matrix for all)
-  uint32_t* rem;          // [sample][8] particles not yet popped, as bits
+  uint32_t* rem;          // [sample] particles not yet popped (at most 32), as bits
   const double* uni;      // [input-order sample][n] uniforms
   const SweepProblem* probs_cur;
   const uint8_t* dmode_cur;  // [sample][32]
@@ -702,13 +702,11 @@ constexpr int kFinWarps = 4;
 constexpr float kMinorsErrF64 = 9.094947e-13f;  // 2^-40
 constexpr float kMinorsErrFF = 5.820766e-11f;   // 2^-34
 
-__device__ __forceinline__ unsigned long long warp_max_u64(unsigned long long v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const unsigned long long y = __shfl_xor_sync(0xffffffffu, v, o);
-    v = y > v ? y : v;
-  }
-  return v;
+// The largest exponent field of the warp's non-negative doubles (0x7ff and above for an
+// infinity or a NaN), or -1 if all are zero.
+__device__ __forceinline__ int warp_max_exponent(unsigned long long b) {
+  const unsigned h = __reduce_max_sync(0xffffffffu, (unsigned)(b >> 32) | (b != 0ull ? 1u : 0u));
+  return h ? (int)(h >> 20) : -1;
 }
 
 __device__ __forceinline__ float warp_sum_f(float v) {
@@ -738,39 +736,14 @@ __device__ __forceinline__ unsigned long long fixed_of_double(double x, int F) {
   return (mant >> -sh) + ((mant >> (-sh - 1)) & 1ull);
 }
 
-// Removes the r-th (0-based) particle still in a 256-bit set held one 32-bit word
-// per lane (lanes 0..7, the rest 0; r is below the set's size: the host drew it
-// with randint(0, remaining)).  Every lane gets the particle's index; the owning
-// lane's word loses its bit.
-__device__ __forceinline__ int pop_particle_warp(uint32_t& remw, int r, int lane) {
-  const int c = (lane < 8) ? __popc(remw) : 0;
-  int incl = c;  // inclusive prefix over the words
-#pragma unroll
-  for (int off = 1; off < 8; off <<= 1) {
-    const int y = __shfl_up_sync(0xffffffffu, incl, off);
-    if (lane >= off) incl += y;
-  }
-  const int excl = incl - c;
-  const unsigned who = __ballot_sync(0xffffffffu, lane < 8 && r >= excl && r < incl);
-  const int q = __ffs(who) - 1;  // the word holding it (r is below the set's size: the host drew it)
-  int pos = 0;
-  if (lane == q) {
-    int rr = r - excl;
-    uint32_t x = remw;
-    for (int s = 16; s > 0; s >>= 1) {  // binary search for the bit
-      const uint32_t lo = x & ((1u << s) - 1u);
-      const int cl = __popc(lo);
-      if (rr >= cl) {
-        rr -= cl;
-        x >>= s;
-        pos += s;
-      } else {
-        x = lo;
-      }
-    }
-    remw &= ~(1u << pos);
-  }
-  return q * 32 + __shfl_sync(0xffffffffu, pos, q);
+// Removes the r-th (0-based) particle still in a set of 32 (the same word in every
+// lane; r is below the set's size: the host drew it with randint(0, remaining)).
+// Every lane gets the particle's index.
+__device__ __forceinline__ int pop_particle_warp(uint32_t& rem, int r, int lane) {
+  const bool here = ((rem >> lane) & 1u) && __popc(rem & ((1u << lane) - 1u)) == r;
+  const int p = __ffs(__ballot_sync(0xffffffffu, here)) - 1;
+  rem &= ~(1u << p);
+  return p;
 }
 
 // (r2 2^54 + r1 2^27 + r0) 2^e rounded to the nearest double (ties to even), in
@@ -880,7 +853,7 @@ struct FinShared {
 struct FinSample {
   size_t drow;    // the row of its replayed draws
   int idxv, pmv;  // lane's randint result and particle mode
-  uint32_t remw;  // particles not yet popped (one word per lane 0..7)
+  uint32_t rem;   // particles not yet popped (at most 32), as bits
 };
 
 // The digits and factors of a sample's next sweep (their modes in FinShared).
@@ -893,9 +866,9 @@ __device__ __forceinline__ FinSample fin_load(const FinalizeArgs& a, int k, int 
   const uint8_t* S = a.S + (size_t)j * m;
   const uint8_t* T = a.T + (size_t)j * m;
   // Everything the particle bookkeeping needs, loaded up front (independent
-  // loads, in flight during the sums below): the occupations, the sample's
-  // randint results and particle modes (one per lane; at most 32 particles), and
-  // its set of particles not yet popped (one word per lane 0..7).
+  // loads, in flight during the sums below): the occupations, the sample's randint
+  // results and particle modes (one per lane; at most 32 particles), and its set of
+  // particles not yet popped.
   FinSample me;
   me.drow = (size_t)a.order[j] * a.n;
   for (int i = lane; i < m; i += 32) {
@@ -904,13 +877,11 @@ __device__ __forceinline__ FinSample fin_load(const FinalizeArgs& a, int k, int 
   }
   me.idxv = (lane < a.n) ? (int)a.idx[me.drow + lane] : 0;
   me.pmv = (lane < a.n) ? (int)a.pmode[me.drow + lane] : 0;
-  me.remw = 0;
   if (k == 1) {
     const int np = a.npart[a.order[j]];
-    const int lo = lane * 32;
-    if (lane < 8) me.remw = (np >= lo + 32) ? 0xffffffffu : (np > lo ? ((1u << (np - lo)) - 1u) : 0u);
-  } else if (lane < 8) {
-    me.remw = a.rem[(size_t)j * 8 + lane];
+    me.rem = np >= 32 ? 0xffffffffu : (1u << np) - 1u;
+  } else {
+    me.rem = a.rem[j];
   }
   __syncwarp();
   return me;
@@ -920,7 +891,7 @@ __device__ __forceinline__ FinSample fin_load(const FinalizeArgs& a, int k, int 
 // (bs_submatrices_permanent_calculator_base.py:157-158).
 __device__ __forceinline__ void fin_first(const FinalizeArgs& a, int j, FinSample& me, FinShared& sh, int lane) {
   uint8_t* S = a.S + (size_t)j * a.m;
-  const int mode = __shfl_sync(0xffffffffu, me.pmv, pop_particle_warp(me.remw, __shfl_sync(0xffffffffu, me.idxv, 0), lane));
+  const int mode = __shfl_sync(0xffffffffu, me.pmv, pop_particle_warp(me.rem, __shfl_sync(0xffffffffu, me.idxv, 0), lane));
   if (lane == 0) {
     sh.srow[mode] = 1;
     S[mode] = 1;
@@ -984,9 +955,9 @@ __device__ __forceinline__ void fin_draw(const FinalizeArgs& a, int k, int j, in
       cv = sh.sub[lane];
       c1 = fabs(cv.x) + fabs(cv.y);
     }
-    const unsigned long long cb = warp_max_u64((unsigned long long)__double_as_longlong(c1));
-    const int Ec = (int)(cb >> 52) - 1023;  // non-negative doubles order as integers
-    const double sc = (cb >> 52) ? __longlong_as_double((long long)(1023 - Ec) << 52) : 1.0;  // 2^-Ec
+    const int ce = max(warp_max_exponent((unsigned long long)__double_as_longlong(c1)), 0);
+    const int Ec = ce - 1023;
+    const double sc = ce ? __longlong_as_double((long long)(1023 - Ec) << 52) : 1.0;  // 2^-Ec
     float cn = 0.0f;
     if (lane < nd) {
       cn = __double2float_ru(c1 * sc);  // in [0, 2)
@@ -1081,16 +1052,16 @@ __device__ __forceinline__ void fin_draw(const FinalizeArgs& a, int k, int j, in
     // The cdf scan in exact 64-bit fixed point: F fraction bits with every entry
     // below 2^54 and the total below 2^62 (m <= 256); each entry is off by at most
     // half a unit (2^-54 of the largest entry).
-    unsigned long long pb = 0;
+    unsigned long long pb = 0;  // non-negative doubles order as integers
     for (int o = lane; o < m; o += 32) {
       const unsigned long long b = (unsigned long long)__double_as_longlong(pmf[o]);
       pb = b > pb ? b : pb;
     }
-    pb = warp_max_u64(pb);
-    if (pb == 0ull || (pb >> 52) >= 0x7ffull) {  // zero total, or an infinite / NaN entry
+    const int pe = warp_max_exponent(pb);
+    if (pe < 0 || pe >= 0x7ff) {  // zero total, or an infinite / NaN entry
       if (lane == 0) atomicOr(a.err, 1);
     } else {
-      const int F = 53 - ((int)(pb >> 52) - 1023);
+      const int F = 53 - (pe - 1023);
       unsigned long long run = 0;
       for (int q = 0; q < K; ++q)
         if (o0 + q < m) run += fixed_of_double(pmf[o0 + q], F);
@@ -1121,8 +1092,7 @@ __device__ __forceinline__ void fin_draw(const FinalizeArgs& a, int k, int j, in
         near |= (o < m - 1) && dlt <= W;
         cnt += (C <= ut) ? 1 : 0;
       }
-#pragma unroll
-      for (int off = 16; off > 0; off >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, off);
+      cnt = __reduce_add_sync(0xffffffffu, cnt);
       idx = cnt < m ? cnt : m - 1;
     }
   } else {
@@ -1301,7 +1271,7 @@ __device__ __forceinline__ FinDigits fin_digits(const FinalizeArgs& a, int k, in
   const int m = a.m;
   uint8_t* S = a.S + (size_t)j * m;
   {
-    const int mode = __shfl_sync(0xffffffffu, me.pmv, pop_particle_warp(me.remw, __shfl_sync(0xffffffffu, me.idxv, k), lane));
+    const int mode = __shfl_sync(0xffffffffu, me.pmv, pop_particle_warp(me.rem, __shfl_sync(0xffffffffu, me.idxv, k), lane));
     if (lane == 0) {
       const uint8_t sv = (uint8_t)(sh.srow[mode] + 1);
       sh.srow[mode] = sv;
@@ -1336,6 +1306,12 @@ __device__ __forceinline__ FinDigits fin_digits(const FinalizeArgs& a, int k, in
   for (int base = 0; base < m; base += 32) {
     const int mode = base + lane;
     const int tv = (mode < m) ? sh.trow[mode] : 0;
+    if (!__any_sync(0xffffffffu, tv > 1)) {
+      const unsigned b1 = __ballot_sync(0xffffffffu, tv == 1);
+      if (tv == 1) sh.fm[nf + __popc(b1 & ((1u << lane) - 1u))] = (uint8_t)mode;
+      nf += __popc(b1);
+      continue;
+    }
     int incl = tv;
 #pragma unroll
     for (int off = 1; off < 32; off <<= 1) {
@@ -1710,7 +1686,7 @@ __global__ void __launch_bounds__(kFinWarps * 32, 8) gccb_finalize_kernel(Finali
   fin_draw<kF64>(a, a.k, j, nd, uu, sh, lane);
   if (j >= a.A_next) return;
   const FinDigits dg = fin_digits(a, a.k, j, me, sh, lane);
-  if (lane < 8) a.rem[(size_t)j * 8 + lane] = me.remw;
+  if (lane == 0) a.rem[j] = me.rem;
   fin_rows(a, j, dg, sh, lane);
 }
 
@@ -1732,12 +1708,12 @@ struct HeadShared {
 };
 
 template <int NF>
-__device__ __forceinline__ void head_walk(int nf, HeadShared& sh, int lane) {
+__device__ __forceinline__ void head_walk(int nf, HeadShared& sh, int at, int len, int lane) {
   if constexpr (NF < kHeadLevels) {
     if (nf == NF)
-      minors_walk<NF, kHeadStride>(sh.P, sh.D, sh.B, lane, sh.M + lane);
+      minors_walk<NF, kHeadStride>(sh.P, sh.D, sh.B, at, len, sh.M + lane);
     else
-      head_walk<NF + 1>(nf, sh, lane);
+      head_walk<NF + 1>(nf, sh, at, len, lane);
   }
 }
 
@@ -1748,46 +1724,46 @@ __device__ __forceinline__ void head_sweep(const FinalizeArgs& a, int j, const F
   const int m = a.m, nf = dg.nf, nd = dg.nd, nds = nd - dg.held;
   const longlong2* U = a.Ufx + (size_t)j * a.mstride;
   const int32_t* rowfx = a.rowfx + (a.mstride ? (size_t)j * m : 0);
-  for (int e = lane; e < nds * nf; e += 32) {
-    const int d = e / nf, f = e - d * nf;
-    const longlong2 u = U[(size_t)sh.f.fm[f] * m + sh.f.dm[d]];
-    sh.D[e] = make_longlong2(pack_row(u.x), pack_row(u.y));
-  }
   int fxsum = 0;
   if (lane < nf) {
+    const longlong2* row = U + (size_t)sh.f.fm[lane] * m;
     long long bx = 0, by = 0;
-#pragma unroll 8  // independent gathers in flight
-    for (int d = 0; d < nd; ++d) {
-      const longlong2 u = U[(size_t)sh.f.fm[lane] * m + sh.f.dm[d]];
-      bx += (long long)sh.f.mult[d] * u.x;
-      by += (long long)sh.f.mult[d] * u.y;
+#pragma unroll
+    for (int d = 0; d < kHeadLevels; ++d) {  // independent gathers in flight
+      if (d < nd) {
+        const longlong2 u = row[sh.f.dm[d]];
+        bx += (long long)sh.f.mult[d] * u.x;
+        by += (long long)sh.f.mult[d] * u.y;
+        if (d < nds) sh.D[d * nf + lane] = make_longlong2(pack_row(u.x), pack_row(u.y));
+      }
     }
     sh.B[lane] = make_longlong2(bx, by);
     fxsum = rowfx[sh.f.fm[lane]];
   }
   fxsum = __reduce_add_sync(0xffffffffu, fxsum);
-  int codes = 1;
-  for (int d = 0; d < nds; ++d) codes *= sh.f.mult[d] + 1;
+  const int nb = dg.nb - dg.held;
+  int codes = 1 << nb;
+  for (int d = nb; d < nds; ++d) codes *= sh.f.mult[d] + 1;
   const int walkers = codes < 32 ? codes : 32;
   sh.P.mult[lane] = lane < nd ? sh.f.mult[lane] : 0;
   if (lane == 0) {
     sh.P.nd = nds;
-    sh.P.nb = dg.nb - dg.held;
+    sh.P.nb = nb;
     sh.P.parity0 = 0;
     sh.P.fx = -fxsum;
     sh.P.has_base = 1;
-    sh.P.n_codes = codes;
-    sh.P.n_threads = walkers;
-    sh.P.align = 0;
     sh.P.fixed_digit = dg.held;
   }
   __syncwarp();
-  head_walk<1>(nf, sh, lane);
+  {  // even shares of the codes
+    const int per = codes < 32 ? 1 : codes >> 5, rem = codes < 32 ? 0 : codes & 31;
+    const int at = lane * per + min(lane, rem);
+    head_walk<1>(nf, sh, at, lane < walkers ? per + (lane < rem ? 1 : 0) : 0, lane);
+  }
   __syncwarp();
   // gs lanes a digit, each every gs-th walker in order, then a butterfly
-  int gs = 32;
-  while (gs * nd > 32) gs >>= 1;
-  const int d = lane / gs, g = lane & (gs - 1);
+  const int lg = min(__clz(nd - 1) - 27, 5), gs = 1 << lg;  // nd << lg <= 32
+  const int d = lane >> lg, g = lane & (gs - 1);
   double x = 0.0, y = 0.0;
   if (d < nd)
     for (int i = g; i < walkers; i += gs) {
@@ -1800,7 +1776,7 @@ __device__ __forceinline__ void head_sweep(const FinalizeArgs& a, int j, const F
     y += __shfl_xor_sync(0xffffffffu, y, off);
   }
   if (d < nd && g == 0) {
-    const double scale = ldexp(1.0, dg.held ? -(nf - 1) : -nf);
+    const double scale = __longlong_as_double((long long)(1023 - (dg.held ? nf - 1 : nf)) << 52);  // 2^-..
     sh.f.sub[d] = make_double2(x * scale, y * scale);
   }
   __syncwarp();
@@ -1820,7 +1796,7 @@ __global__ void __launch_bounds__(kFinWarps * 32, 4) gccb_head_kernel(FinalizeAr
     if (j >= h.A[k + 1]) return;
     const FinDigits dg = fin_digits(a, k, j, me, sh.f, lane);
     if (k == h.levels) {
-      if (lane < 8) a.rem[(size_t)j * 8 + lane] = me.remw;
+      if (lane == 0) a.rem[j] = me.rem;
       fin_rows(a, j, dg, sh.f, lane);
       return;
     }
@@ -2293,7 +2269,7 @@ static int gccb_prepare(Context* cx, const double* matrix, int n_mats, int m, Dr
   if ((st = ensure(B[3], (size_t)A[1] * 32 * 2))) return st;                          // digit modes x2
   if ((st = ensure(B[4], sizeof(longlong2) * (size_t)max_pool * 2 + 512))) return st;  // rows x2
   if ((st = ensure(B[5], sizeof(double2) * (size_t)(max_parts + 32 * max_red)))) return st;  // partials | sums
-  if ((st = ensure(B[6], sizeof(uint32_t) * 8 * (size_t)N))) return st;                // particles left
+  if ((st = ensure(B[6], sizeof(uint32_t) * (size_t)N))) return st;                // particles left
   // U fixed point | U^T (limbs or float pairs) | U^T 1-norms | rows' fraction bits
   if ((st = ensure(B[7], (36 * (size_t)m * m + 4 * (size_t)m) * n_mats + 256))) return st;
   if ((st = ensure_slot_pinned(slot, std::max(arena, al((size_t)N * m) + 256)))) return st;

@@ -102,16 +102,13 @@ constexpr int kMinorsMinBlocks = NF <= 16 ? 4 : 3;
 // (w_before - w_after) R = +-2R.  The kernel accumulates half of every minor
 // (flips add +-R, settles w R / 2); the problem's scale carries the factor 2.
 // Segments of 2^16 codes (and every change of a multi-valued digit) are closed
-// by settle_minors and R restarts from zero.  minors_walk is one thread's part
-// (thread q of the sweep's threads); its minors live in shared memory, row j at
-// M[j * STRIDE].
+// by settle_minors and R restarts from zero.  minors_walk is one thread's part (codes
+// a to a + len - 1); its minors live in shared memory, row j at M[j * STRIDE].
 template <int NF, int STRIDE>
 __device__ __forceinline__ void minors_walk(const SweepProblem& P, const longlong2* __restrict__ D,
-                                            const longlong2* __restrict__ base, int64_t q, double2* M) {
+                                            const longlong2* __restrict__ base, int64_t a, int64_t len, double2* M) {
   const int nd = P.nd + P.fixed_digit;
   for (int j = 0; j < nd; ++j) M[j * STRIDE] = make_double2(0.0, 0.0);
-  int64_t a, len;
-  thread_range_aligned(P, q, P.align, a, len);
   if (len > 0) {
     const int e0 = P.fx;
     const int nb = P.nb;
@@ -175,7 +172,9 @@ __global__ void __launch_bounds__(128, kMinorsMinBlocks<NF>) minors_sweep_kernel
   const int64_t q = gt - P.thread_begin;
   const int nd = P.nd + P.fixed_digit;  // minors written per thread
   double2* M = minors_smem + threadIdx.x;
-  minors_walk<NF, 128>(P, pool + P.mat_off, pool + P.base_off, q, M);
+  int64_t a, len;
+  thread_range_aligned(P, q, P.align, a, len);
+  minors_walk<NF, 128>(P, pool + P.mat_off, pool + P.base_off, a, len, M);
   const int G = P.group;
   if (G > 32) {
     // Groups of 64 or 128 threads (the planner allows them only when the launch's
