@@ -762,7 +762,7 @@ int boss_perm_batch(const double* matrix, int32_t m, const int32_t* input_states
   std::lock_guard<std::mutex> lk(g_api_mutex);
   std::vector<HostSweep> by_class[kSweepClasses];
   std::vector<int> which[kSweepClasses];
-  std::vector<int> small[kSmallPermMax + 1];  // one GPU thread per permanent, no planning
+  std::vector<int> small[kSmallPermMax + 1];  // by particle count; no planning
   bool any = false, any_small = false;
   if (variant < BOSS_RYSER || variant > BOSS_CLASSIC) {
     set_error("unknown permanent variant");

@@ -40,18 +40,22 @@ extern std::mutex g_api_mutex;
 constexpr int kDistMaxL = 10;  // per-thread permanents up to 10 x 10 (512 sign vectors)
 constexpr int kDistMaxDiv = 8;  // divisors (factorials of occupations >= 2) kept per state
 
-// perm(U[rows, cols]) for one L x L matrix: Glynn's formula with the sign of
-// column 0 fixed, columns 1..L-1 walked in binary-reflected Gray order.
+// The permanent of one L x L matrix of doubles, entry (a, b) at A[(b L + a) n]:
+// Glynn's formula with the sign of column 0 fixed, columns 1..L-1 walked in
+// binary-reflected Gray order.
 template <int L>
-__device__ __forceinline__ double2 glynn_small(const double2* __restrict__ U, int m, const int (&row)[L],
-                                              const int (&col)[L]) {
+__device__ __forceinline__ double2 glynn_small(const longlong2* __restrict__ A, int64_t n) {
+  auto entry = [&](int a, int b) {
+    const longlong2 u = A[(b * L + a) * n];
+    return make_double2(__longlong_as_double(u.x), __longlong_as_double(u.y));
+  };
   double sr[L], si[L];
 #pragma unroll
   for (int a = 0; a < L; ++a) {
     double x = 0.0, y = 0.0;
 #pragma unroll
     for (int b = 0; b < L; ++b) {
-      const double2 u = U[(size_t)row[a] * m + col[b]];
+      const double2 u = entry(a, b);
       x += u.x;
       y += u.y;
     }
@@ -83,7 +87,7 @@ __device__ __forceinline__ double2 glynn_small(const double2* __restrict__ U, in
     neg ^= 1u << b;
 #pragma unroll
     for (int a = 0; a < L; ++a) {
-      const double2 u = U[(size_t)row[a] * m + col[b]];
+      const double2 u = entry(a, b);
       sr[a] = fma(c, u.x, sr[a]);
       si[a] = fma(c, u.y, si[a]);
     }
@@ -104,106 +108,101 @@ __host__ __device__ inline int row_fraction_bits(double largest, int terms) {
 }
 
 // The permanents of a batch by particle count: count l has permanents first[l] to
-// first[l + 1] - 1 and, l modes each, entries at[l] on of the rows and columns.
+// first[l + 1] - 1, and their matrices begin at entry mat[l].
 struct SmallClasses {
-  int64_t first[kSmallPermMax + 2], at[kSmallPermMax + 2];
+  int64_t first[kSmallPermMax + 2], mat[kSmallPermMax + 2];
 };
 
-// One warp per row of U: its scale, and its entries in it, packed (pack_row); then one
-// per permanent and side: the modes of its particles, from len occupations.  U and
-// the occupations are in page-locked host memory, and every one is read once.
-__global__ void __launch_bounds__(128) small_prepare_kernel(const double2* __restrict__ U, int m, int terms,
-                                                            longlong2* __restrict__ out, int32_t* __restrict__ rowfx,
+// One warp per permanent: its particles' modes from len occupations (in page-locked
+// host memory, every one read once), and its matrix, every row in the scale that its
+// own entries allow: entry (a, b) of permanent i of n of a class at (b l + a) n + i,
+// packed (pack_row), e0 minus the rows' fraction bits; or as doubles, e0 = kNoScale,
+// where a row has no scale.
+__global__ void __launch_bounds__(128) small_prepare_kernel(const double2* __restrict__ U, int m,
                                                             const uint8_t* __restrict__ T,
                                                             const uint8_t* __restrict__ S, int len, SmallClasses c,
-                                                            uint16_t* __restrict__ rows, uint16_t* __restrict__ cols) {
-  const int64_t r = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
+                                                            longlong2* __restrict__ A, int32_t* __restrict__ e0s) {
+  __shared__ uint16_t modes_s[4][2][kSmallPermMax];
+  __shared__ unsigned long long mx_s[4][kSmallPermMax];
+  const int64_t k = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
-  if (r >= m) {
-    const int64_t k = (r - m) >> 1;
-    if (k >= c.first[kSmallPermMax + 1]) return;
-    int l = 1;
-    while (k >= c.first[l + 1]) ++l;
-    const uint8_t* occ = (((r - m) & 1) ? S : T) + k * len;
-    uint16_t* to = (((r - m) & 1) ? cols : rows) + c.at[l] + (k - c.first[l]) * l;
-    int done = 0;
-    for (int base = 0; base < len && done < l; base += 32) {
-      const int v = base + lane < len ? occ[base + lane] : 0;
-      int incl = v;
+  if (k >= c.first[kSmallPermMax + 1]) return;
+  int l = 1;
+  while (k >= c.first[l + 1]) ++l;
+  uint16_t(&modes)[2][kSmallPermMax] = modes_s[threadIdx.x >> 5];
+  unsigned long long* mx = mx_s[threadIdx.x >> 5];
+  if (lane < kSmallPermMax) mx[lane] = 0ull;
+  int done[2] = {0, 0};
+  for (int base = 0; base < len && min(done[0], done[1]) < l; base += 32) {
+    const bool in = base + lane < len;
+    const int v[2] = {in ? T[k * len + base + lane] : 0, in ? S[k * len + base + lane] : 0};
+#pragma unroll
+    for (int side = 0; side < 2; ++side) {
+      int incl = v[side];
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
         const int y = __shfl_up_sync(0xffffffffu, incl, o);
         if (lane >= o) incl += y;
       }
-      for (int q = 0; q < v; ++q) to[done + incl - v + q] = (uint16_t)(base + lane);
-      done += __shfl_sync(0xffffffffu, incl, 31);
+      for (int q = 0; q < v[side]; ++q) modes[side][done[side] + incl - v[side] + q] = (uint16_t)(base + lane);
+      done[side] += __shfl_sync(0xffffffffu, incl, 31);
     }
-    return;
   }
-  const double2* row = U + (size_t)r * m;
-  double mx = 0.0;
-  bool fine = true;
-  for (int i = lane; i < m; i += 32) {
-    const double2 v = row[i];
-    fine = fine && isfinite(v.x) && isfinite(v.y);
-    mx = fmax(mx, fmax(fabs(v.x), fabs(v.y)));
-  }
+  __syncwarp();
+  constexpr int kPer = (kSmallPermMax * kSmallPermMax + 31) / 32;  // entries per lane
+  double2 v[kPer];
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-  fine = __all_sync(0xffffffffu, fine);
-  const int fx = fine ? row_fraction_bits(mx, terms) : kNoScale;
-  if (lane == 0) rowfx[r] = fx;
-  for (int i = lane; i < m && fx != kNoScale; i += 32) {
-    const double2 v = row[i];
-    out[(size_t)r * m + i] =
-        make_longlong2(pack_row(__double2ll_rn(ldexp(v.x, fx))), pack_row(__double2ll_rn(ldexp(v.y, fx))));
+  for (int i = 0; i < kPer; ++i) {  // independent gathers in flight
+    const int e = lane + 32 * i, b = e / l, a = e - b * l;
+    if (e >= l * l) break;
+    v[i] = U[(size_t)modes[0][a] * m + modes[1][b]];
+    // the row's largest: non-negative doubles order as integers, an infinity above every finite one
+    const double x = isfinite(v[i].x) && isfinite(v[i].y) ? fmax(fabs(v[i].x), fabs(v[i].y)) : __longlong_as_double(0x7ff0000000000000ll);
+    atomicMax(mx + a, (unsigned long long)__double_as_longlong(x));
+  }
+  __syncwarp();
+  int fx = 0;
+  if (lane < l) fx = row_fraction_bits(__longlong_as_double((long long)mx[lane]), l);  // infinite: kNoScale
+  const bool fine = __all_sync(0xffffffffu, fx != kNoScale);
+  const int e0 = fine ? -__reduce_add_sync(0xffffffffu, fx) : kNoScale;
+  if (lane == 0) e0s[k] = e0;
+  const int64_t n = c.first[l + 1] - c.first[l];
+  longlong2* to = A + c.mat[l] + (k - c.first[l]);
+#pragma unroll
+  for (int i = 0; i < kPer; ++i) {
+    const int e = lane + 32 * i, a = e % l;
+    if (32 * i >= l * l) break;  // the whole warp
+    const int f = __shfl_sync(0xffffffffu, fx, a);
+    if (e >= l * l) continue;
+    to[(int64_t)e * n] = fine ? make_longlong2(pack_row(__double2ll_rn(ldexp(v[i].x, f))),
+                                               pack_row(__double2ll_rn(ldexp(v[i].y, f))))
+                              : make_longlong2(__double_as_longlong(v[i].x), __double_as_longlong(v[i].y));
   }
 }
 
-// Small permanents: perm of the L x L matrix with rows rows[k][a] and columns
-// cols[k][b] of A (row stride ld, fixed point, packed).  2^lg lanes per permanent,
-// each over 2^(L - 1 - lg) sign vectors: the last lg columns' signs are the lane's
-// bits, the others walk in Gray order, column 0 stays +.  The products run on the
-// integer pipe (accumulate_product_bf), so a code costs ~45 instructions per factor
-// where FP64 ones hold its pipe for 4 * 64 clocks, and a single permanent has all
-// lanes of a block instead of one thread's chain of dependent FP64 products
-// (n = 8: 248 -> 40 us a call, planning and synchronisation included).  e0: minus the rows' fraction bits if given, else
-// rowfx by row; a permanent with a row that has no scale is summed in FP64 from U by
-// its first lane.
+// Small permanents, each of the L x L matrix that small_prepare_kernel (or, for a few,
+// the host) laid out.  2^lg lanes per permanent, each over 2^(L - 1 - lg) sign vectors:
+// the last lg columns' signs are the lane's bits, the others walk in Gray order, column
+// 0 stays +.  The products run on the integer pipe (accumulate_product_bf), so a code
+// costs ~45 instructions per factor where FP64 ones hold its pipe for 4 * 64 clocks,
+// and a single permanent has all lanes of a block instead of one thread's chain of
+// dependent FP64 products (n = 8: 248 -> 40 us a call, planning and synchronisation
+// included).  A permanent with a row that has no scale is summed in FP64 by its first lane.
 template <int L>
-__global__ void __launch_bounds__(128) small_perm_kernel(const longlong2* __restrict__ A, int ld, int64_t stride,
-                                                         const uint16_t* __restrict__ rows,
-                                                         const uint16_t* __restrict__ cols,
-                                                         const int32_t* __restrict__ rowfx,
-                                                         const int32_t* __restrict__ e0s,
-                                                         const double2* __restrict__ U, int64_t count, int lg,
+__global__ void __launch_bounds__(128) small_perm_kernel(const longlong2* __restrict__ A,
+                                                         const int32_t* __restrict__ e0s, int64_t count, int lg,
                                                          double2* __restrict__ out) {
   __shared__ double2 part[4];
   const int64_t gid = (int64_t)blockIdx.x * 128 + threadIdx.x;
   const int64_t at = gid >> lg;
   const int64_t k = at < count ? at : count - 1;
   const uint32_t mine = (uint32_t)gid & ((1u << lg) - 1u);
-  const uint16_t* ck = cols + k * L;
-  const longlong2* Ak = A + k * stride;
-  int row[L];
-  int e0 = e0s ? e0s[k] : 0;
-  bool fp64 = false;
-#pragma unroll
-  for (int a = 0; a < L; ++a) {
-    row[a] = rows[k * L + a];
-    if (!e0s) {
-      const int fx = rowfx[row[a]];
-      fp64 = fp64 || fx == kNoScale;
-      e0 -= fx;
-    }
-  }
+  const longlong2* Ak = A + k;
+  const int e0 = e0s[k];
   double ar = 0.0, ai = 0.0;
-  if (fp64) {
+  if (e0 == kNoScale) {
     if (mine == 0) {
-      int col[L];
-#pragma unroll
-      for (int b = 0; b < L; ++b) col[b] = ck[b];
-      const double2 p = glynn_small<L>(U, ld, row, col);
+      const double2 p = glynn_small<L>(Ak, count);
       ar = p.x;
       ai = p.y;
     }
@@ -214,10 +213,9 @@ __global__ void __launch_bounds__(128) small_perm_kernel(const longlong2* __rest
     const int low = L - lg;  // columns low .. L - 1 have the lane's signs
     for (int b = 0; b < L; ++b) {
       const int sg = (b >= low && ((mine >> (b - low)) & 1u)) ? -1 : 1;
-      const int c = ck[b];
 #pragma unroll
       for (int a = 0; a < L; ++a) {
-        const longlong2 u = Ak[(size_t)row[a] * ld + c];
+        const longlong2 u = Ak[(b * L + a) * count];
         sr[a] = add_packed(sr[a], u.x, sg);
         si[a] = add_packed(si[a], u.y, sg);
       }
@@ -231,10 +229,9 @@ __global__ void __launch_bounds__(128) small_perm_kernel(const longlong2* __rest
       const int sg = ((neg >> b) & 1u) ? 2 : -2;
       neg ^= 1u << b;
       parity ^= 1u;
-      const int c = ck[b];
 #pragma unroll
       for (int a = 0; a < L; ++a) {
-        const longlong2 u = Ak[(size_t)row[a] * ld + c];
+        const longlong2 u = Ak[(b * L + a) * count];
         sr[a] = add_packed(sr[a], u.x, sg);
         si[a] = add_packed(si[a], u.y, sg);
       }
@@ -742,11 +739,7 @@ static int group_large(Context* cx, const double* matrix, int m, int n, int l, c
 
 struct SmallLaunch {
   const longlong2* A;
-  int ld;
-  int64_t stride;  // between the permanents' own matrices (0: one for all)
-  const uint16_t *rows, *cols;  // L per permanent
-  const int32_t *rowfx, *e0;
-  const double2* U;
+  const int32_t* e0;
   int64_t count;
   double2* out;
 };
@@ -758,8 +751,7 @@ static cudaError_t launch_small(const SmallLaunch& s, int sm_count, cudaStream_t
   int lg = 0;
   while (lg < 7 && lg < L - 1 && (s.count << (lg + 1)) <= (int64_t)sm_count * 256) ++lg;
   const int64_t threads = s.count << lg;
-  small_perm_kernel<L><<<(unsigned)((threads + 127) / 128), 128, 0, st>>>(s.A, s.ld, s.stride, s.rows, s.cols, s.rowfx,
-                                                                          s.e0, s.U, s.count, lg, s.out);
+  small_perm_kernel<L><<<(unsigned)((threads + 127) / 128), 128, 0, st>>>(s.A, s.e0, s.count, lg, s.out);
   return cudaGetLastError();
 }
 
@@ -790,28 +782,28 @@ static void particle_modes(const int32_t* occ, int len, uint16_t* out) {
 // host memory: one launch and one synchronisation, no copies.  done = false: a row
 // has no fixed-point scale, nothing was launched.
 constexpr int64_t kFewPerms = 16;
+// .. and so are more of them while that is not more work for the host than the launch it
+// saves (about 4 us): this many matrix entries, and occupations of one side to look through.
+constexpr int64_t kFewEntries = 600, kFewOccupations = 3072;
 
 static int small_perm_few(Context* cx, const double* matrix, int m, int len, const int32_t* S, const int32_t* T,
                           const std::vector<int>* by_l, int64_t total, double2* results, bool& done) {
   constexpr int L = kSmallPermMax;
   done = false;
-  const size_t o_rows = align256(sizeof(longlong2) * L * L * (size_t)total);
-  const size_t o_cols = o_rows + align256(sizeof(uint16_t) * (size_t)total * L);
-  const size_t o_e0 = o_cols + align256(sizeof(uint16_t) * (size_t)total * L);
+  const size_t o_e0 = align256(sizeof(longlong2) * L * L * (size_t)total);
   const size_t o_out = o_e0 + align256(sizeof(int32_t) * (size_t)total);
   int st;
   if ((st = ensure_pinned(cx, o_out + sizeof(double2) * (size_t)total))) return st;
   char* h = (char*)cx->pinned;
-  uint16_t* hr = (uint16_t*)(h + o_rows);
-  uint16_t* hc = (uint16_t*)(h + o_cols);
-  size_t at = 0;  // rows and columns, l per permanent
   int64_t q = 0;
-  for (int l = 1; l <= L; ++l)
+  for (int l = 1; l <= L; ++l) {
+    longlong2* M = (longlong2*)h + q * L * L;  // the class's matrices, interleaved as on the GPU
+    const int64_t n = (int64_t)by_l[l].size();
+    int64_t at = 0;
     for (int k : by_l[l]) {
       uint16_t r[L], c[L];
       particle_modes(T + (size_t)k * len, len, r);
       particle_modes(S + (size_t)k * len, len, c);
-      longlong2* M = (longlong2*)(h) + q * L * L;
       int e0 = 0;
       for (int a = 0; a < l; ++a) {
         double mx = 0.0;
@@ -826,24 +818,22 @@ static int small_perm_few(Context* cx, const double* matrix, int m, int len, con
         if (fx == kNoScale) return kOk;
         const double scale = std::ldexp(1.0, fx);
         for (int b = 0; b < l; ++b)
-          M[a * L + b] = longlong2{pack_row(std::llrint(row[2 * c[b]] * scale)),
-                                   pack_row(std::llrint(row[2 * c[b] + 1] * scale))};
+          M[(b * l + a) * n + at] = longlong2{pack_row(std::llrint(row[2 * c[b]] * scale)),
+                                              pack_row(std::llrint(row[2 * c[b] + 1] * scale))};
         e0 -= fx;
-        hr[at + a] = hc[at + a] = (uint16_t)a;
       }
-      ((int32_t*)(h + o_e0))[q++] = e0;
-      at += l;
+      ((int32_t*)(h + o_e0))[q + at] = e0;
+      ++at;
     }
-  at = 0;
+    q += n;
+  }
   q = 0;
   for (int l = 1; l <= L; ++l) {
     const int64_t c = (int64_t)by_l[l].size();
     if (!c) continue;
-    const SmallLaunch s{(longlong2*)h + q * L * L, L, L * L, hr + at, hc + at, nullptr, (int32_t*)(h + o_e0) + q, nullptr,
-                        c, (double2*)(h + o_out) + q};
+    const SmallLaunch s{(longlong2*)h + q * L * L, (int32_t*)(h + o_e0) + q, c, (double2*)(h + o_out) + q};
     const cudaError_t e = launch_small_l(l, s, cx->sm_count, cx->stream);
     if (e != cudaSuccess) return fail_cuda(e, "small permanents");
-    at += (size_t)c * l;
     q += c;
   }
   const cudaError_t e = cudaStreamSynchronize(cx->stream);
@@ -860,41 +850,40 @@ static void bytes_of(const int32_t* x, size_t n, uint8_t* out) {  // occupations
   for (size_t i = 0; i < n; ++i) out[i] = (uint8_t)x[i];
 }
 
+// Entries of the matrices of one pass at most (64 MiB); larger batches take several.
+constexpr int64_t kSmallPassEntries = 1 << 22;
+
 int small_perm_batch(Context* cx, const double* matrix, int m, int len, const int32_t* S, const int32_t* T,
                      const std::vector<int>* by_l, double2* results) {
-  int64_t total = 0;
-  int most = 0;
-  size_t particles = 0;
-  for (int l = 1; l <= kSmallPermMax; ++l)
-    if (!by_l[l].empty()) {
-      total += (int64_t)by_l[l].size();
-      particles += (size_t)l * by_l[l].size();
-      most = l;
-    }
+  int64_t first[kSmallPermMax + 2] = {}, entries = 0;  // by particle count
+  for (int l = 1; l <= kSmallPermMax; ++l) {
+    first[l + 1] = first[l] + (int64_t)by_l[l].size();
+    entries += (int64_t)l * l * (int64_t)by_l[l].size();
+  }
+  const int64_t total = first[kSmallPermMax + 1];
   if (total == 0) return kOk;
   int st;
-  if (total <= kFewPerms) {
+  if (total <= kFewPerms || (entries <= kFewEntries && total * len <= kFewOccupations)) {
     bool done = false;
     if ((st = small_perm_few(cx, matrix, m, len, S, T, by_l, total, results, done)) || done) return st;
   }
   // Page-locked: U, the occupations (grouped by particle count) and the results, which
-  // the kernels read and write there; on the device: U in fixed point, its scales and
-  // the particles' modes.  Making the modes here took longer than the permanents
-  // (4000 of 5 particles in 64 modes: 0.69 ms a call, 0.31 when the GPU decodes them).
+  // the kernels read and write there; on the device: the matrices of a pass, and U
+  // where the gathers read its entries often.  Making the modes here took longer than
+  // the permanents (4000 of 5 particles in 64 modes: 0.69 ms a call).
   const size_t mm = (size_t)m * m, occ = (size_t)len;  // a byte each
   const size_t o_T = align256(sizeof(double2) * mm), o_S = o_T + align256(occ * total);
   const size_t o_out = o_S + align256(occ * total);
-  const size_t o_rowfx = align256(sizeof(longlong2) * mm), o_rows = o_rowfx + align256(sizeof(int32_t) * (size_t)m);
-  const size_t o_cols = o_rows + align256(sizeof(uint16_t) * particles);
-  if ((st = ensure(cx->dist[3], o_cols + sizeof(uint16_t) * particles))) return st;
+  const bool copy = entries > 4096 && entries > 4 * (int64_t)mm;
+  const size_t o_A = copy ? align256(sizeof(double2) * mm) : 0;
+  const int64_t pass = std::min(entries, kSmallPassEntries);
+  const size_t o_e0 = o_A + align256(sizeof(longlong2) * (size_t)pass);
+  if ((st = ensure(cx->dist[3], o_e0 + sizeof(int32_t) * (size_t)std::min(total, pass)))) return st;
   if ((st = ensure_pinned(cx, o_out + sizeof(double2) * (size_t)total))) return st;
   char* h = (char*)cx->pinned;
   memcpy(h, matrix, sizeof(double2) * mm);
-  SmallClasses c = {};
-  int64_t q = 0, at = 0;
+  int64_t q = 0;
   for (int l = 1; l <= kSmallPermMax; ++l) {
-    c.first[l] = q;
-    c.at[l] = at;
     const std::vector<int>& ks = by_l[l];
     for (size_t i = 0, e; i < ks.size(); i = e) {  // neighbours in the batch in one go
       for (e = i + 1; e < ks.size() && ks[e] == ks[e - 1] + 1;) ++e;
@@ -902,22 +891,38 @@ int small_perm_batch(Context* cx, const double* matrix, int m, int len, const in
       bytes_of(S + (size_t)ks[i] * len, occ * (e - i), (uint8_t*)h + o_S + q * occ);
       q += e - i;
     }
-    at += (int64_t)l * (int64_t)ks.size();
   }
-  c.first[kSmallPermMax + 1] = q;
   char* d = (char*)cx->dist[3].ptr;
+  longlong2* A = (longlong2*)(d + o_A);
+  int32_t* e0 = (int32_t*)(d + o_e0);
   cudaStream_t s = cx->stream;
-  small_prepare_kernel<<<(unsigned)((m + 2 * total + 3) / 4), 128, 0, s>>>(
-      (const double2*)h, m, most, (longlong2*)d, (int32_t*)(d + o_rowfx), (const uint8_t*)(h + o_T),
-      (const uint8_t*)(h + o_S), len, c, (uint16_t*)(d + o_rows), (uint16_t*)(d + o_cols));
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return fail_cuda(e, "small permanents");
-  for (int l = 1; l <= kSmallPermMax; ++l) {
-    if (by_l[l].empty()) continue;
-    const SmallLaunch a{(const longlong2*)d, m, 0, (const uint16_t*)(d + o_rows) + c.at[l],
-                        (const uint16_t*)(d + o_cols) + c.at[l], (const int32_t*)(d + o_rowfx), nullptr,
-                        (const double2*)h, (int64_t)by_l[l].size(), (double2*)(h + o_out) + c.first[l]};
-    if ((e = launch_small_l(l, a, cx->sm_count, s)) != cudaSuccess) break;
+  cudaError_t e = copy ? cudaMemcpyAsync(d, h, sizeof(double2) * mm, cudaMemcpyHostToDevice, s) : cudaSuccess;
+  for (int64_t a = 0, b; a < total && e == cudaSuccess; a = b) {  // permanents a to b - 1
+    SmallClasses c = {};
+    int64_t left = pass;
+    b = a;
+    for (int l = 1; l <= kSmallPermMax; ++l) {
+      c.first[l] = b - a;
+      c.mat[l] = pass - left;
+      if (b == std::max(a, first[l])) {  // no smaller count had to stop
+        const int64_t n = std::min(first[l + 1] - b, left / (l * l));
+        if (n > 0) {
+          b += n;
+          left -= n * l * l;
+        }
+      }
+    }
+    c.first[kSmallPermMax + 1] = b - a;
+    small_prepare_kernel<<<(unsigned)((b - a + 3) / 4), 128, 0, s>>>((const double2*)(copy ? d : h), m,
+                                                                     (const uint8_t*)h + o_T + a * occ,
+                                                                     (const uint8_t*)h + o_S + a * occ, len, c, A, e0);
+    e = cudaGetLastError();
+    for (int l = 1; l <= kSmallPermMax && e == cudaSuccess; ++l) {
+      const int64_t n = c.first[l + 1] - c.first[l];
+      if (n == 0) continue;
+      const SmallLaunch sl{A + c.mat[l], e0 + c.first[l], n, (double2*)(h + o_out) + a + c.first[l]};
+      e = launch_small_l(l, sl, cx->sm_count, s);
+    }
   }
   const cudaError_t w = cudaStreamSynchronize(s);
   if (e != cudaSuccess || w != cudaSuccess) return fail_cuda(e != cudaSuccess ? e : w, "small permanents");

@@ -8,9 +8,9 @@
 theboss evaluates one outcome at a time: a loop over the lossy inputs, one
 permanent each (the uniform-loss calculator spreads the outcomes over a process
 pool).  Here every requested outcome, with every lossy input, is one call of
-boss_lossy_probabilities (libboss_gb300.so): one GPU thread per (lossy input,
-outcome) pair, then one per outcome for the sum and the normalisation, in
-theboss's operation order.  The permanent calculator passed in is kept for API
+boss_lossy_probabilities (libboss_gb300.so): row sums tabulated per lossy input,
+neighbouring outcomes sharing their prefix products, then one thread per outcome
+for the sum and the normalisation, in theboss's operation order.  The permanent calculator passed in is kept for API
 compatibility; the GPU computes the permanents whatever its type (they agree to
 rounding).
 """
