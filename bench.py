@@ -306,8 +306,8 @@ def single_permanents(peak_tflops, seed, peak32=None):
         ms = float(np.mean(b["sweep_ms"]))
         tf = b["flops"] / (ms / 1e3) / 1e12
         res[str(n)] = {"perms_per_s": 64 / (ms / 1e3), "ms_per_64": ms, "codes": b["codes"], "arithmetic": "fp64",
-                       "arithmetic_note": "the first n - 8 factors of every product in block floating point on "
-                                          "the integer pipe; frac_of_fp64_peak counts FP64-equivalent flops",
+                       "arithmetic_note": "every product in block floating point on the integer pipe; "
+                                          "frac_of_fp64_peak counts FP64-equivalent flops",
                        "achieved_tflops": tf, "frac_of_fp64_peak": tf / peak_tflops, **errors(n, U, S, T, b["results"])}
         prev = _native.perm_arithmetic(_native.FLOAT_PAIRS)
         try:
@@ -518,8 +518,8 @@ def strategies_section(seed):
 # arithmetic of the path (theboss computes in float64)
 DTYPE = "f64"
 DTYPE_NOTE = ("FP64 products, minors, Laplace step, |.|^2 and pmf; row sums in exact 64-bit fixed point; "
-              "the first factors of every product multiplied in block floating point on the integer pipe "
-              "(62-bit mantissas, each product within 2^-56.5 of its magnitude, one rounding to FP64); "
+              "every product multiplied in block floating point on the integer pipe (62-bit mantissas, "
+              "each product within 2^-56.5 of its magnitude, one rounding of the chain to FP64); "
               "cdf decisions by an exact integer scan of the FP64 pmf, theboss's sequential FP64 rule "
               "inside the pmf's error window")
 
@@ -531,11 +531,10 @@ def roofline(b, sweep_s, achieved, peak, peak32, traffic):
     common = {"traffic": traffic, "sweep_ms_per_step": sweep_s * 1e3, "flops_per_step": b["sweep_flops"],
               "flops_note": "9k - 12 flops per Guan code at level k over the codes the Glynn-form all-minors "
                             "sweeps walk (half of theboss's Ryser-form codes for single photons); of these "
-                            "the row-sum updates and the products of the first 8 factors (nf - 8 above 16 "
-                            "factors; block floating point, 62-bit mantissas) run on the integer pipe, the "
-                            "rest on the FP64 pipe, so "
-                            "the FP64-equivalent rate can exceed the FP64 pipe's peak; ryser_form_* count "
-                            "theboss's codes",
+                            "the row-sum updates and the products (block floating point, 62-bit mantissas) run "
+                            "on the integer pipe, so the FP64-equivalent rate can exceed the FP64 pipe's "
+                            "peak; the first eight levels run in one launch with their draws, which "
+                            "sweep_ms_per_step includes; ryser_form_* count theboss's codes",
               "ryser_form_flops_per_step": b["ref_flops"],
               "ryser_form_equivalent_tflops": b["ref_flops"] / sweep_s / 1e12}
     if b["ff_inst"] > 0:
@@ -550,11 +549,12 @@ def roofline(b, sweep_s, achieved, peak, peak32, traffic):
                 "fp32_inst_per_step": b["ff_inst"],
                 "fp64_equivalent": {"achieved_tflops": achieved, "fp64_peak_tflops": peak,
                                     "ratio_to_fp64_peak": achieved / peak}, **common}
-    return {"bound": "fp64", "kernel": "minors_sweep_kernel (all levels of a step)", "achieved": achieved,
+    return {"bound": "fp64", "kernel": "gccb_head_kernel, minors_sweep_kernel, minors_quad_kernel (all levels)",
+            "achieved": achieved,
             "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
             "peak_source": "boss_fp64_peak, measured in this run",
             "frac_note": "FP64-equivalent flops over the FP64 pipe's measured peak; the integer pipe carries "
-                         "part of the products, so a fraction above 1 is reachable", **common}
+                         "the products, so a fraction above 1 is reachable", **common}
 
 
 def float_pair_section(U, inp, w, args, fp64_samples):
