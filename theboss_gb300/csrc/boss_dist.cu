@@ -267,9 +267,13 @@ __global__ void __launch_bounds__(128) small_perm_kernel(const longlong2* __rest
 // (input, sign vector), a warp 32 of them (several sign vectors of one input from
 // L = 6 on, several inputs below), and walks a chunk of outcomes with the partial
 // products in registers: the same control flow in every lane.
-// Bound by the FP64 pipe (4 instructions per product, 2 per outcome for the sum over
-// the lanes).  8 photons in 16 modes, all 735,471 outcomes: 16.5 -> 4.4 ms, FP64 pipe
-// 85 % busy, against one thread per (input, outcome) walking all sign vectors.
+// kFixed: the row sums are exact 64-bit fixed point, each (input, row) in the scale of
+// its own L entries, and the products run on the integer pipe (block floating point,
+// boss_sweep.cuh): about 45 instructions each against four FP64 ones that hold their
+// pipe for 64 clocks.  Otherwise (a matrix with entries that have no scale) both are FP64.
+// 8 photons in 16 modes, all 735,471 outcomes: 16.5 ms with one thread per (input,
+// outcome) walking all sign vectors, 4.4 with this walk in FP64 (pipe 87 % busy), 2.5
+// in fixed point (issue and latency: 190 instructions an outcome and 32 sign vectors).
 // ---------------------------------------------------------------------------
 constexpr int kWalkChunk = 128;  // outcomes per warp at most (a multiple of 8)
 
@@ -295,17 +299,41 @@ __global__ void lossy_rows_kernel(const uint8_t* __restrict__ occ, int m, int64_
   rows[o] = make_uint4(w[0], w[1], w[2], w[3]);
 }
 
-// V[(combo / 32 * m + row) * 32 + combo % 32], combo = input * 2^(L-1) + sign vector.
+// V[(combo / 32 * m + row) * 32 + combo % 32], combo = input * 2^(L-1) + sign vector:
+// doubles, or (fx given) fixed point, each (input, row) with fx[input * m + row] fraction bits.
 __global__ void lossy_table_kernel(const double2* __restrict__ U, int m, int L, const uint8_t* __restrict__ cols,
-                                   int K, int64_t combos, double2* __restrict__ V) {
+                                   int K, int64_t combos, int32_t* __restrict__ fx, double2* __restrict__ V) {
   const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= combos * m) return;
   const int64_t combo = e / ((int64_t)32 * m) * 32 + (e & 31);
   const int row = (int)((e >> 5) % m);
   const int64_t k = combo >> (L - 1);
   double x = 0.0, y = 0.0;
+  const uint32_t d = (uint32_t)combo & ((1u << (L - 1)) - 1u);
+  if (fx) {
+    long long fr = 0, fi = 0;
+    if (k < K) {
+      unsigned long long mx = 0;  // magnitudes order as integers
+      for (int b = 0; b < L; ++b) {
+        const double2 u = U[(size_t)row * m + cols[k * L + b]];
+        mx = max(mx, max((unsigned long long)__double_as_longlong(fabs(u.x)),
+                         (unsigned long long)__double_as_longlong(fabs(u.y))));
+      }
+      const int f = row_fraction_bits(__longlong_as_double((long long)mx), L);
+      if (d == 0) fx[k * m + row] = f;
+      const double scale = __longlong_as_double((long long)(1023 + f) << 52);  // 2^f, |f| < 1000
+      for (int b = 0; b < L; ++b) {
+        const double2 u = U[(size_t)row * m + cols[k * L + b]];
+        const bool neg = b > 0 && ((d >> (b - 1)) & 1u);
+        const long long ur = __double2ll_rn(u.x * scale), ui = __double2ll_rn(u.y * scale);
+        fr += neg ? -ur : ur;
+        fi += neg ? -ui : ui;
+      }
+    }
+    reinterpret_cast<longlong2*>(V)[e] = make_longlong2(fr, fi);
+    return;
+  }
   if (k < K) {
-    const uint32_t d = (uint32_t)combo & ((1u << (L - 1)) - 1u);
     for (int b = 0; b < L; ++b) {
       const double2 u = U[(size_t)row * m + cols[k * L + b]];
       const bool neg = b > 0 && ((d >> (b - 1)) & 1u);
@@ -319,8 +347,9 @@ __global__ void lossy_table_kernel(const double2* __restrict__ U, int m, int L, 
 // One warp per (group of 32 combos of equal input or of several inputs, chunk of
 // outcomes); from L = 6 on a group is one input and its 2^(L-6) blocks of 32 sign
 // vectors are walked one after the other.
-template <int L>
+template <int L, bool kFixed>
 __global__ void __launch_bounds__(128) lossy_walk_kernel(const double2* __restrict__ V, int m,
+                                                         const int32_t* __restrict__ fx,  // kFixed: [K][m]
                                                          const uint4* __restrict__ rows, int64_t O, int K, int groups,
                                                          const double* __restrict__ in_div,    // [K][kDistMaxDiv]
                                                          const int* __restrict__ in_ndiv,      // [K]
@@ -353,14 +382,37 @@ __global__ void __launch_bounds__(128) lossy_walk_kernel(const double2* __restri
     const double2* Vg = V + block * 32 * m + lane;
     const uint32_t d = L >= 6 ? (uint32_t)(j * 32 + lane) : (uint32_t)(lane & (kLanes - 1));
     const uint32_t neg = (__popc(d) & 1) << 31;
-    double2 P[L];
+    const int mine = L >= 6 ? g : min(g * (32 / kLanes) + lane / kLanes, K - 1);  // this lane's input
+    const int32_t* fxk = kFixed ? fx + (size_t)mine * m : nullptr;
+    double2 P[kFixed ? 1 : L];
+    long long pr[kFixed ? L : 1], pi[kFixed ? L : 1];  // normalised, in units of 2^pe
+    int pe[kFixed ? L : 1];
+    double2 x = make_double2(0.0, 0.0);  // the last product
     for (int q = 0; q < n; ++q) {
       const uint4 r = __ldg(rows + o0 + q);
       const uint32_t w[4] = {r.x, r.y, r.z, r.w};
       const int c = q > 0 ? (int)(r.w >> 24) : 0;
       auto step = [&](auto index) {
         constexpr int a = decltype(index)::value;
-        if constexpr (a < L) {
+        if constexpr (a < L && kFixed) {
+          const int row = (int)((w[a >> 2] >> (8 * (a & 3))) & 255u);
+          const longlong2 v = __ldg(reinterpret_cast<const longlong2*>(Vg) + (size_t)row * 32);
+          const int f = __ldg(fxk + row);
+          long long zr = v.x, zi = v.y;
+          int e = -f;
+          if constexpr (a > 0) {
+            bf_mul_high(pr[a - 1], pi[a - 1], v.x, v.y, zr, zi);
+            e += pe[a - 1] + 64;
+          }
+          if constexpr (a < L - 1) {
+            e += bf_renorm(zr, zi) - 29;
+            pr[a] = zr;
+            pi[a] = zi;
+            pe[a] = e;
+          } else {
+            x = make_double2(xor_sign(bf_to_double(zr, e), neg), xor_sign(bf_to_double(zi, e), neg));
+          }
+        } else if constexpr (a < L) {
           const double2 v = __ldg(Vg + (size_t)((w[a >> 2] >> (8 * (a & 3))) & 255u) * 32);
           if constexpr (a == 0) {
             P[0] = make_double2(xor_sign(v.x, neg), xor_sign(v.y, neg));
@@ -368,6 +420,7 @@ __global__ void __launch_bounds__(128) lossy_walk_kernel(const double2* __restri
             const double2 p = P[a - 1];
             P[a] = make_double2(fma(p.x, v.x, -(p.y * v.y)), fma(p.x, v.y, p.y * v.x));
           }
+          if constexpr (a == L - 1) x = P[a];
         }
       };
       // a jump into the chain, not a condition per step: predicated-off FP64
@@ -385,15 +438,15 @@ __global__ void __launch_bounds__(128) lossy_walk_kernel(const double2* __restri
         case 9: step(std::integral_constant<int, 9>{}); break;
         default: break;
       }
-      double2 x = P[L - 1];
       if constexpr (L < 6) {
+        double2 sum = x;
 #pragma unroll
         for (int o = 1; o < kLanes; o <<= 1) {
-          x.x += __shfl_xor_sync(0xffffffffu, x.x, o);
-          x.y += __shfl_xor_sync(0xffffffffu, x.y, o);
+          sum.x += __shfl_xor_sync(0xffffffffu, sum.x, o);
+          sum.y += __shfl_xor_sync(0xffffffffu, sum.y, o);
         }
         const int k = g * (32 / kLanes) + lane / kLanes;
-        if ((lane & (kLanes - 1)) == 0 && k < K) terms[(size_t)k * O + o0 + q] = term(x, k);
+        if ((lane & (kLanes - 1)) == 0 && k < K) terms[(size_t)k * O + o0 + q] = term(sum, k);
       } else {
         // eight outcomes at a time: four lanes add up eight combos each of one outcome
         buf[(q & 7) * 33 + lane] = x;
@@ -537,7 +590,7 @@ static void particle_list(const int32_t* occ, int m, uint8_t* out) {
 }
 
 template <int L>
-static cudaError_t launch_walk(const double2* V, int m, const uint4* rows, int64_t O, int K, int groups,
+static cudaError_t launch_walk(const double2* V, int m, const int32_t* fx, const uint4* rows, int64_t O, int K, int groups,
                                const double* div, const int* ndiv, const double* mult, double* terms,
                                int sm_count, cudaStream_t s) {
   // chunks of outcomes that leave about 16 warps per SM: a walk is serial (a chunk of
@@ -545,25 +598,25 @@ static cudaError_t launch_walk(const double2* V, int m, const uint4* rows, int64
   const int64_t want = O * groups / ((int64_t)sm_count * 16);
   const int chunk = (int)std::min<int64_t>(kWalkChunk, std::max<int64_t>(8, want / 8 * 8));
   const int64_t tasks = (O + chunk - 1) / chunk * groups;
-  lossy_walk_kernel<L><<<(unsigned)((tasks + 3) / 4), 128, 0, s>>>(V, m, rows, O, K, groups, div, ndiv, mult,
-                                                                chunk, terms);
+  auto* kernel = fx ? lossy_walk_kernel<L, true> : lossy_walk_kernel<L, false>;
+  kernel<<<(unsigned)((tasks + 3) / 4), 128, 0, s>>>(V, m, fx, rows, O, K, groups, div, ndiv, mult, chunk, terms);
   return cudaGetLastError();
 }
 
-static cudaError_t launch_walk_l(int l, const double2* V, int m, const uint4* rows, int64_t O, int K, int groups,
+static cudaError_t launch_walk_l(int l, const double2* V, int m, const int32_t* fx, const uint4* rows, int64_t O, int K, int groups,
                                  const double* div, const int* ndiv, const double* mult, double* terms,
                                  int sms, cudaStream_t s) {
   switch (l) {
-    case 1: return launch_walk<1>(V, m, rows, O, K, groups, div, ndiv, mult, terms, sms, s);
-    case 2: return launch_walk<2>(V, m, rows, O, K, groups, div, ndiv, mult, terms, sms, s);
-    case 3: return launch_walk<3>(V, m, rows, O, K, groups, div, ndiv, mult, terms, sms, s);
-    case 4: return launch_walk<4>(V, m, rows, O, K, groups, div, ndiv, mult, terms, sms, s);
-    case 5: return launch_walk<5>(V, m, rows, O, K, groups, div, ndiv, mult, terms, sms, s);
-    case 6: return launch_walk<6>(V, m, rows, O, K, groups, div, ndiv, mult, terms, sms, s);
-    case 7: return launch_walk<7>(V, m, rows, O, K, groups, div, ndiv, mult, terms, sms, s);
-    case 8: return launch_walk<8>(V, m, rows, O, K, groups, div, ndiv, mult, terms, sms, s);
-    case 9: return launch_walk<9>(V, m, rows, O, K, groups, div, ndiv, mult, terms, sms, s);
-    case 10: return launch_walk<10>(V, m, rows, O, K, groups, div, ndiv, mult, terms, sms, s);
+    case 1: return launch_walk<1>(V, m, fx, rows, O, K, groups, div, ndiv, mult, terms, sms, s);
+    case 2: return launch_walk<2>(V, m, fx, rows, O, K, groups, div, ndiv, mult, terms, sms, s);
+    case 3: return launch_walk<3>(V, m, fx, rows, O, K, groups, div, ndiv, mult, terms, sms, s);
+    case 4: return launch_walk<4>(V, m, fx, rows, O, K, groups, div, ndiv, mult, terms, sms, s);
+    case 5: return launch_walk<5>(V, m, fx, rows, O, K, groups, div, ndiv, mult, terms, sms, s);
+    case 6: return launch_walk<6>(V, m, fx, rows, O, K, groups, div, ndiv, mult, terms, sms, s);
+    case 7: return launch_walk<7>(V, m, fx, rows, O, K, groups, div, ndiv, mult, terms, sms, s);
+    case 8: return launch_walk<8>(V, m, fx, rows, O, K, groups, div, ndiv, mult, terms, sms, s);
+    case 9: return launch_walk<9>(V, m, fx, rows, O, K, groups, div, ndiv, mult, terms, sms, s);
+    case 10: return launch_walk<10>(V, m, fx, rows, O, K, groups, div, ndiv, mult, terms, sms, s);
     default: return cudaErrorInvalidValue;
   }
 }
@@ -586,8 +639,14 @@ static int queue_small_groups(Context* cx, const double* matrix, int m, int n, c
   size_t off = 0;
   const size_t o_U = off; off = align256(off + sizeof(double2) * (size_t)m * m);
   const size_t o_fact = off; off = align256(off + sizeof(double) * 256);
+  // fixed point if every entry is zero or of a size that has a scale
+  bool fixed = true;
+  for (size_t i = 0; i < (size_t)2 * m * m; ++i) {
+    const double x = std::fabs(matrix[i]);
+    fixed = fixed && (x == 0.0 || (x < 1e270 && x > 1e-270));
+  }
   size_t o_cols[kDistMaxL + 1], o_div[kDistMaxL + 1], o_ndiv[kDistMaxL + 1], o_mult[kDistMaxL + 1];
-  int64_t most_terms = 1, most_O = 1, most_V = 1;
+  int64_t most_terms = 1, most_O = 1, most_V = 1, most_fx = 1;
   int st;
   for (int l = 1; l <= kDistMaxL; ++l) {
     if (!G.size[l]) continue;
@@ -599,12 +658,14 @@ static int queue_small_groups(Context* cx, const double* matrix, int m, int n, c
     o_mult[l] = off; off = align256(off + sizeof(double) * (size_t)K);
     most_terms = std::max(most_terms, K * G.size[l]);
     most_O = std::max(most_O, G.size[l]);
+    most_fx = std::max(most_fx, K * m);
     const int64_t combos = ((K << (l - 1)) + 31) / 32 * 32;
     most_V = std::max(most_V, std::min(combos * m, std::max<int64_t>(kTableBytes / 16, (int64_t)m << l) + 32 * m));
   }
   if ((st = ensure(cx->dist[0], off))) return st;
   if ((st = ensure(cx->dist[1], sizeof(double) * (size_t)most_terms))) return st;
-  if ((st = ensure(cx->gpart, sizeof(uint4) * (size_t)most_O + sizeof(double2) * (size_t)most_V + 256))) return st;
+  const size_t o_V = align256(sizeof(uint4) * (size_t)most_O), o_fx = o_V + align256(sizeof(double2) * (size_t)most_V);
+  if ((st = ensure(cx->gpart, o_fx + sizeof(int32_t) * (size_t)most_fx))) return st;
   if ((st = ensure_pinned(cx, off))) return st;
   char* h = (char*)cx->pinned;
   memcpy(h + o_U, matrix, sizeof(double2) * (size_t)m * m);
@@ -627,7 +688,8 @@ static int queue_small_groups(Context* cx, const double* matrix, int m, int n, c
   char* d = (char*)cx->dist[0].ptr;
   double* terms = (double*)cx->dist[1].ptr;
   uint4* rows = (uint4*)cx->gpart.ptr;
-  double2* V = (double2*)((char*)cx->gpart.ptr + align256(sizeof(uint4) * (size_t)most_O));
+  double2* V = (double2*)((char*)cx->gpart.ptr + o_V);
+  int32_t* fx = fixed ? (int32_t*)((char*)cx->gpart.ptr + o_fx) : nullptr;
   cudaStream_t s = cx->stream;
   cudaError_t e = cudaMemcpyAsync(d, h, off, cudaMemcpyHostToDevice, s);
   if (e != cudaSuccess) return fail_cuda(e, "H2D distribution tables");
@@ -653,8 +715,8 @@ static int queue_small_groups(Context* cx, const double* matrix, int m, int n, c
       const int64_t combos = l >= 6 ? (int64_t)kn << (l - 1) : (int64_t)groups * 32;
       const uint8_t* cols = (const uint8_t*)(d + o_cols[l]) + k0 * l;
       lossy_table_kernel<<<(unsigned)((combos * m + 127) / 128), 128, 0, s>>>((const double2*)(d + o_U), m, l, cols, kn,
-                                                                             combos, V);
-      e = launch_walk_l(l, V, m, rows, O, kn, groups, (const double*)(d + o_div[l]) + k0 * kDistMaxDiv,
+                                                                             combos, fx ? fx + k0 * m : nullptr, V);
+      e = launch_walk_l(l, V, m, fx ? fx + k0 * m : nullptr, rows, O, kn, groups, (const double*)(d + o_div[l]) + k0 * kDistMaxDiv,
                         (const int*)(d + o_ndiv[l]) + k0, (const double*)(d + o_mult[l]) + k0, terms + k0 * O, cx->sm_count, s);
     }
     lossy_outcome_kernel<<<(unsigned)((O + 127) / 128), 128, 0, s>>>(terms, K, O, m, occ, (const double*)(d + o_fact),
