@@ -160,8 +160,9 @@ BOSS_API int boss_gccb_predraw(const int32_t* input_state, int32_t m, const doub
  * call on the 2m x 2m expanded matrix.  Consumes numpy's MT19937 stream exactly as
  * boss_gccb_predraw describes and returns the advanced state, so the samples are
  * the ones theboss draws with the same seed (given the same probabilities).
- * All samples run level-synchronously: the all-minors sweeps of every sample at
- * one step in one launch, the whole loop as one CUDA graph.
+ * All samples run level-synchronously: the first eight steps in one launch, above them
+ * the all-minors sweeps of every sample at one step in one, the whole loop as one CUDA
+ * graph.
  *   matrix   : m x m complex128, m <= 256;  sum(input_state) <= 32
  *   samples  : n_samples x m int32 output occupations
  */
@@ -207,7 +208,7 @@ BOSS_API int boss_gccb_near_ties(int64_t* count, int32_t reset);
 /*
  * The sampler's autotuner.  On the workload of a boss_gccb_sample call (the same
  * arguments; the MT19937 state is read, not advanced) it times, per level of
- * the sampler, power-of-two shifts of the split (threads per sample) and caps of
+ * the sampler that has launches of its own, power-of-two shifts of the split (threads per sample) and caps of
  * the size of the thread groups that sum their minors inside the sweep, keeps
  * the fastest shape of every level when the whole step gets faster, then times
  * the pipelined parts (the first part's size and the growth of the later ones)
@@ -234,11 +235,11 @@ BOSS_API int boss_gccb_autotune(const double* matrix, int32_t m, const int32_t* 
  * inputs uploaded once, then the captured sampler graph runs n_warmup + n_steps
  * times with inputs resident in GPU memory.  Before every run a flush_bytes
  * memset evicts L2.  Per timed run it writes the graph time (step_ms) and the
- * summed time of its all-minors sweep launches (sweep_ms), both from CUDA events
- * on the library stream.  info[0..6] = flops of the sweeps per run (9k - 12 per
+ * summed time of its all-minors sweep launches (sweep_ms; the first eight levels'
+ * launch counts, with its draws), both from CUDA events on the library stream.  info[0..6] = flops of the sweeps per run (9k - 12 per
  * Guan code at level k, over the codes the Glynn-form sweeps walk), H2D bytes and
- * D2H bytes of one boss_gccb_sample call, kernels per run, sweep launches per
- * run, the deepest level, the same flop count over theboss's Ryser-form codes
+ * D2H bytes of one boss_gccb_sample call, kernels per run, launches per run that
+ * are sweeps alone, the deepest level, the same flop count over theboss's Ryser-form codes
  * (twice as many for single photons), and the FP32 instructions per run of the
  * float-pair sweeps (47.5625 nf per code at nf factors: nf - 1 float-pair
  * complex products of 32, two complex float-pair sums of 16 for the running
