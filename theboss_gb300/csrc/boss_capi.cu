@@ -166,6 +166,7 @@ struct SweepBatch {
   int nd_max = 1;
   SweepLaunch L;
   size_t out_elems = 0;
+  double2* out = nullptr;  // results, in page-locked memory that the reduction writes: no copy down
   double codes = 0.0;  // codes swept per launch
 };
 
@@ -228,9 +229,10 @@ static int sweeps_prepare(Context* cx, const std::vector<HostSweep>& sweeps, boo
   int st;
   if ((st = ensure(cx->plans, arena_bytes))) return st;
   if ((st = ensure(cx->partials, sizeof(double2) * std::max<int64_t>(parts, 1)))) return st;
-  if ((st = ensure(cx->out, sizeof(double2) * B.out_elems))) return st;
-  if ((st = ensure_pinned(cx, std::max(up, sizeof(double2) * B.out_elems)))) return st;
+  const size_t o_out = align_up(up, 256);
+  if ((st = ensure_pinned(cx, o_out + sizeof(double2) * B.out_elems))) return st;
   char* h = (char*)cx->pinned;
+  B.out = (double2*)(h + o_out);
   memcpy(h + o_probs, probs.data(), sizeof(SweepProblem) * n);
   longlong2* hp = (longlong2*)(h + o_pool);
   int max_entries = 0;
@@ -280,18 +282,15 @@ static int sweeps_launch(Context* cx, const SweepBatch& B, cudaEvent_t after_swe
   cudaError_t e = launch_sweep(B.nf, op, B.L, cx->stream);
   if (e != cudaSuccess) return fail_cuda(e, "sweep launch");
   if (after_sweep) cudaEventRecord(after_sweep, cx->stream);
-  e = B.minors ? launch_minors_reduce(B.L.probs, B.n, B.L.rows, B.L.partials, (double2*)cx->out.ptr, B.nd_max, cx->stream, B.ff)
-               : launch_perm_reduce(B.L.probs, B.n, B.L.partials, (double2*)cx->out.ptr, cx->stream, B.ff);
+  e = B.minors ? launch_minors_reduce(B.L.probs, B.n, B.L.rows, B.L.partials, B.out, B.nd_max, cx->stream, B.ff)
+               : launch_perm_reduce(B.L.probs, B.n, B.L.partials, B.out, cx->stream, B.ff);
   return e == cudaSuccess ? kOk : fail_cuda(e, "reduce launch");
 }
 
 static int sweeps_collect(Context* cx, const SweepBatch& B, double2* results_host) {
-  cudaError_t e =
-      cudaMemcpyAsync(cx->pinned, cx->out.ptr, sizeof(double2) * B.out_elems, cudaMemcpyDeviceToHost, cx->stream);
-  if (e != cudaSuccess) return fail_cuda(e, "D2H results");
-  e = cudaStreamSynchronize(cx->stream);
+  const cudaError_t e = cudaStreamSynchronize(cx->stream);
   if (e != cudaSuccess) return fail_cuda(e, "sweep");
-  memcpy(results_host, cx->pinned, sizeof(double2) * B.out_elems);
+  memcpy(results_host, B.out, sizeof(double2) * B.out_elems);
   return kOk;
 }
 
@@ -300,8 +299,11 @@ int run_sweeps(Context* cx, const std::vector<HostSweep>& sweeps, bool minors, i
   if (sweeps.empty()) return kOk;
   SweepBatch B;
   int st = sweeps_prepare(cx, sweeps, minors, nd_max, B, matrix, m);
-  if (st) return st;
-  if ((st = sweeps_launch(cx, B))) return st;
+  if (!st) st = sweeps_launch(cx, B);
+  if (st) {
+    cudaStreamSynchronize(cx->stream);  // nothing queued may outlive the call's staging
+    return st;
+  }
   return sweeps_collect(cx, B, results_host);
 }
 

@@ -154,7 +154,9 @@ __global__ void __launch_bounds__(128) minors_reduce_kernel(const SweepProblem* 
   sr[threadIdx.x] = ar;
   si[threadIdx.x] = ai;
   __syncthreads();
-  for (int s = 64; s > 0; s >>= 1) {
+  int s = 64;
+  while (s >= parts) s >>= 1;  // few partials: the upper sums are zero
+  for (; s > 0; s >>= 1) {
     if ((int)threadIdx.x < s) {
       sr[threadIdx.x] += sr[threadIdx.x + s];
       si[threadIdx.x] += si[threadIdx.x + s];
