@@ -108,6 +108,26 @@ def _layer_entries(m: int):
     return torch.from_numpy(np.concatenate([np.concatenate(b) for b in blocks] + [ones])), len(ones)
 
 
+def _layer_product(theta: torch.Tensor, phi: torch.Tensor, m: int) -> torch.Tensor:
+    """The mesh's layers applied one after the other."""
+    ctype = torch.complex128
+    M = torch.eye(m, dtype=ctype, device=theta.device)
+    pos = 0
+    for ks in clements_layers(m):
+        k = torch.from_numpy(ks).to(theta.device)
+        n = len(ks)
+        th = theta[pos:pos + n]
+        ep = torch.exp(1j * phi[pos:pos + n].to(ctype))
+        pos += n
+        c = torch.cos(th).to(ctype)
+        s = torch.sin(th).to(ctype)
+        top, bot = M[k], M[k + 1]
+        new_top = (ep * c)[:, None] * top - s[:, None] * bot
+        new_bot = (ep * s)[:, None] * top + c[:, None] * bot
+        M = M.index_copy(0, k, new_top).index_copy(0, k + 1, new_bot)
+    return M
+
+
 def clements_unitary(theta: torch.Tensor, phi: torch.Tensor, output_phases: torch.Tensor = None) -> torch.Tensor:
     """U = D * T_L ... T_1 with T(theta, phi) on modes (k, k+1):
     [[e^{i phi} cos theta, -sin theta], [e^{i phi} sin theta, cos theta]]."""
@@ -116,12 +136,14 @@ def clements_unitary(theta: torch.Tensor, phi: torch.Tensor, output_phases: torc
     if m * (m - 1) // 2 != n_mzi or phi.shape[0] != n_mzi:
         raise ValueError("theta and phi need m(m-1)/2 entries each")
     ctype = torch.complex128
-    ep, c, s = torch.exp(1j * phi.to(ctype)), torch.cos(theta).to(ctype), torch.sin(theta).to(ctype)
-    if m <= _DENSE_LAYERS:
+    if m <= _DENSE_LAYERS and torch.is_grad_enabled() and (theta.requires_grad or phi.requires_grad):
         # every layer as a dense m x m matrix, multiplied pairwise: 2 log2(m) batched
-        # products instead of some fifteen small operations per layer, whose dispatch
-        # was the whole time (forward and backward, CPU: m = 24 9.6 -> 1.3 ms, m = 96
-        # 70 -> 10.5 ms; beyond that the m^3 entries grow past what it saves)
+        # products instead of some fifteen small operations per layer for autograd to
+        # follow, whose dispatch was the whole time (forward and backward, CPU: m = 24
+        # 9.6 -> 1.3 ms, m = 96 70 -> 10.5 ms; beyond that the m^3 entries grow past what
+        # it saves).  Its value is replaced by the layers' own product, in their order:
+        # derivatives of the logarithm of a small probability magnify the last bits of U.
+        ep, c, s = torch.exp(1j * phi.to(ctype)), torch.cos(theta).to(ctype), torch.sin(theta).to(ctype)
         at, ones = _layer_entries(m)
         v = torch.cat([ep * c, -s, ep * s, c, torch.ones(ones, dtype=ctype, device=theta.device)])
         L = torch.zeros(m * m * m, dtype=ctype, device=theta.device).index_copy(0, at.to(theta.device), v)
@@ -130,18 +152,11 @@ def clements_unitary(theta: torch.Tensor, phi: torch.Tensor, output_phases: torc
             n = L.shape[0]
             P = L[1::2] @ L[0:n - n % 2:2]  # the later layer on the left
             L = torch.cat([P, L[-1:]]) if n % 2 else P
-        M = L[0]
+        with torch.no_grad():
+            value = _layer_product(theta.detach(), phi.detach(), m)
+        M = L[0] + (value - L[0].detach())
     else:
-        M = torch.eye(m, dtype=ctype, device=theta.device)
-        pos = 0
-        for ks in clements_layers(m):
-            k = torch.from_numpy(ks).to(theta.device)
-            q = slice(pos, pos + len(ks))
-            pos += len(ks)
-            top, bot = M[k], M[k + 1]
-            new_top = (ep[q] * c[q])[:, None] * top - s[q][:, None] * bot
-            new_bot = (ep[q] * s[q])[:, None] * top + c[q][:, None] * bot
-            M = M.index_copy(0, k, new_top).index_copy(0, k + 1, new_bot)
+        M = _layer_product(theta, phi, m)
     if output_phases is not None:
         M = torch.exp(1j * output_phases.to(ctype))[:, None] * M
     return M
