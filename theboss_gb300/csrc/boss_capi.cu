@@ -361,15 +361,14 @@ int g_perm_arith = 1;
 
 static longlong2 packed(Cx64 v) { return longlong2{pack_row(v.re), pack_row(v.im)}; }
 static longlong2 plain(Cx64 v) { return longlong2{v.re, v.im}; }
-static Cx64 times(Cx64 v, long long k) { return Cx64{v.re * k, v.im * k}; }
 
 // The rows, base and constants of boss_quad.cuh.  u[a * nf + f]: every digit's
 // fixed-point u (binary digits first, the held one at `drop`).
 static void fill_quad(HostSweep& hs, const Side& dig, int drop, bool glynn, const std::vector<Cx64>& u) {
-  const int nf = hs.nf, slots = quad_slots(nf), W = 4 * slots, nd_all = (int)dig.modes.size(), ndo = hs.nd - 2;
+  const int nf = hs.nf, slots = quad_slots(nf), W = quad_width(nf), nd_all = (int)dig.modes.size(), ndo = hs.nd - 2;
   const Cx64 zero{0, 0};
   hs.D.assign((size_t)ndo * W, longlong2{0, 0});
-  hs.base.assign((size_t)W + 2 * slots, longlong2{0, 0});
+  hs.base.assign((size_t)quad_base(nf), longlong2{0, 0});
   longlong2* consts = hs.base.data() + W;
   for (int g = 0; g < slots; ++g) {
     const bool unit = 2 * g + 1 >= nf;  // an odd last factor's partner, the constant 1
@@ -382,16 +381,17 @@ static void fill_quad(HostSweep& hs, const Side& dig, int drop, bool glynn, cons
       Cx64 rp, rm;
       quad_row(uf, ug, f0, f1, g0, g1, rp, rm);
       if (a != drop) {
-        longlong2* r = &hs.D[(size_t)(row++) * W + 4 * g];
+        longlong2* r = &hs.D[(size_t)(row++) * W + kQuadRow * g];
         r[0] = packed(uf);
         r[1] = packed(ug);
         r[2] = packed(rp);
         r[3] = packed(rm);
+        r[4] = quad_low(rp, rm);
       }
-      of = cx_add(of, times(uf, dig.mult[a]));
-      og = cx_add(og, times(ug, dig.mult[a]));
-      ep = cx_add(ep, times(rp, dig.mult[a]));
-      em = cx_add(em, times(rm, dig.mult[a]));
+      of = cx_add(of, cx_times(uf, dig.mult[a]));
+      og = cx_add(og, cx_times(ug, dig.mult[a]));
+      ep = cx_add(ep, cx_times(rp, dig.mult[a]));
+      em = cx_add(em, cx_times(rm, dig.mult[a]));
     }
     if (!glynn) {  // Ryser: no base, and r = (1 - d) / 2 leaves -(u0 + u1)
       of = cx_sub(zero, cx_add(f0, f1));
@@ -402,15 +402,13 @@ static void fill_quad(HostSweep& hs, const Side& dig, int drop, bool glynn, cons
       og = Cx64{kQuadOne, 0};
       quad_row(zero, og, f0, f1, zero, zero, ep, em);
     }
-    longlong2* b = &hs.base[4 * g];
+    longlong2* b = &hs.base[kQuadRow * g];
     b[0] = plain(of);
     b[1] = plain(og);
     b[2] = plain(ep);
     b[3] = plain(em);
-    Cx64 cp, cm;
-    quad_const(f0, f1, g0, g1, cp, cm);
-    consts[2 * g] = plain(cp);
-    consts[2 * g + 1] = plain(cm);
+    b[4] = quad_low(ep, em);
+    quad_constants(f0, f1, g0, g1, consts + kQuadConst * g);
   }
   if (nf & 1) hs.fx_sum += 62;
 }
@@ -487,7 +485,7 @@ static int fill_sweep(HostSweep& hs, const Side& dig, const Side& col, int kind,
   if (hs.on_device) {
     const int Fg = grad_factors(hs.nf), W = quad_width(hs.nf);
     hs.D_size = hs.layout == kRowsGrad ? (size_t)hs.nd * Fg : (size_t)(hs.nd - 2) * W;
-    hs.base_size = hs.layout == kRowsGrad ? (size_t)Fg + Fg / 4 : (size_t)W + W / 2;
+    hs.base_size = hs.layout == kRowsGrad ? (size_t)Fg + Fg / 4 : (size_t)quad_base(hs.nf);
     return kOk;
   }
   // |row sum| <= sum_a mult_a * max component of the entries

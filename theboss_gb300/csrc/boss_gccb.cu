@@ -1376,7 +1376,7 @@ __device__ __forceinline__ void fin_rows(const FinalizeArgs& a, int j, const Fin
     return cx(u.x, u.y);
   };
   if (a.next_quad) {
-    const int slots = quad_slots(nf), W = 4 * slots, ndo = nds - 2;
+    const int slots = quad_slots(nf), W = quad_width(nf), ndo = nds - 2;
     base_off = (int64_t)ndo * W;
     longlong2* B = D + base_off;
     longlong2* consts = B + W;
@@ -1387,11 +1387,12 @@ __device__ __forceinline__ void fin_rows(const FinalizeArgs& a, int j, const Fin
       const Cx64 uf = entry(2 * g, d + 2), ug = second(g, d + 2);
       Cx64 ep, em;
       quad_row(uf, ug, entry(2 * g, 0), entry(2 * g, 1), second(g, 0), second(g, 1), ep, em);
-      longlong2* r = D + (size_t)d * W + 4 * g;
+      longlong2* r = D + (size_t)d * W + kQuadRow * g;
       r[0] = make_longlong2(pack_row(uf.re), pack_row(uf.im));
       r[1] = make_longlong2(pack_row(ug.re), pack_row(ug.im));
       r[2] = make_longlong2(pack_row(ep.re), pack_row(ep.im));
       r[3] = make_longlong2(pack_row(em.re), pack_row(em.im));
+      r[4] = quad_low(ep, em);
     }
     __syncwarp();  // the rows just written by other lanes
     for (int f = lane; f < nf; f += 32) {  // the factors' outer sums
@@ -1402,32 +1403,32 @@ __device__ __forceinline__ void fin_rows(const FinalizeArgs& a, int j, const Fin
         const long long mu = sh.mult[d];
         o = cx(o.re + mu * u.re, o.im + mu * u.im);
       }
-      B[4 * (f >> 1) + (f & 1)] = make_longlong2(o.re, o.im);
+      B[kQuadRow * (f >> 1) + (f & 1)] = make_longlong2(o.re, o.im);
       fxsum += rowfx[sh.fm[f]];
     }
     for (int g = lane; g < slots; g += 32) {  // the pairs' E+-: the rows' coefficients and the held digit's
       const Cx64 f0 = entry(2 * g, 0), f1 = entry(2 * g, 1), g0 = second(g, 0), g1 = second(g, 1);
       Cx64 ep = cx(0, 0), em = cx(0, 0);
       if (2 * g + 1 >= nf) {
-        B[4 * g + 1] = make_longlong2(kQuadOne, 0);
+        B[kQuadRow * g + 1] = make_longlong2(kQuadOne, 0);
         quad_row(cx(0, 0), cx(kQuadOne, 0), f0, f1, cx(0, 0), cx(0, 0), ep, em);
         fxsum += 62;
       } else {
         if (held) quad_row(entry(2 * g, nds), second(g, nds), f0, f1, g0, g1, ep, em);
 #pragma unroll 4
         for (int d = 0; d < ndo; ++d) {
-          const longlong2 p = D[(size_t)d * W + 4 * g + 2], q = D[(size_t)d * W + 4 * g + 3];
-          const long long mu = sh.mult[d + 2];
-          ep = cx(ep.re + mu * unpack_row(p.x), ep.im + mu * unpack_row(p.y));
-          em = cx(em.re + mu * unpack_row(q.x), em.im + mu * unpack_row(q.y));
+          const longlong2* r = D + (size_t)d * W + kQuadRow * g;
+          const longlong2 p = r[2], q = r[3];
+          const int4 low = *reinterpret_cast<const int4*>(r + 4);
+          const int mu = sh.mult[d + 2];
+          ep = cx_add(ep, cx_times(Cx64{unpack_row(p.x), unpack_row(p.y), low.x, low.y}, mu));
+          em = cx_add(em, cx_times(Cx64{unpack_row(q.x), unpack_row(q.y), low.z, low.w}, mu));
         }
       }
-      B[4 * g + 2] = make_longlong2(ep.re, ep.im);
-      B[4 * g + 3] = make_longlong2(em.re, em.im);
-      Cx64 cp, cm;
-      quad_const(f0, f1, g0, g1, cp, cm);
-      consts[2 * g] = make_longlong2(cp.re, cp.im);
-      consts[2 * g + 1] = make_longlong2(cm.re, cm.im);
+      B[kQuadRow * g + 2] = make_longlong2(ep.re, ep.im);
+      B[kQuadRow * g + 3] = make_longlong2(em.re, em.im);
+      B[kQuadRow * g + 4] = quad_low(ep, em);
+      quad_constants(f0, f1, g0, g1, consts + kQuadConst * g);
     }
   } else {
     base_off = (int64_t)nds * nf;

@@ -3,12 +3,10 @@
 // kQuadMinMinorFactors).  The templated kernels of boss_sweep_kernels.cuh take the
 // others.
 //
-// Measured (64 permanents, input-side digits): n = 20 1.41 ms, n = 24 24.0 ms, n = 28
-// 486 ms, against 1.71, 33.5 and about 640 ms with the templated kernel; the
-// benchmark's output-side batches n = 28 104 ms against 154.  45 instructions per
-// factor and code (58 there); the FMA pipe 61 % busy, the ALU pipe 51 %, the rest
-// dispatch and fixed-latency stalls at 16 warps per SM, which more warps do not
-// lessen.
+// Measured (calls of 64 permanents, input-side digits): n = 20 1.82 ms, n = 24 29.1 ms;
+// with the pairs in 62 bits, which lost weakly coupled networks' digits, 1.52 and 24.5.
+// 8 of n = 28 73 ms (61).  Bound by fixed latencies of one dependent chain a lane at 12
+// to 16 warps per SM, which more warps do not lessen.
 #include <algorithm>
 
 #include "boss_internal.h"
@@ -16,17 +14,17 @@
 
 namespace boss {
 
-// Blocks of 128 per SM the kernels are compiled for: the state is 16 registers per
-// four slots.  One block more or fewer at any size is no faster (64 permanents at
-// n = 20: 4 blocks 1.41 ms, 3 blocks 1.47; n = 28: 3 or 4 blocks 104 ms).
-constexpr int quad_blocks(int slots) { return slots <= 4 ? 5 : slots <= 12 ? 4 : 3; }
+// Blocks of 128 per SM the kernels are compiled for: the state is 20 registers per
+// four slots.  64 permanents at n = 20: 3 blocks 1.82 ms, 4 blocks (spills) 1.88; n = 24
+// 29.1 and 30.3; 8 of n = 28: 3 blocks 73.1 ms, 2 blocks 78.4.
+constexpr int quad_blocks(int slots) { return slots <= 4 ? 5 : slots <= 8 ? 4 : 3; }
 
 // A lane's slots are 4 i + (lane & 3) of its walker, i = 0 .. ceil(S / 4) - 1, their
 // state in registers (lanes past the last slot repeat it, so that no lane
-// branches).  Shared memory, 16-byte entries: two buffers for the slots' four
-// values on their way to the chains' lanes, value v of thread t at
-// [v * kQuadXStride + t] (the odd stride puts a walker's four readers in different
-// banks).
+// branches).  Shared memory, two buffers for the slots' four values on their way to
+// the chains' lanes, 16-byte entries, value v of thread t at [v * kQuadXStride + t]
+// (the odd stride puts a walker's four readers in different banks).  Their exponents
+// stay with the slots' lanes, summed, two 16-bit sums a register (low + 2^16 high).
 constexpr int kQuadXStride = kQuadBlock + 1;
 constexpr int kQuadX = 4 * kQuadXStride;
 template <int S>
@@ -39,29 +37,59 @@ struct QuadState {
   }
 };
 
+// A pair's state moved by sg times its entries of a row.
+__device__ __forceinline__ void quad_move(Cx64 (&v)[4], const longlong2* __restrict__ row, int sg) {
+  const int4 low = __ldg(reinterpret_cast<const int4*>(row + 4));
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    const longlong2 d = __ldg(row + c);
+    v[c].re = add_packed(v[c].re, d.x, sg);
+    v[c].im = add_packed(v[c].im, d.y, sg);
+  }
+  v[2].fr += sg * low.x;
+  v[2].fi += sg * low.y;
+  v[3].fr += sg * low.z;
+  v[3].fi += sg * low.w;
+}
+
+// The small ones among a pair's four values formed from its factors, in place (rare:
+// out of line; con: the pair's constants).  Takes and returns the exponents' pairs.
+__device__ __noinline__ int2 quad_redo(longlong2* vals, int2 ls, const longlong2* __restrict__ con, long long fr,
+                                       long long fi, long long gr, long long gi) {
+  auto at = [&](int c) {
+    const longlong2 x = con[3 + c];
+    return cx(x.x, x.y);
+  };
+  int l[4] = {(short)ls.x, (ls.x - (short)ls.x) >> 16, (short)ls.y, (ls.y - (short)ls.y) >> 16};
+  for (int k = 0; k < 4; ++k) {
+    if (l[k] >= kQuadLeast) continue;
+    Cx64 q;
+    l[k] = quad_small(k, cx(fr, fi), cx(gr, gi), at(0), at(1), at(2), at(3), q);
+    vals[k * kQuadXStride] = make_longlong2(q.re, q.im);
+  }
+  return make_int2(l[0] + l[1] * 65536, l[2] + l[3] * 65536);
+}
+
 // The walk at outer code t, and this lane's state.
 template <int S>
 __device__ __forceinline__ void quad_decode(const SweepProblem& P, const longlong2* __restrict__ rows,
                                             const longlong2* __restrict__ base, uint64_t t, QuadState<S>& st, QuadWalk& k) {
-  constexpr int W = 4 * S;
+  constexpr int W = kQuadRow * S;
   const int nb = P.nb;
   quad_walk_at(P, t, k);
 #pragma unroll
-  for (int i = 0; i < QuadState<S>::kRounds; ++i)
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      const longlong2 b = base[4 * QuadState<S>::slot(i) + c];
-      st.v[i][c] = cx(b.x, b.y);
-    }
+  for (int i = 0; i < QuadState<S>::kRounds; ++i) {
+    const longlong2* b = base + kQuadRow * QuadState<S>::slot(i);
+    const int4 low = *reinterpret_cast<const int4*>(b + 4);
+    st.v[i][0] = cx(b[0].x, b[0].y);
+    st.v[i][1] = cx(b[1].x, b[1].y);
+    st.v[i][2] = Cx64{b[2].x, b[2].y, low.x, low.y};
+    st.v[i][3] = Cx64{b[3].x, b[3].y, low.z, low.w};
+  }
   auto add = [&](int d, int sg) {
-    const longlong2* row = rows + (int64_t)d * W;
 #pragma unroll
     for (int i = 0; i < QuadState<S>::kRounds; ++i)
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        const longlong2 x = __ldg(row + 4 * QuadState<S>::slot(i) + c);
-        st.v[i][c] = cx(add_packed(st.v[i][c].re, x.x, sg), add_packed(st.v[i][c].im, x.y, sg));
-      }
+      quad_move(st.v[i], rows + (int64_t)d * W + kQuadRow * QuadState<S>::slot(i), sg);
   };
   for (uint64_t bits = k.g; bits; bits &= bits - 1ull) add(__ffsll((long long)bits) - 1, -2);
   for (int d = nb; d < P.nd; ++d)
@@ -77,23 +105,24 @@ __device__ __forceinline__ void quad_eval(QuadState<S>& st, longlong2* xbuf, con
                                           int& e) {
   constexpr int kRounds = (S + 3) / 4;
   const int kk = threadIdx.x & 3;
-  longlong2* mine = xbuf + threadIdx.x;
-  const longlong2* from = xbuf + kk * kQuadXStride + (threadIdx.x & ~3);
-  int ls = 0, ps = 0;  // leading bits: of this lane's slots, of its chain
+  int2 ls = make_int2(0, 0);  // exponents of this lane's values
+  const int from = kk * kQuadXStride + (threadIdx.x & ~3);
+  int ps = 0;  // and of its chain
   auto prepare = [&](int i) {
-    const int s = QuadState<S>::slot(i);
-    const longlong2 cp = __ldg(consts + 2 * s), cm = __ldg(consts + 2 * s + 1);
+    const int s = QuadState<S>::slot(i), at = (i & 1) * kQuadX + (int)threadIdx.x;
+    const longlong2* con = consts + kQuadConst * s;
+    const longlong2 cp = __ldg(con), cm = __ldg(con + 1);
+    const int4 low = __ldg(reinterpret_cast<const int4*>(con + 2));
     Cx64(&v)[4] = st.v[i];
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      const longlong2 d = __ldg(row + 4 * s + c);
-      v[c] = cx(add_packed(v[c].re, d.x, sg), add_packed(v[c].im, d.y, sg));
-    }
+    quad_move(v, row + kQuadRow * s, sg);
     Cx64 q[4];
-    const int l = quad_pair(v[0], v[1], v[2], v[3], cx(cp.x, cp.y), cx(cm.x, cm.y), q);
-    ls += (4 * i + 4 <= S || 4 * i + kk < S) ? l : 0;
+    int l[4];
+    const int least = quad_values(v[0], v[1], v[2], v[3], Cx64{cp.x, cp.y, low.x, low.y}, Cx64{cm.x, cm.y, low.z, low.w}, q, l);
+    int2 lv = make_int2(l[0] + l[1] * 65536, l[2] + l[3] * 65536);
 #pragma unroll
-    for (int c = 0; c < 4; ++c) mine[(i & 1) * kQuadX + c * kQuadXStride] = make_longlong2(q[c].re, q[c].im);
+    for (int c = 0; c < 4; ++c) xbuf[at + c * kQuadXStride] = make_longlong2(q[c].re, q[c].im);
+    if (least < kQuadLeast) lv = quad_redo(xbuf + at, lv, con, v[0].re, v[0].im, v[1].re, v[1].im);
+    if (4 * i + 4 <= S || 4 * i + kk < S) ls = make_int2(ls.x + lv.x, ls.y + lv.y);
   };
   prepare(0);
   __syncwarp();
@@ -103,14 +132,18 @@ __device__ __forceinline__ void quad_eval(QuadState<S>& st, longlong2* xbuf, con
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       if (4 * i + j >= S) break;
-      const longlong2 q = from[(i & 1) * kQuadX + j];
+      const longlong2 q = xbuf[(i & 1) * kQuadX + from + j];
       ps += (i + j == 0) ? quad_chain_first(re, im, q.x, q.y) : quad_chain(re, im, q.x, q.y);
     }
     __syncwarp();
   }
-  ls += __shfl_xor_sync(0xffffffffu, ls, 1);
-  ls += __shfl_xor_sync(0xffffffffu, ls, 2);
-  e = quad_exponent(e0, ls, S) + ps;
+#pragma unroll
+  for (int o = 1; o < 4; o <<= 1) {
+    ls.x += __shfl_xor_sync(0xffffffffu, ls.x, o);
+    ls.y += __shfl_xor_sync(0xffffffffu, ls.y, o);
+  }
+  const int l = (kk & 2) ? ls.y : ls.x, low = (short)l;  // the sum of this chain's values
+  e = quad_exponent(e0, (kk & 1) ? (l - low) >> 16 : low, S) + ps;
 }
 
 // One permanent per sweep problem; every group of walkers writes one complex partial.
@@ -126,7 +159,7 @@ __global__ void __launch_bounds__(kQuadBlock, quad_blocks(S)) perm_quad_kernel(c
   const int64_t walker = live ? at : total_walkers - 1;
   const SweepProblem& P = probs[find_problem(probs, n_probs, walker)];
   const QuadRange R = quad_range(P, walker, live);
-  constexpr int W = 4 * S;
+  constexpr int W = kQuadRow * S;
   const longlong2* rows = pool + P.mat_off;
   const longlong2* base = pool + P.base_off;
   QuadState<S> st;
@@ -179,7 +212,7 @@ __global__ void __launch_bounds__(kQuadBlock, quad_blocks(S)) minors_quad_kernel
   const SweepProblem& P =
       probs[uniform_walkers > 0 ? (int)(walker / uniform_walkers) : find_problem(probs, n_probs, walker)];
   const QuadRange R = quad_range(P, walker, live);
-  constexpr int W = 4 * S;
+  constexpr int W = kQuadRow * S;
   const int ndo = P.nd, nb = P.nb;
   const longlong2* rows = pool + P.mat_off;
   const longlong2* base = pool + P.base_off;
@@ -266,8 +299,7 @@ __global__ void __launch_bounds__(kQuadBlock, quad_blocks(S)) minors_quad_kernel
 
 static size_t quad_smem_bytes(int slots, int rows) {
   const int rounds = (slots + 3) / 4;
-  return sizeof(longlong2) *
-         (size_t)std::max((rounds > 1 ? 2 : 1) * kQuadX, rows * kQuadBlock);
+  return sizeof(longlong2) * (size_t)std::max((rounds > 1 ? 2 : 1) * kQuadX, rows * kQuadBlock);
 }
 
 constexpr int kQuadMaxSlots = (kMaxFactors + 1) / 2;

@@ -9,28 +9,34 @@
 //     E+- = o_f (u_g0 +- u_g1) + o_g (u_f0 +- u_f1),
 // so its four values are K+ + E+, K+ - E+, K- + E-, K- - E-: one product for four
 // codes instead of four, and E+-, linear in the outer digits, walks by additions
-// like the row sums do.  Per factor and code that leaves 9 instead of 15 holds of
-// the FMA pipe (which bounds the sweeps: a 32 x 32 + 64-bit multiply-add holds it
-// for 4 cycles a warp).
+// like the row sums do.
 //
 // Four lanes walk together (a walker): each prepares a quarter of the pairs (moves
 // their state, forms the four values, hands them over through shared memory) and
 // multiplies one code's chain over all pairs.  A lane's share of the state then fits
 // in registers; one thread doing all four codes kept it in shared memory, 8 to 16
-// warps per SM and 40 % of the issue slots (n = 20: 1.52 ms against 1.41).
+// warps per SM and 40 % of the issue slots.
 //
 // Fixed point: factor f in units 2^-fx_f, its largest possible sum (every digit
 // included) below 2^62; a pair's K and E in units 2^(64 - fx_f - fx_g), below 2^61
-// (a component of s_f s_g is below 2 * 2^62 * 2^62).  E's coefficients and C+- are
-// rounded once from exact 128-bit products; o_f o_g is truncated (bf_mul_high).
+// (a component of s_f s_g is below 2 * 2^62 * 2^62), with 16 bits more below them.  A
+// value K +- E that comes out far below its largest possible size (2^-17 of it: a
+// network's weakly coupled modes) has lost those bits, and is formed from the two
+// factor sums instead (quad_small, exact 128-bit product): every value handed to a chain is
+// within 2^-55 of the pair's product.  (With K and E in 62 bits alone, 12 photons whose
+// modes couple by 1e-4 and are doubly occupied at the output: 4.7e-9; now
+// 3e-14.)  Haar matrices at 28 photons take the second way
+// for a few values in 10^6.
 //
 // Layout of a sweep in the pool (longlong2 = one complex), slots = ceil(nf / 2)
 // pairs (an odd last factor is paired with the constant 1 = 2^62 in its units),
-// W = 4 slots:
-//   rows, one per outer digit: per pair u_f u_g e+ e-, packed (pack_row); the walk
-//     adds -2 r times a row (r: the digit's value);
-//   base, W: o_f o_g E+ E- per pair at r = 0 (unpacked);
-//   constants, 2 per pair: C+, C- - C+.
+// W = kQuadRow slots:
+//   rows, one per outer digit: per pair u_f u_g e+ e-, packed (pack_row), and the e's
+//     16 low bits (int4: e+ re im, e- re im); the walk adds -2 r times a row (r: the
+//     digit's value);
+//   base, W: o_f o_g E+ E- and the E's low parts per pair at r = 0 (unpacked);
+//   constants, kQuadConst per pair: C+, C- - C+, their low parts (int4, 0 .. 2^16 - 1), and the low
+//     digits' u_f0 u_f1 u_g0 u_g1.
 #pragma once
 #include "boss_sweep.cuh"
 
@@ -41,28 +47,46 @@ constexpr int kQuadBlock = 128;                          // threads per block
 constexpr int kQuadWalkers = kQuadBlock / kQuadLanes;    // walkers per block
 constexpr long long kQuadOne = 1ll << 62;                // the constant factor, 62 fraction bits
 
+constexpr int kQuadRow = 5;    // entries per pair of a row, of the base
+constexpr int kQuadConst = 7;  // and of the constants
 __host__ __device__ __forceinline__ int quad_slots(int nf) { return (nf + 1) >> 1; }
-__host__ __device__ __forceinline__ int quad_width(int nf) { return 4 * quad_slots(nf); }
-// Pool entries of a quad sweep over ndo outer digits.
+__host__ __device__ __forceinline__ int quad_width(int nf) { return kQuadRow * quad_slots(nf); }
+// Entries of the base and the constants; of a quad sweep over ndo outer digits.
+__host__ __device__ __forceinline__ int quad_base(int nf) { return quad_width(nf) + kQuadConst * quad_slots(nf); }
 __host__ __device__ __forceinline__ int64_t quad_pool(int ndo, int nf) {
-  return (int64_t)(ndo + 1) * quad_width(nf) + 2 * quad_slots(nf);
+  return (int64_t)ndo * quad_width(nf) + quad_base(nf);
 }
 
-struct Cx64 {  // complex fixed point
+struct Cx64 {  // complex fixed point: re + fr 2^-16, im + fi 2^-16 (the low parts: of pairs' E and C only)
   long long re, im;
+  int fr = 0, fi = 0;  // sums of at most 2^14 coefficients' 0 .. 2^16
 };
 __host__ __device__ __forceinline__ Cx64 cx(long long re, long long im) { return Cx64{re, im}; }
-__host__ __device__ __forceinline__ Cx64 cx_add(Cx64 a, Cx64 b) { return Cx64{a.re + b.re, a.im + b.im}; }
-__host__ __device__ __forceinline__ Cx64 cx_sub(Cx64 a, Cx64 b) { return Cx64{a.re - b.re, a.im - b.im}; }
+__host__ __device__ __forceinline__ Cx64 cx_add(Cx64 a, Cx64 b) {
+  return Cx64{a.re + b.re, a.im + b.im, a.fr + b.fr, a.fi + b.fi};
+}
+__host__ __device__ __forceinline__ Cx64 cx_sub(Cx64 a, Cx64 b) {
+  return Cx64{a.re - b.re, a.im - b.im, a.fr - b.fr, a.fi - b.fi};
+}
+__host__ __device__ __forceinline__ Cx64 cx_times(Cx64 v, int k) {
+  return Cx64{v.re * k, v.im * k, v.fr * k, v.fi * k};
+}
+// Two complex low parts as one pool entry (int4 in memory).
+__host__ __device__ __forceinline__ longlong2 quad_low(Cx64 a, Cx64 b) {
+  longlong2 v;
+  v.x = join32((unsigned)a.fi, (unsigned)a.fr);
+  v.y = join32((unsigned)b.fi, (unsigned)b.fr);
+  return v;
+}
 
-// (a b + c d) 2^-64 rounded to nearest, from exact 128-bit sums.
-__host__ __device__ __forceinline__ long long round_hi(I128 v) { return v.hi + (long long)(v.lo >> 63); }
+// v 2^-64 in 64 + 16 bits, rounded to nearest.
+__host__ __device__ __forceinline__ int low16(I128 v) { return (int)(v.lo >> 48) + (int)((v.lo >> 47) & 1ull); }
 __host__ __device__ __forceinline__ Cx64 quad_coef(Cx64 a, Cx64 b, Cx64 c, Cx64 d) {
   const I128 re = add128(sub128(mul_s64(a.re, b.re), mul_s64(a.im, b.im)),
                          sub128(mul_s64(c.re, d.re), mul_s64(c.im, d.im)));
   const I128 im = add128(add128(mul_s64(a.re, b.im), mul_s64(a.im, b.re)),
                          add128(mul_s64(c.re, d.im), mul_s64(c.im, d.re)));
-  return cx(round_hi(re), round_hi(im));
+  return Cx64{re.hi, im.hi, low16(re), low16(im)};
 }
 // E+ and E- coefficients of one outer digit: uf, ug its entries; f0 f1 g0 g1 the low digits'.
 __host__ __device__ __forceinline__ void quad_row(Cx64 uf, Cx64 ug, Cx64 f0, Cx64 f1, Cx64 g0, Cx64 g1, Cx64& ep,
@@ -77,39 +101,123 @@ __host__ __device__ __forceinline__ void quad_const(Cx64 f0, Cx64 f1, Cx64 g0, C
   cm_cp = cx_sub(quad_coef(cx_sub(f0, f1), cx_sub(g0, g1), z, z), cp);
 }
 
-__host__ __device__ __forceinline__ long long shl64(long long x, int s) {  // 0 <= s < 32
-  return join32(fshl32(lo32(x), hi32(x), s), lo32(x) << (s & 31));
+__host__ __device__ __forceinline__ Cx64 quad_carry(Cx64 v) {
+  return Cx64{v.re + (v.fr >> 16), v.im + (v.fi >> 16), v.fr & 0xffff, v.fi & 0xffff};
+}
+// A pair's constants as they lie in the pool.
+__host__ __device__ __forceinline__ void quad_constants(Cx64 f0, Cx64 f1, Cx64 g0, Cx64 g1, longlong2* out) {
+  Cx64 v[6];
+  quad_const(f0, f1, g0, g1, v[0], v[1]);
+  v[0] = quad_carry(v[0]);
+  v[1] = quad_carry(v[1]);
+  out[2] = quad_low(v[0], v[1]);
+  v[2] = f0;
+  v[3] = f1;
+  v[4] = g0;
+  v[5] = g1;
+  for (int c = 0; c < 6; ++c) {
+    out[c < 2 ? c : c + 1].x = v[c].re;
+    out[c < 2 ? c : c + 1].y = v[c].im;
+  }
 }
 
-// The four values q, order (+,+), (-,-), (+,-), (-,+), from K+- and E+- (all below
-// 2^61), which are normalised together first, so that no bit is left to the gap
-// between the largest possible sum and the sums as they are.  Returns the leading
-// bit's position, which quad_exponent takes back.
-__host__ __device__ __forceinline__ int quad_values(Cx64 kp, Cx64 km, Cx64 ep, Cx64 em, Cx64 (&q)[4]) {
-  const int l0 = lead_bit((int)hi32(kp.re)), l1 = lead_bit((int)hi32(kp.im));
-  const int l2 = lead_bit((int)hi32(km.re)), l3 = lead_bit((int)hi32(km.im));
-  const int l4 = lead_bit((int)hi32(ep.re)), l5 = lead_bit((int)hi32(ep.im));
-  const int l6 = lead_bit((int)hi32(em.re)), l7 = lead_bit((int)hi32(em.im));
-  auto mx = [](int a, int b) { return a > b ? a : b; };
-  const int l = mx(mx(mx(l0, l1), mx(l2, l3)), mx(mx(l4, l5), mx(l6, l7)));
-  const int s = 28 - l;  // 0 .. 29: components below 2^61, their sums below 2^62
-  kp = cx(shl64(kp.re, s), shl64(kp.im, s));
-  km = cx(shl64(km.re, s), shl64(km.im, s));
-  ep = cx(shl64(ep.re, s), shl64(ep.im, s));
-  em = cx(shl64(em.re, s), shl64(em.im, s));
-  q[0] = cx_add(kp, ep);
-  q[1] = cx_sub(kp, ep);
-  q[2] = cx_add(km, em);
-  q[3] = cx_sub(km, em);
+// 96-bit integers: w2 the highest word.
+struct Q96 {
+  unsigned w0, w1, w2;
+};
+__host__ __device__ __forceinline__ Q96 q96(long long hi, unsigned lo) { return Q96{lo, lo32(hi), hi32(hi)}; }
+__host__ __device__ __forceinline__ Q96 q96_add(Q96 a, Q96 b) {
+#ifdef __CUDA_ARCH__
+  Q96 r;
+  asm("add.cc.u32 %0, %3, %6;\n\taddc.cc.u32 %1, %4, %7;\n\taddc.u32 %2, %5, %8;"
+      : "=r"(r.w0), "=r"(r.w1), "=r"(r.w2)
+      : "r"(a.w0), "r"(a.w1), "r"(a.w2), "r"(b.w0), "r"(b.w1), "r"(b.w2));
+  return r;
+#else
+  const unsigned lo = a.w0 + b.w0;
+  return q96((long long)((unsigned long long)join32(a.w2, a.w1) + (unsigned long long)join32(b.w2, b.w1) + (lo < b.w0 ? 1u : 0u)), lo);
+#endif
+}
+__host__ __device__ __forceinline__ Q96 q96_sub(Q96 a, Q96 b) {
+#ifdef __CUDA_ARCH__
+  Q96 r;
+  asm("sub.cc.u32 %0, %3, %6;\n\tsubc.cc.u32 %1, %4, %7;\n\tsubc.u32 %2, %5, %8;"
+      : "=r"(r.w0), "=r"(r.w1), "=r"(r.w2)
+      : "r"(a.w0), "r"(a.w1), "r"(a.w2), "r"(b.w0), "r"(b.w1), "r"(b.w2));
+  return r;
+#else
+  return q96((long long)((unsigned long long)join32(a.w2, a.w1) - (unsigned long long)join32(b.w2, b.w1) - (a.w0 < b.w0 ? 1u : 0u)), a.w0 - b.w0);
+#endif
+}
+// hi + f 2^-16 in units 2^-32.
+__host__ __device__ __forceinline__ Q96 q96_of(long long hi, int f) { return q96(hi + (f >> 16), (unsigned)f << 16); }
+__host__ __device__ __forceinline__ int mulhi_s32(int a, int b) {
+#ifdef __CUDA_ARCH__
+  return __mulhi(a, b);
+#else
+  return (int)(((long long)a * (long long)b) >> 32);
+#endif
+}
+// (x y) 2^-64 in units 2^-32, within 2 of them: bf_mul_high with the cross products'
+// low words and the low products' high ones.
+__host__ __device__ __forceinline__ void quad_product(Cx64 x, Cx64 y, Q96& re, Q96& im) {
+  const Limbs a = limbs_of(x.re), b = limbs_of(x.im), c = limbs_of(y.re), d = limbs_of(y.im);
+  const long long p = mad_wide(a.l, c.h, mad_wide(a.h, c.l, mulhi_s32(a.l, c.l)));
+  const long long q = mad_wide(b.l, d.h, mad_wide(b.h, d.l, mulhi_s32(b.l, d.l)));
+  const long long r = mad_wide(b.l, c.h, mad_wide(b.h, c.l, mad_wide(a.l, d.h, mad_wide(a.h, d.l,
+                          (long long)mulhi_s32(a.l, d.l) + mulhi_s32(b.l, c.l)))));
+  const long long t = p - q;
+  re = q96(mad_wide(-b.h, d.h, mul_wide(a.h, c.h)) + (int)hi32(t), lo32(t));
+  im = q96(mad_wide(b.h, c.h, mul_wide(a.h, d.h)) + (int)hi32(r), lo32(r));
+}
+
+// A value below 2^(32 + kQuadLeast) of its possible 2^61 is formed again (quad_small):
+// above, the 16 low bits (off by a few units: the coefficients' roundings) leave it
+// within 2^-55 (32 particles).
+constexpr int kQuadLeast = 12;
+// re, im in units 2^-32 normalised to 61 bits: (qr + i qi) 2^(l - 28), l the leading bit's
+// position in the high word (below kQuadLeast: the value is not to be used).
+__host__ __device__ __forceinline__ int quad_value(Q96 re, Q96 im, Cx64& q) {
+  const int pr = lead_bit((int)re.w2), pi = lead_bit((int)im.w2);
+  const int l = pr > pi ? pr : pi;
+  const int s = 28 - l;  // 0 .. 29
+  q = cx(join32(fshl32(re.w1, re.w2, s), fshl32(re.w0, re.w1, s)), join32(fshl32(im.w1, im.w2, s), fshl32(im.w0, im.w1, s)));
   return l;
 }
-// A pair: of, og the outer sums, ep, em = E+-, cp, cm_cp the constants.
-__host__ __device__ __forceinline__ int quad_pair(Cx64 of, Cx64 og, Cx64 ep, Cx64 em, Cx64 cp, Cx64 cm_cp,
-                                                  Cx64 (&q)[4]) {
-  Cx64 kp;
-  bf_mul_high(of.re, of.im, og.re, og.im, kp.re, kp.im);
-  kp = cx_add(kp, cp);
-  return quad_values(kp, cx_add(kp, cm_cp), ep, em, q);
+// A pair's four values q, order (+,+), (-,-), (+,-), (-,+), each q 2^(l - 28), from of,
+// og the outer sums, ep, em = E+-, cp, cm_cp the constants (low parts 0 .. 2^16 - 1,
+// quad_carry).  Returns the smallest l.
+__host__ __device__ __forceinline__ int quad_values(Cx64 of, Cx64 og, Cx64 ep, Cx64 em, Cx64 cp, Cx64 cm_cp, Cx64 (&q)[4],
+                                                    int (&l)[4]) {
+  Q96 pr, pi;
+  quad_product(of, og, pr, pi);
+  const Q96 kpr = q96_add(pr, q96(cp.re, (unsigned)cp.fr << 16)), kpi = q96_add(pi, q96(cp.im, (unsigned)cp.fi << 16));
+  const Q96 kmr = q96_add(kpr, q96(cm_cp.re, (unsigned)cm_cp.fr << 16));
+  const Q96 kmi = q96_add(kpi, q96(cm_cp.im, (unsigned)cm_cp.fi << 16));
+  const Q96 epr = q96_of(ep.re, ep.fr), epi = q96_of(ep.im, ep.fi), emr = q96_of(em.re, em.fr), emi = q96_of(em.im, em.fi);
+  l[0] = quad_value(q96_add(kpr, epr), q96_add(kpi, epi), q[0]);
+  l[1] = quad_value(q96_sub(kpr, epr), q96_sub(kpi, epi), q[1]);
+  l[2] = quad_value(q96_add(kmr, emr), q96_add(kmi, emi), q[2]);
+  l[3] = quad_value(q96_sub(kmr, emr), q96_sub(kmi, emi), q[3]);
+  const int x = l[0] < l[1] ? l[0] : l[1], y = l[2] < l[3] ? l[2] : l[3];
+  return x < y ? x : y;
+}
+// Value k of a pair from its factors: the exact product, normalised to 62 bits.
+__host__ __device__ __forceinline__ int quad_small(int k, Cx64 of, Cx64 og, Cx64 f0, Cx64 f1, Cx64 g0, Cx64 g1, Cx64& q) {
+  const int d0 = (k & 1) ? -1 : 1, d1 = (k == 1 || k == 2) ? -1 : 1;
+  const Cx64 f = cx(of.re + d0 * f0.re + d1 * f1.re, of.im + d0 * f0.im + d1 * f1.im);
+  const Cx64 g = cx(og.re + d0 * g0.re + d1 * g1.re, og.im + d0 * g0.im + d1 * g1.im);
+  const BFloat z = bf_pair(f.re, f.im, g.re, g.im, 0);
+  q = cx(z.re, z.im);
+  return z.e - 36;  // z 2^-64 = q 2^(l - 28)
+}
+// The same four over one exponent, the largest l (returned), for a check of quad_values.
+inline int quad_pair(Cx64 of, Cx64 og, Cx64 ep, Cx64 em, Cx64 cp, Cx64 cm_cp, Cx64 (&q)[4]) {
+  int l[4], most = -1;
+  quad_values(of, og, ep, em, quad_carry(cp), quad_carry(cm_cp), q, l);
+  for (int k = 0; k < 4; ++k) most = l[k] > most ? l[k] : most;
+  for (int k = 0; k < 4; ++k) q[k] = cx(q[k].re >> (most - l[k]), q[k].im >> (most - l[k]));
+  return most;
 }
 // One code's running product over the slots: a normal
 // value (larger component in [2^61, 2^62], or zero); returns what its exponent
@@ -125,7 +233,7 @@ __host__ __device__ __forceinline__ int quad_chain(long long& re, long long& im,
 }
 // Exponent of a chain beyond its own sum: e0 = minus the factors' fraction bits, 64
 // per pair product and per chain product, the shifts (28 - l a slot, 29 - p a
-// chain step) taken back; ls: the slots' leading bits.
+// chain step) taken back; ls: the values' leading bits l.
 __host__ __device__ __forceinline__ int quad_exponent(int e0, int ls, int slots) {
   return e0 + ls + (64 - 28 + 64 - 29) * slots - 64;
 }
