@@ -23,20 +23,28 @@ def _matrix(m, eps, seed):
     return U + eps * (rng.normal(size=(m, m)) + 1j * rng.normal(size=(m, m))) / np.sqrt(2.0 * m)
 
 
+def _exact_matrix(m, eps, seed):
+    """The same with entries that fixed point and FP64 sums hold exactly: multiples of 2^-50
+    (a row's largest sum is below 8), so that the products' own error is all there is."""
+    U = _matrix(m, eps, seed)
+    U[:2, :2] *= 0.75 / np.sqrt(0.5)
+    return np.round(U * 2.0 ** 50) / 2.0 ** 50
+
+
 def _int(x):
     v = Fraction(float(x)) * 2 ** BITS
     assert v.denominator == 1
     return v.numerator
 
 
-def _glynn(U, cols, rows, minors):
+def _glynn(U, cols, rows, minors, exact=False):
     """Glynn's sum over the signs of the particles `cols` and the factors `rows`: the
     permanent, or every column's minor; and the bound on its error."""
     n = len(cols)
     E = [[(_int(U[r, c].real), _int(U[r, c].imag)) for c in cols] for r in rows]
     F = U[np.ix_(rows, cols)]
     # the entries' roundings: half a unit each, 2^-61 of the largest possible sum at most
-    delta = n * np.sqrt(0.5) * 2.0 ** -61 * np.maximum(abs(F.real), abs(F.imag)).sum(axis=1)
+    delta = (0 if exact else n) * np.sqrt(0.5) * 2.0 ** -61 * np.maximum(abs(F.real), abs(F.imag)).sum(axis=1)
     out = [[0, 0] for _ in range(n if minors else 1)]
     tol = 0.0
     for tail in itertools.product((1, -1), repeat=n - 1):
@@ -91,3 +99,33 @@ def test_minors(eps):
     assert tol < 1e-4 * max(map(abs, ref))
     got = _native.submatrices_batch(U, S[None, :], T[None, :], _native.CHIN_HUH)[0]
     assert np.abs(got - np.array(ref)).max() <= tol, (eps, np.abs(got - np.array(ref)).max(), tol, np.abs(ref).max())
+
+
+EXACT = [1e-3, 1e-6, 1e-9]
+
+
+@pytest.mark.parametrize("eps", EXACT)
+@pytest.mark.parametrize("k", [6, 11, 15])
+def test_minors_of_exact_entries(k, eps):
+    from theboss_gb300 import _native
+
+    U = _exact_matrix(k, eps, k)
+    T = np.array([2, 2] + [1] * (k - 5) + [0] * 3, dtype=np.int32)
+    ref, tol = _glynn(U, list(range(k)), np.repeat(np.arange(k), T).tolist(), True, exact=True)
+    got = _native.submatrices_batch(U, np.ones((1, k), dtype=np.int32), T[None, :], _native.CHIN_HUH)[0]
+    assert np.abs(got - np.array(ref)).max() <= tol, (np.abs(got - np.array(ref)).max(), tol, np.abs(ref).max())
+
+
+@pytest.mark.parametrize("eps", EXACT)
+@pytest.mark.parametrize("S", [[1] * 8, [2, 2, 2, 2, 2, 1], [1] * 12], ids=["small", "multiple", "single"])
+def test_permanents_of_exact_entries(S, eps):
+    from theboss_gb300 import _native
+
+    n = sum(S)
+    U = _exact_matrix(n, eps, n)
+    S = np.array(S + [0] * (n - len(S)), dtype=np.int32)
+    T = np.array([2, 2] + [1] * (n - 4) + [0] * 2, dtype=np.int32)
+    (ref,), tol = _glynn(U, np.repeat(np.arange(n), S).tolist(), np.repeat(np.arange(n), T).tolist(), False, exact=True)
+    for count in (1, 40):
+        got = _native.perm_batch(U, np.tile(S, (count, 1)), np.tile(T, (count, 1)), _native.CHIN_HUH)
+        assert np.abs(got - ref).max() <= tol, (count, got[0], ref, tol)

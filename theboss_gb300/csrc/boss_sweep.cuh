@@ -276,19 +276,14 @@ __host__ __device__ __forceinline__ I128 sub128(I128 x, I128 y) {
 //     a unit, is dropped), then one normalising shift.  Of two normal values
 //     |product| >= 2^122 before the >> 64, off by less than 2 units a component:
 //     relative error below 2^-56.5 of the product's magnitude;
-//   * bf_mul_high with a fixed-point factor as it is (|re|, |im| < 2^62, its own scale
-//     2^fx_f such that its largest possible sum has 62 bits): the same absolute
-//     error, under 2^-58 of (the first value's magnitude times that largest
-//     sum), so a factor that happens to be small costs nothing extra to scale;
+//   * so every factor, a fixed-point sum below 2^62 in its own scale, is normalised
+//     before it is multiplied: as it is, the error would be relative to its largest
+//     possible sum, and a factor far below that (weakly coupled modes) lose its digits;
 //   * bf_to_double: one rounding to FP64 (2^-53) at the end.
-// An FP64 complex product errs by up to about 2^-52 of its magnitude, so a chain
-// of these products is more accurate than the FP64 chain it replaces (64
-// permanents at n = 28: 9.9e-14 from 64-bit values against 1.5e-13 with the last
-// 8 factors multiplied in FP64).
+// An FP64 complex product errs by up to about 2^-52 of its magnitude, these by less
+// than 2^-56.5.
 // Measured, 64 permanents (input-side digits, 2^(n-1) codes each) with the templated
-// kernel: n = 20 1.71 ms, n = 24 33.5 ms (2.08 and 39.3 ms with the limb products left
-// to the compiler).  Bound by the FMA pipe (a 32 x 32 + 64-bit multiply-add holds it
-// for 4 cycles a warp, 66 % busy) and dependent latency at 3 warps per scheduler.
+// kernel: n = 20 2.39 ms, n = 24 40.0 ms a call (33.5 with the factors as they are).
 // ---------------------------------------------------------------------------
 struct BFloat {
   long long re, im;
@@ -452,10 +447,18 @@ __host__ __device__ __forceinline__ double bf_to_double(long long x, int e) {
   if (be >= 1 && be <= 2046 && ax != 0) return bits_to_double((sgn << 63) | ((unsigned long long)be << 52) | mant);
   return ax ? ldexp((double)x, e) : 0.0;
 }
+// prod_f s_f with a factor below 2^32 (2^-30 of its possible size), whose digits
+// bf_renorm's one shift leaves below the product's last place.
+__device__ __noinline__ inline BFloat product_of_small(const long long* sr, const long long* si, int nf, int e0) {
+  BFloat x = bf_norm(sr[0], si[0], e0);
+  for (int f = 1; f < nf; ++f) x = bf_mul(x, bf_norm(sr[f], si[f], 0));
+  return x;
+}
 // acc += sign * prod_f s_f, every product on the integer pipe, two FP64 adds.  The
 // factors are split over two chains (two independent chains of dependent
-// instructions hide each other's latency); a chain starts from a normalised
-// factor and takes the others as they are.  e0: minus the factors' fraction bits.
+// instructions hide each other's latency), each factor normalised first: a factor far
+// below its largest possible sum keeps its digits (as it is, it cost 6 % less of the
+// 10^4-sample step and up to 2^-60 of that largest sum).  e0: minus the factors' fraction bits.
 template <int NF>
 __device__ __forceinline__ void accumulate_product_bf(const long long (&sr)[NF], const long long (&si)[NF], int e0,
                                                       uint32_t neg_mask, double& ar, double& ai) {
@@ -465,24 +468,46 @@ __device__ __forceinline__ void accumulate_product_bf(const long long (&sr)[NF],
   } else {
     constexpr int H = NF < 4 ? NF : (NF + 1) / 2;  // first chain: factors 0 .. H - 1
     long long xr = sr[0], xi = si[0], yr, yi;
-    int e = e0;
-    e += bf_renorm(xr, xi) - 29;
+    int e = e0, least = 0;  // the sign of the factors' leading bits
+    auto normal = [&](long long& re, long long& im) {
+      const int p = bf_renorm(re, im);
+      least = p < least ? p : least;
+      e += p - 29;
+    };
+    normal(xr, xi);
     if constexpr (H < NF) {
       yr = sr[H];
       yi = si[H];
-      e += bf_renorm(yr, yi) - 29;
+      normal(yr, yi);
     }
 #pragma unroll
     for (int k = 1; k < H; ++k) {
-      bf_mul_high(xr, xi, sr[k], si[k], xr, xi);
+      long long fr = sr[k], fi = si[k];
+      normal(fr, fi);
+      bf_mul_high(xr, xi, fr, fi, xr, xi);
       if (k < H - 1 || H < NF) e += 35 + bf_renorm(xr, xi);
       if (H + k < NF) {
-        bf_mul_high(yr, yi, sr[H + k], si[H + k], yr, yi);
+        fr = sr[H + k];
+        fi = si[H + k];
+        normal(fr, fi);
+        bf_mul_high(yr, yi, fr, fi, yr, yi);
         e += 35 + bf_renorm(yr, yi);
       }
     }
     if constexpr (H < NF) bf_mul_high(xr, xi, yr, yi, xr, xi);
     e += 64;  // the last product stays unnormalised: each component is rounded on its own
+    if (least < 0 && (xr | xi) != 0) {  // rare
+      long long tr[NF], ti[NF];
+#pragma unroll
+      for (int f = 0; f < NF; ++f) {
+        tr[f] = sr[f];
+        ti[f] = si[f];
+      }
+      const BFloat z = product_of_small(tr, ti, NF, e0);
+      xr = z.re;
+      xi = z.im;
+      e = z.e;
+    }
     ar += xor_sign(bf_to_double(xr, e), neg_mask);
     ai += xor_sign(bf_to_double(xi, e), neg_mask);
   }
