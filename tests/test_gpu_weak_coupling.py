@@ -129,3 +129,21 @@ def test_permanents_of_exact_entries(S, eps):
     for count in (1, 40):
         got = _native.perm_batch(U, np.tile(S, (count, 1)), np.tile(T, (count, 1)), _native.CHIN_HUH)
         assert np.abs(got - ref).max() <= tol, (count, got[0], ref, tol)
+
+
+@pytest.mark.parametrize("eps", EXACT)
+def test_gradients_of_exact_entries(eps):
+    from theboss_gb300 import _native
+
+    n = 8
+    U = _exact_matrix(n, eps, 80)
+    # the sweep takes the inputs' digits: 2^2 3^3 / 2 codes against 2^8 / 2
+    S, T = np.array([1, 1, 2, 2, 2, 0, 0, 0], dtype=np.int32), np.ones(n, dtype=np.int32)
+    got = _native.perm_grad_batch(U, S[None, :], T[None, :])[1][0]
+    cols = np.repeat(np.arange(n), S).tolist()
+    for j in np.nonzero(T)[0]:  # d perm / d U[j, i] = T_j S_i minor(T - e_j, S - e_i)
+        rows = np.repeat(np.arange(n), T - (np.arange(n) == j)).tolist()
+        ref, tol = _glynn(U, cols, rows, True, exact=True)
+        for i in np.nonzero(S)[0]:
+            want = T[j] * sum(ref[q] for q in range(n) if cols[q] == i)
+            assert abs(got[j, i] - want) <= T[j] * S[i] * tol, (j, i, got[j, i], want, tol)

@@ -31,15 +31,9 @@ struct GradMant {  // (re + i im) 2^e, normal (bf_renorm)
   long long re, im;
   int e;
 };
-__device__ __forceinline__ GradMant grad_norm(Cx64 s) {
+__device__ __forceinline__ GradMant grad_norm(Cx64 s) {  // of a factor's sum (fully where |s| >= 2^32)
   GradMant r{s.re, s.im, 0};
   r.e = bf_renorm(r.re, r.im) - 29;
-  return r;
-}
-__device__ __forceinline__ GradMant grad_mul(const GradMant& a, Cx64 s) {  // by a factor as it is
-  GradMant r;
-  bf_mul_high(a.re, a.im, s.re, s.im, r.re, r.im);
-  r.e = a.e + 35 + bf_renorm(r.re, r.im);
   return r;
 }
 __device__ __forceinline__ GradMant grad_mul(const GradMant& a, const GradMant& b) {
@@ -123,12 +117,25 @@ __global__ void __launch_bounds__(128, M <= 3 ? 5 : M <= 5 ? 4 : 3) grad_sweep_k
       move(b, -2 * dr);
     }
     // suffixes within the lane, the lane's product, the other lanes'
-    GradMant suf[M];  // suf[i]: factors after i of this lane (i < M - 1)
-    GradMant A = grad_norm(s[M - 1]);
+    int least = 0;
+    GradMant n[M], suf[M];  // the factors; suf[i]: factors after i of this lane (i < M - 1)
+#pragma unroll
+    for (int i = 0; i < M; ++i) {
+      n[i] = grad_norm(s[i]);
+      least = min(least, n[i].e);
+    }
+    if (least < -29) {  // rare: a factor below 2^32
+#pragma unroll
+      for (int i = 0; i < M; ++i) {
+        const BFloat z = bf_norm(s[i].re, s[i].im, 0);
+        n[i] = GradMant{z.re, z.im, z.e};
+      }
+    }
+    GradMant A = n[M - 1];
 #pragma unroll
     for (int i = M - 2; i >= 0; --i) {
       suf[i] = A;
-      A = grad_mul(A, s[i]);
+      A = grad_mul(A, n[i]);
     }
     const GradMant A1 = grad_from(A, 1);
     const GradMant B = grad_mul(A, A1);
@@ -140,7 +147,7 @@ __global__ void __launch_bounds__(128, M <= 3 ? 5 : M <= 5 ? 4 : 3) grad_sweep_k
       const int e = L.e + P.fx + fx[i];
       R[i].x = fma(w, bf_to_double(L.re, e), R[i].x);
       R[i].y = fma(w, bf_to_double(L.im, e), R[i].y);
-      pre = grad_mul(pre, s[i]);
+      pre = grad_mul(pre, n[i]);
     }
     pr = fma(w, bf_to_double(pre.re, pre.e + P.fx), pr);
     pi = fma(w, bf_to_double(pre.im, pre.e + P.fx), pi);
