@@ -147,3 +147,15 @@ def test_gradients_of_exact_entries(eps):
         for i in np.nonzero(S)[0]:
             want = T[j] * sum(ref[q] for q in range(n) if cols[q] == i)
             assert abs(got[j, i] - want) <= T[j] * S[i] * tol, (j, i, got[j, i], want, tol)
+
+
+@pytest.mark.parametrize("eps", EXACT)
+def test_distributions_of_exact_entries(eps):
+    from theboss_gb300 import _native
+
+    n = 7
+    U = _exact_matrix(n, eps, 70)
+    S, T = np.ones(n, dtype=np.int32), np.array([2, 2] + [1] * (n - 4) + [0] * 2, dtype=np.int32)
+    (ref,), tol = _glynn(U, list(range(n)), np.repeat(np.arange(n), T).tolist(), False, exact=True)
+    got = _native.lossy_probabilities(U, S, T[None, :])[0] * 4.0
+    assert abs(got - abs(ref) ** 2) <= 2.0 * abs(ref) * tol + tol ** 2 + 2.0 ** -50 * abs(ref) ** 2, (got, abs(ref) ** 2, tol)

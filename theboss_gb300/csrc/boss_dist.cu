@@ -300,9 +300,10 @@ __global__ void lossy_rows_kernel(const uint8_t* __restrict__ occ, int m, int64_
 }
 
 // V[(combo / 32 * m + row) * 32 + combo % 32], combo = input * 2^(L-1) + sign vector:
-// doubles, or (fx given) fixed point, each (input, row) with fx[input * m + row] fraction bits.
+// doubles, or (ve given) 62-bit mantissas with the exponents ve at the same places, of
+// exact fixed-point sums, each (input, row) in the scale of its own entries.
 __global__ void lossy_table_kernel(const double2* __restrict__ U, int m, int L, const uint8_t* __restrict__ cols,
-                                   int K, int64_t combos, int32_t* __restrict__ fx, double2* __restrict__ V) {
+                                   int K, int64_t combos, int32_t* __restrict__ ve, double2* __restrict__ V) {
   const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= combos * m) return;
   const int64_t combo = e / ((int64_t)32 * m) * 32 + (e & 31);
@@ -310,8 +311,9 @@ __global__ void lossy_table_kernel(const double2* __restrict__ U, int m, int L, 
   const int64_t k = combo >> (L - 1);
   double x = 0.0, y = 0.0;
   const uint32_t d = (uint32_t)combo & ((1u << (L - 1)) - 1u);
-  if (fx) {
+  if (ve) {
     long long fr = 0, fi = 0;
+    int exp = 0;
     if (k < K) {
       unsigned long long mx = 0;  // magnitudes order as integers
       for (int b = 0; b < L; ++b) {
@@ -320,7 +322,6 @@ __global__ void lossy_table_kernel(const double2* __restrict__ U, int m, int L, 
                          (unsigned long long)__double_as_longlong(fabs(u.y))));
       }
       const int f = row_fraction_bits(__longlong_as_double((long long)mx), L);
-      if (d == 0) fx[k * m + row] = f;
       const double scale = __longlong_as_double((long long)(1023 + f) << 52);  // 2^f, |f| < 1000
       for (int b = 0; b < L; ++b) {
         const double2 u = U[(size_t)row * m + cols[k * L + b]];
@@ -329,7 +330,12 @@ __global__ void lossy_table_kernel(const double2* __restrict__ U, int m, int L, 
         fr += neg ? -ur : ur;
         fi += neg ? -ui : ui;
       }
+      const BFloat z = bf_norm(fr, fi, -f);
+      fr = z.re;
+      fi = z.im;
+      exp = z.e;
     }
+    ve[e] = exp;
     reinterpret_cast<longlong2*>(V)[e] = make_longlong2(fr, fi);
     return;
   }
@@ -349,7 +355,7 @@ __global__ void lossy_table_kernel(const double2* __restrict__ U, int m, int L, 
 // vectors are walked one after the other.
 template <int L, bool kFixed>
 __global__ void __launch_bounds__(128) lossy_walk_kernel(const double2* __restrict__ V, int m,
-                                                         const int32_t* __restrict__ fx,  // kFixed: [K][m]
+                                                         const int32_t* __restrict__ ve,  // kFixed: V's exponents
                                                          const uint4* __restrict__ rows, int64_t O, int K, int groups,
                                                          const double* __restrict__ in_div,    // [K][kDistMaxDiv]
                                                          const int* __restrict__ in_ndiv,      // [K]
@@ -382,8 +388,7 @@ __global__ void __launch_bounds__(128) lossy_walk_kernel(const double2* __restri
     const double2* Vg = V + block * 32 * m + lane;
     const uint32_t d = L >= 6 ? (uint32_t)(j * 32 + lane) : (uint32_t)(lane & (kLanes - 1));
     const uint32_t neg = (__popc(d) & 1) << 31;
-    const int mine = L >= 6 ? g : min(g * (32 / kLanes) + lane / kLanes, K - 1);  // this lane's input
-    const int32_t* fxk = kFixed ? fx + (size_t)mine * m : nullptr;
+    const int32_t* eg = kFixed ? ve + block * 32 * m + lane : nullptr;
     double2 P[kFixed ? 1 : L];
     long long pr[kFixed ? L : 1], pi[kFixed ? L : 1];  // normalised, in units of 2^pe
     int pe[kFixed ? L : 1];
@@ -397,15 +402,14 @@ __global__ void __launch_bounds__(128) lossy_walk_kernel(const double2* __restri
         if constexpr (a < L && kFixed) {
           const int row = (int)((w[a >> 2] >> (8 * (a & 3))) & 255u);
           const longlong2 v = __ldg(reinterpret_cast<const longlong2*>(Vg) + (size_t)row * 32);
-          const int f = __ldg(fxk + row);
           long long zr = v.x, zi = v.y;
-          int e = -f;
+          int e = __ldg(eg + (size_t)row * 32);
           if constexpr (a > 0) {
             bf_mul_high(pr[a - 1], pi[a - 1], v.x, v.y, zr, zi);
             e += pe[a - 1] + 64;
           }
           if constexpr (a < L - 1) {
-            e += bf_renorm(zr, zi) - 29;
+            if constexpr (a > 0) e += bf_renorm(zr, zi) - 29;
             pr[a] = zr;
             pi[a] = zi;
             pe[a] = e;
@@ -590,7 +594,7 @@ static void particle_list(const int32_t* occ, int m, uint8_t* out) {
 }
 
 template <int L>
-static cudaError_t launch_walk(const double2* V, int m, const int32_t* fx, const uint4* rows, int64_t O, int K, int groups,
+static cudaError_t launch_walk(const double2* V, int m, const int32_t* ve, const uint4* rows, int64_t O, int K, int groups,
                                const double* div, const int* ndiv, const double* mult, double* terms,
                                int sm_count, cudaStream_t s) {
   // chunks of outcomes that leave about 16 warps per SM: a walk is serial (a chunk of
@@ -598,25 +602,25 @@ static cudaError_t launch_walk(const double2* V, int m, const int32_t* fx, const
   const int64_t want = O * groups / ((int64_t)sm_count * 16);
   const int chunk = (int)std::min<int64_t>(kWalkChunk, std::max<int64_t>(8, want / 8 * 8));
   const int64_t tasks = (O + chunk - 1) / chunk * groups;
-  auto* kernel = fx ? lossy_walk_kernel<L, true> : lossy_walk_kernel<L, false>;
-  kernel<<<(unsigned)((tasks + 3) / 4), 128, 0, s>>>(V, m, fx, rows, O, K, groups, div, ndiv, mult, chunk, terms);
+  auto* kernel = ve ? lossy_walk_kernel<L, true> : lossy_walk_kernel<L, false>;
+  kernel<<<(unsigned)((tasks + 3) / 4), 128, 0, s>>>(V, m, ve, rows, O, K, groups, div, ndiv, mult, chunk, terms);
   return cudaGetLastError();
 }
 
-static cudaError_t launch_walk_l(int l, const double2* V, int m, const int32_t* fx, const uint4* rows, int64_t O, int K, int groups,
+static cudaError_t launch_walk_l(int l, const double2* V, int m, const int32_t* ve, const uint4* rows, int64_t O, int K, int groups,
                                  const double* div, const int* ndiv, const double* mult, double* terms,
                                  int sms, cudaStream_t s) {
   switch (l) {
-    case 1: return launch_walk<1>(V, m, fx, rows, O, K, groups, div, ndiv, mult, terms, sms, s);
-    case 2: return launch_walk<2>(V, m, fx, rows, O, K, groups, div, ndiv, mult, terms, sms, s);
-    case 3: return launch_walk<3>(V, m, fx, rows, O, K, groups, div, ndiv, mult, terms, sms, s);
-    case 4: return launch_walk<4>(V, m, fx, rows, O, K, groups, div, ndiv, mult, terms, sms, s);
-    case 5: return launch_walk<5>(V, m, fx, rows, O, K, groups, div, ndiv, mult, terms, sms, s);
-    case 6: return launch_walk<6>(V, m, fx, rows, O, K, groups, div, ndiv, mult, terms, sms, s);
-    case 7: return launch_walk<7>(V, m, fx, rows, O, K, groups, div, ndiv, mult, terms, sms, s);
-    case 8: return launch_walk<8>(V, m, fx, rows, O, K, groups, div, ndiv, mult, terms, sms, s);
-    case 9: return launch_walk<9>(V, m, fx, rows, O, K, groups, div, ndiv, mult, terms, sms, s);
-    case 10: return launch_walk<10>(V, m, fx, rows, O, K, groups, div, ndiv, mult, terms, sms, s);
+    case 1: return launch_walk<1>(V, m, ve, rows, O, K, groups, div, ndiv, mult, terms, sms, s);
+    case 2: return launch_walk<2>(V, m, ve, rows, O, K, groups, div, ndiv, mult, terms, sms, s);
+    case 3: return launch_walk<3>(V, m, ve, rows, O, K, groups, div, ndiv, mult, terms, sms, s);
+    case 4: return launch_walk<4>(V, m, ve, rows, O, K, groups, div, ndiv, mult, terms, sms, s);
+    case 5: return launch_walk<5>(V, m, ve, rows, O, K, groups, div, ndiv, mult, terms, sms, s);
+    case 6: return launch_walk<6>(V, m, ve, rows, O, K, groups, div, ndiv, mult, terms, sms, s);
+    case 7: return launch_walk<7>(V, m, ve, rows, O, K, groups, div, ndiv, mult, terms, sms, s);
+    case 8: return launch_walk<8>(V, m, ve, rows, O, K, groups, div, ndiv, mult, terms, sms, s);
+    case 9: return launch_walk<9>(V, m, ve, rows, O, K, groups, div, ndiv, mult, terms, sms, s);
+    case 10: return launch_walk<10>(V, m, ve, rows, O, K, groups, div, ndiv, mult, terms, sms, s);
     default: return cudaErrorInvalidValue;
   }
 }
@@ -646,7 +650,7 @@ static int queue_small_groups(Context* cx, const double* matrix, int m, int n, c
     fixed = fixed && (x == 0.0 || (x < 1e270 && x > 1e-270));
   }
   size_t o_cols[kDistMaxL + 1], o_div[kDistMaxL + 1], o_ndiv[kDistMaxL + 1], o_mult[kDistMaxL + 1];
-  int64_t most_terms = 1, most_O = 1, most_V = 1, most_fx = 1;
+  int64_t most_terms = 1, most_O = 1, most_V = 1;
   int st;
   for (int l = 1; l <= kDistMaxL; ++l) {
     if (!G.size[l]) continue;
@@ -658,14 +662,13 @@ static int queue_small_groups(Context* cx, const double* matrix, int m, int n, c
     o_mult[l] = off; off = align256(off + sizeof(double) * (size_t)K);
     most_terms = std::max(most_terms, K * G.size[l]);
     most_O = std::max(most_O, G.size[l]);
-    most_fx = std::max(most_fx, K * m);
     const int64_t combos = ((K << (l - 1)) + 31) / 32 * 32;
     most_V = std::max(most_V, std::min(combos * m, std::max<int64_t>(kTableBytes / 16, (int64_t)m << l) + 32 * m));
   }
   if ((st = ensure(cx->dist[0], off))) return st;
   if ((st = ensure(cx->dist[1], sizeof(double) * (size_t)most_terms))) return st;
-  const size_t o_V = align256(sizeof(uint4) * (size_t)most_O), o_fx = o_V + align256(sizeof(double2) * (size_t)most_V);
-  if ((st = ensure(cx->gpart, o_fx + sizeof(int32_t) * (size_t)most_fx))) return st;
+  const size_t o_V = align256(sizeof(uint4) * (size_t)most_O), o_ve = o_V + align256(sizeof(double2) * (size_t)most_V);
+  if ((st = ensure(cx->gpart, o_ve + sizeof(int32_t) * (size_t)most_V))) return st;
   if ((st = ensure_pinned(cx, off))) return st;
   char* h = (char*)cx->pinned;
   memcpy(h + o_U, matrix, sizeof(double2) * (size_t)m * m);
@@ -689,7 +692,7 @@ static int queue_small_groups(Context* cx, const double* matrix, int m, int n, c
   double* terms = (double*)cx->dist[1].ptr;
   uint4* rows = (uint4*)cx->gpart.ptr;
   double2* V = (double2*)((char*)cx->gpart.ptr + o_V);
-  int32_t* fx = fixed ? (int32_t*)((char*)cx->gpart.ptr + o_fx) : nullptr;
+  int32_t* ve = fixed ? (int32_t*)((char*)cx->gpart.ptr + o_ve) : nullptr;
   cudaStream_t s = cx->stream;
   cudaError_t e = cudaMemcpyAsync(d, h, off, cudaMemcpyHostToDevice, s);
   if (e != cudaSuccess) return fail_cuda(e, "H2D distribution tables");
@@ -715,8 +718,8 @@ static int queue_small_groups(Context* cx, const double* matrix, int m, int n, c
       const int64_t combos = l >= 6 ? (int64_t)kn << (l - 1) : (int64_t)groups * 32;
       const uint8_t* cols = (const uint8_t*)(d + o_cols[l]) + k0 * l;
       lossy_table_kernel<<<(unsigned)((combos * m + 127) / 128), 128, 0, s>>>((const double2*)(d + o_U), m, l, cols, kn,
-                                                                             combos, fx ? fx + k0 * m : nullptr, V);
-      e = launch_walk_l(l, V, m, fx ? fx + k0 * m : nullptr, rows, O, kn, groups, (const double*)(d + o_div[l]) + k0 * kDistMaxDiv,
+                                                                             combos, ve, V);
+      e = launch_walk_l(l, V, m, ve, rows, O, kn, groups, (const double*)(d + o_div[l]) + k0 * kDistMaxDiv,
                         (const int*)(d + o_ndiv[l]) + k0, (const double*)(d + o_mult[l]) + k0, terms + k0 * O, cx->sm_count, s);
     }
     lossy_outcome_kernel<<<(unsigned)((O + 127) / 128), 128, 0, s>>>(terms, K, O, m, occ, (const double*)(d + o_fact),
