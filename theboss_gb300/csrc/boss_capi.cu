@@ -480,7 +480,7 @@ static int fill_sweep(HostSweep& hs, const Side& dig, const Side& col, int kind,
                                                                        : kRowsPacked;
   hs.scale = glynn ? std::ldexp(1.0, -dig.n) * (drop >= 0 ? 2.0 : 1.0) : 1.0;
   hs.parity0 = glynn ? 0 : (dig.n & 1);
-  hs.has_base = glynn || hs.layout != kRowsPlain;
+  hs.has_base = glynn;  // (the quad and gradient layouts carry one always)
   hs.on_device = on_device && (hs.layout == kRowsQuad || hs.layout == kRowsGrad);
   if (hs.on_device) {
     const int Fg = grad_factors(hs.nf), W = quad_width(hs.nf);

@@ -63,16 +63,17 @@ struct SweepProblem {
   int64_t ff_off;    // float-pair all-minors only: nb x nf rows of D as float pairs (float4: re hi, re lo,
                      // im hi, im lo, each factor in its own scale), then nf int32 exponent biases
   double scale;      // final real scale
-  int32_t fixed_digit;  // gradients, all-minors: a binary digit held at r = 0 (Glynn halving) adds a weight-1 row
-  int32_t group;     // each aligned group of `group` threads (all-minors: 1, 2, 4, .., 128; above 32 only when the
+  int16_t fixed_digit;  // gradients, all-minors: a binary digit held at r = 0 (Glynn halving) adds a weight-1 row
+  int16_t group;     // each aligned group of `group` threads (all-minors: 1, 2, 4, .., 128; above 32 only when the
                      // launch's threads fill whole blocks; low = 2: walkers, permanents up to 8, all-minors up
                      // to 32; the templated permanents 1) sums its partials, so there are n_threads / group of
                      // them; n_threads and thread_begin are multiples of it, and every sweep of the launch has
                      // the same
-  int32_t align;     // permanents, all-minors: ranges start at multiples of 2^align codes (range_align)
-  int32_t low;       // 2: two more binary digits, all four of whose values are taken at every step (boss_quad.cuh)
+  int16_t align;     // permanents, all-minors: ranges start at multiples of 2^align codes (range_align)
+  int16_t low;       // 2: two more binary digits, all four of whose values are taken at every step (boss_quad.cuh)
   uint8_t mult[kMaxDigits];
 };
+static_assert(sizeof(SweepProblem) == 168, "the allocation-free entry point's scratch holds one a permanent");
 
 // A row entry of the integer-pipe sweeps (permanents, all-minors): u = -D / 2, the
 // 64-bit value hi 2^32 + lo with lo taken as a SIGNED word (hi carries its sign
