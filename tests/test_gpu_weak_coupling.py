@@ -79,7 +79,7 @@ def test_permanents(eps):
     (ref,), tol = _glynn(U, list(range(n)), rows, False)
     assert tol < 1e-4 * abs(ref)
     got = list(_native.perm_batch(U, S[None, :], T[None, :], _native.CHIN_HUH))
-    got += list(_native.perm_batch(U, np.tile(S, (4, 1)), np.tile(T, (4, 1)), _native.CHIN_HUH))  # rows made on the GPU
+    got += list(_native.perm_batch(U, np.tile(S, (40, 1)), np.tile(T, (40, 1)), _native.CHIN_HUH))  # rows made on the GPU
     for g in got:
         assert abs(g - ref) <= tol, (eps, g, ref, abs(g - ref) / abs(ref), tol / abs(ref))
     # Glynn's form takes the outputs' signs here (fewer codes), whose products do not vanish with eps

@@ -133,10 +133,20 @@ static int split_threads(const std::vector<HostSweep>& sweeps, int64_t resident,
 static size_t rows_of(const HostSweep& h) { return h.on_device ? h.D_size : h.D.size(); }
 static size_t base_of(const HostSweep& h) { return h.on_device ? h.base_size : h.base.size(); }
 
-// Whether a call's sweeps have their rows made on the GPU: from four permanents on,
-// while the matrix is a small upload (64 permanents at n = 16: 340 -> 150 us a call; a
-// single one is planned on the host in the time of the extra launch).
-static bool plan_on_device(int m, int count) { return count >= 4 && m <= 512; }
+// Whether a call's sweeps have their rows made on the GPU: where planning them on the
+// host (17 ns per digit and factor, judged by the first request) takes longer than the
+// extra launch (15 us) and the matrix's way there (0.78 ns an entry).  Calls in us, host / GPU
+// rows: 64 of n = 16 in 32 modes 443 / 178, 4 of n = 12 in 32 modes 42 / 49, in 512 modes
+// 51 / 261, 64 there 379 / 462, 128 745 / 639.
+static bool plan_on_device(int m, int count, int len, const int32_t* S, const int32_t* T) {
+  if (count < 4 || m > 512) return false;
+  int ni = 0, no = 0;
+  for (int i = 0; i < len; ++i) {
+    ni += std::max(S[i], 0);
+    no += std::max(T[i], 0);
+  }
+  return 22.0 * count * ni * no > 20000.0 + (double)m * m;
+}
 
 static void describe_plan(const HostSweep& h, int64_t mat_off, int64_t base_off, PlanItem& I) {
   I.layout = h.layout;
@@ -764,6 +774,7 @@ int boss_perm_batch(const double* matrix, int32_t m, const int32_t* input_states
   std::vector<int> which[kSweepClasses];
   std::vector<int> small[kSmallPermMax + 1];  // by particle count; no planning
   bool any = false, any_small = false;
+  const bool on_device = count > 0 && plan_on_device(m, count, len, input_states, output_states);
   if (variant < BOSS_RYSER || variant > BOSS_CLASSIC) {
     set_error("unknown permanent variant");
     return kErrArg;
@@ -788,7 +799,7 @@ int boss_perm_batch(const double* matrix, int32_t m, const int32_t* input_states
     HostSweep hs;
     bool need = false;
     double2 v = make_double2(0.0, 0.0);
-    const int st = plan_permanent(matrix, m, Sk, Tk, len, variant, hs, need, v, kPlanAny, plan_on_device(m, count));
+    const int st = plan_permanent(matrix, m, Sk, Tk, len, variant, hs, need, v, kPlanAny, on_device);
     if (st) return st;
     if (need) {
       const int c = sweep_class(hs);
@@ -885,13 +896,14 @@ int boss_perm_grad_batch(const double* matrix, int32_t m, const int32_t* input_s
   std::vector<HostSweep> by_nf[kMaxFactors + 1];
   std::vector<int> which[kMaxFactors + 1];
   bool any = false;
+  const bool on_device = count > 0 && plan_on_device(m, count, len, input_states, output_states);
   for (int k = 0; k < count; ++k) {
     HostSweep hs;
     bool need = false;
     double2 v = make_double2(0.0, 0.0);
     const int32_t* S = input_states + (size_t)k * len;
     const int32_t* T = output_states + (size_t)k * len;
-    int st = plan_permanent(matrix, m, S, T, len, BOSS_GLYNN, hs, need, v, kPlanGrad, plan_on_device(m, count));
+    int st = plan_permanent(matrix, m, S, T, len, BOSS_GLYNN, hs, need, v, kPlanGrad, on_device);
     if (st) return st;
     if (!need) {  // no particles: perm = 1, gradient 0
       P2[k] = v;
