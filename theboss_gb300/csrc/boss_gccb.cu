@@ -1934,9 +1934,11 @@ __global__ void __launch_bounds__(128) fixed_rows_kernel(const double2* __restri
 // sample, from the level's code count and the resident threads of the kernel)
 // and the size G of the thread groups that sum their minors inside the sweep.
 // boss_gccb_autotune times candidate shapes on the caller's workload and keeps,
-// per (arithmetic, level, sample-count bucket), the split's power-of-two shift
+// per (kernel, arithmetic, level, sample-count bucket), the split's power-of-two shift
 // and G's cap that ran fastest; the winners are cached in-process and on disk,
-// keyed by the GPU's name.
+// keyed by the GPU's name.  A level's kernel is minors_sweep_kernel (threads) or
+// minors_quad_kernel (walkers of four lanes), by the samples' inputs; kTuneKernels
+// grows when their work per thread changes, and entries of other values are not read.
 // ---------------------------------------------------------------------------
 struct LevelTune {
   int shift = 0;  // threads per sample = heuristic * 2^shift (clamped to [1, codes])
@@ -1955,8 +1957,16 @@ static inline int sample_bucket(int64_t A) {
   while ((A >> (b + 1)) > 0 && b < 40) ++b;
   return b;  // floor(log2(A))
 }
-static inline uint64_t tune_key(bool f64, int k, int64_t A) {
-  return ((uint64_t)(f64 ? 1 : 0) << 32) | ((uint64_t)k << 16) | (uint64_t)sample_bucket(A);
+constexpr uint64_t kTuneKernels = 1;
+static inline uint64_t tune_key(bool f64, bool quad, int k, int64_t A) {
+  return (kTuneKernels << 40) | ((uint64_t)(quad ? 1 : 0) << 33) | ((uint64_t)(f64 ? 1 : 0) << 32) |
+         ((uint64_t)k << 16) | (uint64_t)sample_bucket(A);
+}
+// Whether level k runs four codes per step: an FP64 sweep of enough factors whose every
+// sample has two binary digits besides the held one (singles: the fewest modes with one
+// particle of a sample's input there).
+static inline bool level_is_quad(bool f64, int k, bool binned, int singles) {
+  return !(!f64 && minors_ff_available(k - 1)) && k - 1 >= kQuadMinMinorFactors && (!binned || singles >= 3);
 }
 static std::string tune_path() {
   const char* p = getenv("BOSS_TUNE_CACHE");
@@ -1989,6 +1999,7 @@ static void tune_load(int device) {
       if (x >= 1 && x <= 6) g_pipeline_shift = x;
       if (y >= 1 && y <= 4) g_pipeline_growth = y;
     } else if (sscanf(rest.c_str(), "%llu|%d|%d", &key, &x, &y) == 3) {
+      if (key >> 40 != kTuneKernels) continue;
       g_level_tune[(uint64_t)key] = LevelTune{std::max(-3, std::min(x, 3)), std::max(0, std::min(y, 128))};
     }
   }
@@ -2015,10 +2026,10 @@ static void tune_save() {
   fprintf(f, "%s|pipeline|%d|%d\n", g_tune_gpu.c_str(), g_pipeline_shift, g_pipeline_growth);
   fclose(f);
 }
-static LevelTune level_tune(bool f64, int k, int64_t A) {
+static LevelTune level_tune(bool f64, bool quad, int k, int64_t A) {
   if (g_tune_force) return *g_tune_force;
   if (k < (int)g_tune_force_level.size()) return g_tune_force_level[k];
-  const auto it = g_level_tune.find(tune_key(f64, k, A));
+  const auto it = g_level_tune.find(tune_key(f64, quad, k, A));
   return it == g_level_tune.end() ? LevelTune{} : it->second;
 }
 
@@ -2133,10 +2144,8 @@ static int gccb_prepare(Context* cx, const double* matrix, int n_mats, int m, Dr
       for (int k = 0; k < L[s]; ++k) occ[D.modes[(size_t)s * n + k]] = 0;
     }
   }
-  // Levels that run four codes per step: FP64 sweeps of two factors at least whose
-  // every sample has two binary digits besides the held one.
   std::vector<char> quad(Lmax + 2, 0);
-  for (int k = 3; k <= Lmax; ++k) quad[k] = !ffl[k] && k - 1 >= kQuadMinMinorFactors && (!D.binned || lvl_singles[k] >= 3);
+  for (int k = 3; k <= Lmax; ++k) quad[k] = level_is_quad(f64, k, D.binned, lvl_singles[k]);
   std::vector<char> uniform(Lmax + 2, 0);
   std::vector<LevelSample> uni_lvl(Lmax + 2);
   std::vector<int> grp(Lmax + 2, 1);
@@ -2170,7 +2179,7 @@ static int gccb_prepare(Context* cx, const double* matrix, int n_mats, int m, Dr
       const double total = (double)code0 * Ak;
       const double want = std::max<double>(Ak, std::min<double>((double)resident, total / min_codes_per_thread(total, kMinCodesPerThread >> low, 1, block, cx->sm_count)));
       int64_t tps = std::max<int64_t>(1, std::min<int64_t>((int64_t)code0, (int64_t)(want / Ak)));
-      const LevelTune lt = level_tune(f64, k, Ak);
+      const LevelTune lt = level_tune(f64, quad[k], k, Ak);
       if (lt.shift > 0) tps = std::min<int64_t>((int64_t)code0, tps << lt.shift);
       if (lt.shift < 0) tps = std::max<int64_t>(1, tps >> -lt.shift);
       // Each aligned group of G threads of a sample sums its minors inside the sweep:
@@ -2203,7 +2212,7 @@ static int gccb_prepare(Context* cx, const double* matrix, int n_mats, int m, Dr
     }
     std::vector<int64_t> nthr;
     {
-      const LevelTune lt = level_tune(f64, k, Ak);
+      const LevelTune lt = level_tune(f64, quad[k], k, Ak);
       const int64_t res = lt.shift >= 0 ? resident << lt.shift : std::max<int64_t>(1, resident >> -lt.shift);
       std::vector<uint64_t> steps(codes);
       double total = 0.0;
@@ -2613,6 +2622,26 @@ static std::vector<int64_t> level_counts(const Draws& D) {
   return A;
 }
 
+// Whether each level of these draws runs four codes per step, as gccb_prepare decides.
+static std::vector<char> quad_levels(Draws& D, int m, bool f64, int Lmax) {
+  if (D.binned && D.modes.empty()) modes_from_draws(D);
+  std::vector<int> fewest(Lmax + 2, 256);
+  std::vector<uint8_t> occ(m, 0);
+  for (size_t s = 0; D.binned && s < D.L.size(); ++s) {
+    const uint8_t* modes = &D.modes[s * D.n];
+    for (int k = 1, singles = 0; k <= D.L[s]; ++k) {
+      uint8_t& o = occ[modes[k - 1]];
+      singles += o == 0 ? 1 : o == 1 ? -1 : 0;
+      ++o;
+      fewest[k] = std::min(fewest[k], singles);
+    }
+    for (int k = 0; k < D.L[s]; ++k) occ[modes[k]] = 0;
+  }
+  std::vector<char> quad(Lmax + 2, 0);
+  for (int k = 3; k <= Lmax; ++k) quad[k] = level_is_quad(f64, k, D.binned, fewest[k]);
+  return quad;
+}
+
 // Whether every level of this workload (the draws of `count` samples from a copy
 // of `mt`) already has a tuned entry.
 static bool workload_tuned(const int32_t* input_state, int m, const double* weights, int nw, const MT19937& mt,
@@ -2622,8 +2651,9 @@ static bool workload_tuned(const int32_t* input_state, int m, const double* weig
   if (predraw(input_state, m, weights, nw, t, count, D)) return true;  // errors surface in the call itself
   const std::vector<int64_t> A = level_counts(D);
   const bool f64 = (g_minors_arith != 0);
+  const std::vector<char> quad = quad_levels(D, m, f64, (int)A.size() - 2);
   for (int k = 2; k + 1 < (int)A.size(); ++k)
-    if (A[k] > 0 && !g_level_tune.count(tune_key(f64, k, A[k]))) return false;
+    if (A[k] > 0 && !g_level_tune.count(tune_key(f64, quad[k], k, A[k]))) return false;
   return true;
 }
 
@@ -2746,10 +2776,11 @@ static int gccb_autotune_locked(Context* cx, const double* matrix, int m, const 
   g_tune_force_level.clear();
   const bool keep = step1 < step0;
   int changed = 0;
+  const std::vector<char> quad = quad_levels(D, m, f64, Lmax);
   for (int k = 2; k <= Lmax; ++k) {
     if (A[k] <= 0) continue;
     const LevelTune v = keep ? best[k] : LevelTune{};
-    g_level_tune[tune_key(f64, k, A[k])] = v;
+    g_level_tune[tune_key(f64, quad[k], k, A[k])] = v;
     changed += (v.shift != 0 || v.gmax != 0) ? 1 : 0;
   }
   report[0] = step0;
