@@ -38,6 +38,7 @@
 #include <mutex>
 #include <string>
 #include <numeric>
+#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -210,7 +211,8 @@ static void modes_from_draws(Draws& D) {
 
 // Host threads for the replay, created on first use and never destroyed (the
 // process ends with them parked).  run(T, fn) runs fn(1..T-1) on the pool and
-// fn(0) on the caller, and returns when all have finished.  A process forked
+// fn(0) on the caller, and returns when all have finished; where the system grants no
+// threads the caller runs all of them in order (one may wait for fn(0) only).  A process forked
 // from one with a pool inherits the object but not its threads: its first
 // replay makes a pool of its own and leaves the inherited one untouched.
 class HostPool {
@@ -228,9 +230,14 @@ class HostPool {
   }
   void run(int T, const std::function<void(int)>& fn) {
     std::lock_guard<std::mutex> serial(run_mu_);
-    while (nthreads_ < T - 1) {
-      const int id = ++nthreads_;
-      std::thread([this, id] { worker(id); }).detach();
+    try {
+      for (int id; nthreads_ < T - 1; nthreads_ = id) {
+        id = nthreads_ + 1;
+        std::thread([this, id] { worker(id); }).detach();
+      }
+    } catch (const std::system_error&) {  // no more threads to be had
+      for (int t = 0; t < T; ++t) fn(t);
+      return;
     }
     {
       std::lock_guard<std::mutex> lk(mu_);
