@@ -105,7 +105,8 @@ def _layer_entries(m: int):
         alone = np.setdiff1d(np.arange(m), np.concatenate([k, k + 1]))
         ones.append(base + alone * m + alone)
     ones = np.concatenate(ones)
-    return torch.from_numpy(np.concatenate([np.concatenate(b) for b in blocks] + [ones])), len(ones)
+    # arrays, not tensors: a tensor made while a call is traced would be the tracer's
+    return np.concatenate([np.concatenate(b) for b in blocks] + [ones]), len(ones)
 
 
 def _layer_product(theta: torch.Tensor, phi: torch.Tensor, m: int) -> torch.Tensor:
@@ -128,6 +129,23 @@ def _layer_product(theta: torch.Tensor, phi: torch.Tensor, m: int) -> torch.Tens
     return M
 
 
+def _dense_product(theta: torch.Tensor, phi: torch.Tensor, m: int) -> torch.Tensor:
+    """The same from every layer as a dense m x m matrix, multiplied pairwise: 2 log2(m)
+    batched products instead of some fifteen small operations per layer for autograd to
+    follow."""
+    ctype = torch.complex128
+    ep, c, s = torch.exp(1j * phi.to(ctype)), torch.cos(theta).to(ctype), torch.sin(theta).to(ctype)
+    at, ones = _layer_entries(m)
+    v = torch.cat([ep * c, -s, ep * s, c, torch.ones(ones, dtype=ctype, device=theta.device)])
+    L = torch.zeros(m * m * m, dtype=ctype, device=theta.device).index_copy(0, torch.from_numpy(at).to(theta.device), v)
+    L = L.view(m, m, m)
+    while L.shape[0] > 1:
+        n = L.shape[0]
+        P = L[1::2] @ L[0:n - n % 2:2]  # the later layer on the left
+        L = torch.cat([P, L[-1:]]) if n % 2 else P
+    return L[0]
+
+
 def clements_unitary(theta: torch.Tensor, phi: torch.Tensor, output_phases: torch.Tensor = None) -> torch.Tensor:
     """U = D * T_L ... T_1 with T(theta, phi) on modes (k, k+1):
     [[e^{i phi} cos theta, -sin theta], [e^{i phi} sin theta, cos theta]]."""
@@ -137,24 +155,16 @@ def clements_unitary(theta: torch.Tensor, phi: torch.Tensor, output_phases: torc
         raise ValueError("theta and phi need m(m-1)/2 entries each")
     ctype = torch.complex128
     if m <= _DENSE_LAYERS and torch.is_grad_enabled() and (theta.requires_grad or phi.requires_grad):
-        # every layer as a dense m x m matrix, multiplied pairwise: 2 log2(m) batched
-        # products instead of some fifteen small operations per layer for autograd to
-        # follow, whose dispatch was the whole time (forward and backward, CPU: m = 24
-        # 9.6 -> 1.3 ms, m = 96 70 -> 10.5 ms; beyond that the m^3 entries grow past what
-        # it saves).  Its value is replaced by the layers' own product, in their order:
-        # derivatives of the logarithm of a small probability magnify the last bits of U.
-        ep, c, s = torch.exp(1j * phi.to(ctype)), torch.cos(theta).to(ctype), torch.sin(theta).to(ctype)
-        at, ones = _layer_entries(m)
-        v = torch.cat([ep * c, -s, ep * s, c, torch.ones(ones, dtype=ctype, device=theta.device)])
-        L = torch.zeros(m * m * m, dtype=ctype, device=theta.device).index_copy(0, at.to(theta.device), v)
-        L = L.view(m, m, m)
-        while L.shape[0] > 1:
-            n = L.shape[0]
-            P = L[1::2] @ L[0:n - n % 2:2]  # the later layer on the left
-            L = torch.cat([P, L[-1:]]) if n % 2 else P
+        # The derivatives of the dense layers' product, whose few operations autograd
+        # follows in less time than the loop's (forward and backward, CPU: m = 24 8.3 -> 3.5 ms,
+        # m = 96 72 -> 35; at m = 192 353 -> 282, with 113 MB in each of its m x m x m
+        # steps: the line lies before that).  The value is the layers' own product, in
+        # their order: derivatives of the logarithm of a small probability magnify the last
+        # bits of U.
+        dense = _dense_product(theta, phi, m)
         with torch.no_grad():
             value = _layer_product(theta.detach(), phi.detach(), m)
-        M = L[0] + (value - L[0].detach())
+        M = value + (dense - dense.detach())
     else:
         M = _layer_product(theta, phi, m)
     if output_phases is not None:
