@@ -56,9 +56,8 @@ int grad_reduce_parts(int64_t walkers, int n_probs, int row_stride, int sm_count
 cudaError_t launch_grad_reduce(int nf, const SweepProblem* probs, int n_probs, const double2* gpart,
                                const double2* ppart, double2* mid, int parts, double2* grad_out, double2* perm_out,
                                int row_stride, cudaStream_t st);
-// Whether the float-pair all-minors / single-permanent kernel exists for nf factors.
+// Whether the float-pair all-minors kernel exists for nf factors.
 bool minors_ff_available(int nf);
-bool perm_ff_available(int nf);
 cudaError_t launch_sweep(int nf, SweepOp op, const SweepLaunch& L, cudaStream_t st);
 cudaError_t launch_perm_reduce(const SweepProblem* probs, int n_probs, const double2* partials, double2* out,
                                cudaStream_t st, bool ff = false);

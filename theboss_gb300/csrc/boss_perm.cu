@@ -36,7 +36,6 @@ cudaError_t prepare_sweep_kernels() {
   return prepare_grad_kernels();
 }
 
-bool perm_ff_available(int nf) { return nf >= 1 && nf <= kMaxFactors && g_perm_ff_occ[nf] > 0; }
 
 bool minors_ff_available(int nf) { return nf >= 1 && nf <= kMaxFactors && g_minors_ff_occ[nf][kMaxMinorDigits] > 0; }
 
