@@ -186,10 +186,12 @@ __global__ void __launch_bounds__(128) small_prepare_kernel(const double2* __res
 // 0 stays +.  The products run on the integer pipe (accumulate_product_bf), so a code
 // costs ~45 instructions per factor where FP64 ones hold its pipe for 4 * 64 clocks,
 // and a single permanent has all lanes of a block instead of one thread's chain of
-// dependent FP64 products (n = 8: 248 -> 40 us a call, planning and synchronisation
-// included).  A permanent with a row that has no scale is summed in FP64 by its first lane.
+// dependent FP64 products (n = 8: 248 -> 27 us a call, planning and synchronisation
+// included).  Compiled for 5 to 6 blocks per SM although few run: with the 80 to 94
+// registers of no bound, one of n = 10 takes 41.7 us a call instead of 36.7, 31 of n = 9
+// 44.4 instead of 39.6.  A permanent with a row that has no scale is summed in FP64 by its first lane.
 template <int L>
-__global__ void __launch_bounds__(128) small_perm_kernel(const longlong2* __restrict__ A,
+__global__ void __launch_bounds__(128, L <= 9 ? 6 : 5) small_perm_kernel(const longlong2* __restrict__ A,
                                                          const int32_t* __restrict__ e0s, int64_t count, int lg,
                                                          double2* __restrict__ out) {
   __shared__ double2 part[4];

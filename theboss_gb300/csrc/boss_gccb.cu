@@ -706,8 +706,10 @@ constexpr int kFinWarps = 4;
 // Stated relative error bounds of the all-minors sweeps (absolute error of every
 // minor against the exact value, over the largest minor of the step), used by the
 // finalize kernel's cdf guard.  Measured against the double-double oracle at
-// k = 8..22 input particles: FP64 sweeps at most 8.1e-15, float-pair sweeps at
-// most 3.0e-12; the bounds hold 110x and 19x of margin.
+// k = 8..22 input particles of Haar matrices: FP64 sweeps at most 3.5e-15, float-pair
+// sweeps at most 3.0e-12 (260x and 19x of margin).  Two modes coupled to the rest by eps
+// only and doubly occupied, FP64: 2.5e-15 at eps = 1e-3, 1.4e-13 at 1e-5, and 1.2e-12, above
+// the bound, at 1e-6: the entries' own rounding to fixed point.
 constexpr float kMinorsErrF64 = 9.094947e-13f;  // 2^-40
 constexpr float kMinorsErrFF = 5.820766e-11f;   // 2^-34
 
