@@ -38,8 +38,8 @@ def test_values_keep_their_digits(tmp_path):
                 assert re == 0 and im == 0
                 seen["zero"] += 1
                 continue
-            assert max(abs(re), abs(im)) >= 2 ** 60 - 1
+            assert max(abs(re), abs(im)) >= 2 ** 61 - 1
             for c, got in enumerate((re, im)):
                 # 16 roundings of the coefficients at most (half a unit of 2^48 each) over 2^108, truncations 2^-60
-                assert abs(F(got) * F(2) ** (l + 36) - exact[c]) <= F(size) * F(2) ** -55, (nd, k, small, l)
+                assert abs(F(got) * F(2) ** (l + 35) - exact[c]) <= F(size) * F(2) ** -55, (nd, k, small, l)
     assert min(seen.values()) > 100

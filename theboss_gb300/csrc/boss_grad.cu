@@ -42,6 +42,12 @@ __device__ __forceinline__ GradMant grad_mul(const GradMant& a, const GradMant& 
   r.e = a.e + b.e + 35 + bf_renorm(r.re, r.im);
   return r;
 }
+__device__ __forceinline__ GradMant grad_last(const GradMant& a, const GradMant& b) {  // a product that is only converted
+  GradMant r;
+  bf_mul_high(a.re, a.im, b.re, b.im, r.re, r.im);
+  r.e = a.e + b.e + 64;
+  return r;
+}
 __device__ __forceinline__ GradMant grad_from(const GradMant& a, int o) {  // lane ^ o's
   GradMant r;
   r.re = __shfl_xor_sync(0xffffffffu, a.re, o);
@@ -143,7 +149,7 @@ __global__ void __launch_bounds__(128, M <= 3 ? 5 : M <= 5 ? 4 : 3) grad_sweep_k
     const double w = it < Q.len ? xor_sign(k.w, k.parity << 31) : 0.0;
 #pragma unroll
     for (int i = 0; i < M; ++i) {
-      const GradMant L = i < M - 1 ? grad_mul(pre, suf[i]) : pre;
+      const GradMant L = i < M - 1 ? grad_last(pre, suf[i]) : pre;
       const int e = L.e + P.fx + fx[i];
       R[i].x = fma(w, bf_to_double(L.re, e), R[i].x);
       R[i].y = fma(w, bf_to_double(L.im, e), R[i].y);

@@ -93,12 +93,13 @@ int range_align(int64_t n_codes, int64_t n_threads, int nb);
 // Host-side sweep description.
 // ---------------------------------------------------------------------------
 // Factors from which a sweep with two binary digits takes four codes per step
-// (boss_quad.cuh) instead of the templated kernel.  Permanents: always (64
-// permanents: n = 12 18 against 20 us, n = 16 86 against 109, n = 18 354 against 400,
-// n = 24 24.0 against 33.5 ms).  All-minors: from 14 (the sampler's levels of 10^4
-// samples, n = 20: 13 factors 186 against 197 us but its rows cost the finalize 8 us
-// more to plan; 12 factors 197 against 200, 11 factors 199 against 172, 14 factors
-// 125 against 135).
+// (boss_quad.cuh) instead of the templated kernel.  Permanents: always (sweeps of 64
+// permanents: n = 12 18.4 against 17.7 us, n = 16 89 against 116, n = 18 416 against 433,
+// n = 20 1.67 against 1.94 ms, n = 24 28.1 against 37.0).  All-minors: from 14, by the
+// sampler's levels (300 samples of 18 photons, eta 0.9, with the line at 13, 14, 15, 16, none:
+// 1.76, 1.77, 1.79, 1.84, 1.93 ms a call; 10^4 of 20 at 0.5: 2.72, 2.74, 2.73, 2.74, 2.69).
+// Calls planned on the host share the line, though theirs would lie higher: one call of 14
+// factors 44 against 40 us, of 17 66 against 54, of 20 112 against 125.
 constexpr int kQuadMinFactors = 2;
 constexpr int kQuadMinMinorFactors = 14;
 enum RowLayout : int {

@@ -3,10 +3,10 @@
 // kQuadMinMinorFactors).  The templated kernels of boss_sweep_kernels.cuh take the
 // others.
 //
-// Measured (calls of 64 permanents, input-side digits): n = 20 1.82 ms, n = 24 29.1 ms;
-// with the pairs in 62 bits, which lost weakly coupled networks' digits, 1.52 and 24.5.
-// 8 of n = 28 73 ms (61).  Bound by fixed latencies of one dependent chain a lane at 12
-// to 16 warps per SM, which more warps do not lessen.
+// Measured (sweeps of 64 permanents, input-side digits): n = 16 89 us, n = 20 1.67 ms, n = 24
+// 28.1; with the pairs in 62 bits, which lost weakly coupled networks' digits, 88, 1.41 and
+// 24.4.  The benchmark's output-side batch n = 28 120 ms (104).  Bound by fixed latencies
+// of one dependent chain a lane at 12 to 16 warps per SM, which more warps do not lessen.
 #include <algorithm>
 
 #include "boss_internal.h"
@@ -15,8 +15,8 @@
 namespace boss {
 
 // Blocks of 128 per SM the kernels are compiled for: the state is 20 registers per
-// four slots.  64 permanents at n = 20: 3 blocks 1.82 ms, 4 blocks (spills) 1.88; n = 24
-// 29.1 and 30.3; 8 of n = 28: 3 blocks 73.1 ms, 2 blocks 78.4.
+// four slots.  Calls of 64 permanents n = 20: 3 blocks 1.82 ms, 4 blocks (spills) 1.88; n = 24
+// 29.1 and 30.3; 8 of n = 28: 3 blocks 73.1 ms, 2 blocks 78.4 (every product shifted then).
 constexpr int quad_blocks(int slots) { return slots <= 4 ? 5 : slots <= 8 ? 4 : 3; }
 
 // A lane's slots are 4 i + (lane & 3) of its walker, i = 0 .. ceil(S / 4) - 1, their
@@ -133,7 +133,10 @@ __device__ __forceinline__ void quad_eval(QuadState<S>& st, longlong2* xbuf, con
     for (int j = 0; j < 4; ++j) {
       if (4 * i + j >= S) break;
       const longlong2 q = xbuf[(i & 1) * kQuadX + from + j];
-      ps += (i + j == 0) ? quad_chain_first(re, im, q.x, q.y) : quad_chain(re, im, q.x, q.y);
+      const int n = 4 * i + j;
+      ps += n == 0 ? quad_chain_first(re, im, q.x, q.y)
+            : n % 2 ? quad_chain_raw(re, im, q.x, q.y)
+                    : quad_chain(re, im, q.x, q.y);
     }
     __syncwarp();
   }

@@ -175,16 +175,16 @@ __host__ __device__ __forceinline__ void quad_product(Cx64 x, Cx64 y, Q96& re, Q
 // above, the 16 low bits (off by a few units: the coefficients' roundings) leave it
 // within 2^-55 (32 particles).
 constexpr int kQuadLeast = 12;
-// re, im in units 2^-32 normalised to 61 bits: (qr + i qi) 2^(l - 28), l the leading bit's
+// re, im in units 2^-32 normalised to 62 bits: (qr + i qi) 2^(l - 29), l the leading bit's
 // position in the high word (below kQuadLeast: the value is not to be used).
 __host__ __device__ __forceinline__ int quad_value(Q96 re, Q96 im, Cx64& q) {
   const int pr = lead_bit((int)re.w2), pi = lead_bit((int)im.w2);
   const int l = pr > pi ? pr : pi;
-  const int s = 28 - l;  // 0 .. 29
+  const int s = 29 - l;  // 1 .. 30
   q = cx(join32(fshl32(re.w1, re.w2, s), fshl32(re.w0, re.w1, s)), join32(fshl32(im.w1, im.w2, s), fshl32(im.w0, im.w1, s)));
   return l;
 }
-// A pair's four values q, order (+,+), (-,-), (+,-), (-,+), each q 2^(l - 28), from of,
+// A pair's four values q, order (+,+), (-,-), (+,-), (-,+), each q 2^(l - 29), from of,
 // og the outer sums, ep, em = E+-, cp, cm_cp the constants (low parts 0 .. 2^16 - 1,
 // quad_carry).  Returns the smallest l.
 __host__ __device__ __forceinline__ int quad_values(Cx64 of, Cx64 og, Cx64 ep, Cx64 em, Cx64 cp, Cx64 cm_cp, Cx64 (&q)[4],
@@ -209,7 +209,7 @@ __host__ __device__ __forceinline__ int quad_small(int k, Cx64 of, Cx64 og, Cx64
   const Cx64 g = cx(og.re + d0 * g0.re + d1 * g1.re, og.im + d0 * g0.im + d1 * g1.im);
   const BFloat z = bf_pair(f.re, f.im, g.re, g.im, 0);
   q = cx(z.re, z.im);
-  return z.e - 36;  // z 2^-64 = q 2^(l - 28)
+  return z.e - 35;  // z 2^-64 = q 2^(l - 29)
 }
 // The same four over one exponent, the largest l (returned), for a check of quad_values.
 inline int quad_pair(Cx64 of, Cx64 og, Cx64 ep, Cx64 em, Cx64 cp, Cx64 cm_cp, Cx64 (&q)[4]) {
@@ -231,11 +231,17 @@ __host__ __device__ __forceinline__ int quad_chain(long long& re, long long& im,
   bf_mul_high(re, im, qr, qi, re, im);
   return bf_renorm(re, im);
 }
+// The same without the shift (which 29 stands for): the value stays above 2^58, and the
+// next step, within 2^-54 of its product then, shifts.
+__host__ __device__ __forceinline__ int quad_chain_raw(long long& re, long long& im, long long qr, long long qi) {
+  bf_mul_high(re, im, qr, qi, re, im);
+  return 29;
+}
 // Exponent of a chain beyond its own sum: e0 = minus the factors' fraction bits, 64
-// per pair product and per chain product, the shifts (28 - l a slot, 29 - p a
+// per pair product and per chain product, the shifts (29 - l a slot, 29 - p a
 // chain step) taken back; ls: the values' leading bits l.
 __host__ __device__ __forceinline__ int quad_exponent(int e0, int ls, int slots) {
-  return e0 + ls + (64 - 28 + 64 - 29) * slots - 64;
+  return e0 + ls + 2 * (64 - 29) * slots - 64;
 }
 
 // The walk over a sweep's (outer) digits: the reflected mixed-radix Gray code changes one

@@ -281,10 +281,12 @@ __host__ __device__ __forceinline__ I128 sub128(I128 x, I128 y) {
 //     before it is multiplied: as it is, the error would be relative to its largest
 //     possible sum, and a factor far below that (weakly coupled modes) lose its digits;
 //   * bf_to_double: one rounding to FP64 (2^-53) at the end.
-// An FP64 complex product errs by up to about 2^-52 of its magnitude, these by less
-// than 2^-56.5.
-// Measured, 64 permanents (input-side digits, 2^(n-1) codes each) with the templated
-// kernel: n = 20 2.39 ms, n = 24 40.0 ms a call (33.5 with the factors as they are).
+//   * in a chain only every second product is shifted back to the normal form: the one
+//     between stays above 2^58, and the next is within 2^-54 of its magnitude.
+// An FP64 complex product errs by up to about 2^-52 of its magnitude.
+// Measured, sweeps of 64 permanents (input-side digits, 2^(n-1) codes each) with the
+// templated kernel: n = 20 1.94 ms, n = 24 37.0 (every product shifted: 2.1 and 39; the
+// factors as they are, losing digits: 1.71 and 33.5).
 // ---------------------------------------------------------------------------
 struct BFloat {
   long long re, im;
@@ -458,8 +460,8 @@ __device__ __noinline__ inline BFloat product_of_small(const long long* sr, cons
 // acc += sign * prod_f s_f, every product on the integer pipe, two FP64 adds.  The
 // factors are split over two chains (two independent chains of dependent
 // instructions hide each other's latency), each factor normalised first: a factor far
-// below its largest possible sum keeps its digits (as it is, it cost 6 % less of the
-// 10^4-sample step and up to 2^-60 of that largest sum).  e0: minus the factors' fraction bits.
+// below its largest possible sum keeps its digits (as it is, it would lose up to 2^-60 of
+// that largest sum).  e0: minus the factors' fraction bits.
 template <int NF>
 __device__ __forceinline__ void accumulate_product_bf(const long long (&sr)[NF], const long long (&si)[NF], int e0,
                                                       uint32_t neg_mask, double& ar, double& ai) {
@@ -486,17 +488,22 @@ __device__ __forceinline__ void accumulate_product_bf(const long long (&sr)[NF],
       long long fr = sr[k], fi = si[k];
       normal(fr, fi);
       bf_mul_high(xr, xi, fr, fi, xr, xi);
-      if (k < H - 1 || H < NF) e += 35 + bf_renorm(xr, xi);
+      if ((H < NF && k == H - 1) || (k < H - 1 && k % 2 == 0))  // every second, and the last of two chains
+        e += 35 + bf_renorm(xr, xi);
+      else
+        e += 64;
       if (H + k < NF) {
         fr = sr[H + k];
         fi = si[H + k];
         normal(fr, fi);
         bf_mul_high(yr, yi, fr, fi, yr, yi);
-        e += 35 + bf_renorm(yr, yi);
+        e += (H + k == NF - 1 || k % 2 == 0) ? 35 + bf_renorm(yr, yi) : 64;
       }
     }
-    if constexpr (H < NF) bf_mul_high(xr, xi, yr, yi, xr, xi);
-    e += 64;  // the last product stays unnormalised: each component is rounded on its own
+    if constexpr (H < NF) {
+      bf_mul_high(xr, xi, yr, yi, xr, xi);
+      e += 64;
+    }
     if (least < 0 && (xr | xi) != 0) {  // rare
       long long tr[NF], ti[NF];
 #pragma unroll
