@@ -519,7 +519,7 @@ def strategies_section(seed):
 DTYPE = "f64"
 DTYPE_NOTE = ("FP64 products, minors, Laplace step, |.|^2 and pmf; row sums in exact 64-bit fixed point; "
               "every product multiplied in block floating point on the integer pipe (62-bit mantissas, "
-              "each product within 2^-56.5 of its magnitude, one rounding of the chain to FP64); "
+              "each product within 2^-54 of its magnitude, one rounding of the chain to FP64); "
               "cdf decisions by an exact integer scan of the FP64 pmf, theboss's sequential FP64 rule "
               "inside the pmf's error window")
 

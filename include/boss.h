@@ -179,9 +179,10 @@ BOSS_API int boss_gccb_sample(const double* matrix, int32_t m, const int32_t* in
 // pairs (two FP32 values, about 47 significant bits) on the FP32 pipe, for
 // sweeps of at most 24 product-side particles (larger ones stay FP64); -1: query
 // only.  *previous (if not null) receives the mode in force before the call.  Row
-// sums are exact 64-bit fixed point in both; in mode 1 every product is multiplied
-// in block floating point on the integer pipe (62-bit mantissas, each product within
-// 2^-56.5 of its magnitude, the chain rounded once to FP64).
+// sums are exact 64-bit fixed point in both (of entries rounded once, to 2^-62 of the
+// factor's largest possible sum); in mode 1 every product is multiplied in block floating
+// point on the integer pipe (62-bit mantissas, each product within 2^-54 of its
+// magnitude, the chain rounded once to FP64).
 BOSS_API int boss_minors_arithmetic(int32_t mode, int32_t* previous);
 
 // The same choice for the single-permanent sweeps of boss_perm_batch and

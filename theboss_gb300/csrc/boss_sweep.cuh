@@ -285,8 +285,8 @@ __host__ __device__ __forceinline__ I128 sub128(I128 x, I128 y) {
 //     between stays above 2^58, and the next is within 2^-54 of its magnitude.
 // An FP64 complex product errs by up to about 2^-52 of its magnitude.
 // Measured, sweeps of 64 permanents (input-side digits, 2^(n-1) codes each) with the
-// templated kernel: n = 20 1.94 ms, n = 24 37.0 (every product shifted: 2.1 and 39; the
-// factors as they are, losing digits: 1.71 and 33.5).
+// templated kernel: n = 20 1.94 ms, n = 24 37.0 (the factors as they are, losing digits: 1.71
+// and 33.5); whole calls 2.31 and 37.5 ms (with every product shifted 2.39 and 40.0).
 // ---------------------------------------------------------------------------
 struct BFloat {
   long long re, im;
