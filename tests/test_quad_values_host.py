@@ -22,10 +22,10 @@ def test_values_keep_their_digits(tmp_path):
     seen = {0: 0, 1: 0, "zero": 0}
     for line in subprocess.run([exe, "5", "6000"], check=True, capture_output=True, text=True).stdout.splitlines():
         v = list(map(int, line.split()))
-        nd, u = v[0], [v[17 + 5 * a:22 + 5 * a] for a in range(v[0])]
+        nd, one, u = v[0], v[1], [v[18 + 5 * a:23 + 5 * a] for a in range(v[0])]
         for k, (d0, d1) in enumerate(LOW):
-            re, im, l, small = v[1 + 4 * k:5 + 4 * k]
-            s = [0, 0, 0, 0]
+            re, im, l, small = v[2 + 4 * k:6 + 4 * k]
+            s = [0, 0, one, 0]
             for a in range(nd):
                 d = (d0, d1)[a] if a < 2 else u[a][0]
                 for c in range(4):

@@ -52,22 +52,16 @@ __device__ __forceinline__ void quad_move(Cx64 (&v)[4], const longlong2* __restr
   v[3].fi += sg * low.w;
 }
 
-// The small ones among a pair's four values formed from its factors, in place (rare:
-// out of line; con: the pair's constants).  Takes and returns the exponents' pairs.
-__device__ __noinline__ int2 quad_redo(longlong2* vals, int2 ls, const longlong2* __restrict__ con, long long fr,
-                                       long long fi, long long gr, long long gi) {
-  auto at = [&](int c) {
-    const longlong2 x = con[3 + c];
-    return cx(x.x, x.y);
-  };
-  int l[4] = {(short)ls.x, (ls.x - (short)ls.x) >> 16, (short)ls.y, (ls.y - (short)ls.y) >> 16};
-  for (int k = 0; k < 4; ++k) {
-    if (l[k] >= kQuadLeast) continue;
-    Cx64 q;
-    l[k] = quad_small(k, cx(fr, fi), cx(gr, gi), at(0), at(1), at(2), at(3), q);
-    vals[k * kQuadXStride] = make_longlong2(q.re, q.im);
-  }
-  return make_int2(l[0] + l[1] * 65536, l[2] + l[3] * 65536);
+// Two of a pair's values, 2 half and 2 half + 1, formed from its factors, in place (con: the
+// pair's constants); returns their exponents as one pair.
+__device__ __forceinline__ int quad_redo(longlong2* vals, int half, const longlong2* __restrict__ con, Cx64 of, Cx64 og) {
+  const longlong2 f = __ldg(con + 3 + half), g = __ldg(con + 5 + half);
+  Cx64 q[2];
+  int l[2];
+  quad_small(of, og, cx(f.x, f.y), cx(g.x, g.y), q, l);
+#pragma unroll
+  for (int k = 0; k < 2; ++k) vals[(2 * half + k) * kQuadXStride] = make_longlong2(q[k].re, q[k].im);
+  return l[0] + l[1] * 65536;
 }
 
 // The walk at outer code t, and this lane's state.
@@ -118,10 +112,18 @@ __device__ __forceinline__ void quad_eval(QuadState<S>& st, longlong2* xbuf, con
     Cx64 q[4];
     int l[4];
     const int least = quad_values(v[0], v[1], v[2], v[3], Cx64{cp.x, cp.y, low.x, low.y}, Cx64{cm.x, cm.y, low.z, low.w}, q, l);
-    int2 lv = make_int2(l[0] + l[1] * 65536, l[2] + l[3] * 65536);
 #pragma unroll
     for (int c = 0; c < 4; ++c) xbuf[at + c * kQuadXStride] = make_longlong2(q[c].re, q[c].im);
-    if (least < kQuadLeast) lv = quad_redo(xbuf + at, lv, con, v[0].re, v[0].im, v[1].re, v[1].im);
+    int2 lv = make_int2(l[0] + l[1] * 65536, l[2] + l[3] * 65536);
+    if (least < kQuadLeast) {  // rare but for weakly coupled modes: the half of the values that has the small one
+      const int half = min(l[0], l[1]) < kQuadLeast ? 0 : 1;
+      const bool both = half == 0 && min(l[2], l[3]) < kQuadLeast;
+#pragma unroll 1
+      for (int h = half; h <= (both ? 1 : half); ++h) {
+        const int x = quad_redo(xbuf + at, h, con, v[0], v[1]);
+        lv = h ? make_int2(lv.x, x) : make_int2(x, lv.y);
+      }
+    }
     if (4 * i + 4 <= S || 4 * i + kk < S) ls = make_int2(ls.x + lv.x, ls.y + lv.y);
   };
   prepare(0);

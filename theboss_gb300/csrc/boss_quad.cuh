@@ -22,11 +22,13 @@
 // (a component of s_f s_g is below 2 * 2^62 * 2^62), with 16 bits more below them.  A
 // value K +- E that comes out far below its largest possible size (2^-17 of it: a
 // network's weakly coupled modes) has lost those bits, and is formed from the two
-// factor sums instead (quad_small, exact 128-bit product): every value handed to a chain is
+// factor sums instead (quad_small): every value handed to a chain is
 // within 2^-55 of the pair's product.  (With K and E in 62 bits alone, 12 photons whose
 // modes couple by 1e-4 and are doubly occupied at the output: 4.7e-9; now
-// 3e-14.)  Haar matrices at 28 photons take the second way
-// for a few values in 10^6.
+// 3e-14.)  Haar matrices at 28 photons take the second way for a few values in 10^6; 64
+// permanents of n = 22 7.0 ms, with two modes coupled by 1e-6 9.7, a Fourier matrix 9.7, 50:50
+// splitters on all pairs of modes 8.8 (exact zeros), these coupled by 1e-9, where every value
+// is small, 17.9.
 //
 // Layout of a sweep in the pool (longlong2 = one complex), slots = ceil(nf / 2)
 // pairs (an odd last factor is paired with the constant 1 = 2^62 in its units),
@@ -35,8 +37,8 @@
 //     16 low bits (int4: e+ re im, e- re im); the walk adds -2 r times a row (r: the
 //     digit's value);
 //   base, W: o_f o_g E+ E- and the E's low parts per pair at r = 0 (unpacked);
-//   constants, kQuadConst per pair: C+, C- - C+, their low parts (int4, 0 .. 2^16 - 1), and the low
-//     digits' u_f0 u_f1 u_g0 u_g1.
+//   constants, kQuadConst per pair: C+, C- - C+, their low parts (int4, 0 .. 2^16 - 1), and
+//     u_f0 + u_f1, u_f0 - u_f1, u_g0 + u_g1, u_g0 - u_g1.
 #pragma once
 #include "boss_sweep.cuh"
 
@@ -111,10 +113,10 @@ __host__ __device__ __forceinline__ void quad_constants(Cx64 f0, Cx64 f1, Cx64 g
   v[0] = quad_carry(v[0]);
   v[1] = quad_carry(v[1]);
   out[2] = quad_low(v[0], v[1]);
-  v[2] = f0;
-  v[3] = f1;
-  v[4] = g0;
-  v[5] = g1;
+  v[2] = cx_add(f0, f1);
+  v[3] = cx_sub(f0, f1);
+  v[4] = cx_add(g0, g1);
+  v[5] = cx_sub(g0, g1);
   for (int c = 0; c < 6; ++c) {
     out[c < 2 ? c : c + 1].x = v[c].re;
     out[c < 2 ? c : c + 1].y = v[c].im;
@@ -202,14 +204,44 @@ __host__ __device__ __forceinline__ int quad_values(Cx64 of, Cx64 og, Cx64 ep, C
   const int x = l[0] < l[1] ? l[0] : l[1], y = l[2] < l[3] ? l[2] : l[3];
   return x < y ? x : y;
 }
-// Value k of a pair from its factors: the exact product, normalised to 62 bits.
-__host__ __device__ __forceinline__ int quad_small(int k, Cx64 of, Cx64 og, Cx64 f0, Cx64 f1, Cx64 g0, Cx64 g1, Cx64& q) {
-  const int d0 = (k & 1) ? -1 : 1, d1 = (k == 1 || k == 2) ? -1 : 1;
-  const Cx64 f = cx(of.re + d0 * f0.re + d1 * f1.re, of.im + d0 * f0.im + d1 * f1.im);
-  const Cx64 g = cx(og.re + d0 * g0.re + d1 * g1.re, og.im + d0 * g0.im + d1 * g1.im);
-  const BFloat z = bf_pair(f.re, f.im, g.re, g.im, 0);
-  q = cx(z.re, z.im);
-  return z.e - 35;  // z 2^-64 = q 2^(l - 29)
+// A factor's sum normalised, also where its high word is empty, or the constant factor
+// (2^62, one place too high); the exponent.
+__host__ __device__ __forceinline__ int quad_normal(Cx64& s) {
+  auto lead = [&] {
+    const int pr = lead_bit((int)hi32(s.re)), pi = lead_bit((int)hi32(s.im));
+    return pr > pi ? pr : pi;
+  };
+  auto up = [&] { s = cx((long long)((unsigned long long)s.re << 30), (long long)((unsigned long long)s.im << 30)); };
+  int e = -29;
+  const int p = lead();
+  if ((unsigned)p > 29u) {  // rare
+    if (p > 29) {
+      s = cx(s.re >> 1, s.im >> 1);
+      e += 1;
+    } else {
+      up();
+      e -= 30;
+      if (lead() < 0) {
+        up();
+        e -= 30;
+      }
+    }
+  }
+  return e + bf_renorm(s.re, s.im);
+}
+// Values 2 h and 2 h + 1 of a pair from its factors: the low digits' part is +-low_f,
+// +-low_g, u_0 + u_1 for h = 0, u_0 - u_1 for h = 1.  Each within 2^-56 of the product.
+__host__ __device__ __forceinline__ void quad_small(Cx64 of, Cx64 og, Cx64 low_f, Cx64 low_g, Cx64 (&q)[2], int (&l)[2]) {
+  Cx64 f[2] = {cx_add(of, low_f), cx_sub(of, low_f)}, g[2] = {cx_add(og, low_g), cx_sub(og, low_g)};
+  auto zero = [](Cx64 s) { return (s.re | s.im) == 0; };
+  l[0] = l[1] = 0;
+  q[0] = q[1] = cx(0, 0);
+  if ((zero(f[0]) || zero(g[0])) && (zero(f[1]) || zero(g[1]))) return;
+  for (int k = 0; k < 2; ++k) {
+    l[k] = quad_normal(f[k]) + quad_normal(g[k]);
+    bf_mul_high(f[k].re, f[k].im, g[k].re, g[k].im, q[k].re, q[k].im);
+    l[k] += bf_renorm(q[k].re, q[k].im);  // the product 2^-64 = q 2^(l - 29)
+  }
 }
 // The same four over one exponent, the largest l (returned), for a check of quad_values.
 inline int quad_pair(Cx64 of, Cx64 og, Cx64 ep, Cx64 em, Cx64 cp, Cx64 cm_cp, Cx64 (&q)[4]) {
